@@ -7,13 +7,15 @@
 //   [W1 (h1 x d_in), b1 (h1), W2 (h2 x h1), b2 (h2), W3 (d_out x h2), b3 (d_out)]
 // with a bf16 copy of the same layout; forward passes multiply by the bf16
 // weights with FP32 accumulation and FP32 biases.  The layer products run on
-// the CUDA cores (64 x 64 output tiles, 16-deep K slices staged in shared
-// memory, 4 x 4 outputs per thread): they are a few hundred MFLOP per step,
-// small beside the exact HLR pass.
+// the CUDA cores (mlp_gemm_kernel), every output one chain of multiply-adds
+// in k order: they are a few hundred MFLOP per step, small beside the exact
+// HLR pass.
 //
 //   forward   P1 = X W1^T + b1, A1 = gelu(P1), P2 = A1 W2^T + b2,
-//             A2 = gelu(P2), Y = A2 W3^T + b3 — one fused launch, a few rows
-//             per block with the activations in shared memory
+//             A2 = gelu(P2), Y = A2 W3^T + b3 — a product per layer when the
+//             activations are kept for the backward pass, otherwise one fused
+//             launch, a few rows per block with the activations in shared
+//             memory
 //   loss      mean squared error against a target, dY = 2 (Y - T) / (B d_out)
 //   backward  dW3 = dY^T A2, db3 = colsum dY, dP2 = (dY W3) . gelu'(P2), ...
 //   Adam      on the master vector, refreshing the bf16 copy.
@@ -25,10 +27,9 @@
 namespace ab {
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16;
-
-__device__ __forceinline__ float ld(const float* p) { return *p; }
-__device__ __forceinline__ float ld(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+constexpr int TM = 32, TN = 32, TK = 32;       // output tile and K slice of mlp_gemm_kernel
+constexpr int GEMM_THREADS = 128;
+constexpr int GROUPS = TK * TM / 4 / GEMM_THREADS;   // four-element groups of a slice a thread loads
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad(float x) {
@@ -40,78 +41,190 @@ enum { EPI_STORE = 0, EPI_GELU = 1, EPI_GELU_GRAD = 2 };
 // C[m][n] = sum_k A(m, k) B(k, n) (+ bias[n]) with A(m, k) = A[m*sam + k*sak]
 // and B(k, n) = B[k*sbk + n*sbn].  EPI_GELU also stores P (pre-activation)
 // to C and gelu(P) to C2; EPI_GELU_GRAD multiplies by gelu'(P[m][n]).
-template <typename TB, int EPI>
-__global__ void __launch_bounds__(256) mlp_gemm_kernel(int M, int N, int K, const float* __restrict__ A, int sam,
-                                                       int sak, const TB* __restrict__ B, int sbk, int sbn,
-                                                       const float* __restrict__ bias, float* __restrict__ C,
-                                                       int ldc, float* __restrict__ C2, const float* __restrict__ P,
-                                                       int ldp) {
-  __shared__ float As[TK][TM + 4];
-  __shared__ float Bs[TK][TN + 4];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-  float acc[4][4];
+// `colsum`, when given, receives sum_k A(m, k) for every m.
+struct GemmJob {
+  int M, N, K, epi;
+  const float* A;
+  int sam, sak;
+  const void* B;   // float, or bf16 (b_bf16)
+  int b_bf16, sbk, sbn;
+  const float* bias;
+  float* C;
+  int ldc;
+  float* C2;
+  const float* P;
+  int ldp;
+  float* colsum;
+  int a_vec, b_vec;   // set by gemm(): 16-byte (bf16: 8-byte) loads along the unit-stride dimension
+};
+
+// Up to two independent products in one launch (a layer's weight gradient
+// beside the gradient handed to the layer below).
+struct GemmJobs {
+  GemmJob j[2];
+  int tiles0;      // 32 x 32 output tiles of j[0]
+};
+
+// A group of four elements of one operand as loaded (raw bits, so that a
+// prefetched group waits for its load only when it is stored).
+__device__ __forceinline__ uint4 ld4(const float* p) { return *reinterpret_cast<const uint4*>(p); }
+__device__ __forceinline__ uint4 ld4(const __nv_bfloat16* p) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  return make_uint4(r.x, r.y, 0u, 0u);
+}
+__device__ __forceinline__ uint4 pack4(const float* p, size_t su, int n) {
+  return make_uint4(__float_as_uint(p[0]), n > 1 ? __float_as_uint(p[su]) : 0u, n > 2 ? __float_as_uint(p[2 * su]) : 0u,
+                    n > 3 ? __float_as_uint(p[3 * su]) : 0u);
+}
+__device__ __forceinline__ uint4 pack4(const __nv_bfloat16* p, size_t su, int n) {
+  const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+  const uint32_t a = h[0], b = n > 1 ? h[su] : 0u, c = n > 2 ? h[2 * su] : 0u, d = n > 3 ? h[3 * su] : 0u;
+  return make_uint4(a | (b << 16), c | (d << 16), 0u, 0u);
+}
+template <bool BF16>
+__device__ __forceinline__ float4 to_f32(const uint4& r) {
+  if (BF16)
+    return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16),
+                       __uint_as_float(r.y & 0xffff0000u));
+  return make_float4(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z), __uint_as_float(r.w));
+}
+
+// A staged K slice is [TK][32] floats; the float4 holding rows (m or n)
+// 4g..4g+3 of k lies at group g ^ ((k >> 2) & 7), which keeps both kinds of
+// store below and the reads free of bank conflicts.
+__device__ __forceinline__ int slot(int k, int r) { return k * 32 + ((((r >> 2) ^ (k >> 2)) & 7) << 2) + (r & 3); }
+
+// The next K slice of one operand into registers, GROUPS groups of four
+// elements along its unit-stride dimension a thread.  (r, k) is an element's
+// row (m or n) and K index; rows at or past R and k at or past K are zero.
+// `vec`: whole groups are in or out of range and aligned, one load each.
+template <typename T>
+__device__ __forceinline__ void fetch_slice(uint4 (&v)[GROUPS], const T* __restrict__ X, bool vec, int r0, int R,
+                                            int sr, int k0, int K, int sk) {
+  const bool k_unit = sk == 1;
+  const int u = 4 * (threadIdx.x & 7), o = threadIdx.x >> 3;   // along, across the unit-stride dimension
+  const int u_left = (k_unit ? K - k0 : R - r0) - u, o_left = (k_unit ? R - r0 : K - k0) - o;
+  const size_t so = k_unit ? sr : sk, su = k_unit ? sk : sr;
+  const T* p = X + (size_t)r0 * sr + (size_t)k0 * sk + (size_t)o * so + (size_t)u * su;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-  // consecutive threads walk the operand's unit-stride dimension
-  const bool a_k_unit = sak == 1, b_k_unit = sbk == 1;
-  for (int k0 = 0; k0 < K; k0 += TK) {
-    for (int e = threadIdx.x; e < TK * TM; e += 256) {
-      const int kk = a_k_unit ? e % TK : e / TM, mm = a_k_unit ? e / TK : e % TM;
-      const int m = m0 + mm, k = k0 + kk;
-      As[kk][mm] = (m < M && k < K) ? A[(size_t)m * sam + (size_t)k * sak] : 0.0f;
-    }
-    for (int e = threadIdx.x; e < TK * TN; e += 256) {
-      const int kk = b_k_unit ? e % TK : e / TN, nn = b_k_unit ? e / TK : e % TN;
-      const int n = n0 + nn, k = k0 + kk;
-      Bs[kk][nn] = (n < N && k < K) ? ld(B + (size_t)k * sbk + (size_t)n * sbn) : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
+  for (int i = 0; i < GROUPS; ++i, p += (GEMM_THREADS / 8) * so) {
+    v[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (o_left > (GEMM_THREADS / 8) * i && u_left > 0) v[i] = vec ? ld4(p) : pack4(p, su, u_left);
   }
+}
+
+template <bool BF16>
+__device__ __forceinline__ void put_slice(float* S, const uint4 (&v)[GROUPS], bool k_unit) {
+  const int u = 4 * (threadIdx.x & 7), o = threadIdx.x >> 3;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty + 16 * i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx + 16 * j;
-      if (n >= N) continue;
-      float v = acc[i][j];
-      if (EPI != EPI_GELU_GRAD && bias) v += bias[n];
-      if (EPI == EPI_STORE) {
-        C[(size_t)m * ldc + n] = v;
-      } else if (EPI == EPI_GELU) {
-        C[(size_t)m * ldc + n] = v;
-        C2[(size_t)m * ldc + n] = gelu(v);
-      } else {
-        C[(size_t)m * ldc + n] = v * gelu_grad(P[(size_t)m * ldp + n]);
-      }
+  for (int i = 0; i < GROUPS; ++i) {
+    const int oo = o + (GEMM_THREADS / 8) * i;
+    const float4 f = to_f32<BF16>(v[i]);
+    if (k_unit) {
+      S[slot(u, oo)] = f.x;
+      S[slot(u + 1, oo)] = f.y;
+      S[slot(u + 2, oo)] = f.z;
+      S[slot(u + 3, oo)] = f.w;
+    } else {
+      *reinterpret_cast<float4*>(S + slot(oo, u)) = f;
     }
   }
 }
 
-// out[n] = sum_m X[m][n], sequential over m (deterministic).
-__global__ void colsum_kernel(int M, int N, const float* __restrict__ X, int ldx, float* __restrict__ out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float s = 0.0f;
-  for (int m = 0; m < M; ++m) s += X[(size_t)m * ldx + n];
-  out[n] = s;
+// One 32 x 32 output tile per CTA of 128 threads, 4 x 2 outputs a thread, so
+// that the layers of a 512-256-256-512 network and a batch of 512 give 64 to
+// 256 CTAs a launch (64 x 64 tiles gave 16 to 32 and left most SMs idle).  Each
+// output is one chain of fused multiply-adds in k order, whatever the tile:
+// the K slices are only fetched ahead, into registers, while the current one
+// is multiplied out of shared memory (two buffers, one barrier a slice).
+// Bound: the serial walk over K with one or two warps a scheduler (issue
+// 29-40 %): 1340 us for ten training steps of batch 512 through
+// 512-256-256-512, 5030 before.  64 threads with 4 x 4 outputs measured 1660,
+// 256 threads with 2 x 2 outputs 1410, and three slices in flight 1370.
+__global__ void __launch_bounds__(GEMM_THREADS) mlp_gemm_kernel(const __grid_constant__ GemmJobs jobs) {
+  __shared__ __align__(16) float As[2][TK * TM];
+  __shared__ __align__(16) float Bs[2][TK * TN];
+  const bool second = (int)blockIdx.x >= jobs.tiles0;
+  const GemmJob& q = jobs.j[second ? 1 : 0];
+  const int tile = (int)blockIdx.x - (second ? jobs.tiles0 : 0);
+  const int tiles_n = (q.N + TN - 1) / TN;
+  const int M = q.M, N = q.N, K = q.K;
+  const int m0 = tile / tiles_n * TM, n0 = tile % tiles_n * TN;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const bool ak = q.sak == 1, bk = q.sbk == 1, av = q.a_vec, bv = q.b_vec;
+  uint4 va[GROUPS], vb[GROUPS];
+  auto fetch = [&](int k0) {
+    fetch_slice(va, q.A, av, m0, M, q.sam, k0, K, q.sak);
+    if (q.b_bf16) fetch_slice(vb, static_cast<const __nv_bfloat16*>(q.B), bv, n0, N, q.sbn, k0, K, q.sbk);
+    else fetch_slice(vb, static_cast<const float*>(q.B), bv, n0, N, q.sbn, k0, K, q.sbk);
+  };
+  float acc[4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.0f;
+  float csum = 0.0f;   // sum_k A(m0 + tid, k), threads below TM of the first column of tiles
+  const bool want_sum = q.colsum != nullptr && n0 == 0 && threadIdx.x < TM;
+  fetch(0);
+  for (int k0 = 0, buf = 0; k0 < K; k0 += TK, buf ^= 1) {
+    put_slice<false>(As[buf], va, ak);
+    if (q.b_bf16) put_slice<true>(Bs[buf], vb, bk);
+    else put_slice<false>(Bs[buf], vb, bk);
+    __syncthreads();
+    if (k0 + TK < K) fetch(k0 + TK);
+    const float* as = As[buf];
+    const float* bs = Bs[buf];
+    // fragments of four k at a time, the next four read while these multiply
+    float4 fa[2][4];
+    float2 fb[2][4];
+    auto frag = [&](int g, int k) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        fa[g][j] = *reinterpret_cast<const float4*>(as + slot(k + j, 4 * ty));
+        fb[g][j] = *reinterpret_cast<const float2*>(bs + slot(k + j, 2 * tx));
+      }
+    };
+    frag(0, 0);
+#pragma unroll
+    for (int k4 = 0; k4 < TK / 4; ++k4) {
+      const int g = k4 & 1;
+      if (k4 + 1 < TK / 4) frag(g ^ 1, 4 * k4 + 4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float a[4] = {fa[g][j].x, fa[g][j].y, fa[g][j].z, fa[g][j].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          acc[i][0] = fmaf(a[i], fb[g][j].x, acc[i][0]);
+          acc[i][1] = fmaf(a[i], fb[g][j].y, acc[i][1]);
+        }
+      }
+    }
+    if (want_sum) {
+      const int nk = min(TK, K - k0);
+#pragma unroll 8
+      for (int kk = 0; kk < nk; ++kk) csum += as[slot(kk, threadIdx.x)];
+    }
+  }
+  if (want_sum && m0 + (int)threadIdx.x < M) q.colsum[m0 + threadIdx.x] = csum;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + 4 * ty + i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int n = n0 + 2 * tx + j;
+      if (n >= N) continue;
+      float v = acc[i][j];
+      if (q.epi != EPI_GELU_GRAD && q.bias) v += q.bias[n];
+      float* out = q.C + (size_t)m * q.ldc + n;
+      if (q.epi == EPI_STORE) {
+        *out = v;
+      } else if (q.epi == EPI_GELU) {
+        *out = v;
+        q.C2[(size_t)m * q.ldc + n] = gelu(v);
+      } else {
+        *out = v * gelu_grad(q.P[(size_t)m * q.ldp + n]);
+      }
+    }
+  }
 }
 
 // dY = 2 (Y - T) / (B d), and the per-row squared error (FP64).
@@ -180,7 +293,7 @@ __global__ void sur_post_kernel(int C, int D, const float* __restrict__ theta, c
 template <int G>
 __device__ __forceinline__ void dense_layer(const float* __restrict__ in, int din, const __nv_bfloat16* __restrict__ W,
                                             const float* __restrict__ b, int dout, float* __restrict__ out,
-                                            float* __restrict__ pre, bool gelu_act) {
+                                            bool gelu_act) {
   for (int j = threadIdx.x; j < dout; j += blockDim.x) {
     float acc[G];
 #pragma unroll
@@ -216,7 +329,6 @@ __device__ __forceinline__ void dense_layer(const float* __restrict__ in, int di
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       const float v = acc[g] + bj;
-      if (pre) pre[g * dout + j] = v;
       out[g * dout + j] = gelu_act ? gelu(v) : v;
     }
   }
@@ -224,24 +336,20 @@ __device__ __forceinline__ void dense_layer(const float* __restrict__ in, int di
 
 // The whole network for G rows per block.  SUR: input theta with the
 // surrogate's input map z = (theta - mu) * inv_s, output the gradient
-// estimate a + h (theta - mu) + o * y; otherwise input x, output y, and the
-// activations (P1, A1, P2, A2 by rows) saved for the backward pass when act
-// is not NULL.
+// estimate a + h (theta - mu) + o * y; otherwise input x, output y.
 template <int G, bool SUR>
 __global__ void __launch_bounds__(256) mlp_fused_kernel(int B, int din, int h1, int h2, int dout,
                                                         const float* __restrict__ x, int ldx,
                                                         const __nv_bfloat16* __restrict__ wb,
                                                         const float* __restrict__ w, float* __restrict__ y, int ldy,
-                                                        float* __restrict__ act, const float* __restrict__ mu,
+                                                        const float* __restrict__ mu,
                                                         const float* __restrict__ inv_s, const float* __restrict__ sa,
                                                         const float* __restrict__ sh, const float* __restrict__ so) {
   extern __shared__ float sm[];
   float* z = sm;                       // [G][din]
   float* a1 = z + G * din;             // [G][h1]
   float* a2 = a1 + G * h1;             // [G][h2]
-  float* p1 = a2 + G * h2;             // [G][h1]
-  float* p2 = p1 + G * h1;             // [G][h2]
-  float* o3 = p2 + G * h2;             // [G][dout]
+  float* o3 = a2 + G * h2;             // [G][dout]
   const int r0 = blockIdx.x * G;
   const size_t ow1 = 0, ob1 = (size_t)h1 * din, ow2 = ob1 + h1, ob2 = ow2 + (size_t)h2 * h1, ow3 = ob2 + h2,
                ob3 = ow3 + (size_t)dout * h2;
@@ -255,12 +363,11 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(int B, int din, int h1, 
     z[i] = v;
   }
   __syncthreads();
-  const bool save = !SUR && act;
-  dense_layer<G>(z, din, wb + ow1, w + ob1, h1, a1, save ? p1 : nullptr, true);
+  dense_layer<G>(z, din, wb + ow1, w + ob1, h1, a1, true);
   __syncthreads();
-  dense_layer<G>(a1, h1, wb + ow2, w + ob2, h2, a2, save ? p2 : nullptr, true);
+  dense_layer<G>(a1, h1, wb + ow2, w + ob2, h2, a2, true);
   __syncthreads();
-  dense_layer<G>(a2, h2, wb + ow3, w + ob3, dout, o3, nullptr, false);
+  dense_layer<G>(a2, h2, wb + ow3, w + ob3, dout, o3, false);
   __syncthreads();
   for (int i = threadIdx.x; i < G * dout; i += blockDim.x) {
     const int g = i / dout, j = i % dout, r = r0 + g;
@@ -272,41 +379,30 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(int B, int din, int h1, 
     }
     y[(size_t)r * ldy + j] = v;
   }
-  if (save) {
-    float* P1 = act;
-    float* A1 = P1 + (size_t)B * h1;
-    float* P2 = A1 + (size_t)B * h1;
-    float* A2 = P2 + (size_t)B * h2;
-    for (int i = threadIdx.x; i < G * h1; i += blockDim.x) {
-      const int g = i / h1, j = i % h1, r = r0 + g;
-      if (r < B) {
-        P1[(size_t)r * h1 + j] = p1[i];
-        A1[(size_t)r * h1 + j] = a1[i];
-      }
-    }
-    for (int i = threadIdx.x; i < G * h2; i += blockDim.x) {
-      const int g = i / h2, j = i % h2, r = r0 + g;
-      if (r < B) {
-        P2[(size_t)r * h2 + j] = p2[i];
-        A2[(size_t)r * h2 + j] = a2[i];
-      }
-    }
-  }
 }
 
 constexpr int FUSED_G = 4;
 
+inline size_t fused_smem(const ab_mlp_desc* d) {
+  return sizeof(float) * FUSED_G * ((size_t)d->d_in + 2 * d->h1 + 2 * d->h2 + d->d_out);
+}
+
+int check_fused(const ab_mlp_desc* d) {
+  AB_REQUIRE(fused_smem(d) <= 200 * 1024, AB_ERR_ARG, "mlp: layers too wide for the fused kernel");
+  return AB_OK;
+}
+
 template <bool SUR>
-int launch_fused(const ab_mlp_desc* d, int B, const float* x, int ldx, float* y, int ldy, float* act,
-                 const float* mu, const float* inv_s, const float* a, const float* h, const float* o,
-                 cudaStream_t st) {
-  const size_t smem = sizeof(float) * FUSED_G * ((size_t)d->d_in + 2 * d->h1 + 2 * d->h2 + d->d_out);
-  AB_REQUIRE(smem <= 200 * 1024, AB_ERR_ARG, "mlp: layers too wide for the fused kernel");
+int launch_fused(const ab_mlp_desc* d, int B, const float* x, int ldx, float* y, int ldy, const float* mu,
+                 const float* inv_s, const float* a, const float* h, const float* o, cudaStream_t st) {
+  int rc = check_fused(d);
+  if (rc) return rc;
+  const size_t smem = fused_smem(d);
   AB_CUDA(cudaFuncSetAttribute(mlp_fused_kernel<FUSED_G, SUR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem));
   mlp_fused_kernel<FUSED_G, SUR><<<ceil_div(B, FUSED_G), 256, smem, st>>>(
-      B, d->d_in, d->h1, d->h2, d->d_out, x, ldx, static_cast<const __nv_bfloat16*>(d->wb), d->w, y, ldy, act, mu,
-      inv_s, a, h, o);
+      B, d->d_in, d->h1, d->h2, d->d_out, x, ldx, static_cast<const __nv_bfloat16*>(d->wb), d->w, y, ldy, mu, inv_s,
+      a, h, o);
   AB_LAUNCH_CHECK("mlp_fused_kernel");
   return AB_OK;
 }
@@ -328,11 +424,22 @@ Offsets offsets(const ab_mlp_desc* d) {
   return o;
 }
 
-template <typename TB, int EPI>
-int gemm(int M, int N, int K, const float* A, int sam, int sak, const TB* B, int sbk, int sbn, const float* bias,
-         float* C, int ldc, float* C2, const float* P, int ldp, cudaStream_t st) {
-  dim3 grid(ceil_div(N, TN), ceil_div(M, TM));
-  mlp_gemm_kernel<TB, EPI><<<grid, 256, 0, st>>>(M, N, K, A, sam, sak, B, sbk, sbn, bias, C, ldc, C2, P, ldp);
+inline int gemm_tiles(const GemmJob& q) { return (int)(ceil_div(q.M, TM) * ceil_div(q.N, TN)); }
+
+// Whether an operand's groups of four along its unit-stride dimension (n_unit
+// elements, the other dimension `stride` elements apart) can be loaded whole.
+inline int can_vec(const void* p, int unit_stride, int n_unit, int stride, int elem) {
+  return unit_stride == 1 && n_unit % 4 == 0 && stride % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & (4 * elem - 1)) == 0;
+}
+
+int gemm(GemmJob a, const GemmJob* b, cudaStream_t st) {
+  GemmJobs jobs{{a, b ? *b : a}, gemm_tiles(a)};
+  for (GemmJob& q : jobs.j) {
+    q.a_vec = q.sak == 1 ? can_vec(q.A, q.sak, q.K, q.sam, 4) : can_vec(q.A, q.sam, q.M, q.sak, 4);
+    const int es = q.b_bf16 ? 2 : 4;
+    q.b_vec = q.sbk == 1 ? can_vec(q.B, q.sbk, q.K, q.sbn, es) : can_vec(q.B, q.sbn, q.N, q.sbk, es);
+  }
+  mlp_gemm_kernel<<<jobs.tiles0 + (b ? gemm_tiles(*b) : 0), GEMM_THREADS, 0, st>>>(jobs);
   AB_LAUNCH_CHECK("mlp_gemm_kernel");
   return AB_OK;
 }
@@ -368,8 +475,28 @@ extern "C" int ab_mlp_forward(const ab_mlp_desc* d, int B, const float* x, int l
   if (rc) return rc;
   AB_REQUIRE(B > 0 && x && y && ldx >= d->d_in && ldy >= d->d_out && ldx % 4 == 0, AB_ERR_ARG,
              "ab_mlp_forward: bad arguments");
-  return launch_fused<false>(d, B, x, ldx, y, ldy, act, nullptr, nullptr, nullptr, nullptr, nullptr,
-                             as_stream(stream));
+  cudaStream_t st = as_stream(stream);
+  if (!act) return launch_fused<false>(d, B, x, ldx, y, ldy, nullptr, nullptr, nullptr, nullptr, nullptr, st);
+  // the activations are wanted anyway: one tiled product per layer, which
+  // spreads every layer over the GPU (three launches, the same values; for a
+  // batch of 512 through 512-256-256-512 47 us cold and 49 in the fused kernel,
+  // whose CTAs each read every weight)
+  if ((rc = check_fused(d))) return rc;
+  const Offsets o = offsets(d);
+  const __nv_bfloat16* wb = static_cast<const __nv_bfloat16*>(d->wb);
+  const int h1 = d->h1, h2 = d->h2, din = d->d_in, dout = d->d_out;
+  float* P1 = act;
+  float* A1 = P1 + (size_t)B * h1;
+  float* P2 = A1 + (size_t)B * h1;
+  float* A2 = P2 + (size_t)B * h2;
+  if ((rc = gemm(GemmJob{B, h1, din, EPI_GELU, x, ldx, 1, wb + o.w1, 1, 1, din, d->w + o.b1, P1, h1, A1, nullptr, 0,
+                         nullptr}, nullptr, st)))
+    return rc;
+  if ((rc = gemm(GemmJob{B, h2, h1, EPI_GELU, A1, h1, 1, wb + o.w2, 1, 1, h1, d->w + o.b2, P2, h2, A2, nullptr, 0,
+                         nullptr}, nullptr, st)))
+    return rc;
+  return gemm(GemmJob{B, dout, h2, EPI_STORE, A2, h2, 1, wb + o.w3, 1, 1, h2, d->w + o.b3, y, ldy, nullptr, nullptr, 0,
+                      nullptr}, nullptr, st);
 }
 
 extern "C" int ab_sur_predict(const ab_mlp_desc* d, int C, const float* theta, int ldt, const float* mu,
@@ -380,7 +507,7 @@ extern "C" int ab_sur_predict(const ab_mlp_desc* d, int C, const float* theta, i
   AB_REQUIRE(d->d_in == d->d_out, AB_ERR_ARG, "ab_sur_predict: the network must map D to D");
   AB_REQUIRE(C > 0 && theta && mu && inv_s && a && h && o && g && ldt >= d->d_in && ldg >= d->d_out, AB_ERR_ARG,
              "ab_sur_predict: bad arguments");
-  return launch_fused<true>(d, C, theta, ldt, g, ldg, nullptr, mu, inv_s, a, h, o, as_stream(stream));
+  return launch_fused<true>(d, C, theta, ldt, g, ldg, mu, inv_s, a, h, o, as_stream(stream));
 }
 
 extern "C" int ab_mlp_mse(int B, int D, const float* y, int ldy, const float* target, int ldt, float* dy,
@@ -413,31 +540,23 @@ extern "C" int ab_mlp_backward(const ab_mlp_desc* d, int B, const float* x, int 
   float* dP2 = scratch;                        // [B][h2]
   float* dP1 = scratch + (size_t)B * d->h2;    // [B][h1]
   const int h1 = d->h1, h2 = d->h2, din = d->d_in, dout = d->d_out;
-  // dW3[o][j] = sum_b dY[b][o] A2[b][j];  db3 = colsum dY
-  if ((rc = gemm<float, EPI_STORE>(dout, h2, B, dy, 1, dout, A2, h2, 1, nullptr, grad + o.w3, h2, nullptr, nullptr, 0,
-                                   st)))
-    return rc;
-  colsum_kernel<<<ceil_div(dout, 128), 128, 0, st>>>(B, dout, dy, dout, grad + o.b3);
-  AB_LAUNCH_CHECK("colsum_kernel");
+  // dW3[o][j] = sum_b dY[b][o] A2[b][j], db3 = colsum dY; beside it
   // dP2 = (dY W3) . gelu'(P2)
-  if ((rc = gemm<__nv_bfloat16, EPI_GELU_GRAD>(B, h2, dout, dy, dout, 1, wb + o.w3, h2, 1, nullptr, dP2, h2, nullptr,
-                                               P2, h2, st)))
-    return rc;
-  if ((rc = gemm<float, EPI_STORE>(h2, h1, B, dP2, 1, h2, A1, h1, 1, nullptr, grad + o.w2, h1, nullptr, nullptr, 0,
-                                   st)))
-    return rc;
-  colsum_kernel<<<ceil_div(h2, 128), 128, 0, st>>>(B, h2, dP2, h2, grad + o.b2);
-  AB_LAUNCH_CHECK("colsum_kernel");
-  // dP1 = (dP2 W2) . gelu'(P1)
-  if ((rc = gemm<__nv_bfloat16, EPI_GELU_GRAD>(B, h1, h2, dP2, h2, 1, wb + o.w2, h1, 1, nullptr, dP1, h1, nullptr, P1,
-                                               h1, st)))
-    return rc;
-  if ((rc = gemm<float, EPI_STORE>(h1, din, B, dP1, 1, h1, x, ldx, 1, nullptr, grad + o.w1, din, nullptr, nullptr, 0,
-                                   st)))
-    return rc;
-  colsum_kernel<<<ceil_div(h1, 128), 128, 0, st>>>(B, h1, dP1, h1, grad + o.b1);
-  AB_LAUNCH_CHECK("colsum_kernel");
-  return AB_OK;
+  const GemmJob w3{dout, h2, B, EPI_STORE, dy, 1, dout, A2, 0, h2, 1, nullptr, grad + o.w3, h2, nullptr, nullptr, 0,
+                   grad + o.b3};
+  const GemmJob p2{B, h2, dout, EPI_GELU_GRAD, dy, dout, 1, wb + o.w3, 1, h2, 1, nullptr, dP2, h2, nullptr, P2, h2,
+                   nullptr};
+  if ((rc = gemm(w3, &p2, st))) return rc;
+  // dW2, db2; beside them dP1 = (dP2 W2) . gelu'(P1)
+  const GemmJob w2{h2, h1, B, EPI_STORE, dP2, 1, h2, A1, 0, h1, 1, nullptr, grad + o.w2, h1, nullptr, nullptr, 0,
+                   grad + o.b2};
+  const GemmJob p1{B, h1, h2, EPI_GELU_GRAD, dP2, h2, 1, wb + o.w2, 1, h1, 1, nullptr, dP1, h1, nullptr, P1, h1,
+                   nullptr};
+  if ((rc = gemm(w2, &p1, st))) return rc;
+  // dW1, db1
+  const GemmJob w1{h1, din, B, EPI_STORE, dP1, 1, h1, x, 0, ldx, 1, nullptr, grad + o.w1, din, nullptr, nullptr, 0,
+                   grad + o.b1};
+  return gemm(w1, nullptr, st);
 }
 
 extern "C" int ab_mlp_adam(const ab_mlp_desc* d, const float* grad, float* m, float* v, int step, float lr, float b1,

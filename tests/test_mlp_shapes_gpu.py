@@ -1,0 +1,43 @@
+"""The surrogate network's layer products at ragged batch and layer sizes
+(remainders of the 32 x 32 output tiles and 32-deep K slices, one partial
+tile, unaligned operands) against the FP64 oracle."""
+import numpy as np
+import pytest
+import torch
+
+from augurv2_b200 import hlrb as H
+from oracle import batched as B
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D,h1,h2,Bn,pad", [(8, 8, 8, 1, 0), (16, 24, 40, 31, 0), (40, 32, 64, 33, 4), (136, 72, 256, 65, 0),
+                                            (64, 264, 128, 512, 8), (24, 16, 8, 7, 0)])
+def test_forward_backward_match_fp64_at_ragged_sizes(D, h1, h2, Bn, pad):
+    sur = H.MlpSurrogate(D, h1, h2, seed=D + Bn)
+    gen = torch.Generator("cuda").manual_seed(Bn)
+    # rows of x `pad` elements longer than the layer; dy starts 4 bytes off a
+    # 16-byte boundary, so its groups are loaded element by element
+    x = torch.randn(Bn, D + pad, device="cuda", generator=gen)
+    dy_mem = torch.randn(Bn * D + 1, device="cuda", generator=gen)
+    dy = dy_mem[1:]
+    sc = sur._scratch(Bn)
+    L = H.N.lib()
+    H.N.check(L.ab_mlp_forward(H.C.byref(sur.desc), Bn, H.N.ptr(x), D + pad, H.N.ptr(sc["out"]), D, H.N.ptr(sc["act"]), None))
+    H.N.check(L.ab_mlp_backward(H.C.byref(sur.desc), Bn, H.N.ptr(x), D + pad, dy.data_ptr(), H.N.ptr(sc["act"]),
+                                H.N.ptr(sur.gw), H.N.ptr(sc["bsc"]), None))
+    torch.cuda.synchronize()
+    wmat, w = sur.wb.double().cpu().numpy(), sur.w.double().cpu().numpy()
+    x64 = x[:, :D].double().cpu().numpy()
+    Y, _ = B.mlp_forward(wmat, w, x64, D, h1, h2, D)
+    out = sc["out"].double().cpu().numpy()
+    assert np.max(np.abs(out - Y)) <= 1e-4 * max(1.0, np.max(np.abs(Y)))
+    # the oracle's loss gradient at the target that gives this dy (FP64 outputs
+    # differ from the device's by rounding only)
+    t64 = Y - dy.double().cpu().numpy().reshape(Bn, D) * (0.5 * Bn * D)
+    _, g = B.mlp_loss_grad(wmat, w, x64, t64, D, h1, h2, D)
+    gd = sur.gw.double().cpu().numpy()
+    n1, n2 = h1 * D, h2 * h1
+    offs = [0, n1, n1 + h1, n1 + h1 + n2, n1 + h1 + n2 + h2, n1 + h1 + n2 + h2 + D * h2, len(g)]
+    for a, b in zip(offs[:-1], offs[1:]):
+        assert np.max(np.abs(gd[a:b] - g[a:b])) <= 1e-4 * np.max(np.abs(g[a:b])), (a, b)
