@@ -60,66 +60,6 @@ __device__ void w_chol(double* A, int d) {
   }
 }
 
-// augur_mat_lower_trmi (:335-345).  In the in-place loop the entries above
-// the diagonal of column c come out as exact zeros before any lower entry of
-// the column is formed, so each column is an independent forward
-// substitution over the original factor; the zero terms it skips change
-// nothing.  One lane per column; T receives the original factor, which the
-// sequential loop would still see in the columns not yet processed.
-__device__ void w_trmi(double* L, double* T, int d) {
-  const int lane = threadIdx.x & 31;
-  for (int e = lane; e < d * d; e += 32) T[e] = L[e];
-  __syncwarp();
-  for (int c = lane; c < d; c += 32) {
-    for (int m = c; m < d; ++m) {
-      double b = (c == m) ? 1.0 : 0.0;
-#pragma unroll 4
-      for (int i = c; i < m; ++i) b = __dadd_rn(b, -__dmul_rn(GM(T, m, i), GM(L, i, c)));
-      GM(L, m, c) = __ddiv_rn(b, GM(T, m, m));
-    }
-  }
-  __syncwarp();
-  for (int e = lane; e < d * d; e += 32) {
-    const int r = e / d, c = e - r * d;
-    if (r < c) L[e] = 0.0;
-  }
-  __syncwarp();
-}
-
-// augur_mat_cholesky_invert (:363-375): trmi, then for each column c and row
-// r >= c (in order) A[r][c] = sum_{k=c}^{d-1} A[k][r] A[k][c] with the
-// column's earlier rows already replaced, then the lower part mirrored.
-// After trmi the factor's upper triangle is zero, so the terms k < r are
-// zero products: starting from +0.0 they leave the sum +0.0, and the entry
-// is the sum over k = r .. d-1 of M[k][r] M[k][c] (M the inverse factor, kept
-// in T), in k order - independent of every other entry (while the entries
-// are finite).  The d(d+1)/2 entries are dealt to the lanes in turn, which
-// balances their d - r terms (column 0 alone used to take d^2 / 2 steps of
-// one lane).
-__device__ void w_cholinv(double* A, double* T, int d) {
-  const int lane = threadIdx.x & 31;
-  w_trmi(A, T, d);
-  for (int e = lane; e < d * d; e += 32) T[e] = A[e];
-  __syncwarp();
-  const int ntri = d * (d + 1) / 2;
-  for (int idx = lane; idx < ntri; idx += 32) {
-    int r = (int)((sqrtf(8.0f * (float)idx + 1.0f) - 1.0f) * 0.5f);
-    while (r * (r + 1) / 2 > idx) --r;
-    while ((r + 1) * (r + 2) / 2 <= idx) ++r;
-    const int c = idx - r * (r + 1) / 2;
-    double acc = 0.0;
-#pragma unroll 4
-    for (int k = r; k < d; ++k) acc = __dadd_rn(acc, __dmul_rn(GM(T, k, r), GM(T, k, c)));
-    GM(A, r, c) = acc;
-  }
-  __syncwarp();
-  for (int e = lane; e < d * d; e += 32) {
-    const int r = e / d, c = e - r * d;
-    if (r < c) A[e] = GM(A, c, r);
-  }
-  __syncwarp();
-}
-
 // augur_mat_trvm (:398-406): v = L v (row i uses the original v[0..i]).
 __device__ void w_trvm(const double* L, double* v, double* tmp, int d) {
   const int lane = threadIdx.x & 31;
@@ -131,35 +71,6 @@ __device__ void w_trvm(const double* L, double* v, double* tmp, int d) {
   }
   __syncwarp();
   for (int i = lane; i < d; i += 32) v[i] = tmp[i];
-  __syncwarp();
-}
-
-// augur_mat_mvm (:412-420): dst = A v.
-__device__ void w_mvm(double* dst, const double* A, const double* v, int d) {
-  const int lane = threadIdx.x & 31;
-  for (int i = lane; i < d; i += 32) {
-    double s = 0.0;
-#pragma unroll 4
-    for (int j = 0; j < d; ++j) s = __dadd_rn(s, __dmul_rn(GM(A, i, j), v[j]));
-    dst[i] = s;
-  }
-  __syncwarp();
-}
-
-// augur_mat_trtrmm (:381-392): L2 = L1 L2 (rows below i are original when row
-// i is formed).
-__device__ void w_trtrmm(const double* L1, double* L2, double* tmp, int d) {
-  const int lane = threadIdx.x & 31;
-  for (int e = lane; e < d * d; e += 32) {
-    const int i = e / d, j = e - i * d;
-    double s = 0.0;
-#pragma unroll 4
-    for (int k = 0; k < i; ++k) s = __dadd_rn(s, __dmul_rn(GM(L1, i, k), GM(L2, k, j)));
-    s = __dadd_rn(s, __dmul_rn(GM(L1, i, i), GM(L2, i, j)));
-    tmp[e] = s;
-  }
-  __syncwarp();
-  for (int e = lane; e < d * d; e += 32) L2[e] = tmp[e];
   __syncwarp();
 }
 
@@ -182,28 +93,188 @@ __device__ void w_mvn_sample(const Stream& s, double* result, const double* mean
   __syncwarp();
 }
 
+// ---- thread-group matrix routines -----------------------------------------
+// The same factorisations by a group of `nt` threads (a whole CTA, or one of
+// two equal halves that factor different matrices in step), t the thread's
+// index in it.  Every thread of the CTA calls them together: they use
+// __syncthreads.  The lower-triangle entries (i, j) are dealt to the threads,
+// NE at most each, and every entry's sum over k is carried in a register and
+// extended as soon as the column (or row) k it needs is final: the same
+// additions in the same order as the reference's loop, so the same values,
+// but the chain is one column after another - a reciprocal root, two barriers
+// and one product - instead of all of a column's products in turn.
+// Their matrices have rows of pitch(d) doubles: a column is read by many
+// lanes at once, and an odd pitch spreads it over the banks (with rows of d =
+// 32 doubles every such read was a 32-way conflict).
+__host__ __device__ __forceinline__ int pitch(int d) { return d | 1; }
+#define GP(A, i, j) (A)[(i) * (d | 1) + (j)]
+
+template <int NE>
+struct Tri {
+  int ij[NE];    // i << 8 | j, or -1
+  __device__ __forceinline__ void deal(int t, int nt, int d) {
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+      const int e = t + q * nt;
+      if (e >= d * (d + 1) / 2) { ij[q] = -1; continue; }
+      int r = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+      while (r * (r + 1) / 2 > e) --r;
+      while ((r + 1) * (r + 2) / 2 <= e) ++r;
+      ij[q] = r << 8 | (e - r * (r + 1) / 2);
+    }
+  }
+};
+
+// sqrt(x) and 1 / sqrt(x)'s rounded root, both correctly rounded: the
+// reciprocal root (CUDA's rsqrt, within an ulp) gives the root by one
+// residual step and seeds the reciprocal, which a second one rounds
+// (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  Far shorter a chain than a square root and a
+// division in turn; values outside its range take those.
+__device__ __forceinline__ void root_recip(double x, double& root, double& rec) {
+  if (x > 0x1p-900 && x < 0x1p900) {
+    const double y = rsqrt(x);
+    const double g = __dmul_rn(x, y);
+    root = __fma_rn(__fma_rn(-g, g, x), __dmul_rn(0.5, y), g);
+    rec = __fma_rn(__fma_rn(-root, y, 1.0), y, y);
+  } else {
+    root = __dsqrt_rn(x);
+    rec = __ddiv_rn(1.0, root);
+  }
+}
+
+// b / v given rec = 1 / v correctly rounded: the quotient's residual rounds it
+// correctly (the same theorem) while nothing under- or overflows.
+__device__ __forceinline__ double quotient(double b, double v, double rec) {
+  const double ab = fabs(b), av = fabs(v);
+  if ((ab > 0x1p-400 && ab < 0x1p400 && av > 0x1p-400 && av < 0x1p400) || b == 0.0) {
+    const double q = __dmul_rn(b, rec);
+    return __fma_rn(__fma_rn(-q, v, b), rec, q);
+  }
+  return __ddiv_rn(b, v);
+}
+
+// augur_mat_cholesky (:312-328) of A, in place (lower triangle; the upper one
+// is left as it is, as the reference leaves it) and, with INV,
+// augur_mat_lower_trmi (:335-345) of the factor into O, lower triangle, in the
+// same walk: once column k of the factor is final, so is row k of its inverse.
+// Entry (i, j) first sums A[i][k] A[j][k] over k < j, becomes final at k = j,
+// then subtracts L[i][k] O[k][j] over j <= k < i from the identity's entry and
+// gives O[i][j] at k = i.  piv: [d] scratch.
+template <int NE, bool INV>
+__device__ __forceinline__ void g_factor(const Tri<NE>& T, double* A, double* O, double* piv, int d) {
+  double acc[NE];
+#pragma unroll
+  for (int q = 0; q < NE; ++q) acc[q] = 0.0;
+  __syncthreads();
+  for (int k = 0; k < d; ++k) {
+    // the pivot A[k][k] - sum, published by its owner
+#pragma unroll
+    for (int q = 0; q < NE; ++q)
+      if (T.ij[q] == (k << 8 | k)) piv[k] = __dadd_rn(GP(A, k, k), -acc[q]);
+    __syncthreads();
+    double root, rec;
+    root_recip(piv[k], root, rec);
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+      const int i = T.ij[q] >> 8, j = T.ij[q] & 255;
+      if (T.ij[q] < 0) continue;
+      if (j == k) {
+        GP(A, i, k) = i == k ? root : __dmul_rn(rec, __dadd_rn(GP(A, i, k), -acc[q]));
+        if (INV && i == k) GP(O, k, k) = rec;
+        acc[q] = 0.0;
+      } else if (INV && i == k) {
+        GP(O, k, j) = quotient(acc[q], root, rec);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+      const int i = T.ij[q] >> 8, j = T.ij[q] & 255;
+      if (T.ij[q] < 0 || i <= k || (!INV && j <= k)) continue;
+      const double p = __dmul_rn(GP(A, i, k), j > k ? GP(A, j, k) : GP(O, k, j));
+      acc[q] = __dadd_rn(acc[q], j > k ? p : -p);
+    }
+  }
+  __syncthreads();
+}
+
+// augur_mat_lower_trmi (:335-345) of a given factor L into O, lower triangle.
+template <int NE>
+__device__ __forceinline__ void g_trmi(const Tri<NE>& T, const double* L, double* O, double* recs, int t, int nt,
+                                       int d) {
+  double b[NE];
+#pragma unroll
+  for (int q = 0; q < NE; ++q) b[q] = (T.ij[q] >> 8) == (T.ij[q] & 255) ? 1.0 : 0.0;
+  __syncthreads();
+  for (int i = t; i < d; i += nt) recs[i] = __ddiv_rn(1.0, GP(L, i, i));
+  __syncthreads();
+  for (int r = 0; r < d; ++r) {
+#pragma unroll
+    for (int q = 0; q < NE; ++q)
+      if (T.ij[q] >= 0 && (T.ij[q] >> 8) == r) GP(O, r, T.ij[q] & 255) = quotient(b[q], GP(L, r, r), recs[r]);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+      const int m = T.ij[q] >> 8, c = T.ij[q] & 255;
+      if (T.ij[q] >= 0 && m > r && c <= r) b[q] = __dadd_rn(b[q], -__dmul_rn(GP(L, m, r), GP(O, r, c)));
+    }
+  }
+  __syncthreads();
+}
+
+// The product of augur_mat_cholesky_invert (:363-375) from the inverse factor
+// M (lower triangle): A[r][c] = sum_{k >= r} M[k][r] M[k][c] in k order (the
+// reference's terms k < r are zero products), mirrored.
+template <int NE>
+__device__ __forceinline__ void g_inverse(const Tri<NE>& T, const double* M, double* A, int d) {
+#pragma unroll
+  for (int q = 0; q < NE; ++q) {
+    if (T.ij[q] < 0) continue;
+    const int r = T.ij[q] >> 8, c = T.ij[q] & 255;
+    double acc = 0.0;
+#pragma unroll 8
+    for (int k = r; k < d; ++k) acc = __dadd_rn(acc, __dmul_rn(GP(M, k, r), GP(M, k, c)));
+    GP(A, r, c) = acc;
+    GP(A, c, r) = acc;
+  }
+  __syncthreads();
+}
+
+// augur_mat_mvm (:412-420) by threads t = 0 .. d-1 of the group.
+__device__ __forceinline__ void g_mvm(double* dst, const double* A, const double* v, int t, int nt, int d) {
+  for (int i = t; i < d; i += nt) {
+    double s = 0.0;
+#pragma unroll 8
+    for (int j = 0; j < d; ++j) s = __dadd_rn(s, __dmul_rn(GP(A, i, j), v[j]));
+    dst[i] = s;
+  }
+}
+
 // ---- per-component tables for the assignment draw -------------------------
 // Linv = lower_trmi(chol(cov_k)) and hdet = 0.5 * log((prod L_ii)^2), the
 // quantities augur_mvnormal_ll (augur_dist.c:548-568) derives from cov.
-__global__ void __launch_bounds__(32)
+template <int DT>
+__global__ void __launch_bounds__(GMM_THREADS)
 gmm_prep_kernel(int d, const double* __restrict__ cov, double* __restrict__ Linv, double* __restrict__ hdet) {
+  constexpr int NE = (DT * (DT + 1) / 2 + GMM_THREADS - 1) / GMM_THREADS;
   extern __shared__ double sm[];
-  const int k = blockIdx.x;
+  __shared__ double piv[DT];
+  const int k = blockIdx.x, tid = threadIdx.x;
   double* L = sm;
-  double* T = sm + d * d;
-  const int lane = threadIdx.x;
-  for (int e = lane; e < d * d; e += 32) L[e] = cov[(size_t)k * d * d + e];
-  __syncwarp();
-  w_chol(L, d);
-  if (lane == 0) {
+  double* O = sm + d * pitch(d);
+  for (int e = tid; e < d * d; e += GMM_THREADS) GP(L, e / d, e % d) = cov[(size_t)k * d * d + e];
+  Tri<NE> T;
+  T.deal(tid, GMM_THREADS, d);
+  g_factor<NE, true>(T, L, O, piv, d);
+  for (int e = tid; e < d * d; e += GMM_THREADS)
+    Linv[(size_t)k * d * d + e] = e / d >= e % d ? GP(O, e / d, e % d) : 0.0;
+  if (tid == GMM_THREADS - 1) {
     double det = 1.0;
-    for (int i = 0; i < d; ++i) det = __dmul_rn(det, GM(L, i, i));
+    for (int i = 0; i < d; ++i) det = __dmul_rn(det, GP(L, i, i));
     det = __dmul_rn(det, det);
     hdet[k] = __dmul_rn(0.5, log(det));
   }
-  __syncwarp();
-  w_trmi(L, T, d);
-  for (int e = lane; e < d * d; e += 32) Linv[(size_t)k * d * d + e] = L[e];
 }
 
 // ---- assignment draw --------------------------------------------------------
@@ -724,56 +795,80 @@ __global__ void gmm_conj_pis_kernel(int K, const double* __restrict__ alpha, con
 }
 
 // augur_mvnormal_mvnormal_conj (augur_dist.c:633-669) for component k, one
-// warp, substream (k, iter, 8|comp<<8).
-__global__ void __launch_bounds__(64)
+// CTA, substream (k, iter, 8|comp<<8).  The two halves of the CTA invert the
+// prior and the component covariance in step, then all of it inverts and
+// factors the posterior precision.  Bound: the chain of the d columns of three
+// factorisations, about 1400 cycles each (157 -> 81 us at d = 32, K = 16; one
+// warp per matrix before).
+template <int DT>
+__global__ void __launch_bounds__(GMM_THREADS)
 gmm_conj_mu_kernel(int d, int shared_cov, const double* __restrict__ mu0, const double* __restrict__ cov0,
                    const int* __restrict__ cnt, const double* __restrict__ sum, const double* __restrict__ cov,
                    double* __restrict__ mu, uint64_t seed, uint32_t iter, uint32_t comp) {
+  constexpr int HALF = GMM_THREADS / 2;
+  constexpr int TE = DT * (DT + 1) / 2;
+  constexpr int NH = (TE + HALF - 1) / HALF, NE = (TE + GMM_THREADS - 1) / GMM_THREADS;
   extern __shared__ double sm[];
-  const int k = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int dd = d * d;
+  __shared__ double piv[2][DT];
+  const int k = blockIdx.x, tid = threadIdx.x;
+  const int half = tid / HALF, t = tid - half * HALF;
+  const int dd = d * d, dp = d * pitch(d);
   double* L0 = sm;
-  double* L = L0 + dd;
-  double* T = L + dd;
-  double* T2 = T + dd;
-  double* res = T2 + dd;
+  double* L = L0 + dp;
+  double* M0 = L + dp;
+  double* M1 = M0 + dp;
+  double* res = M1 + dp;
   double* w0 = res + d;
   double* mean = w0 + d;
   double* sk = mean + d;
-  double* tmp = sk + d;
-  double* mu0s = tmp + d;
+  double* nrm = sk + d;
+  double* mu0s = nrm + d;
   const double* ck = cov + (size_t)(shared_cov ? 0 : k) * dd;
-  for (int e = threadIdx.x; e < dd; e += blockDim.x) { L0[e] = cov0[e]; L[e] = ck[e]; }
-  for (int i = threadIdx.x; i < d; i += blockDim.x) { sk[i] = sum[(size_t)k * d + i]; mu0s[i] = mu0[i]; }
-  __syncthreads();
-  // the two inverses are independent: one warp each (each the reference's
-  // sequential routine, so the values are unchanged), then warp 0 alone
-  if (warp == 0) {
-    w_chol(L0, d);
-    w_cholinv(L0, T, d);
+  const int n = cnt[k];
+  const double sc = n == 0 ? 1.0 : __ddiv_rn(1.0, (double)n);                       // augur_vec_scale
+  for (int e = tid; e < dd; e += GMM_THREADS) {
+    GP(L0, e / d, e % d) = cov0[e];
+    GP(L, e / d, e % d) = ck[e];
+  }
+  for (int i = tid; i < d; i += GMM_THREADS) {
+    sk[i] = __dmul_rn(sc, sum[(size_t)k * d + i]);
+    mu0s[i] = mu0[i];
+    Stream s = make_stream(seed, (uint32_t)k, iter, TAG_MU | (comp << 8));
+    s.pos = (uint32_t)i;
+    nrm[i] = s.normal();
+  }
+  double* A = half ? L : L0;
+  double* M = half ? M1 : M0;
+  {
+    Tri<NH> T;
+    T.deal(t, HALF, d);
+    g_factor<NH, true>(T, A, M, piv[half], d);
+    g_inverse(T, M, A, d);
+  }
+  if (half) {
+    for (int e = t; e < dp; e += HALF) L[e] = __dmul_rn((double)n, L[e]);           // augur_mat_ms
   } else {
-    w_chol(L, d);
-    w_cholinv(L, T2, d);
+    g_mvm(res, L0, mu0s, t, HALF, d);
   }
   __syncthreads();
-  if (warp != 0) return;
-  const int n = cnt[k];
-  for (int e = lane; e < dd; e += 32) L[e] = __dmul_rn((double)n, L[e]);           // augur_mat_ms
-  __syncwarp();
-  w_mvm(res, L0, mu0s, d);
-  const double sc = n == 0 ? 1.0 : __ddiv_rn(1.0, (double)n);                       // augur_vec_scale
-  for (int i = lane; i < d; i += 32) sk[i] = __dmul_rn(sc, sk[i]);
-  __syncwarp();
-  w_mvm(w0, L, sk, d);
-  for (int i = lane; i < d; i += 32) res[i] = __dadd_rn(res[i], w0[i]);
-  for (int e = lane; e < dd; e += 32) L0[e] = __dadd_rn(L0[e], L[e]);              // augur_mat_plus
-  __syncwarp();
-  w_chol(L0, d);
-  w_cholinv(L0, T, d);
-  w_mvm(mean, L0, res, d);
-  const Stream s = make_stream(seed, (uint32_t)k, iter, TAG_MU | (comp << 8));
-  w_mvn_sample(s, res, mean, L0, L, tmp, d);
-  for (int i = lane; i < d; i += 32) mu[(size_t)k * d + i] = res[i];
+  if (half) g_mvm(w0, L, sk, t, HALF, d);
+  __syncthreads();
+  for (int i = tid; i < d; i += GMM_THREADS) res[i] = __dadd_rn(res[i], w0[i]);
+  for (int e = tid; e < dp; e += GMM_THREADS) L0[e] = __dadd_rn(L0[e], L[e]);      // augur_mat_plus
+  Tri<NE> T;
+  T.deal(tid, GMM_THREADS, d);
+  g_factor<NE, true>(T, L0, M0, piv[0], d);
+  g_inverse(T, M0, L0, d);
+  g_mvm(mean, L0, res, tid, GMM_THREADS, d);
+  // augur_mvnormal_sample (augur_dist.c:622-630): chol(cov) nrm + mean
+  for (int e = tid; e < dp; e += GMM_THREADS) L[e] = L0[e];
+  g_factor<NE, false>(T, L, nullptr, piv[1], d);
+  for (int i = tid; i < d; i += GMM_THREADS) {
+    double s = 0.0;
+#pragma unroll 8
+    for (int j = 0; j <= i; ++j) s = __dadd_rn(s, __dmul_rn(GP(L, i, j), nrm[j]));
+    mu[(size_t)k * d + i] = __dadd_rn(s, mean[i]);
+  }
 }
 
 // Bartlett diagonal for the inverse-Wishart draw (bartlett_decomp,
@@ -813,52 +908,56 @@ gmm_bartlett_chi_kernel(int d, int df, const int* __restrict__ cnt, double* __re
 // chi-square of n - i normals follows its row's off-diagonal normals).  The
 // chi-square sums of up to cnt + df squares come from
 // gmm_bartlett_chi_kernel (chi[k * sk + i * si]), added in a fixed tree order
-// instead of sequentially (a rounding-level difference); the d x d algebra
-// runs on warp 0.
+// instead of sequentially (a rounding-level difference).  Bound: the chain of
+// the d columns of two factorisations and one inverse (126 -> 51 us at d = 32).
+template <int DT>
 __global__ void __launch_bounds__(GMM_THREADS)
 gmm_conj_cov_kernel(int d, int df, const double* __restrict__ scale0, const int* __restrict__ cnt,
                     const double* __restrict__ obs, const double* chi, int sk, int si, double* cov, uint64_t seed,
                     uint32_t iter, uint32_t comp) {
+  constexpr int NE = (DT * (DT + 1) / 2 + GMM_THREADS - 1) / GMM_THREADS;
   extern __shared__ double sm[];
+  __shared__ double piv[DT];
   const int k = blockIdx.x, tid = threadIdx.x;
-  const int dd = d * d;
-  double* S = sm;          // obs + scale0
-  double* L = S + dd;
-  double* A = L + dd;
-  double* T = A + dd;
-  for (int e = tid; e < dd; e += blockDim.x) {
-    S[e] = __dadd_rn(obs[(size_t)k * dd + e], scale0[e]);
-    L[e] = S[e];
-  }
-  __syncthreads();
+  const int dd = d * d, dp = d * pitch(d);
+  double* L = sm;          // obs + scale0, then its inverse's factor
+  double* M = L + dp;
+  double* A = M + dp;
+  double* P = A + dp;
+  for (int e = tid; e < dd; e += GMM_THREADS) GP(L, e / d, e % d) = __dadd_rn(obs[(size_t)k * dd + e], scale0[e]);
   const int n = cnt[k] + df;
-  if (tid < 32) {
-    w_chol(L, d);
-    w_cholinv(L, T, d);
-    w_chol(L, d);
-  }
   // Bartlett factor: element (i, j < i) is the normal at position i*n + j;
   // the diagonal (i, i) is the square root of the row's chi-square sum.
   const Stream s0 = make_stream(seed, (uint32_t)k, iter, TAG_COV | (comp << 8));
-  for (int e = tid; e < dd; e += blockDim.x) {
+  for (int e = tid; e < dd; e += GMM_THREADS) {
     const int i = e / d, j = e - i * d;
     if (j < i) {
       Stream s = s0;
       s.pos = (uint32_t)(i * n + j);
-      A[e] = s.normal();
+      GP(A, i, j) = s.normal();
     } else if (j > i) {
-      A[e] = 0.0;
+      GP(A, i, j) = 0.0;
     } else {
-      A[e] = __dsqrt_rn(chi[(size_t)k * sk + (size_t)i * si]);
+      GP(A, i, j) = __dsqrt_rn(chi[(size_t)k * sk + (size_t)i * si]);
     }
   }
-  __syncthreads();
-  if (tid < 32) {
-    w_trtrmm(L, A, T, d);
-    w_cholinv(A, T, d);
+  Tri<NE> T;
+  T.deal(tid, GMM_THREADS, d);
+  g_factor<NE, true>(T, L, M, piv, d);
+  g_inverse(T, M, L, d);
+  g_factor<NE, false>(T, L, nullptr, piv, d);
+  // augur_mat_trtrmm (:381-392): the entries above the diagonal of L are not
+  // read; A's are zeros, so the product's upper entries are sums of zeros
+  for (int e = tid; e < dd; e += GMM_THREADS) {
+    const int i = e / d, j = e - i * d;
+    double s = 0.0;
+#pragma unroll 8
+    for (int q = 0; q <= i; ++q) s = __dadd_rn(s, __dmul_rn(GP(L, i, q), GP(A, q, j)));
+    GP(P, i, j) = s;
   }
-  __syncthreads();
-  for (int e = tid; e < dd; e += blockDim.x) cov[(size_t)k * dd + e] = A[e];
+  g_trmi(T, P, M, piv, tid, GMM_THREADS, d);
+  g_inverse(T, M, L, d);
+  for (int e = tid; e < dd; e += GMM_THREADS) cov[(size_t)k * dd + e] = GP(L, e / d, e % d);
 }
 
 // ---- ESlice / MWG on the means ---------------------------------------------------
@@ -996,6 +1095,7 @@ gmm_mwg_kernel(int N, int d, int shared_cov, const float* __restrict__ Y, const 
 }
 
 #undef GM
+#undef GP
 
 // ---- launchers -------------------------------------------------------------------
 static int gmm_check(int N, int d, int K) {
@@ -1070,12 +1170,24 @@ int launch_gmm_z_screened(int N, int d, int K, int shared, const float* Y, const
   return AB_OK;
 }
 
-int launch_gmm_prep(int Kc, int d, const double* cov, double* Linv, double* hdet, cudaStream_t st) {
-  const size_t smem = sizeof(double) * 2 * (size_t)d * d;
-  AB_CUDA(cudaFuncSetAttribute(gmm_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gmm_prep_kernel<<<Kc, 32, smem, st>>>(d, cov, Linv, hdet);
+// The thread-group kernels are built for d <= 16, 32 and 64 (the entries a
+// thread carries in registers).
+#define AB_GMM_BY_D(d, CALL) \
+  ((d) <= 16 ? CALL(16) : (d) <= 32 ? CALL(32) : CALL(GMM_MAX_D))
+
+template <int DT>
+static int launch_prep_t(int Kc, int d, const double* cov, double* Linv, double* hdet, cudaStream_t st) {
+  const size_t smem = sizeof(double) * 2 * (size_t)d * pitch(d);
+  AB_CUDA(cudaFuncSetAttribute(gmm_prep_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  gmm_prep_kernel<DT><<<Kc, GMM_THREADS, smem, st>>>(d, cov, Linv, hdet);
   AB_LAUNCH_CHECK("gmm_prep_kernel");
   return AB_OK;
+}
+
+int launch_gmm_prep(int Kc, int d, const double* cov, double* Linv, double* hdet, cudaStream_t st) {
+#define AB_CALL(DT) launch_prep_t<DT>(Kc, d, cov, Linv, hdet, st)
+  return AB_GMM_BY_D(d, AB_CALL);
+#undef AB_CALL
 }
 
 size_t gmm_stats_scratch(int d, int K) {
@@ -1101,14 +1213,23 @@ int launch_gmm_stats(int N, int d, int K, const float* Y, const int* z, const do
   return AB_OK;
 }
 
+template <int DT>
+static int launch_conj_mu_t(int K, int d, int shared, const double* mu0, const double* cov0, const int* cnt,
+                            const double* sum, const double* cov, double* mu, uint64_t seed, uint32_t iter,
+                            uint32_t comp, cudaStream_t st) {
+  const size_t smem = sizeof(double) * (4 * (size_t)d * pitch(d) + 6 * (size_t)d);
+  AB_CUDA(cudaFuncSetAttribute(gmm_conj_mu_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  gmm_conj_mu_kernel<DT><<<K, GMM_THREADS, smem, st>>>(d, shared, mu0, cov0, cnt, sum, cov, mu, seed, iter, comp);
+  AB_LAUNCH_CHECK("gmm_conj_mu_kernel");
+  return AB_OK;
+}
+
 int launch_gmm_conj_mu(int K, int d, int shared, const double* mu0, const double* cov0, const int* cnt,
                        const double* sum, const double* cov, double* mu, uint64_t seed, uint32_t iter,
                        uint32_t comp, cudaStream_t st) {
-  const size_t smem = sizeof(double) * (4 * (size_t)d * d + 6 * (size_t)d);
-  AB_CUDA(cudaFuncSetAttribute(gmm_conj_mu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gmm_conj_mu_kernel<<<K, 64, smem, st>>>(d, shared, mu0, cov0, cnt, sum, cov, mu, seed, iter, comp);
-  AB_LAUNCH_CHECK("gmm_conj_mu_kernel");
-  return AB_OK;
+#define AB_CALL(DT) launch_conj_mu_t<DT>(K, d, shared, mu0, cov0, cnt, sum, cov, mu, seed, iter, comp, st)
+  return AB_GMM_BY_D(d, AB_CALL);
+#undef AB_CALL
 }
 
 // The Bartlett chi-square sums into chi (chi == nullptr: cov's diagonal).
@@ -1122,20 +1243,27 @@ int launch_gmm_bartlett(int K, int d, int df, const int* cnt, double* chi, doubl
   return AB_OK;
 }
 
+template <int DT>
+static int launch_conj_cov_t(int K, int d, int df, const double* scale0, const int* cnt, const double* obs,
+                             const double* chi, int sk, int si, double* cov, uint64_t seed, uint32_t iter,
+                             uint32_t comp, cudaStream_t st) {
+  const size_t smem = sizeof(double) * 4 * (size_t)d * pitch(d);
+  AB_CUDA(cudaFuncSetAttribute(gmm_conj_cov_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  gmm_conj_cov_kernel<DT><<<K, GMM_THREADS, smem, st>>>(d, df, scale0, cnt, obs, chi, sk, si, cov, seed, iter, comp);
+  AB_LAUNCH_CHECK("gmm_conj_cov_kernel");
+  return AB_OK;
+}
+
 // The inverse-Wishart draw from the chi-square sums in chi (chi == nullptr:
 // cov's diagonal).
 int launch_gmm_conj_cov_from(int K, int d, int df, const double* scale0, const int* cnt, const double* obs,
                              const double* chi, double* cov, uint64_t seed, uint32_t iter, uint32_t comp,
                              cudaStream_t st) {
-  const size_t smem = sizeof(double) * 4 * (size_t)d * d;
-  AB_CUDA(cudaFuncSetAttribute(gmm_conj_cov_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (chi != nullptr)
-    gmm_conj_cov_kernel<<<K, GMM_THREADS, smem, st>>>(d, df, scale0, cnt, obs, chi, d, 1, cov, seed, iter, comp);
-  else
-    gmm_conj_cov_kernel<<<K, GMM_THREADS, smem, st>>>(d, df, scale0, cnt, obs, cov, d * d, d + 1, cov, seed, iter,
-                                                      comp);
-  AB_LAUNCH_CHECK("gmm_conj_cov_kernel");
-  return AB_OK;
+  const int sk = chi != nullptr ? d : d * d, si = chi != nullptr ? 1 : d + 1;
+  if (chi == nullptr) chi = cov;
+#define AB_CALL(DT) launch_conj_cov_t<DT>(K, d, df, scale0, cnt, obs, chi, sk, si, cov, seed, iter, comp, st)
+  return AB_GMM_BY_D(d, AB_CALL);
+#undef AB_CALL
 }
 
 int launch_gmm_conj_cov(int K, int d, int df, const double* scale0, const int* cnt, const double* obs,

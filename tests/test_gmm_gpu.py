@@ -90,6 +90,47 @@ def test_conj_cov_in_two_calls_equals_one(K, d):
     assert torch.isfinite(one).all()
 
 
+@pytest.mark.parametrize("d", [1, 2, 15, 16, 17, 31, 32, 33, 62, 64])
+def test_factorisations_at_the_edges_of_the_dimension_ranges(orc, d):
+    """Component tables and conjugate draws at the smallest and largest d and
+    around the d (16, 32) at which the kernels change, counts of zero and one
+    among them; tables also where the pivots leave the range of the short
+    reciprocal root (covariances scaled by 2^-930 and 2^930)."""
+    K = 3
+    rng = np.random.default_rng(d)
+    A = rng.standard_normal((K, d, d + 3))
+    covs = np.einsum("kij,klj->kil", A, A) / (d + 3) + 0.1 * np.eye(d)
+    L = N.lib()
+    st = N.stream_ptr()
+    for scale in (1.0, 2.0 ** -930, 2.0 ** 930):
+        cov_t = torch.as_tensor(covs * scale).cuda()
+        Linv = torch.full((K, d, d), float("nan"), dtype=torch.float64, device="cuda")
+        hdet = torch.zeros(K, dtype=torch.float64, device="cuda")
+        N.check(L.ab_gmm_prep(K, d, N.ptr(cov_t), N.ptr(Linv), N.ptr(hdet), st), "prep")
+        ref = np.linalg.inv(np.linalg.cholesky(covs)) / np.sqrt(scale)
+        got = Linv.cpu().numpy()
+        assert np.all(got[:, np.triu_indices(d, 1)[0], np.triu_indices(d, 1)[1]] == 0.0)
+        np.testing.assert_allclose(got, ref, rtol=1e-9, atol=1e-9 * np.abs(ref).max())
+        if scale == 1.0:
+            np.testing.assert_allclose(hdet.cpu().numpy(), 0.5 * np.linalg.slogdet(covs)[1], rtol=1e-9, atol=1e-9)
+    cnt = np.array([0, 1, 900], np.int32)
+    s = rng.standard_normal((K, d)) * cnt[:, None]
+    obs = covs * cnt[:, None, None]
+    om = O.GmmModel(rng.standard_normal((4, d)), K, np.zeros(d), 25 * np.eye(d), False, alpha=np.ones(K), df=d + 2,
+                    scale0=np.eye(d))
+    dev = lambda a: torch.as_tensor(np.ascontiguousarray(a)).cuda()
+    cnt_t, s_t, obs_t, cov_t = dev(cnt), dev(s), dev(obs), dev(covs)
+    mu0, cov0, scale0 = dev(np.zeros(d)), dev(25 * np.eye(d)), dev(np.eye(d))
+    mu = torch.zeros((K, d), dtype=torch.float64, device="cuda")
+    cov = torch.zeros((K, d, d), dtype=torch.float64, device="cuda")
+    N.check(L.ab_gmm_conj_mu(K, d, 0, N.ptr(mu0), N.ptr(cov0), N.ptr(cnt_t), N.ptr(s_t), N.ptr(cov_t), N.ptr(mu), 9, 2, 0,
+                             st), "mu")
+    np.testing.assert_allclose(mu.cpu().numpy(), O.gmm_conj_mu(orc, om, cnt, s, covs, 9, 2), rtol=1e-9, atol=1e-9)
+    N.check(L.ab_gmm_conj_cov(K, d, d + 2, N.ptr(scale0), N.ptr(cnt_t), N.ptr(obs_t), N.ptr(cov), 9, 2, 0, st), "cov")
+    want = O.gmm_conj_cov(orc, om, cnt, obs, 9, 2)
+    np.testing.assert_allclose(cov.cpu().numpy(), want, rtol=1e-9, atol=1e-9 * np.abs(want).max())
+
+
 @pytest.mark.parametrize("N_,K,d", [(300_000, 16, 32), (250_000, 3, 40), (1, 2, 3), (900, 16, 2)])
 def test_stats_sizes(orc, N_, K, d):
     """Statistics at sizes where a CTA's chunk spans several shared-memory
