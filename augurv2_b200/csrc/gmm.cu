@@ -17,6 +17,8 @@
 // are produced changes.  The per-point log-density uses the Cholesky inverse
 // of the component covariance computed once per sweep — the same binary64
 // values the reference recomputes for every (point, component).
+#include <algorithm>
+
 #include "common.cuh"
 #include "dist.cuh"
 
@@ -25,7 +27,6 @@ namespace ab {
 constexpr int GMM_MAX_D = 64;
 constexpr int GMM_MAX_K = 64;
 constexpr int GMM_THREADS = 256;
-constexpr int GMM_STAT_CTAS = 296;
 
 // d <= GMM_MAX_D, so a shared-memory matrix index fits 32 bits
 #define GM(A, i, j) (A)[(i) * d + (j)]
@@ -340,7 +341,7 @@ gmm_z_kernel(int N, int d, int K, int shared_cov, const float* __restrict__ Y, c
 //   gmm_zs_prep_kernel  per component (once per call): the lower triangle of
 //                       Linv_k and mu_k rounded to binary32, and the constants
 //                       of the error bound below; log(pis_k) + c - hdet_k;
-//   gmm_zs_kernel       one thread per point: t_k = log p_k in binary32 with a
+//   gmm_zs_kernel       two points a thread: t_k = log p_k in binary32 with a
 //                       rigorous bound eps_k on its error against the exact
 //                       value, p_k / p_max = exp(t_k - t_max), the running
 //                       sums, and the reference's draw when u lies outside the
@@ -350,13 +351,15 @@ gmm_z_kernel(int N, int d, int K, int shared_cov, const float* __restrict__ Y, c
 //                       rows of Linv w on the lanes, every sum in its order),
 //                       so every draw equals gmm_z_kernel's bit for bit.
 // Error bound (u = 2^-24; all quantities of component k; L~, w~ the binary32
-// values, w~_j = fl32(y_j - mu_j) with the difference formed in binary64):
-//   |w~_j - w_j| <= u |w~_j| (1 + 2^-28);
-//   row i of Linv w (i + 1 products, fused multiply-adds; zero padding adds
-//   exact zeros): |s~_i - s_i| <= delta_i = u (1 + 4u) (i + 3) A_i,
-//     A_i = sum_j |L~_ij||w~_j| <= R_i W (R_i >= ||L~_i||, W >= ||w~||);
+// values; mu_j = mh_j + ml_j + r_j, two binary32 parts, |r_j| <= 2^-48 |mu_j|;
+// w~_j = fl(fl(y_j - mh_j) - ml_j)):
+//   |w~_j - w_j| <= 2u |w~_j| (1 + 4u) + 2^-47 |mu_j| (1 + 4u);
+//   row i of Linv w (i + 1 products, fused multiply-adds in two interleaved
+//   chains, then their sum; zero padding adds exact zeros): |s~_i - s_i| <=
+//   delta_i = u (1 + 4u) (i + 4) A_i, A_i = sum_j |L~_ij| (|w~_j| + 2^-23 |mu_j|)
+//     <= R_i W (R_i >= ||L~_i||, W >= ||w~|| + 2^-23 ||mu||);
 //   expon = sum_i s_i^2: |e~ - e| <= (d + 1) u e~ + sum_i (2 |s~_i| delta_i + delta_i^2),
-//     with sum_i |s~_i| a_i (a_i = (i + 3) R_i) accumulated beside the rows
+//     with sum_i |s~_i| a_i (a_i = (i + 4) R_i) accumulated beside the rows
 //     and sum_i delta_i^2 <= u^2 (1 + 4u)^2 W^2 S_aa, S_aa = sum_i a_i^2;
 //   t_k = fl(lpc_k - e~ / 2), lpc_k = fl32(log pis_k + c - hdet_k): |t_k - log p_k|
 //     <= eps_k = E_k / 2 + u (|lpc_k| + |t_k|) + 2^-40 (|lpc_k| + e~ + 1) (the last
@@ -378,26 +381,35 @@ constexpr int GMM_ZS_MAXK = 32;
 constexpr int GMM_ZS_THREADS = 128;
 
 // Per component, floats: L~ with row i padded to whole float4s (zeros) at
-// gmm_zs_row(i), a [d], then lpc, S_aa; the stride is whole float4s.
+// gmm_zs_row(i), then a, mh and ml, each padded to whole float4s (zeros), then
+// lpc, S_aa and 2^-23 ||mu|| (rounded up); the stride is whole float4s.
 __host__ __device__ constexpr int gmm_zs_row(int i) { return 4 * (i / 4 + 1) * (2 * (i / 4) + i % 4); }
-__host__ __device__ inline int gmm_zs_stride(int d) { return (gmm_zs_row(d) + d + 2 + 3) / 4 * 4; }
+__host__ __device__ constexpr int gmm_zs_dq(int d) { return (d + 3) / 4 * 4; }
+__host__ __device__ inline int gmm_zs_stride(int d) { return gmm_zs_row(d - 1) + gmm_zs_dq(d) + 3 * gmm_zs_dq(d) + 4; }
 
-// tab: K float tables of gmm_zs_stride(d), then the means, binary64 [K][d].
+// tab: K float tables of gmm_zs_stride(d).
 __global__ void __launch_bounds__(64) gmm_zs_prep_kernel(int d, int K, int shared_cov, const double* __restrict__ pis,
                                                          const double* __restrict__ mu,
                                                          const double* __restrict__ Linv,
                                                          const double* __restrict__ hdet, float* __restrict__ tab,
                                                          int* __restrict__ flag) {
-  __shared__ double red[1][64];
+  __shared__ double red[2][64];
   const int k = blockIdx.x, kc = shared_cov ? 0 : k;
   const double* Lk = Linv + (size_t)kc * d * d;
   const double* mk = mu + (size_t)k * d;
   float* t = tab + (size_t)k * gmm_zs_stride(d);
-  const int T = gmm_zs_row(d);
+  const int dq = gmm_zs_dq(d);
   float* L32 = t;
-  float* a = t + T;
-  float* sc = a + d;
-  for (int i = threadIdx.x; i < d; i += blockDim.x) {
+  float* a = t + gmm_zs_row(d - 1) + dq;
+  float* mh = a + dq;
+  float* ml = mh + dq;
+  float* sc = ml + dq;
+  double saa = 0.0, mm = 0.0;
+  for (int i = threadIdx.x; i < dq; i += blockDim.x) {
+    if (i >= d) {
+      a[i] = mh[i] = ml[i] = 0.0f;
+      continue;
+    }
     double r2 = 0.0;
     const int row = gmm_zs_row(i), len = (i / 4 + 1) * 4;
     for (int j = 0; j < len; ++j) {
@@ -406,149 +418,295 @@ __global__ void __launch_bounds__(64) gmm_zs_prep_kernel(int d, int K, int share
       r2 += (double)l * (double)l;
     }
     // rounded up, with a relative slack for the binary64 sums' own rounding
-    a[i] = __fmul_ru((float)(i + 3), __double2float_ru(sqrt(r2) * (1.0 + 1e-12)));
-    reinterpret_cast<double*>(tab + (size_t)K * gmm_zs_stride(d))[(size_t)k * d + i] = mk[i];
+    a[i] = __fmul_ru((float)(i + 4), __double2float_ru(sqrt(r2) * (1.0 + 1e-12)));
+    saa += (double)a[i] * a[i];
+    const double m = mk[i];
+    const float h = __double2float_rn(m);
+    mh[i] = -h;                                             // stored negated: w = (y + mh) + ml
+    ml[i] = -__double2float_rn(__dadd_rn(m, -(double)h));
+    mm += m * m;
   }
-  __syncthreads();
-  double saa = 0.0;
-  for (int i = threadIdx.x; i < d; i += blockDim.x) saa += (double)a[i] * a[i];
   red[0][threadIdx.x] = saa;
+  red[1][threadIdx.x] = mm;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int i = 1; i < (int)blockDim.x; ++i) saa += red[0][i];
+    for (int i = 1; i < (int)blockDim.x; ++i) {
+      saa += red[0][i];
+      mm += red[1][i];
+    }
     const double c = -0.5 * (double)d * log(2.0 * 3.14159265358979323846264338327950288);
     const double llc = c - hdet[kc];
     const double pk = pis[k];
     sc[0] = pk > 0.0 ? __double2float_rn(log(pk) + llc) : -INFINITY;
     sc[1] = __double2float_ru(saa * (1.0 + 1e-12));
+    sc[2] = __double2float_ru(sqrt(mm) * (0x1p-23 * (1.0 + 0x1p-16)));
+    sc[3] = 0.0f;
     if (!(pk >= 0.0) || !(llc <= 700.0) || !isfinite(llc)) atomicExch(flag, 1);
   }
 }
 
+// Two binary32 operations per instruction, each rounded as the scalar one.
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  return (unsigned long long)__float_as_uint(y) << 32 | __float_as_uint(x);
+}
+__device__ __forceinline__ float lo2(unsigned long long a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float hi2(unsigned long long a) { return __uint_as_float((unsigned)(a >> 32)); }
+
+// A thread takes two points at a time, so that every 16-byte read of the
+// factor's rows (a shared-memory broadcast) feeds eight multiply-adds, and
+// pairs of a row's columns go through one packed multiply-add: 338 -> 210 us
+// for N = 200,000, K = 16, d = 32, where one point a thread with scalar
+// operations waited for the factor reads and for the conversions of a
+// binary64 y - mu.  Warps walk the points 64 at a time over a grid of three
+// CTAs per SM, each of which reads the tables once.
 template <int DT>
-__global__ void __launch_bounds__(GMM_ZS_THREADS, 5)   // 5 CTAs of 43 KB per SM
-gmm_zs_kernel(int N, int d, int K, const float* __restrict__ Y, const double* __restrict__ mu,
-              const float* __restrict__ tab,
-              const int* __restrict__ flag, int* __restrict__ queue, int* __restrict__ qn, int* __restrict__ z,
+__global__ void __launch_bounds__(GMM_ZS_THREADS, 3)
+gmm_zs_kernel(int N, int d, int K, int vec, const float* __restrict__ Y, const float* __restrict__ tab,
+              const int* __restrict__ perm, const int* __restrict__ flag, int* __restrict__ queue, int* __restrict__ qn, int* __restrict__ z,
               uint64_t seed, uint32_t iter, uint32_t comp) {
-  extern __shared__ float ts[];   // the K components' tables, then the binary64 means
-  const int stride = gmm_zs_stride(d);
+  extern __shared__ __align__(16) float ts[];   // the K components' tables
+  constexpr int DW = (DT + 3) / 4 * 4;          // whole float4s of row entries
+  const int stride = gmm_zs_stride(d), dq = gmm_zs_dq(d);
   {
-    // K * stride is whole float4s, the means 2 K d floats
     const float4* src = reinterpret_cast<const float4*>(tab);
     float4* dst = reinterpret_cast<float4*>(ts);
-    const int nf = K * stride + 2 * K * d, n4 = nf / 4;
-    for (int e = threadIdx.x; e < n4; e += blockDim.x) dst[e] = src[e];
-    for (int e = 4 * n4 + threadIdx.x; e < nf; e += blockDim.x) ts[e] = tab[e];
+    for (int e = threadIdx.x; e < K * stride / 4; e += GMM_ZS_THREADS) dst[e] = src[e];
   }
   __syncthreads();
-  const double* mus = reinterpret_cast<const double*>(ts + (size_t)K * stride);
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
   const float u32 = 5.9604644775390625e-8f;   // 2^-24
-  bool exact = *flag != 0;
-  float tk[GMM_ZS_MAXK], ek[GMM_ZS_MAXK];
-  float tmax = -INFINITY;
-  if (!exact) {
-    float y[DT];
+  const bool all_exact = *flag != 0;
+  const int lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (GMM_ZS_THREADS / 32);
+  for (int tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; tile < (N + 63) / 64; tile += warps) {
+    int n2[2];
 #pragma unroll
-    for (int j = 0; j < DT; ++j) y[j] = j < d ? Y[(size_t)n * d + j] : 0.0f;
-    const int T = gmm_zs_row(d);
-    for (int k = 0; k < K; ++k) {
-      const float* L32 = ts + k * stride;
-      const float* a = L32 + T;
-      const double* mk = mus + (size_t)k * d;
-      const float* sc = a + d;
-      const float lpc = sc[0];
-      if (lpc == -INFINITY) {   // weight 0: the term is exactly 0 here and in the reference
-        tk[k] = -INFINITY;
-        ek[k] = 0.0f;
-        continue;
-      }
-      constexpr int DW = (DT + 3) / 4 * 4;   // whole float4s of row entries
-      float w[DW];
-      float W2 = 0.0f;
+    for (int h = 0; h < 2; ++h) {
+      const int i = tile * 64 + lane + 32 * h;
+      n2[h] = i < N ? (perm ? perm[i] : i) : -1;
+    }
+    bool exact[2] = {all_exact, all_exact};
+    float tk[2][GMM_ZS_MAXK], ek[2][GMM_ZS_MAXK];
+    float tmax[2] = {-INFINITY, -INFINITY};
+    if (!all_exact) {
+      unsigned long long y[2][DW / 2];
 #pragma unroll
-      for (int j = 0; j < DW; ++j) {
-        w[j] = (j < DT && j < d) ? __double2float_rn(__dadd_rn((double)y[j < DT ? j : 0], -mk[j])) : 0.0f;
-        W2 = __fmaf_rn(w[j], w[j], W2);
-      }
-      float e = 0.0f, t1 = 0.0f;
+      for (int h = 0; h < 2; ++h) {
+        const float* yr = Y + (size_t)max(n2[h], 0) * d;
+        if (vec) {   // d a multiple of 4, rows 16-byte aligned
 #pragma unroll
-      for (int i = 0; i < DT; ++i) {
-        if (i < d) {
-          // row i in float4s; its padding is zero (exact zero products)
-          const float4* Li = reinterpret_cast<const float4*>(L32 + gmm_zs_row(i));
-          float s = 0.0f;
-#pragma unroll
-          for (int q = 0; q <= i / 4; ++q) {
-            const float4 l = Li[q];
-            s = __fmaf_rn(l.x, w[4 * q], s);
-            s = __fmaf_rn(l.y, w[4 * q + 1], s);
-            s = __fmaf_rn(l.z, w[4 * q + 2], s);
-            s = __fmaf_rn(l.w, w[4 * q + 3], s);
+          for (int q = 0; q < DW / 4; ++q) {
+            const float4 f = 4 * q < d ? reinterpret_cast<const float4*>(yr)[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+            y[h][2 * q] = pack2(f.x, f.y);
+            y[h][2 * q + 1] = pack2(f.z, f.w);
           }
-          e = __fmaf_rn(s, s, e);
-          t1 = __fmaf_rn(fabsf(s), a[i], t1);
+        } else {
+#pragma unroll
+          for (int q = 0; q < DW / 2; ++q)
+            y[h][q] = pack2(2 * q < d ? yr[2 * q] : 0.0f, 2 * q + 1 < d ? yr[2 * q + 1] : 0.0f);
         }
       }
-      // W >= ||w~|| (the sum of squares' rounding and the root's covered)
-      const float W = __fsqrt_ru(__fmul_ru(W2, 1.0f + (float)(DT + 2) * u32));
-      const float sd2 = __fmul_ru(__fmul_ru(W, W), sc[1]);
-      const float E = __fmul_ru(__fadd_ru(__fadd_ru(__fmul_ru((float)(d + 1) * u32, e),
-                                                    __fmul_ru(2.0f * u32, __fmul_ru(W, t1))),
-                                          __fmul_ru(u32 * u32 * 1.01f, sd2)),
-                                1.0f + 0x1p-16f);
-      const float t = __fmaf_rn(-0.5f, e, lpc);
-      const float eps = __fadd_ru(__fadd_ru(__fmul_ru(0.5f, E), __fmul_ru(u32, fabsf(lpc) + fabsf(t))),
-                                  __fmul_ru(0x1p-40f, fabsf(lpc) + e + 1.0f));
-      tk[k] = t;
-      ek[k] = eps;
-      if (!(t < INFINITY) || !(eps < INFINITY)) exact = true;   // non-finite
-      tmax = fmaxf(tmax, t);
-    }
-    if (!(tmax >= -690.0f && tmax <= 690.0f)) exact = true;
-  }
-  int zk = -1;
-  if (!exact) {
-    // p~_k and an absolute bound A_k on |p~_k - p_k / p_max| (the exact value
-    // lies in [exp(dt - x), exp(dt + x)], x = eps_k + u |dt| + 4u, binary32
-    // exp within 4u); far components, whose bands are wide, weigh their width
-    // by their tiny size
-    float C[GMM_ZS_MAXK];
-    float acc = 0.0f, err = 0.0f;
-    for (int k = 0; k < K; ++k) {
-      float p = 0.0f;
-      if (tk[k] != -INFINITY) {
-        const float dt = __fsub_rn(tk[k], tmax);
-        p = expf(dt);
-        const float x = __fadd_ru(__fadd_ru(ek[k], __fmul_ru(u32, fabsf(dt))), 4.0f * u32);
-        const float up = __fmul_ru(expf(__fadd_ru(dt, x)), 1.0f + 8.0f * u32);
-        const float dn = __fmul_rd(expf(__fsub_rd(dt, x)), 1.0f - 8.0f * u32);
-        err = __fadd_ru(err, fmaxf(__fsub_ru(up, p), __fsub_ru(p, dn)));
+      // In label order the tile's points have few labels between them, mostly
+      // their draws too: those components first, then - where a point does not
+      // look like any of them - the component its first coordinates suggest,
+      // so that the other components can be found far away early.
+      float low[2] = {-INFINITY, -INFINITY};   // a lower bound of log p_max so far
+      bool likely[2] = {n2[0] < 0, n2[1] < 0};
+      unsigned todo = K == 32 ? 0xffffffffu : (1u << K) - 1u, pend = todo;
+      bool suggest = perm != nullptr;
+      if (perm) {
+        unsigned m = 0u;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int l = n2[h] >= 0 ? z[n2[h]] : -1;
+          m |= l >= 0 && l < K ? 1u << l : 0u;
+        }
+        pend = __reduce_or_sync(0xffffffffu, m);
       }
-      acc = __fadd_rn(acc, p);
-      C[k] = acc;
+      while (todo) {
+        if (pend == 0u && suggest) {
+          suggest = false;
+          if (__any_sync(0xffffffffu, !likely[0] || !likely[1])) {
+            float best[2] = {-INFINITY, -INFINITY};
+            int at[2] = {0, 0};
+            for (int k = 0; k < K; ++k) {
+              const float* L32 = ts + k * stride;
+              const float* a = L32 + gmm_zs_row(d - 1) + dq;
+              const ulonglong2 mh = *reinterpret_cast<const ulonglong2*>(a + dq);
+              const float lpc = a[3 * dq];
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const unsigned long long w0 = add2(y[h][0], mh.x), w1 = DW > 2 ? add2(y[h][1], mh.y) : 0ull;
+                float e = 0.0f;
+#pragma unroll
+                for (int i = 0; i < (DT < 4 ? DT : 4); ++i) {
+                  const ulonglong2 l = *reinterpret_cast<const ulonglong2*>(L32 + gmm_zs_row(i));
+                  const unsigned long long sr = fma2(l.y, w1, fma2(l.x, w0, 0ull));
+                  const float r = lo2(sr) + hi2(sr);
+                  e += r * r;
+                }
+                if (lpc - 0.5f * e > best[h]) {
+                  best[h] = lpc - 0.5f * e;
+                  at[h] = k;
+                }
+              }
+            }
+            pend = __reduce_or_sync(0xffffffffu, (likely[0] ? 0u : 1u << at[0]) | (likely[1] ? 0u : 1u << at[1])) & todo;
+          }
+        }
+        if (pend == 0u) pend = todo;
+        const int k = __ffs(pend) - 1;
+        pend &= pend - 1u;
+        todo &= ~(1u << k);
+        const float* L32 = ts + k * stride;
+        const float* a = L32 + gmm_zs_row(d - 1) + dq;
+        const float4 sc = *reinterpret_cast<const float4*>(a + 3 * dq);
+        const float lpc = sc.x;
+        if (lpc == -INFINITY) {   // weight 0: the term is exactly 0 here and in the reference
+          tk[0][k] = tk[1][k] = -INFINITY;
+          ek[0][k] = ek[1][k] = 0.0f;
+          continue;
+        }
+        unsigned long long w[2][DW / 2], W2[2] = {0ull, 0ull};
+        float e[2] = {0.0f, 0.0f}, t1[2] = {0.0f, 0.0f};
+        float4 a4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        bool far = false;
+#pragma unroll
+        for (int i = 0; i < DT; ++i) {
+          if (i < d && !far) {
+            if (i % 4 == 0) {
+              // the next four coordinates of w, and of a
+              const ulonglong2 mh = reinterpret_cast<const ulonglong2*>(a + dq)[i / 4];
+              const ulonglong2 ml = reinterpret_cast<const ulonglong2*>(a + 2 * dq)[i / 4];
+              a4 = reinterpret_cast<const float4*>(a)[i / 4];
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                w[h][i / 2] = add2(add2(y[h][i / 2], mh.x), ml.x);
+                w[h][i / 2 + 1] = add2(add2(y[h][i / 2 + 1], mh.y), ml.y);
+                W2[h] = fma2(w[h][i / 2], w[h][i / 2], W2[h]);
+                W2[h] = fma2(w[h][i / 2 + 1], w[h][i / 2 + 1], W2[h]);
+              }
+            }
+            // row i in float4s; its padding is zero (exact zero products)
+            const ulonglong2* Li = reinterpret_cast<const ulonglong2*>(L32 + gmm_zs_row(i));
+            unsigned long long s0 = 0ull, s1 = 0ull;
+#pragma unroll
+            for (int q = 0; q <= i / 4; ++q) {
+              const ulonglong2 l = Li[q];
+              s0 = fma2(l.x, w[0][2 * q], s0);
+              s1 = fma2(l.x, w[1][2 * q], s1);
+              s0 = fma2(l.y, w[0][2 * q + 1], s0);
+              s1 = fma2(l.y, w[1][2 * q + 1], s1);
+            }
+            const float r0 = __fadd_rn(lo2(s0), hi2(s0)), r1 = __fadd_rn(lo2(s1), hi2(s1));
+            const float ai = i % 4 == 0 ? a4.x : i % 4 == 1 ? a4.y : i % 4 == 2 ? a4.z : a4.w;
+            e[0] = __fmaf_rn(r0, r0, e[0]);
+            e[1] = __fmaf_rn(r1, r1, e[1]);
+            t1[0] = __fmaf_rn(fabsf(r0), ai, t1[0]);
+            t1[1] = __fmaf_rn(fabsf(r1), ai, t1[1]);
+            // After 4, 8 and 16 rows: log p_k <= lpc - (1 - 2^-9) e~ / 2 + 1 (e's
+            // remaining terms are nonnegative, its error far below 2^-9 e~ + 1
+            // while |lpc| < 2^20 and the bound on e~'s error is below 1), so
+            // a component 41 below the largest so far for all of the warp's
+            // points adds less than 2^-59 of p_max to the sums - all of them
+            // far less than the band's own rounding slack of 2^-38 - and its
+            // remaining rows are left out.
+            if ((i == 3 || i == 7 || i == 15) && perm) {
+              bool f = true;
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const float W = __fadd_ru(__fsqrt_ru(2.0f * __fadd_ru(lo2(W2[h]), hi2(W2[h]))), sc.z);
+                const float err = __fmul_ru(4.0f * u32, __fmul_ru(W, t1[h]));
+                f = f && err < 0.25f + 0x1p-11f * e[h] && fabsf(lpc) < 0x1p20f &&
+                    lpc - 0.4990234375f * e[h] < low[h] - 42.0f;
+              }
+              far = __all_sync(0xffffffffu, f);
+            }
+          }
+        }
+        if (far) {
+          tk[0][k] = tk[1][k] = -INFINITY;
+          ek[0][k] = ek[1][k] = 0.0f;
+          continue;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          // W >= ||w~|| + 2^-23 ||mu|| (the sum of squares' rounding and the root's covered)
+          const float ww = __fadd_ru(lo2(W2[h]), hi2(W2[h]));
+          const float W = __fadd_ru(__fsqrt_ru(__fmul_ru(ww, 1.0f + (float)(DT + 2) * u32)), sc.z);
+          const float sd2 = __fmul_ru(__fmul_ru(W, W), sc.y);
+          const float E = __fmul_ru(__fadd_ru(__fadd_ru(__fmul_ru((float)(d + 1) * u32, e[h]),
+                                                        __fmul_ru(2.0f * u32, __fmul_ru(W, t1[h]))),
+                                              __fmul_ru(u32 * u32 * 1.01f, sd2)),
+                                    1.0f + 0x1p-16f);
+          const float t = __fmaf_rn(-0.5f, e[h], lpc);
+          const float eps = __fadd_ru(__fadd_ru(__fmul_ru(0.5f, E), __fmul_ru(u32, fabsf(lpc) + fabsf(t))),
+                                      __fmul_ru(0x1p-40f, fabsf(lpc) + e[h] + 1.0f));
+          tk[h][k] = t;
+          ek[h][k] = eps;
+          if (!(t < INFINITY) || !(eps < INFINITY)) exact[h] = true;   // non-finite
+          tmax[h] = fmaxf(tmax[h], t);
+          low[h] = fmaxf(low[h], __fsub_rd(t, eps));
+          likely[h] = likely[h] || e[h] < (float)(3 * d + 30);
+        }
+      }
     }
-    // band: the terms' errors, the running sums' and u * norm's roundings,
-    // the comparisons' own roundings, the reference's running quotient sums
-    const float Nt = C[K - 1];
-    const float band = __fmul_ru(__fadd_ru(__fadd_ru(err, __fmul_ru((float)(K + 6) * u32, Nt)),
-                                           __fmul_ru(0x1p-40f, Nt)), 1.0f + 0x1p-16f);
-    Stream s = make_stream(seed, (uint32_t)n, iter, TAG_Z | (comp << 8));
-    const double u = s.uniform();
-    const float un = __fmul_rn(__double2float_rn(u), Nt);
-    int i = 0;
-    while (i < K - 1 && !(un < C[i])) ++i;
-    const bool above_prev = i == 0 || __fadd_ru(C[i - 1], band) < __fsub_rd(un, band);
-    const bool below_this = i == K - 1 || __fadd_ru(un, band) < __fsub_rd(C[i], band);
-    if (above_prev && below_this && Nt >= 1.0f && band < INFINITY) zk = i;
-  }
-  if (zk >= 0) {
-    z[n] = zk;
-  } else {
-    const int slot = atomicAdd(qn, 1);
-    queue[slot] = n;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int n = n2[h];
+      if (n < 0) continue;
+      if (!(tmax[h] >= -690.0f && tmax[h] <= 690.0f)) exact[h] = true;
+      int zk = -1;
+      if (!exact[h]) {
+        // p~_k and an absolute bound A_k on |p~_k - p_k / p_max| (the exact value
+        // lies in [exp(dt - x), exp(dt + x)], x = eps_k + u |dt| + 4u, binary32
+        // exp within 4u); far components, whose bands are wide, weigh their width
+        // by their tiny size
+        float C[GMM_ZS_MAXK];
+        float acc = 0.0f, err = 0.0f;
+        for (int k = 0; k < K; ++k) {
+          float p = 0.0f;
+          if (tk[h][k] != -INFINITY) {
+            const float dt = __fsub_rn(tk[h][k], tmax[h]);
+            p = expf(dt);
+            const float x = __fadd_ru(__fadd_ru(ek[h][k], __fmul_ru(u32, fabsf(dt))), 4.0f * u32);
+            const float up = __fmul_ru(expf(__fadd_ru(dt, x)), 1.0f + 8.0f * u32);
+            const float dn = __fmul_rd(expf(__fsub_rd(dt, x)), 1.0f - 8.0f * u32);
+            err = __fadd_ru(err, fmaxf(__fsub_ru(up, p), __fsub_ru(p, dn)));
+          }
+          acc = __fadd_rn(acc, p);
+          C[k] = acc;
+        }
+        // band: the terms' errors, the running sums' and u * norm's roundings,
+        // the comparisons' own roundings, the reference's running quotient sums
+        const float Nt = C[K - 1];
+        const float band = __fmul_ru(__fadd_ru(__fadd_ru(err, __fmul_ru((float)(K + 6) * u32, Nt)),
+                                               __fmul_ru(0x1p-40f, Nt)), 1.0f + 0x1p-16f);
+        Stream s = make_stream(seed, (uint32_t)n, iter, TAG_Z | (comp << 8));
+        const double u = s.uniform();
+        const float un = __fmul_rn(__double2float_rn(u), Nt);
+        int i = 0;
+        while (i < K - 1 && !(un < C[i])) ++i;
+        const bool above_prev = i == 0 || __fadd_ru(C[i - 1], band) < __fsub_rd(un, band);
+        const bool below_this = i == K - 1 || __fadd_ru(un, band) < __fsub_rd(C[i], band);
+        if (above_prev && below_this && Nt >= 1.0f && band < INFINITY) zk = i;
+      }
+      if (zk >= 0) {
+        z[n] = zk;
+      } else {
+        const int slot = atomicAdd(qn, 1);
+        queue[slot] = n;
+      }
+    }
   }
 }
 
@@ -609,170 +767,323 @@ gmm_zx_kernel(int d, int K, int shared_cov, const float* __restrict__ Y, const d
 }
 
 // ---- conjugate statistics ----------------------------------------------------
-// CTA b accumulates points [b*chunk, (b+1)*chunk): counts, sum of y
-// (want_sum) and the lower triangle of sum (y - mu_z)(y - mu_z)^T
-// (want_obs; the reference's full-matrix update augur_mat_atm_inc_vtmt is
-// symmetric elementwise).  The chunk is taken in sub-chunks of at most
-// `sub` points: a sub-chunk's rows of Y are read with coalesced loads (all
-// in flight at once) into shared memory, as binary32 rows when the sums are
-// wanted and, for the scatter, centred once per point in binary64
-// (c_i = y_i - mu_z,i, the value every scatter entry of the point uses);
-// the points are sorted by component with a stable counting sort (warp 0,
-// match_any ranks), and the components are walked one at a time: each
-// thread owns fixed table entries and accumulates them in registers over
-// the component's points in point order (a count is the component's number
-// of points, the same double as adding 1.0 per point), adding the
-// sub-chunk's sum to its partial.  Partials go to scratch [CTA][K][W] and
-// gmm_stats_reduce_kernel adds them in CTA order (deterministic; the
-// reference adds in point order).
-constexpr int GMM_STAT_THREADS = 512;  // at d = 32 no thread owns more than two of the 529 scatter entries
-constexpr int GMM_STAT_MAXE = 4;       // table entries per thread (W <= 4 * GMM_STAT_THREADS)
-constexpr int GMM_STAT_SMEM = 96 * 1024;
+// Counts, sums of y and scatter matrices sum (y - mu_k)(y - mu_k)^T (the
+// reference's full-matrix update augur_mat_atm_inc_vtmt is symmetric
+// elementwise) of the points of each component, in four launches:
+//   order    the points are brought in component order, stable in the point
+//            index: counts per chunk of 1024 points (gmm_count_kernel), then
+//            every chunk's ranks behind the counts before it
+//            (gmm_place_kernel);
+//   segments one CTA per segment of at most `seg` points of one component
+//            (gmm_segment_kernel): all its partial sums stay in registers for
+//            the whole segment, and only one row of them is written;
+//   reduce   the rows of each component added in a fixed order
+//            (gmm_stats_reduce_kernel).
+// Deterministic; the reference adds in point order.  Before, each of 296 CTAs
+// kept a table of all components over its own points, so every pass wrote and
+// read back 296 K-component tables (20 MB at K = 16, d = 32) and summed them in
+// a chain of 296.  Points with a label outside [0, K) are not counted.
+// Sums pass 74 -> 28 us and scatter pass 157 -> 54 us at K = 16, d = 32,
+// N = 200,000 (16 of either are the ordering); bound by the gathered rows' round
+// trips and, for the scatter, the binary64 pipe.
+constexpr int GMM_STAT_W = 2048;            // widest row of statistics (count, sums, scatter) taken
+constexpr int GMM_ORDER_CHUNK = 1024;       // points of an ordering CTA
+constexpr int GMM_SLAB = 1 << 20;           // points ordered at a time (bounds the scratch)
+constexpr int GMM_ORDER_CHUNKS = GMM_SLAB / GMM_ORDER_CHUNK;
+constexpr int GMM_SEGMENTS = 444;           // segments aimed at: three CTAs per SM
+constexpr int GMM_SEG_TILE = 64;            // points of a segment staged at a time
+constexpr int GMM_SEG_GROUPS = 32;          // at most: thread groups of a CTA that share a segment's points
 
-// bytes of shared memory per point of a sub-chunk: label and rank, the
-// binary32 row (sums), the centred binary64 row (scatter)
-__host__ __device__ inline int gmm_stat_point_bytes(int d, int want_sum, int want_obs) {
-  return 8 + (want_sum ? 4 * d : 0) + (want_obs ? 8 * d : 0);
+// The ordering's buckets: labels [0, K), and those outside in bucket K
+// (B = K + 1 buckets) or left out (B = K).
+__device__ __forceinline__ int gmm_bucket(int label, int K, int B) {
+  return label >= 0 && label < K ? label : (B == K ? -1 : K);
 }
 
-__host__ __device__ inline int gmm_stat_sub(int d, int chunk, int want_sum, int want_obs) {
-  const int fit = GMM_STAT_SMEM / gmm_stat_point_bytes(d, want_sum, want_obs);
-  return chunk < fit ? chunk : fit;
-}
-
-__global__ void __launch_bounds__(GMM_STAT_THREADS)
-gmm_stats_kernel(int N, int d, int K, const float* __restrict__ Y, const int* __restrict__ z,
-                 const double* __restrict__ mu, int want_sum, int want_obs, int chunk,
-                 double* __restrict__ part) {
-  extern __shared__ double sdbl[];       // cs [sub][d] (double), then zs [sub], perm [sub], ys [sub][d] (float)
-  __shared__ int koff[GMM_MAX_K + 1];
-  const int sub = gmm_stat_sub(d, chunk, want_sum, want_obs);
-  double* cs = sdbl;
-  int* zs = reinterpret_cast<int*>(cs + (want_obs ? (size_t)sub * d : 0));
-  int* perm = zs + sub;
-  float* ys = reinterpret_cast<float*>(perm + sub);
-  const int T = d * (d + 1) / 2;
-  const int W = 1 + (want_sum ? d : 0) + (want_obs ? T : 0);
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int n0 = blockIdx.x * chunk, n1 = min(N, n0 + chunk);
-  // entries owned by this thread: kind 0 count, 1 sum of y_i, 2 scatter (i, j)
-  int ekind[GMM_STAT_MAXE], ei[GMM_STAT_MAXE], ej[GMM_STAT_MAXE];
-  int ne = 0;
-  for (int e = tid; e < W && ne < GMM_STAT_MAXE; e += blockDim.x, ++ne) {
-    if (e == 0) { ekind[ne] = 0; ei[ne] = 0; ej[ne] = 0; }
-    else if (want_sum && e <= d) { ekind[ne] = 1; ei[ne] = e - 1; ej[ne] = 0; }
-    else {
-      int t = e - 1 - (want_sum ? d : 0);
-      int i = 0;
-      while (t >= i + 1) { t -= i + 1; ++i; }
-      ekind[ne] = 2; ei[ne] = i; ej[ne] = t;
-    }
+// cnt [B][GMM_ORDER_CHUNKS]: counts of chunk blockIdx.x.
+__global__ void __launch_bounds__(GMM_THREADS)
+gmm_count_kernel(int n, int K, int B, const int* __restrict__ z, int* __restrict__ cnt) {
+  __shared__ int h[GMM_MAX_K + 1];
+  for (int k = threadIdx.x; k < B; k += GMM_THREADS) h[k] = 0;
+  __syncthreads();
+  const int n0 = blockIdx.x * GMM_ORDER_CHUNK, n1 = min(n, n0 + GMM_ORDER_CHUNK);
+  for (int p = n0 + threadIdx.x; p < n1; p += GMM_THREADS) {
+    const int k = gmm_bucket(z[p], K, B);
+    if (k >= 0) atomicAdd(&h[k], 1);
   }
-  for (int base = n0; base < n1 || base == n0; base += sub) {
-    const int m = max(0, min(sub, n1 - base));
-    for (int p = tid; p < m; p += blockDim.x) {
-      const int k = z[base + p];
-      zs[p] = (k >= 0 && k < K) ? k : -1;    // a label outside [0, K) is not counted
+  __syncthreads();
+  for (int k = threadIdx.x; k < B; k += GMM_THREADS) cnt[k * GMM_ORDER_CHUNKS + blockIdx.x] = h[k];
+}
+
+// perm: the slab's points (plus `first`) in bucket order; start [B + 1], if
+// given: where each bucket's begin.
+__global__ void __launch_bounds__(GMM_THREADS)
+gmm_place_kernel(int n, int K, int B, int first, const int* __restrict__ z, const int* __restrict__ cnt,
+                 int* __restrict__ perm, int* __restrict__ start) {
+  constexpr int NW = GMM_THREADS / 32, PER = GMM_ORDER_CHUNK / NW;
+  __shared__ int tot[GMM_MAX_K + 1], before[GMM_MAX_K + 1], cur[NW][GMM_MAX_K + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b = blockIdx.x;
+  for (int k = warp; k < B; k += NW) {
+    int t = 0, f = 0;
+    for (int c = lane; c < (int)gridDim.x; c += 32) {
+      const int v = cnt[k * GMM_ORDER_CHUNKS + c];
+      t += v;
+      f += c < b ? v : 0;
     }
-    if (want_sum)
-      for (int e = tid; e < m * d; e += blockDim.x) ys[e] = Y[(size_t)base * d + e];
-    __syncthreads();
-    if (want_obs) {
-      // the centred rows, one binary64 subtraction per coordinate
-      for (int e = tid; e < m * d; e += blockDim.x) {
-        const int p = e / d, i = e - p * d;
-        const int k = zs[p];
-        cs[e] = k >= 0 ? __dadd_rn((double)Y[(size_t)base * d + e], -mu[(size_t)k * d + i]) : 0.0;
-      }
-    }
-    if (tid < 32) {
-      // stable counting sort of the sub-chunk by component
-      for (int k = lane; k <= K; k += 32) koff[k] = 0;
-      __syncwarp();
-      for (int p = lane; p < m; p += 32)
-        if (zs[p] >= 0) atomicAdd(&koff[zs[p] + 1], 1);
-      __syncwarp();
-      if (lane == 0)
-        for (int k = 0; k < K; ++k) koff[k + 1] += koff[k];
-      __syncwarp();
-      for (int p0 = 0; p0 < m; p0 += 32) {       // koff[k] serves as component k's cursor
-        const int p = p0 + lane;
-        const int k = p < m ? zs[p] : -1;
-        const bool act = k >= 0;
-        const unsigned mask = __ballot_sync(0xffffffffu, act);
-        if (act) {
-          const unsigned peers = __match_any_sync(mask, k);
-          const int rank = __popc(peers & ((1u << lane) - 1u));
-          perm[koff[k] + rank] = p;
-          __syncwarp(mask);
-          if (lane == __ffs(peers) - 1) koff[k] += __popc(peers);
-        }
-        __syncwarp();
-      }
-      if (lane == 0) {                           // cursors back to start offsets
-        for (int k = K; k > 0; --k) koff[k] = koff[k - 1];
-        koff[0] = 0;
-      }
-    }
-    __syncthreads();
-    for (int k = 0; k < K; ++k) {
-      const int p0 = koff[k], p1 = koff[k + 1];
+    t = __reduce_add_sync(0xffffffffu, t);
+    f = __reduce_add_sync(0xffffffffu, f);
+    if (lane == 0) { tot[k] = t; before[k] = f; }
+  }
+  // this warp's points, and its counts by component
+  const int p0 = b * GMM_ORDER_CHUNK + warp * PER;
+  int kk[PER / 32];
+  for (int k = lane; k < B; k += 32) cur[warp][k] = 0;
+  __syncwarp();
 #pragma unroll
-      for (int q = 0; q < GMM_STAT_MAXE; ++q) {
-        if (q >= ne) continue;
-        double acc = 0.0;
-        if (ekind[q] == 0) {
-          acc = (double)(p1 - p0);                 // exactly the sum of p1 - p0 ones
-        } else if (ekind[q] == 1) {
-          const int i = ei[q];
-          for (int p = p0; p < p1; ++p) acc = __dadd_rn(acc, (double)ys[perm[p] * d + i]);
-        } else {
-          const int i = ei[q], j = ej[q];
-#pragma unroll 4
-          for (int p = p0; p < p1; ++p) {
-            const double* c = cs + perm[p] * d;
-            acc = __dadd_rn(acc, __dmul_rn(c[i], c[j]));
-          }
-        }
-        double* dst = part + ((size_t)blockIdx.x * K + k) * W + tid + q * blockDim.x;
-        *dst = base == n0 ? acc : __dadd_rn(*dst, acc);
-      }
+  for (int q = 0; q < PER / 32; ++q) {
+    const int p = p0 + q * 32 + lane;
+    kk[q] = p < n ? gmm_bucket(z[p], K, B) : -1;
+    if (kk[q] >= 0) atomicAdd(&cur[warp][kk[q]], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x < (unsigned)B) {
+    int s = 0;
+    for (int k = 0; k < (int)threadIdx.x; ++k) s += tot[k];
+    if (b == 0 && start != nullptr) {
+      start[threadIdx.x] = s;
+      if ((int)threadIdx.x == B - 1) start[B] = s + tot[B - 1];
     }
-    __syncthreads();                             // the next sub-chunk reuses shared memory
-    if (m == 0) break;
+    s += before[threadIdx.x];
+    for (int w = 0; w < NW; ++w) {   // counts become cursors
+      const int c = cur[w][threadIdx.x];
+      cur[w][threadIdx.x] = s;
+      s += c;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < PER / 32; ++q) {
+    const bool act = kk[q] >= 0;
+    const unsigned mask = __ballot_sync(0xffffffffu, act);
+    if (act) {
+      const unsigned peers = __match_any_sync(mask, kk[q]);
+      const int rank = __popc(peers & ((1u << lane) - 1u));
+      const int base = cur[warp][kk[q]];
+      perm[base + rank] = first + p0 + q * 32 + lane;
+      __syncwarp(mask);
+      if (rank == 0) cur[warp][kk[q]] = base + __popc(peers);
+    }
+    __syncwarp();
   }
 }
 
-__global__ void gmm_stats_reduce_kernel(int d, int K, int want_sum, int want_obs, int nparts,
-                                        const double* __restrict__ part, int* __restrict__ cnt,
-                                        double* __restrict__ sum, double* __restrict__ obs) {
-  const int T = d * (d + 1) / 2;
-  const int W = 1 + (want_sum ? d : 0) + (want_obs ? T : 0);
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= K * W) return;
-  // CTA-order sum; eight partials are loaded ahead of their additions
+// The segment blockIdx.x: its component and its number in it, found by the
+// first warp (lane l takes components l and l + 32; start: [K + 1]); k = -1 past
+// the last segment.
+__device__ __forceinline__ void gmm_find_segment(const int* __restrict__ start, int K, int seg, int r, int* out) {
+  const int lane = threadIdx.x & 31;
+  int base = 0, k = -1, i = 0;
+#pragma unroll
+  for (int h = 0; h < GMM_MAX_K; h += 32) {
+    const int q = h + lane;
+    const int ns = q < K ? (start[q + 1] - start[q] + seg - 1) / seg : 0;
+    int inc = ns;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, r >= base + inc - ns && r < base + inc);
+    if (hit) {
+      k = h + __ffs(hit) - 1;
+      i = r - base - __shfl_sync(0xffffffffu, inc - ns, __ffs(hit) - 1);
+    }
+    base += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  if (lane == 0) {
+    out[0] = k;
+    out[1] = i;
+    out[2] = k >= 0 ? start[k] + i * seg : 0;
+    out[3] = k >= 0 ? min(seg, start[k + 1] - start[k] - i * seg) : 0;
+  }
+}
+
+__host__ __device__ inline int gmm_obs_tiles(int d) { const int t = (d + 3) / 4; return t * (t + 1) / 2; }
+__host__ __device__ inline int gmm_obs_groups(int d) {
+  const int g = GMM_THREADS / gmm_obs_tiles(d);
+  return g < GMM_SEG_GROUPS ? g : GMM_SEG_GROUPS;
+}
+__host__ __device__ inline int gmm_seg_pitch(int d) { return (d + 3) / 4 * 4 + 2; }
+
+// One row of part per segment: sums [d] if wanted, then the scatter's lower
+// triangle, row by row, if wanted.
+// Sums: a group of pow2(d) lanes (32 lanes taking two coordinates each past
+// d = 32) takes points in turn, one coordinate a lane.
+// Scatter: the points are centred in binary64 once each, 64 at a time, into
+// shared memory; a thread owns a 4 x 4 tile of the lower triangle (8
+// values read for 16 multiply-adds), and as many groups of threads as fit
+// the CTA share the points; the groups' tiles are added in group order.
+// CW (16, 32 or 64, at least d): coordinates staged side by side.  All loads of
+// a round are issued together, their indices clamped into the segment rather
+// than guarded one by one (guarded loads waited for each other: 71 us for the
+// scatter pass at K = 16, d = 32, N = 200,000).
+template <int CW>
+__global__ void __launch_bounds__(GMM_THREADS)
+gmm_segment_kernel(int d, int K, int seg, int want_sum, int want_obs, const float* __restrict__ Y,
+                   const double* __restrict__ mu, const int* __restrict__ perm, const int* __restrict__ start,
+                   double* __restrict__ part, int pts_at) {
+  extern __shared__ __align__(16) double sh[];
+  __shared__ double mk[GMM_MAX_D];
+  __shared__ int where[4];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < 32) gmm_find_segment(start, K, seg, blockIdx.x, where);
+  __syncthreads();
+  const int k = where[0], m = where[3];
+  if (k < 0) return;   // uniform
+  int* pts = reinterpret_cast<int*>(sh + pts_at);
+  for (int p = tid; p < m; p += GMM_THREADS) pts[p] = perm[where[2] + p];
+  __syncthreads();
+  const int W = (want_sum ? d : 0) + (want_obs ? d * (d + 1) / 2 : 0);
+  double* row = part + (size_t)blockIdx.x * W;
+  if (want_sum) {
+    int dp = 1;
+    while (dp < d && dp < 32) dp <<= 1;
+    const int c = lane & (dp - 1), per = 32 / dp;             // coordinate, points of a warp at a time
+    const int step = per * (GMM_THREADS / 32);
+    double s0 = 0.0, s1 = 0.0;
+    const int c0 = min(c, d - 1), c1 = min(c + 32, d - 1);
+    for (int p = warp * per + lane / dp; p < m; p += 8 * step) {
+      float y0[8], y1[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float* y = Y + (size_t)pts[min(p + q * step, m - 1)] * d;
+        y0[q] = y[c0];
+        if (CW > 32) y1[q] = y[c1];
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (p + q * step < m) {
+          s0 = __dadd_rn(s0, (double)y0[q]);
+          if (CW > 32) s1 = __dadd_rn(s1, (double)y1[q]);
+        }
+    }
+    for (int o = 16; o >= dp; o >>= 1) s0 = __dadd_rn(s0, __shfl_xor_sync(0xffffffffu, s0, o));   // s1: dp == 32
+    if (lane < dp) {
+      if (c < d) sh[warp * GMM_MAX_D + c] = s0;
+      if (c + 32 < d) sh[warp * GMM_MAX_D + c + 32] = s1;
+    }
+    __syncthreads();
+    if (tid < d) {
+      double a = 0.0;
+      for (int w = 0; w < GMM_THREADS / 32; ++w) a = __dadd_rn(a, sh[w * GMM_MAX_D + tid]);
+      row[tid] = a;
+    }
+    __syncthreads();
+    row += d;
+  }
+  if (!want_obs) return;
+  const int pd = gmm_seg_pitch(d), dz = pd - 2;                // pitch, d rounded up to tiles
+  const int nt = gmm_obs_tiles(d), G = gmm_obs_groups(d);
+  const int g = tid / nt, tile = tid - g * nt;
+  int ti = 0;
+  while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
+  const int tj = tile - ti * (ti + 1) / 2;
+  double acc[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+  if (tid < d) mk[tid] = mu[(size_t)k * d + tid];
+  __syncthreads();
+  // a thread stages one coordinate of every (256 / CW)-th point; the next
+  // tile's values are loaded while this one's products are formed
+  constexpr int PSTEP = GMM_THREADS / CW, NQ = GMM_SEG_TILE / PSTEP;
+  const int c = tid & (CW - 1), pr = tid / CW;
+  const float* yc = Y + min(c, d - 1);
+  // a point's coordinates 4t, 4t + 1 of all t, then its 4t + 2, 4t + 3: the
+  // tiles' 16-byte reads are then side by side
+  const int cp = ((c >> 1) & 1) * (dz / 2) + 2 * (c >> 2) + (c & 1);
+  float v[NQ];
+  auto fetch = [&](int p0) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) v[q] = yc[(size_t)pts[min(p0 + pr + q * PSTEP, m - 1)] * d];
+  };
+  fetch(0);
+  const double mc = c < d ? mk[c] : 0.0;
+  for (int p0 = 0; p0 < m; p0 += GMM_SEG_TILE) {
+    const int np = min(GMM_SEG_TILE, m - p0);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      if (c < dz) sh[(pr + q * PSTEP) * pd + cp] = c < d ? __dadd_rn((double)v[q], -mc) : 0.0;
+    if (p0 + GMM_SEG_TILE < m) fetch(p0 + GMM_SEG_TILE);
+    __syncthreads();
+    if (g < G) {
+      for (int p = g; p < np; p += G) {
+        const double2* x = reinterpret_cast<const double2*>(sh + p * pd) + ti;
+        const double2* y = reinterpret_cast<const double2*>(sh + p * pd) + tj;
+        const double2 x0 = x[0], x1 = x[dz / 4], y0 = y[0], y1 = y[dz / 4];
+        const double xa[4] = {x0.x, x0.y, x1.x, x1.y}, ya[4] = {y0.x, y0.y, y1.x, y1.y};
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) acc[a][b] = __fma_rn(xa[a], ya[b], acc[a][b]);
+      }
+    }
+    __syncthreads();
+  }
+  if (g < G) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) sh[(g * nt + tile) * 16 + 4 * a + b] = acc[a][b];
+  }
+  __syncthreads();
+  for (int e = tid; e < nt * 16; e += GMM_THREADS) {
+    double a = 0.0;
+    for (int q = 0; q < G; ++q) a = __dadd_rn(a, sh[q * nt * 16 + e]);
+    int t = e >> 4, r = 0;
+    while (t >= r + 1) { t -= r + 1; ++r; }
+    const int ii = 4 * r + ((e >> 2) & 3), jj = 4 * t + (e & 3);
+    if (ii < d && jj <= ii) row[ii * (ii + 1) / 2 + jj] = a;
+  }
+}
+
+// Component blockIdx.y's rows added: 32 entries per CTA, eight interleaved
+// partial sums of each, then those in order; `add`: onto an earlier slab's.
+__global__ void __launch_bounds__(GMM_THREADS)
+gmm_stats_reduce_kernel(int d, int K, int seg, int want_sum, int want_obs, const double* __restrict__ part,
+                        const int* __restrict__ start, int add, int* __restrict__ cnt, double* __restrict__ sum,
+                        double* __restrict__ obs) {
+  __shared__ double red[8][33];
+  const int k = blockIdx.y, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  int r0 = 0;
+  for (int q = 0; q < k; ++q) r0 += (start[q + 1] - start[q] + seg - 1) / seg;
+  const int n = start[k + 1] - start[k], ns = (n + seg - 1) / seg;
+  if (blockIdx.x == 0 && threadIdx.x == 0) cnt[k] = n + (add ? cnt[k] : 0);
+  const int W = (want_sum ? d : 0) + (want_obs ? d * (d + 1) / 2 : 0);
+  const int e = blockIdx.x * 32 + tx;
   double a = 0.0;
-  const size_t stride = (size_t)K * W;
-  int b = 0;
-  for (; b + 8 <= nparts; b += 8) {
-    double v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = __ldg(part + (size_t)(b + q) * stride + e);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) a = __dadd_rn(a, v[q]);
+  if (e < W) {
+#pragma unroll 8
+    for (int r = ty; r < ns; r += 8) a = __dadd_rn(a, __ldg(part + (size_t)(r0 + r) * W + e));
   }
-  for (; b < nparts; ++b) a = __dadd_rn(a, __ldg(part + (size_t)b * stride + e));
-  const int k = e / W, f = e - k * W;
-  if (f == 0) {
-    cnt[k] = (int)a;
-  } else if (want_sum && f <= d) {
-    sum[(size_t)k * d + f - 1] = a;
+  red[ty][tx] = a;
+  __syncthreads();
+  if (ty != 0 || e >= W) return;
+  a = red[0][tx];
+#pragma unroll
+  for (int q = 1; q < 8; ++q) a = __dadd_rn(a, red[q][tx]);
+  if (want_sum && e < d) {
+    double* o = sum + (size_t)k * d + e;
+    *o = add ? __dadd_rn(*o, a) : a;
   } else {
-    int t = f - 1 - (want_sum ? d : 0);
+    int t = e - (want_sum ? d : 0);
     int i = 0;
     while (t >= i + 1) { t -= i + 1; ++i; }
-    obs[(size_t)k * d * d + (size_t)i * d + t] = a;
-    obs[(size_t)k * d * d + (size_t)t * d + i] = a;
+    double* o = obs + (size_t)k * d * d;
+    if (add) a = __dadd_rn(o[(size_t)i * d + t], a);
+    o[(size_t)i * d + t] = a;
+    o[(size_t)t * d + i] = a;
   }
 }
 
@@ -1128,19 +1439,31 @@ int launch_gmm_z(int N, int d, int K, int shared, const float* Y, const double* 
 // Scratch of the screened draw: the component tables, the exact-path flag
 // and queue length, the queue.
 static inline size_t gmm_al256(size_t x) { return (x + 255) & ~(size_t)255; }
-static inline size_t gmm_zs_smem(int d, int K) {
-  return sizeof(float) * (size_t)K * gmm_zs_stride(d) + sizeof(double) * (size_t)K * d;
+static inline size_t gmm_zs_smem(int d, int K) { return sizeof(float) * (size_t)K * gmm_zs_stride(d); }
+// Whether the screened draw takes the points in the order of their current
+// labels (two small launches, about 11 us at 200,000 points): then a warp's
+// points are near one component and the others' rows are mostly left out.
+// Worth it where the whole triangular products take several times that: the
+// whole draw 227 -> 145 us at N = 200,000, K = 16, d = 32 (3.3e9 here) with
+// components apart, 250 us while 5 % of the labels are wrong; at 20,011
+// points, K = 7, d = 13 (2.4e7) the draw takes 27 us, no more than the two
+// launches would leave to gain.
+static inline bool gmm_zs_ordered(int N, int d, int K) { return d > 8 && K > 2 && (double)N * K * d * d >= 4e8; }
+static inline size_t gmm_zs_queue_bytes(int N) { return gmm_al256(sizeof(int) * (size_t)N); }
+size_t gmm_zs_scratch(int N, int d, int K) {
+  return gmm_al256(gmm_zs_smem(d, K)) + 256 + gmm_zs_queue_bytes(N) +
+         (gmm_zs_ordered(N, d, K) ? gmm_zs_queue_bytes(N) + sizeof(int) * (size_t)(K + 1) * GMM_ORDER_CHUNKS : 0);
 }
-size_t gmm_zs_scratch(int N, int d, int K) { return gmm_al256(gmm_zs_smem(d, K)) + 256 + gmm_al256(sizeof(int) * (size_t)N); }
 bool gmm_zs_fits(int d, int K) { return K <= GMM_ZS_MAXK && d <= 32 && gmm_zs_smem(d, K) <= 100 * 1024; }
 
 template <int DT>
-static int launch_zs_t(int N, int d, int K, const float* Y, const double* mu, const float* tab, const int* flag,
+static int launch_zs_t(int N, int d, int K, const float* Y, const float* tab, const int* perm, const int* flag,
                        int* queue, int* qn, int* z, uint64_t seed, uint32_t iter, uint32_t comp, cudaStream_t st) {
   const size_t smem = gmm_zs_smem(d, K);
   AB_CUDA(cudaFuncSetAttribute(gmm_zs_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gmm_zs_kernel<DT><<<ceil_div(N, GMM_ZS_THREADS), GMM_ZS_THREADS, smem, st>>>(N, d, K, Y, mu, tab, flag, queue, qn,
-                                                                              z, seed, iter, comp);
+  const int vec = d % 4 == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
+  const unsigned grid = std::min(ceil_div(N, 64), 148u * 3u);   // few points: a warp's tile each
+  gmm_zs_kernel<DT><<<grid, GMM_ZS_THREADS, smem, st>>>(N, d, K, vec, Y, tab, perm, flag, queue, qn, z, seed, iter, comp);
   AB_LAUNCH_CHECK("gmm_zs_kernel");
   return AB_OK;
 }
@@ -1158,12 +1481,24 @@ int launch_gmm_z_screened(int N, int d, int K, int shared, const float* Y, const
   AB_CUDA(cudaMemsetAsync(ctl, 0, 2 * sizeof(int), st));
   gmm_zs_prep_kernel<<<K, 64, 0, st>>>(d, K, shared, pis, mu, Linv, hdet, tab, flag);
   AB_LAUNCH_CHECK("gmm_zs_prep_kernel");
+  int* perm = nullptr;
+  if (gmm_zs_ordered(N, d, K)) {
+    perm = reinterpret_cast<int*>(reinterpret_cast<char*>(queue) + gmm_zs_queue_bytes(N));
+    int* chunk_cnt = reinterpret_cast<int*>(reinterpret_cast<char*>(perm) + gmm_zs_queue_bytes(N));
+    for (int n0 = 0; n0 < N; n0 += GMM_SLAB) {
+      const int n = std::min(GMM_SLAB, N - n0), chunks = (int)ceil_div(n, GMM_ORDER_CHUNK);
+      gmm_count_kernel<<<chunks, GMM_THREADS, 0, st>>>(n, K, K + 1, z + n0, chunk_cnt);
+      AB_LAUNCH_CHECK("gmm_count_kernel");
+      gmm_place_kernel<<<chunks, GMM_THREADS, 0, st>>>(n, K, K + 1, n0, z + n0, chunk_cnt, perm + n0, nullptr);
+      AB_LAUNCH_CHECK("gmm_place_kernel");
+    }
+  }
   int rc;
-  if (d <= 2) rc = launch_zs_t<2>(N, d, K, Y, mu, tab, flag, queue, qn, z, seed, iter, comp, st);
-  else if (d <= 4) rc = launch_zs_t<4>(N, d, K, Y, mu, tab, flag, queue, qn, z, seed, iter, comp, st);
-  else if (d <= 8) rc = launch_zs_t<8>(N, d, K, Y, mu, tab, flag, queue, qn, z, seed, iter, comp, st);
-  else if (d <= 16) rc = launch_zs_t<16>(N, d, K, Y, mu, tab, flag, queue, qn, z, seed, iter, comp, st);
-  else rc = launch_zs_t<32>(N, d, K, Y, mu, tab, flag, queue, qn, z, seed, iter, comp, st);
+  if (d <= 2) rc = launch_zs_t<2>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
+  else if (d <= 4) rc = launch_zs_t<4>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
+  else if (d <= 8) rc = launch_zs_t<8>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
+  else if (d <= 16) rc = launch_zs_t<16>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
+  else rc = launch_zs_t<32>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
   if (rc) return rc;
   gmm_zx_kernel<<<592, 32 * K, 0, st>>>(d, K, shared, Y, pis, mu, Linv, hdet, queue, qn, z, seed, iter, comp);
   AB_LAUNCH_CHECK("gmm_zx_kernel");
@@ -1190,26 +1525,59 @@ int launch_gmm_prep(int Kc, int d, const double* cov, double* Linv, double* hdet
 #undef AB_CALL
 }
 
-size_t gmm_stats_scratch(int d, int K) {
-  const size_t W = 1 + (size_t)d + (size_t)d * (d + 1) / 2;
-  return sizeof(double) * GMM_STAT_CTAS * (size_t)K * W;
+// Scratch of the statistics: the component order, chunk counts, component
+// starts, and a row of partial sums per segment.
+struct GmmStatScratch {
+  size_t perm, cnt, start, part, total;
+};
+static GmmStatScratch gmm_stat_layout(int d, int K) {
+  GmmStatScratch L;
+  const size_t W = (size_t)d + (size_t)d * (d + 1) / 2;
+  L.perm = 0;
+  L.cnt = L.perm + sizeof(int) * (size_t)GMM_SLAB;
+  L.start = L.cnt + sizeof(int) * (size_t)K * GMM_ORDER_CHUNKS;
+  L.part = L.start + gmm_al256(sizeof(int) * ((size_t)K + 1));
+  L.total = L.part + sizeof(double) * ((size_t)GMM_SEGMENTS + K) * W;
+  return L;
 }
+size_t gmm_stats_scratch(int d, int K) { return gmm_stat_layout(d, K).total; }
 
 int launch_gmm_stats(int N, int d, int K, const float* Y, const int* z, const double* mu, int want_sum,
-                     int want_obs, int* cnt, double* sum, double* obs, double* part, cudaStream_t st) {
-  const int T = d * (d + 1) / 2;
-  const int W = 1 + (want_sum ? d : 0) + (want_obs ? T : 0);
-  AB_REQUIRE(W <= GMM_STAT_MAXE * GMM_STAT_THREADS, AB_ERR_ARG, "gmm: d too large for the statistics pass");
-  const int chunk = (N + GMM_STAT_CTAS - 1) / GMM_STAT_CTAS;
-  const int nparts = (N + chunk - 1) / chunk;
-  const int sub = gmm_stat_sub(d, chunk, want_sum, want_obs);
-  const size_t smem = (size_t)gmm_stat_point_bytes(d, want_sum, want_obs) * (size_t)sub;
-  AB_CUDA(cudaFuncSetAttribute(gmm_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gmm_stats_kernel<<<nparts, GMM_STAT_THREADS, smem, st>>>(N, d, K, Y, z, mu, want_sum, want_obs, chunk, part);
-  AB_LAUNCH_CHECK("gmm_stats_kernel");
-  gmm_stats_reduce_kernel<<<ceil_div((size_t)K * W, 256), 256, 0, st>>>(d, K, want_sum, want_obs, nparts, part,
-                                                                        cnt, sum, obs);
-  AB_LAUNCH_CHECK("gmm_stats_reduce_kernel");
+                     int want_obs, int* cnt, double* sum, double* obs, void* scratch, cudaStream_t st) {
+  const int W = (want_sum ? d : 0) + (want_obs ? d * (d + 1) / 2 : 0);
+  AB_REQUIRE(1 + W <= GMM_STAT_W, AB_ERR_ARG, "gmm: d too large for the statistics pass");
+  const GmmStatScratch L = gmm_stat_layout(d, K);
+  char* base = static_cast<char*>(scratch);
+  int* perm = reinterpret_cast<int*>(base + L.perm);
+  int* chunk_cnt = reinterpret_cast<int*>(base + L.cnt);
+  int* start = reinterpret_cast<int*>(base + L.start);
+  double* part = reinterpret_cast<double*>(base + L.part);
+  size_t smem = want_sum ? sizeof(double) * (GMM_THREADS / 32) * GMM_MAX_D : 0;
+  if (want_obs) {
+    smem = std::max(smem, sizeof(double) * (size_t)GMM_SEG_TILE * gmm_seg_pitch(d));
+    smem = std::max(smem, sizeof(double) * 16 * (size_t)gmm_obs_groups(d) * gmm_obs_tiles(d));
+  }
+  const int pts_at = (int)(smem / sizeof(double));   // then the segment's points
+  smem += sizeof(int) * (size_t)std::max(32, (int)ceil_div(std::min(N, GMM_SLAB), GMM_SEGMENTS));
+  const auto segments = d <= 16 ? gmm_segment_kernel<16> : d <= 32 ? gmm_segment_kernel<32> : gmm_segment_kernel<64>;
+  AB_CUDA(cudaFuncSetAttribute(segments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  for (int n0 = 0; n0 < N; n0 += GMM_SLAB) {
+    const int n = std::min(GMM_SLAB, N - n0);
+    const int chunks = (int)ceil_div(n, GMM_ORDER_CHUNK);
+    const int seg = std::max(32, (int)ceil_div(n, GMM_SEGMENTS));   // at most GMM_SEGMENTS + K segments
+    gmm_count_kernel<<<chunks, GMM_THREADS, 0, st>>>(n, K, K, z + n0, chunk_cnt);
+    AB_LAUNCH_CHECK("gmm_count_kernel");
+    gmm_place_kernel<<<chunks, GMM_THREADS, 0, st>>>(n, K, K, 0, z + n0, chunk_cnt, perm, start);
+    AB_LAUNCH_CHECK("gmm_place_kernel");
+    if (W > 0) {
+      segments<<<ceil_div(n, seg) + K, GMM_THREADS, smem, st>>>(d, K, seg, want_sum, want_obs, Y + (size_t)n0 * d, mu,
+                                                                perm, start, part, pts_at);
+      AB_LAUNCH_CHECK("gmm_segment_kernel");
+    }
+    gmm_stats_reduce_kernel<<<dim3(std::max(1u, ceil_div(W, 32)), K), GMM_THREADS, 0, st>>>(
+        d, K, seg, want_sum, want_obs, part, start, n0 > 0, cnt, sum, obs);
+    AB_LAUNCH_CHECK("gmm_stats_reduce_kernel");
+  }
   return AB_OK;
 }
 
@@ -1331,7 +1699,7 @@ extern "C" int ab_gmm_stats(int N, int d, int K, const float* Y, const int* z, c
   AB_REQUIRE(Y && z && cnt && scratch, AB_ERR_ARG, "ab_gmm_stats: null pointer");
   AB_REQUIRE(!obs || mu, AB_ERR_ARG, "ab_gmm_stats: the scatter matrices need mu");
   return launch_gmm_stats(N, d, K, Y, z, mu, sum != nullptr, obs != nullptr, cnt, sum, obs,
-                          static_cast<double*>(scratch), as_stream(stream));
+                          scratch, as_stream(stream));
 }
 
 extern "C" int ab_gmm_conj_pis(int K, const double* alpha, const int* cnt, double* pis, uint64_t seed,

@@ -256,7 +256,9 @@ int ab_gmm_disc_z(int N, int d, int K, int shared_cov, const float* Y, const dou
  * draw wherever the uniform lies outside their uncertainty band; the other
  * points (a few in 10^4), and every point of a call with extreme
  * log-densities, run the reference's binary64 loop.  Equal to
- * ab_gmm_disc_z bit for bit.  scratch: ab_gmm_z_scratch_bytes(N, d, K)
+ * ab_gmm_disc_z bit for bit, whatever z holds on entry: at large sizes the
+ * points are taken in the order of those labels, which only decides how much
+ * work can be left out.  scratch: ab_gmm_z_scratch_bytes(N, d, K)
  * bytes, 256-byte aligned (component tables and the queue of points the
  * screen leaves).  Shapes outside K <= 32, d <= 32 run ab_gmm_disc_z's
  * kernel. */
@@ -271,7 +273,8 @@ int ab_gmm_disc_z_screened(int N, int d, int K, int shared_cov, const float* Y, 
 /* Conjugate statistics of z (CgConj.hs:186-246): counts cnt int32 [K] always;
  * sum f64 [K][d] of y if `sum` is non-NULL; obs f64 [K][d][d] =
  * sum (y - mu[z])(y - mu[z])^T if `obs` is non-NULL (needs mu).  scratch:
- * ab_gmm_stats_scratch_bytes(d, K) bytes (per-block partial tables). */
+ * ab_gmm_stats_scratch_bytes(d, K) bytes (the points in component order, and
+ * rows of partial sums). */
 size_t ab_gmm_stats_scratch_bytes(int d, int K);
 int ab_gmm_stats(int N, int d, int K, const float* Y, const int* z, const double* mu, int* cnt, double* sum,
                  double* obs, void* scratch, void* stream);

@@ -15,7 +15,7 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 
-def _draws(Y, pis, mus, covs, shared, seed=4, it=6):
+def _draws(Y, pis, mus, covs, shared, seed=4, it=6, labels=None):
     L = N.lib()
     N_, d = Y.shape
     K = len(pis)
@@ -29,6 +29,8 @@ def _draws(Y, pis, mus, covs, shared, seed=4, it=6):
     pd, md = dev(pis, torch.float64), dev(mus, torch.float64)
     z0 = torch.full((N_,), -1, dtype=torch.int32, device="cuda")
     z1 = torch.full((N_,), -1, dtype=torch.int32, device="cuda")
+    if labels is not None:
+        z1.copy_(torch.as_tensor(labels))
     N.check(L.ab_gmm_disc_z(N_, d, K, int(shared), N.ptr(Yd), N.ptr(pd), N.ptr(md), N.ptr(Linv), N.ptr(hdet),
                             N.ptr(z0), seed, it, 0, N.stream_ptr()), "disc_z")
     scratch = torch.zeros(int(L.ab_gmm_z_scratch_bytes(N_, d, K)), dtype=torch.uint8, device="cuda")
@@ -60,6 +62,31 @@ def test_screen_equals_binary64_on_the_benchmark_shape():
 def test_screen_equals_binary64(N_, K, d, shared, seed):
     Y, z, mus, covs, pis = O.gmm_synthetic(N_, K, d, seed)
     a, b, _ = _draws(Y, pis, mus, covs, shared, seed=seed)
+    np.testing.assert_array_equal(b, a)
+
+
+@pytest.mark.parametrize("N_,K,d,spread,labels", [(90_001, 9, 24, 5.0, "generating"), (90_001, 9, 24, 5.0, "none"),
+                                                  (90_001, 9, 24, 0.4, "random"), (600_001, 9, 9, 5.0, "random"),
+                                                  (13_101, 32, 32, 5.0, "generating"), (13_101, 32, 31, 0.4, "generating"),
+                                                  (1_060_000, 5, 10, 3.0, "generating")])
+def test_screen_in_label_order_equals_binary64(N_, K, d, spread, labels):
+    """Sizes at which the screen takes the points in the order of the labels z
+    holds on entry and leaves out rows of components found far away: apart
+    and overlapping components, entry labels of every kind (some or all outside
+    [0, K)), a last partial tile, more points than are ordered at a time."""
+    rng = np.random.default_rng(N_ + d)
+    mus = rng.standard_normal((K, d)) * spread
+    A = rng.standard_normal((K, d, d + 2))
+    covs = np.einsum("kij,klj->kil", A, A) / (d + 2) + 0.05 * np.eye(d)
+    pis = rng.dirichlet(np.ones(K))
+    z = rng.choice(K, size=N_, p=pis)
+    Y = rng.standard_normal((N_, d))
+    for k in range(K):
+        m = z == k
+        Y[m] = mus[k] + Y[m] @ np.linalg.cholesky(covs[k]).T
+    Y[::1000] = 50.0 * rng.standard_normal((len(Y[::1000]), d))        # far from every component
+    on_entry = {"generating": z, "none": np.full(N_, -1), "random": rng.integers(-2, K + 2, N_)}[labels].astype(np.int32)
+    a, b, _ = _draws(Y.astype(np.float32), pis, mus, covs, False, seed=9, labels=on_entry)
     np.testing.assert_array_equal(b, a)
 
 
