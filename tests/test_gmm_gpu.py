@@ -215,6 +215,32 @@ def test_mvgmm_moves(orc, move):
         np.testing.assert_array_equal(st["z"], O.gmm_disc_z(orc, om, pis, st["mu"], covs, 2, it))
 
 
+@pytest.mark.parametrize("move", ["eslice", "mwg"])
+@pytest.mark.parametrize("N_,K,d", [(1, 2, 1), (6, 3, 1), (300, 3, 17), (1000, 64, 4), (700, 4, 33), (300, 2, 64),
+                                    (9000, 5, 6)])
+def test_mean_moves_at_ragged_sizes(orc, move, N_, K, d):
+    """Fewer points than CTAs that add them, empty components, the widest d,
+    the d at which the kernels change, labels outside [0, K): the moved means
+    equal the oracle's, which evaluates every point at every candidate."""
+    rng = np.random.default_rng(N_ + d)
+    centres = rng.standard_normal((K, d)) * 2
+    A = rng.standard_normal((d, d + 2))
+    covs = A @ A.T / (d + 2) + 0.1 * np.eye(d)
+    z = rng.integers(0, max(1, K - 1), N_).astype(np.int32)          # the last component is empty
+    Y = (centres[z] + rng.standard_normal((N_, d))).astype(np.float32)
+    om = O.GmmModel(Y.astype(np.float64), K, 0.1 * np.ones(d), 4 * np.eye(d), True)
+    mu = centres + 0.1 * rng.standard_normal((K, d))
+    prop = 0.02 * (np.eye(d) + 0.3)
+    g = GmmGibbs(Y, K, 0.1 * np.ones(d), 4 * np.eye(d), pis=np.full(K, 1.0 / K), covs=covs, mu=mu, z=z, move=move,
+                 prop_cov=prop, seed=2)
+    for it in range(3):
+        prev = g.mu.cpu().numpy()
+        g.z.copy_(torch.as_tensor(z))
+        g.sweep(1)
+        want = O.gmm_eslice(orc, om, prev, covs, z, 2, it) if move == "eslice" else O.gmm_mwg(orc, om, prev, covs, z, prop, 2, it)
+        np.testing.assert_allclose(g.mu.cpu().numpy(), want, rtol=1e-9, atol=1e-9)
+
+
 def test_bench_shape_properties():
     """K=16, d=32, N=2e5 (the benchmark shape): statistics sum to N, the
     covariances stay symmetric positive definite, assignments recover most
