@@ -13,8 +13,8 @@
 // par f64 [C][D+2].
 //
 // Engine: one CTA per chain runs whole iterations of the schedule on chip
-// (hlr_chain_kernel).  A data pass computes, at the chain's current theta
-// and b, ll_data = sum_n log Bern(y_n | sigmoid(t_n)) and its gradient
+// (hlr_chain_kernel), with X in shared memory where it fits.  A data pass
+// computes, at the chain's current theta and b, ll_data = sum_n log Bern(y_n | sigmoid(t_n)) and its gradient
 //   d/dtheta_k = sum_n r_n x_nk,  d/db = sum_n r_n,  r_n = y_n - sigmoid(t_n)
 // in FP32 per row (numerically stable logistic terms), with Kahan-compensated
 // per-thread sums and fixed-order FP64 block reductions, so the result is
@@ -28,7 +28,8 @@
 
 namespace ab {
 
-constexpr int HLR_THREADS = 256;
+constexpr int HLR_THREADS = 256;         // threads that walk the rows: each row's place in the compensated sums
+constexpr int HLR_BLOCK = HLR_THREADS + 32;   // and a warp for the prior and, past D = 30, the log-likelihood sums
 constexpr int HLR_CHUNK = 1024;          // rows per data-pass chunk (r buffer)
 constexpr int HLR_MAX_COLS = 4;          // columns per thread in the gradient pass
 constexpr int HLR_MAX_D = HLR_THREADS * HLR_MAX_COLS - 1;
@@ -45,6 +46,7 @@ struct HlrModelDev {
   int lik;              // AB_LIK_*
   float inv_var;        // AB_LIK_NORMAL: 1 / obs_var
   double ll_add;        // AB_LIK_NORMAL: N times the per-row normaliser, added once
+  double vp_const;      // the variance prior's normaliser: log(lam), or a0 log(s0) - lgamma(a0)
   const float* yr;
 };
 
@@ -66,31 +68,36 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
 }
 
 // Stable log Bern(y | sigmoid(t)) and its derivative, FP32.
-__device__ __forceinline__ void bern_terms(int y, float t, float& ll, float& r) {
-  const float sp = fmaxf(t, 0.0f) + log1pf(__expf(-fabsf(t)));
-  ll = y ? t - sp : -sp;
+__device__ __forceinline__ void bern_terms(bool want_ll, int y, float t, float& ll, float& r) {
+  if (want_ll) {
+    const float sp = fmaxf(t, 0.0f) + log1pf(__expf(-fabsf(t)));
+    ll = y ? t - sp : -sp;
+  }
   const float sg = 1.0f / (1.0f + __expf(-t));
   r = (float)y - sg;
 }
 
-// Data factor of row n at t and its derivative in t, FP32: the logistic
-// terms above, Poisson(exp(t)): y t - exp(t) - lgamma(y + 1) and y - exp(t)
-// (the reference's y log(rate) - rate - sum_{k <= y} log k and its adjoint
-// through exp), Normal(t, obs_var): -(y - t)^2 / (2 var) and (y - t) / var
-// (the normaliser is added once per pass, ll_add).
-__device__ __forceinline__ void lik_terms(const HlrModelDev& m, int n, float t, float& ll, float& r) {
+// Data factor of a row at t (if wanted) and its derivative in t, FP32: the logistic terms above, Poisson(exp(t)): y t - exp(t) -
+// lgamma(y + 1) and y - exp(t) (the reference's y log(rate) - rate -
+// sum_{k <= y} log k and its adjoint through exp), Normal(t, obs_var):
+// -(y - t)^2 / (2 var) and (y - t) / var (the normaliser is added once per
+// pass, ll_add).  lab: the row's label, as the bits of y or yr.
+__device__ __forceinline__ void lik_terms(const HlrModelDev& m, bool want_ll, int lab, float t, float& ll, float& r) {
   if (m.lik == AB_LIK_POISSON) {
-    const int y = m.y[n];
     const float rate = expf(t);
-    ll = (float)y * t - rate - lgammaf((float)y + 1.0f);
-    r = (float)y - rate;
+    if (want_ll) ll = (float)lab * t - rate - lgammaf((float)lab + 1.0f);
+    r = (float)lab - rate;
   } else if (m.lik == AB_LIK_NORMAL) {
-    const float d = m.yr[n] - t;
-    ll = -0.5f * d * d * m.inv_var;
+    const float d = __int_as_float(lab) - t;
+    if (want_ll) ll = -0.5f * d * d * m.inv_var;
     r = d * m.inv_var;
   } else {
-    bern_terms(m.y[n], t, ll, r);
+    bern_terms(want_ll, lab, t, ll, r);
   }
+}
+
+__device__ __forceinline__ int load_label(const HlrModelDev& m, int n) {
+  return m.lik == AB_LIK_NORMAL ? __float_as_int(m.yr[n]) : m.y[n];
 }
 
 // Shared-memory workspace of one chain CTA (sizes fixed by D).
@@ -106,17 +113,26 @@ struct Ws {
   double* aux2;    // [D+2]
   double* aux3;    // [D+2]
   double* aux4;    // [D+2]
-  double* pt_ll;   // [D+2]  per-coordinate prior terms (log density)
-  double* pt_dot;  // [D+2]  per-coordinate prior terms (d/dvar)
   double* gpart;   // [HLR_THREADS] per-thread partials (double)
   float* th;       // [D]    theta in FP32 for the data pass
-  float* r;        // [HLR_CHUNK]
+  float* r;        // [HLR_CHUNK] residuals of a chunk of rows
+  float* l;        // [HLR_CHUNK] their log-likelihood terms
   double* red;     // [34]
   double* bcast;   // [8]   broadcast slots
   int* ibcast;     // [8]
+  int* idx;        // [D+2]  block indices of the running component
+  double* gfr;     // [3][P] NUTS: gradients at both frontiers and at the walk's position
+  // the copy of X in shared memory, float or bf16 (null: it stays in global
+  // memory), and of the labels
+  void* xs;
+  int* lab;
+  int xpitch;
 };
 
-__device__ __forceinline__ double cta_sum(double v, double* red) { return block_sum_f64(v, red); }
+// Which parameters a block moves.
+struct BlockInfo {
+  bool th, b, v;
+};
 
 // Small-D pass widths: D gradient columns, the bias column, the
 // log-likelihood; 16 columns for D + 2 <= 16, else 32.
@@ -141,148 +157,209 @@ __device__ __forceinline__ void warp_transpose_sum(double (&v)[COLS], int lane) 
   if (COLS == 16) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
 }
 
+// Where the rows are read: global memory, or the shared copy in X's type.
+enum { X_GLOBAL = 0, X_F32 = 1, X_BF16 = 2 };
+template <int RES>
+__device__ __forceinline__ float row_x(const HlrModelDev& m, const Ws& ws, int i, int k) {
+  if (RES == X_F32) return static_cast<const float*>(ws.xs)[i * ws.xpitch + k];
+  if (RES == X_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(ws.xs)[i * ws.xpitch + k]);
+  return load_x(m, (size_t)i * m.ldx + k);
+}
+template <int RES>
+__device__ __forceinline__ int row_label(const HlrModelDev& m, const Ws& ws, int i) {
+  return RES ? ws.lab[i] : load_label(m, i);
+}
+
 // Data pass for D + 2 <= COLS: one row per thread (t, the log-likelihood term
 // and the residual's contributions to all D + 1 gradient columns in
 // registers, Kahan-compensated), then one transposed warp reduction and a
-// fixed-order sum over the warps, all in FP64.  The row-per-thread walk
-// keeps every thread busy at small N, where the segmented pass below is
-// bound by its per-row shuffle latency.
-template <int COLS>
-__device__ double data_pass_small(const HlrModelDev& m, const double* par, Ws& ws, bool want_grad) {
-  const int D = m.D, N = m.N;
+// fixed-order sum over the warps, all in FP64: the row-per-thread walk keeps
+// every thread busy at small N.  By the row threads; leaves the sums in ws.g and
+// ws.red[33].
+template <int COLS, int RES>
+__device__ __forceinline__ void data_rows_small(const HlrModelDev& m, bool want_ll, bool want_grad, float bias, const Ws& ws) {
+  const int D = m.D;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int k = tid; k < D; k += blockDim.x) ws.th[k] = (float)par[k];
-  const float bias = m.has_b ? (float)par[D] : 0.0f;
-  __syncthreads();
-  float th[COLS - 2];
+  if (tid < HLR_THREADS) {
+    float th[COLS - 2];
 #pragma unroll
-  for (int k = 0; k < COLS - 2; ++k) th[k] = k < D ? ws.th[k] : 0.0f;
-  float s[COLS], c[COLS];
+    for (int k = 0; k < COLS - 2; ++k) th[k] = k < D ? ws.th[k] : 0.0f;
+    float s[COLS], c[COLS];
 #pragma unroll
-  for (int j = 0; j < COLS; ++j) { s[j] = 0.0f; c[j] = 0.0f; }
-  for (int n = tid; n < N; n += blockDim.x) {
-    const size_t rb = (size_t)n * m.ldx;
-    float x[COLS - 2];
-    float t = 0.0f;
+    for (int j = 0; j < COLS; ++j) { s[j] = 0.0f; c[j] = 0.0f; }
+#pragma unroll 1
+    for (int i = tid; i < m.N; i += HLR_THREADS) {
+      float x[COLS - 2];
+      float t = 0.0f;
 #pragma unroll
-    for (int k = 0; k < COLS - 2; ++k) {
-      x[k] = k < D ? load_x(m, rb + k) : 0.0f;
-      t += x[k] * th[k];
+      for (int k = 0; k < COLS - 2; ++k) {
+        x[k] = k < D ? row_x<RES>(m, ws, i, k) : 0.0f;
+        t += x[k] * th[k];
+      }
+      float llv, rv;
+      lik_terms(m, want_ll, row_label<RES>(m, ws, i), t + bias, llv, rv);
+      if (want_ll) kahan_add(s[COLS - 1], c[COLS - 1], llv);
+      if (want_grad) {
+#pragma unroll
+        for (int k = 0; k < COLS - 2; ++k)
+          if (k < D) kahan_add(s[k], c[k], rv * x[k]);
+#pragma unroll
+        for (int k = 0; k < COLS - 1; ++k)
+          if (k == D) kahan_add(s[k], c[k], rv);
+      }
     }
-    float llv, rv;
-    lik_terms(m, n, t + bias, llv, rv);
-    kahan_add(s[COLS - 1], c[COLS - 1], llv);
-    if (want_grad) {
+    double v[COLS];
 #pragma unroll
-      for (int k = 0; k < COLS - 2; ++k)
-        if (k < D) kahan_add(s[k], c[k], rv * x[k]);
-#pragma unroll
-      for (int k = 0; k < COLS - 1; ++k)
-        if (k == D) kahan_add(s[k], c[k], rv);
-    }
+    for (int j = 0; j < COLS; ++j) v[j] = (double)s[j] - (double)c[j];
+    warp_transpose_sum<COLS>(v, lane);
+    if (lane < COLS) ws.gpart[warp * COLS + lane] = v[0];
   }
-  double v[COLS];
-#pragma unroll
-  for (int j = 0; j < COLS; ++j) v[j] = (double)s[j] - (double)c[j];
-  warp_transpose_sum<COLS>(v, lane);
-  __syncthreads();
-  if (lane < COLS) ws.gpart[warp * COLS + lane] = v[0];
   __syncthreads();
   if (tid < COLS) {
-    double acc = 0.0;
-    const int nw = blockDim.x >> 5;
-    for (int w = 0; w < nw; ++w) acc += ws.gpart[w * COLS + tid];
+    constexpr int NW = HLR_THREADS / 32;
+    double a[NW];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) a[w] = ws.gpart[w * COLS + tid];
+    const double acc = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
     if (tid == COLS - 1) ws.red[33] = acc;
-    else if (want_grad && tid <= D) ws.g[tid] = acc;
+    else if (tid <= D) ws.g[tid] = acc;
   }
-  __syncthreads();
-  return ws.red[33];
 }
 
-// Data pass at `par` (theta in par[0..D-1], b = par[D] if has_b).  Writes
-// ll_data (returned, all threads) and, if want_grad, ws.g[0..D] (theta then
-// bias) — the full data gradient.
-__device__ double data_pass(const HlrModelDev& m, const double* par, Ws& ws, bool want_grad) {
+// Data pass for wider D, a chunk of rows at a time: the rows' dot products (X
+// in shared memory: a row per thread, its 32 interleaved partial sums in
+// registers and added as the warp tree of the global-memory walk adds them;
+// otherwise a warp per row) and their terms; then the row threads, owners of
+// gradient columns, walk the chunk's residuals, while eight lanes of the last
+// warp walk its log-likelihood terms.
+template <int RES>
+__device__ __forceinline__ void data_rows_wide(const HlrModelDev& m, bool want_ll, bool want_grad, float bias, const Ws& ws) {
+  constexpr int NW = HLR_THREADS / 32;
   const int D = m.D, N = m.N;
-  if (D + 2 <= 16) return data_pass_small<16>(m, par, ws, want_grad);
-  if (D + 2 <= SMALL_COLS) return data_pass_small<SMALL_COLS>(m, par, ws, want_grad);
-  const int tid = threadIdx.x;
-  for (int k = tid; k < D; k += blockDim.x) ws.th[k] = (float)par[k];
-  const float bias = m.has_b ? (float)par[D] : 0.0f;
-  __syncthreads();
-  // segment of S lanes per row for the row dot products
-  int S = 1;
-  while (S < D && S < 32) S <<= 1;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int segs_per_warp = 32 / S;
-  const int seg = warp * segs_per_warp + lane / S;
-  const int nseg = (blockDim.x >> 5) * segs_per_warp;
-  const int ls = lane % S;
-  // gradient accumulators: thread owns columns c = tid + i*blockDim (cols
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // gradient accumulators: thread owns columns c = tid + i*HLR_THREADS (cols
   // D+1 including the bias column) for rows n = grp (mod ngrp)
   const int ncol = D + 1;
-  const int ngrp = ncol >= (int)blockDim.x ? 1 : (int)blockDim.x / ncol;
-  const int grp = ncol >= (int)blockDim.x ? 0 : tid / ncol;
-  const int col0 = ncol >= (int)blockDim.x ? tid : tid % ncol;
-  const bool gactive = grp < ngrp;
+  const int ngrp = ncol >= HLR_THREADS ? 1 : HLR_THREADS / ncol;
+  const int grp = ncol >= HLR_THREADS ? 0 : tid / ncol;
+  const int col0 = ncol >= HLR_THREADS ? tid : tid % ncol;
+  const bool gactive = tid < HLR_THREADS && grp < ngrp;
   float gs[HLR_MAX_COLS], gc[HLR_MAX_COLS];
 #pragma unroll
   for (int i = 0; i < HLR_MAX_COLS; ++i) { gs[i] = 0.0f; gc[i] = 0.0f; }
-  float lls = 0.0f, llc = 0.0f;
+  float lls = 0.0f, llc = 0.0f;   // log-likelihood terms of rows = lane (mod NW), lanes below NW of the last warp
   for (int n0 = 0; n0 < N; n0 += HLR_CHUNK) {
     const int nc = min(HLR_CHUNK, N - n0);
-    for (int i = seg; i < nc + ((nseg - nc % nseg) % nseg); i += nseg) {
-      const int n = n0 + i;
-      float part = 0.0f;
-      if (i < nc) {
-        const size_t rb = (size_t)n * m.ldx;
-        for (int k = ls; k < D; k += S) part += load_x(m, rb + k) * ws.th[k];
-      }
-      for (int o = S >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-      if (ls == 0 && i < nc) {
+    if (RES) {
+      for (int i = tid; i < nc; i += HLR_BLOCK) {
+        float p[32];
+#pragma unroll
+        for (int q = 0; q < 32; ++q) p[q] = 0.0f;
+        for (int k0 = 0; k0 < D; k0 += 32) {
+#pragma unroll
+          for (int q = 0; q < 32; ++q)
+            if (k0 + q < D) p[q] += row_x<RES>(m, ws, n0 + i, k0 + q) * ws.th[k0 + q];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int q = 0; q < o; ++q) p[q] += p[q + o];
         float llv, rv;
-        lik_terms(m, n, part + bias, llv, rv);
-        kahan_add(lls, llc, llv);
+        lik_terms(m, want_ll, ws.lab[n0 + i], p[0] + bias, llv, rv);
+        if (want_ll) ws.l[i] = llv;
         ws.r[i] = rv;
       }
-    }
-    __syncthreads();
-    if (want_grad && gactive) {
-      for (int i = grp; i < nc; i += ngrp) {
-        const float rv = ws.r[i];
-        const size_t rb = (size_t)(n0 + i) * m.ldx;
+    } else if (warp < NW) {
+      // eight rows of a warp at a time; the transposed reduction adds each
+      // row's 32 partial sums in the tree of a full one (lanes i and i ^ 16, ...)
+      for (int i0 = warp * 8; i0 < nc; i0 += NW * 8) {
+        float part[8];
 #pragma unroll
-        for (int j = 0; j < HLR_MAX_COLS; ++j) {
-          const int c = col0 + j * (ncol >= (int)blockDim.x ? (int)blockDim.x : ncol);
-          if (j > 0 && ncol < (int)blockDim.x) break;
-          if (c < D) kahan_add(gs[j], gc[j], rv * load_x(m, rb + c));
-          else if (c == D) kahan_add(gs[j], gc[j], rv);
+        for (int r = 0; r < 8; ++r) part[r] = 0.0f;
+        for (int k = lane; k < D; k += 32) {
+          const float tk = ws.th[k];
+#pragma unroll
+          for (int r = 0; r < 8; ++r) part[r] += row_x<RES>(m, ws, n0 + min(i0 + r, nc - 1), k) * tk;
+        }
+#pragma unroll
+        for (int o = 16, h = 4; h > 0; o >>= 1, h >>= 1) {
+          const bool up = (lane & o) != 0;
+#pragma unroll
+          for (int r = 0; r < h; ++r) {
+            const float send = up ? part[r] : part[r + h], keep = up ? part[r + h] : part[r];
+            part[r] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+        }
+        part[0] += __shfl_xor_sync(0xffffffffu, part[0], 2);
+        part[0] += __shfl_xor_sync(0xffffffffu, part[0], 1);
+        const int i = i0 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+        if ((lane & 3) == 0 && i < nc) {
+          float llv, rv;
+          lik_terms(m, want_ll, row_label<RES>(m, ws, n0 + i), part[0] + bias, llv, rv);
+          if (want_ll) ws.l[i] = llv;
+          ws.r[i] = rv;
         }
       }
     }
     __syncthreads();
+    if (want_grad && gactive) {
+      if (ncol < HLR_THREADS) {
+        if (col0 < D) {
+          // eight rows' values in flight, added in row order
+          for (int i = grp; i < nc; i += 8 * ngrp) {
+            float xv[8], rv[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const int ii = min(i + q * ngrp, nc - 1);
+              xv[q] = row_x<RES>(m, ws, n0 + ii, col0);
+              rv[q] = ws.r[ii];
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              if (i + q * ngrp < nc) kahan_add(gs[0], gc[0], rv[q] * xv[q]);
+          }
+        } else {
+#pragma unroll 4
+          for (int i = grp; i < nc; i += ngrp) kahan_add(gs[0], gc[0], ws.r[i]);
+        }
+      } else {
+        for (int i = 0; i < nc; ++i) {
+          const float rv = ws.r[i];
+#pragma unroll
+          for (int j = 0; j < HLR_MAX_COLS; ++j) {
+            const int c = col0 + j * HLR_THREADS;
+            if (c < D) kahan_add(gs[j], gc[j], rv * row_x<RES>(m, ws, n0 + i, c));
+            else if (c == D) kahan_add(gs[j], gc[j], rv);
+          }
+        }
+      }
+    }
+    if (want_ll && warp == NW && lane < NW) {
+#pragma unroll 4
+      for (int i = lane; i < nc; i += NW) kahan_add(lls, llc, ws.l[i]);
+    }
+    if (n0 + HLR_CHUNK < N) __syncthreads();
   }
-  const double ll = cta_sum((double)lls - (double)llc, ws.red);
+  if (want_ll && warp == NW) {
+    const double v = warp_sum_f64((double)lls - (double)llc);
+    if (lane == 0) ws.red[33] = v;
+  }
   if (want_grad) {
-    // combine the groups column by column in a fixed order
-    const int stride = ncol >= (int)blockDim.x ? (int)blockDim.x : ncol;
-    for (int j = 0; j < HLR_MAX_COLS; ++j) {
-      const int c0 = j * stride;
-      if (c0 >= ncol) break;
-      ws.gpart[tid] = gactive ? (double)gs[j] - (double)gc[j] : 0.0;
+    if (ncol >= HLR_THREADS) {
+      for (int j = 0; j < HLR_MAX_COLS; ++j)
+        if (gactive && col0 + j * HLR_THREADS < ncol) ws.g[col0 + j * HLR_THREADS] = (double)gs[j] - (double)gc[j];
+    } else {
+      // combine the groups column by column in a fixed order
+      if (tid < HLR_THREADS) ws.gpart[tid] = gactive ? (double)gs[0] - (double)gc[0] : 0.0;
       __syncthreads();
-      if (ncol >= (int)blockDim.x) {
-        const int c = c0 + tid;
-        if (c < ncol) ws.g[c] = ws.gpart[tid];
-      } else if (tid < ncol) {
+      if (tid < ncol) {
         double acc = 0.0;
+#pragma unroll 4
         for (int q = 0; q < ngrp; ++q) acc += ws.gpart[q * ncol + tid];
         ws.g[tid] = acc;
       }
-      __syncthreads();
     }
   }
-  return ll;
 }
 
 // ---- priors (binary64; reference formulas when compat) ----------------------
@@ -292,24 +369,19 @@ __device__ __forceinline__ double normal_ll(const HlrModelDev& m, double pt, dou
   if (!(var > 0.0)) return -INFINITY;
   return -0.5 * log(2.0 * 3.14159265358979323846 * var) - 0.5 * t * t / var;
 }
-__device__ __forceinline__ double normal_dotarg2(const HlrModelDev& m, double pt, double mean, double var) {
-  const double t = pt - mean;
-  return m.compat ? (-0.5 * var) + (0.5 * (t * t) / (var * var))
-                  : (-0.5 / var) + (0.5 * (t * t) / (var * var));
+// d/dvar of the former at mean 0, iv = 1 / var.
+__device__ __forceinline__ double normal_dvar(const HlrModelDev& m, double t, double var, double iv) {
+  return (m.compat ? -0.5 * var : -0.5 * iv) + 0.5 * (t * t) * (iv * iv);
 }
 __device__ __forceinline__ double vprior_ll(const HlrModelDev& m, double v) {
-  if (m.vprior == 0) return (m.lam > 0.0 && v > 0.0) ? log(m.lam) - m.lam * v : (m.compat ? -1e8 : -INFINITY);
+  if (m.vprior == 0) return (m.lam > 0.0 && v > 0.0) ? m.vp_const - m.lam * v : (m.compat ? -1e8 : -INFINITY);
   if (!(v > 0.0)) return m.compat ? -1e8 : -INFINITY;
-  return m.a0 * log(m.s0) - lgamma(m.a0) - (m.a0 + 1.0) * log(v) - m.s0 / v;
+  return m.vp_const - (m.a0 + 1.0) * log(v) - m.s0 / v;
 }
-__device__ __forceinline__ double vprior_dot(const HlrModelDev& m, double v) {
+__device__ __forceinline__ double vprior_dot(const HlrModelDev& m, double v, double iv) {
   if (m.vprior == 0) return (m.lam > 0.0 && v > 0.0) ? -m.lam : 0.0;
-  return -(m.a0 + 1.0) / v + m.s0 / (v * v);
+  return -(m.a0 + 1.0) * iv + m.s0 * (iv * iv);
 }
-
-struct BlockInfo {
-  bool th, b, v;
-};
 
 __device__ __forceinline__ BlockInfo block_info(const HlrModelDev& m, const int* idx, int P) {
   BlockInfo bi{false, false, false};
@@ -322,59 +394,70 @@ __device__ __forceinline__ BlockInfo block_info(const HlrModelDev& m, const int*
   return bi;
 }
 
-// Full conditional of the block at `par` and (optionally) its gradient in
-// block order into ws.blk_g.  Factor order as the generated ll_/grad_
-// functions (CgLike.hs:139-147, CgGrad.hs:165-376).  All threads return ll.
-__device__ double block_ll_grad(const HlrModelDev& m, const double* par, const int* idx, int P,
-                                Ws& ws, bool want_grad) {
-  const int D = m.D;
-  const BlockInfo bi = block_info(m, idx, P);
-  double data_ll = 0.0;
-  if (bi.th || bi.b) data_ll = data_pass(m, par, ws, want_grad) + m.ll_add;
-  const double b = m.has_b ? par[D] : 0.0, v = par[D + 1];
-  // prior terms of the coefficients, one per thread; thread 0 then adds
-  // them in the reference's (sequential) order
-  if (bi.th || bi.v) {
-    for (int k = threadIdx.x; k < D; k += blockDim.x) {
-      ws.pt_ll[k] = normal_ll(m, par[k], 0.0, v);
-      if (bi.v) ws.pt_dot[k] = normal_dotarg2(m, par[k], 0.0, v);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double ll = 0.0, gv = 0.0;
-    if (bi.v) { ll += vprior_ll(m, v); gv += vprior_dot(m, v); }
-    if (m.has_b && (bi.b || bi.v)) {
-      ll += normal_ll(m, b, 0.0, v);
-      if (bi.v) gv += normal_dotarg2(m, b, 0.0, v);
-    }
-    if (bi.th || bi.v) {
-      double s = 0.0;
-      for (int k = 0; k < D; ++k) {
-        s += ws.pt_ll[k];
-        if (bi.v) gv += ws.pt_dot[k];
+// Full conditional of the block at `par` (returned if wanted) and its
+// gradient, if wanted, in block order into ws.blk_g.  Factor order as the
+// generated ll_/grad_ functions (CgLike.hs:139-147, CgGrad.hs:165-376); the
+// coefficients' prior terms are added in a fixed tree.  The last warp forms the
+// prior - its logarithm and the shared 1 / v are the longest chains of binary64
+// operations of an evaluation - while the row threads pass over the data.
+// COLS: the data pass, 16 or 32 columns of the row-per-thread one, or 0 for the
+// wide one.
+template <int RES, int COLS>
+__device__ __forceinline__ double block_eval(const HlrModelDev& m, bool want_ll, bool want_grad, const double* par,
+                                          const BlockInfo bi, int P, Ws& ws) {
+  const int D = m.D, tid = threadIdx.x, lane = tid & 31;
+  const bool data = bi.th || bi.b;
+  const double v = par[D + 1];
+  if (data)
+    for (int k = tid; k < D; k += HLR_BLOCK) ws.th[k] = (float)par[k];
+  const float bias = m.has_b ? (float)par[D] : 0.0f;
+  const double iv = 1.0 / v;
+  __syncthreads();
+  if (tid >= HLR_THREADS && (want_ll || bi.v)) {
+    // the prior: lanes take the coefficients, lane 0 the variance and the bias
+    double pl = 0.0, pd = 0.0;
+    if (bi.th || bi.v)
+      for (int k = lane; k < D; k += 32) {
+        if (want_ll) pl += normal_ll(m, par[k], 0.0, v);
+        if (bi.v) pd += normal_dvar(m, par[k], v, iv);
       }
-      ll += s;
+    if (want_ll) pl = warp_sum_f64(pl);
+    if (bi.v) pd = warp_sum_f64(pd);
+    if (lane == 0) {
+      double ll = 0.0, gv = 0.0;
+      if (bi.v) {
+        if (want_ll) ll += vprior_ll(m, v);
+        gv += vprior_dot(m, v, iv);
+      }
+      if (m.has_b && (bi.b || bi.v)) {
+        if (want_ll) ll += normal_ll(m, par[D], 0.0, v);
+        if (bi.v) gv += normal_dvar(m, par[D], v, iv);
+      }
+      ws.bcast[0] = ll + pl;
+      ws.bcast[1] = gv + pd;
     }
-    ll += data_ll;
-    ws.bcast[0] = ll;
-    ws.bcast[1] = gv;
+  }
+  if (data) {
+    if constexpr (COLS > 0) data_rows_small<COLS, RES>(m, want_ll, want_grad, bias, ws);
+    else data_rows_wide<RES>(m, want_ll, want_grad, bias, ws);
   }
   __syncthreads();
-  const double ll = ws.bcast[0];
   if (want_grad) {
-    const double gv = ws.bcast[1];
-    for (int j = threadIdx.x; j < P; j += blockDim.x) {
-      const int i = idx[j];
-      double gj;
-      if (i < D) gj = -(par[i] - 0.0) / v + ws.g[i];                 // dotpt + data
-      else if (i == D) gj = m.has_b ? -(b - 0.0) / v + ws.g[D] : 0.0;
-      else gj = gv;
-      ws.blk_g[j] = gj;
+    for (int j = tid; j < P; j += HLR_BLOCK) {
+      const int i = ws.idx[j];
+      ws.blk_g[j] = i < D ? -par[i] * iv + ws.g[i] : i == D ? (m.has_b ? -par[D] * iv + ws.g[D] : 0.0) : ws.bcast[1];
     }
   }
+  const double ll = want_ll ? ws.bcast[0] + (data ? ws.red[33] + m.ll_add : 0.0) : 0.0;
   __syncthreads();
   return ll;
+}
+
+// The same as a call, for the moves that evaluate a few times an iteration.
+template <int RES, int COLS>
+__device__ __noinline__ double block_eval_call(const HlrModelDev& m, bool want_ll, bool want_grad, const double* par,
+                                               const BlockInfo bi, int P, Ws& ws) {
+  return block_eval<RES, COLS>(m, want_ll, want_grad, par, bi, P, ws);
 }
 
 __device__ __forceinline__ void set_block(double* par, const int* idx, int P, const double* q) {
@@ -382,12 +465,21 @@ __device__ __forceinline__ void set_block(double* par, const int* idx, int P, co
   __syncthreads();
 }
 
-// Sequential binary64 dot product in element order (thread 0), broadcast.
-__device__ double seq_dot(const double* a, const double* b, int P, Ws& ws) {
-  if (threadIdx.x == 0) {
+// The running component's block indices, next to the other state.
+__device__ __forceinline__ BlockInfo stage_block(const HlrModelDev& m, const int* idx, int P, Ws& ws) {
+  __syncthreads();
+  for (int j = threadIdx.x; j < P; j += blockDim.x) ws.idx[j] = idx[j];
+  __syncthreads();
+  return block_info(m, ws.idx, P);
+}
+
+// Binary64 dot product, by the first warp in a fixed tree, broadcast.
+__device__ double block_dot(const double* a, const double* b, int P, Ws& ws) {
+  if (threadIdx.x < 32) {
     double acc = 0.0;
-    for (int j = 0; j < P; ++j) acc += a[j] * b[j];
-    ws.bcast[2] = acc;
+    for (int j = threadIdx.x; j < P; j += 32) acc += a[j] * b[j];
+    acc = warp_sum_f64(acc);
+    if (threadIdx.x == 0) ws.bcast[2] = acc;
   }
   __syncthreads();
   const double r = ws.bcast[2];
@@ -396,16 +488,20 @@ __device__ double seq_dot(const double* a, const double* b, int P, Ws& ws) {
 }
 
 // ---- HMC: cbits/augur_mcmclib.h:343-424 -------------------------------------
-__device__ int hmc_transition(const HlrModelDev& m, const HlrComp& cp, const int* idx, Ws& ws,
-                              uint64_t seed, uint32_t iter, uint32_t chain, uint32_t ci,
-                              double* cache_ll, bool* cache_ok) {
+// `known`: ws.aux1 and *ll_known hold the block gradient and log density at
+// the current state (left there by the previous iteration of a schedule whose
+// only component this is); on return they hold the new state's.
+template <int RES, int COLS>
+__device__ int hmc_transition(const HlrModelDev& m, const HlrComp& cp, const BlockInfo bi, Ws& ws, uint64_t seed,
+                              uint32_t iter, uint32_t chain, uint32_t ci, bool known, double* ll_known) {
   const int P = cp.P;
   const int tid = threadIdx.x;
+  const int* idx = ws.idx;
   for (int j = tid; j < P; j += blockDim.x) {
     Stream s = make_stream(seed, chain * (uint32_t)P + j, iter, TAG_MOM | (ci << 8));
     ws.p0[j] = s.normal();
   }
-  if (tid == 0) {
+  if (tid == HLR_THREADS) {
     Stream h = make_stream(seed, chain, iter, TAG_HMC | (ci << 8));
     const double scale_eps = 0.8 + h.uniform() * (1.2 - 0.8);
     const double stepsize = scale_eps * cp.eps;
@@ -420,38 +516,47 @@ __device__ int hmc_transition(const HlrModelDev& m, const HlrComp& cp, const int
   const double step = ws.bcast[3];
   const int L = ws.ibcast[0];
   const double u = ws.bcast[4];
-  // gradient (and ll) at the current state
-  const double ll_curr = block_ll_grad(m, ws.par, idx, P, ws, true);
-  for (int j = tid; j < P; j += blockDim.x) {
-    ws.ps[j] = __dadd_rn(ws.p0[j], __dmul_rn(step / 2.0, ws.blk_g[j]));
-    ws.q[j] = ws.par[idx[j]];
-  }
-  __syncthreads();
-  double ll_prop = 0.0;
-  for (int l = 0; l < L; ++l) {
-    for (int j = tid; j < P; j += blockDim.x) ws.q[j] = __dadd_rn(ws.q[j], __dmul_rn(step, ws.ps[j]));
-    __syncthreads();
-    set_block(ws.prop, idx, P, ws.q);
-    if (l != L - 1) {
-      block_ll_grad(m, ws.prop, idx, P, ws, true);
-      for (int j = tid; j < P; j += blockDim.x) ws.ps[j] = __dadd_rn(ws.ps[j], __dmul_rn(step, ws.blk_g[j]));
+  for (int j = tid; j < P; j += blockDim.x) ws.q[j] = ws.par[idx[j]];
+  // l = 0: gradient and log density at the current state, unless known; then
+  // L positions, the log density needed at the last
+  double ll_curr = *ll_known, ll_prop = 0.0;
+  for (int l = known ? 1 : 0;; ++l) {
+    if (l > 0) {
+      // each thread moves its own coordinates
+      for (int j = tid; j < P; j += blockDim.x) {
+        const double* g = l == 1 ? ws.aux1 : ws.blk_g;
+        const double p = __dadd_rn(l == 1 ? ws.p0[j] : ws.ps[j], __dmul_rn(l == 1 ? step / 2.0 : step, g[j]));
+        const double q = __dadd_rn(ws.q[j], __dmul_rn(step, p));
+        ws.ps[j] = p;
+        ws.q[j] = q;
+        ws.prop[idx[j]] = q;
+      }
       __syncthreads();
     }
+    const double v = block_eval<RES, COLS>(m, l == 0 || l == L, true, l == 0 ? ws.par : ws.prop, bi, P, ws);
+    if (l == 0) {
+      ll_curr = v;
+      for (int j = tid; j < P; j += blockDim.x) ws.aux1[j] = ws.blk_g[j];
+    } else if (l == L) {
+      ll_prop = v;
+      break;
+    }
   }
-  ll_prop = block_ll_grad(m, ws.prop, idx, P, ws, true);
   for (int j = tid; j < P; j += blockDim.x) ws.ps[j] = __dadd_rn(ws.ps[j], __dmul_rn(step / 2.0, ws.blk_g[j]));
   __syncthreads();
-  const double k0 = seq_dot(ws.p0, ws.p0, P, ws);
-  const double k1 = seq_dot(ws.ps, ws.ps, P, ws);
+  const double k0 = block_dot(ws.p0, ws.p0, P, ws);
+  const double k1 = block_dot(ws.ps, ws.ps, P, ws);
   const double auxll = k0 / 2.0 - k1 / 2.0;
   const double dlog = ll_prop - ll_curr + auxll;   // minus the energy error
   const int acc = log(u) < dlog;
   // divergent: the energy error passed the bound, or is not finite
   const int div = !(dlog > -AB_DIVERGENCE_DH);
-  if (acc)
+  if (acc) {
     for (int i = tid; i < m.D + 2; i += blockDim.x) ws.par[i] = ws.prop[i];
+    for (int j = tid; j < P; j += blockDim.x) ws.aux1[j] = ws.blk_g[j];
+  }
+  *ll_known = acc ? ll_prop : ll_curr;
   __syncthreads();
-  (void)cache_ll; (void)cache_ok;
   return acc | (div << 1);
 }
 
@@ -467,18 +572,26 @@ __device__ int nuts_update_s(int s, const double* tp, const double* mp, const do
   if (s == 1) {
     for (int j = threadIdx.x; j < P; j += blockDim.x) ws.blk_g[j] = __dadd_rn(tp[j], __dmul_rn(-1.0, tm[j]));
     __syncthreads();
-    const double d1 = seq_dot(ws.blk_g, mp, P, ws);
-    const double d2 = seq_dot(ws.blk_g, mm, P, ws);
+    const double d1 = block_dot(ws.blk_g, mp, P, ws);
+    const double d2 = block_dot(ws.blk_g, mm, P, ws);
     res = (d1 >= 0.0 && d2 >= 0.0) ? 1 : 0;
   }
   return res;
 }
 
-__device__ int nuts_transition(const HlrModelDev& m, const HlrComp& cp, const int* idx, Ws& ws,
+// The gradient at a leaf's start is the one found at the previous leaf's end
+// (the reference evaluates it again): it is kept for the walk (ws.blk_g between
+// leaves, wg) and for both frontiers (gm, gp), so a leaf is one evaluation.
+template <int RES, int COLS>
+__device__ int nuts_transition(const HlrModelDev& m, const HlrComp& cp, const BlockInfo bi, Ws& ws,
                                double* stk, uint64_t seed, uint32_t iter, uint32_t chain, uint32_t ci,
                                int* depth_out, int* leaves_out, int* error_out, int* div_out) {
   const int P = cp.P;
   const int tid = threadIdx.x;
+  const int* idx = ws.idx;
+  double* gm = ws.gfr;                           // gradient at theta_minus
+  double* gp = ws.gfr + P;                       // gradient at theta_plus
+  double* wg = ws.gfr + 2 * P;                   // gradient at the walk's position
   double* tp_stk = stk;                          // theta_prop stack
   double* ts_stk = stk + (size_t)HLR_STK * P;    // theta stack
   double* ms_stk = stk + (size_t)2 * HLR_STK * P;  // mom stack
@@ -501,8 +614,9 @@ __device__ int nuts_transition(const HlrModelDev& m, const HlrComp& cp, const in
   for (int i = tid; i < m.D + 2; i += blockDim.x) ws.prop[i] = ws.par[i];
   __syncthreads();
   // h substream position counter lives in ibcast[1] (read/advanced by thread 0)
-  const double ll0 = block_ll_grad(m, ws.par, idx, P, ws, false);
-  const double mm2 = seq_dot(mm, mm, P, ws);
+  const double ll0 = block_eval<RES, COLS>(m, true, true, ws.par, bi, P, ws);
+  for (int j = tid; j < P; j += blockDim.x) gm[j] = gp[j] = ws.blk_g[j];
+  const double mm2 = block_dot(mm, mm, P, ws);
   if (tid == 0) {
     Stream h = make_stream(seed, chain, iter, TAG_NUTS | (ci << 8));
     const double e = -1.0 * log(h.uniform());
@@ -559,7 +673,10 @@ __device__ int nuts_transition(const HlrModelDev& m, const HlrComp& cp, const in
     const int dir = draw_u() < 0.5 ? 0 : 1;   // 0 = MINUS
     stepsize = dir == 0 ? -cp.eps : cp.eps;
     double* mom = dir == 0 ? mm : mp;
-    for (int j = tid; j < P; j += blockDim.x) thprop[j] = dir == 0 ? thm[j] : thp[j];
+    for (int j = tid; j < P; j += blockDim.x) {
+      thprop[j] = dir == 0 ? thm[j] : thp[j];
+      wg[j] = dir == 0 ? gm[j] : gp[j];
+    }
     __syncthreads();
     // ---- build_tree(thprop, mom, jd, dir) as an explicit post-order walk
     int sp = 0;
@@ -568,21 +685,22 @@ __device__ int nuts_transition(const HlrModelDev& m, const HlrComp& cp, const in
     while (sp >= 0) {
       NutsFrame& F = fr[sp];
       if (F.j == 0) {
-        // leaf: leapfrog1 (:305-325) - gradient, half kick, drift, gradient, half kick
-        set_block(ws.prop, idx, P, thprop);
-        block_ll_grad(m, ws.prop, idx, P, ws, true);
+        // leaf: leapfrog1 (:305-325) - half kick, drift, gradient, half kick
         for (int j = tid; j < P; j += blockDim.x) {
-          mom[j] = __dadd_rn(mom[j], __dmul_rn(stepsize / 2.0, ws.blk_g[j]));
+          mom[j] = __dadd_rn(mom[j], __dmul_rn(stepsize / 2.0, wg[j]));
           thprop[j] = __dadd_rn(thprop[j], __dmul_rn(stepsize, mom[j]));
+          ws.prop[idx[j]] = thprop[j];
         }
         __syncthreads();
-        set_block(ws.prop, idx, P, thprop);
-        const double llp = block_ll_grad(m, ws.prop, idx, P, ws, true);
-        for (int j = tid; j < P; j += blockDim.x) mom[j] = __dadd_rn(mom[j], __dmul_rn(stepsize / 2.0, ws.blk_g[j]));
+        const double llp = block_eval<RES, COLS>(m, true, true, ws.prop, bi, P, ws);
+        for (int j = tid; j < P; j += blockDim.x) {
+          wg[j] = ws.blk_g[j];
+          mom[j] = __dadd_rn(mom[j], __dmul_rn(stepsize / 2.0, wg[j]));
+        }
         __syncthreads();
         if (tid == 0) ws.ibcast[5] += 1;
         push(tp_stk, 2, thprop);
-        const double ll = llp - 0.5 * seq_dot(mom, mom, P, ws);
+        const double ll = llp - 0.5 * block_dot(mom, mom, P, ws);
         rn = logu <= ll ? 1 : 0;
         rs = logu < 1000.0 + ll ? 1 : 0;
         // a leaf outside the slice by the reference's deltaMax (1000) ends
@@ -630,8 +748,10 @@ __device__ int nuts_transition(const HlrModelDev& m, const HlrComp& cp, const in
       --sp;
     }
     // ---- outer loop body (:744-774)
-    if (dir == 0) for (int j = tid; j < P; j += blockDim.x) thm[j] = thprop[j];
-    else for (int j = tid; j < P; j += blockDim.x) thp[j] = thprop[j];
+    for (int j = tid; j < P; j += blockDim.x) {
+      (dir == 0 ? thm : thp)[j] = thprop[j];
+      (dir == 0 ? gm : gp)[j] = wg[j];
+    }
     __syncthreads();
     const int pp = pop(2);
     if (rs == 1) {
@@ -670,10 +790,12 @@ __device__ int nuts_transition(const HlrModelDev& m, const HlrComp& cp, const in
 // at the new point and, outside the slice, a reflection of p0 off the block
 // gradient there (p0 += -2 (p0.g)/(g.g) g, sequential dot products).  The
 // move is kept only if the last point is inside the slice.
-__device__ int rslice_transition(const HlrModelDev& m, const HlrComp& cp, const int* idx, Ws& ws,
+template <int RES, int COLS>
+__device__ int rslice_transition(const HlrModelDev& m, const HlrComp& cp, const BlockInfo bi, Ws& ws,
                                  uint64_t seed, uint32_t iter, uint32_t chain, uint32_t ci, int* refl_out) {
   const int P = cp.P;
   const int tid = threadIdx.x;
+  const int* idx = ws.idx;
   for (int j = tid; j < P; j += blockDim.x) {
     Stream s = make_stream(seed, chain * (uint32_t)P + j, iter, TAG_MOM | (ci << 8));
     ws.p0[j] = s.normal();
@@ -689,7 +811,7 @@ __device__ int rslice_transition(const HlrModelDev& m, const HlrComp& cp, const 
   const double expo = ws.bcast[3];
   const int L = ws.ibcast[0];
   const double step = cp.eps;
-  const double z = block_ll_grad(m, ws.par, idx, P, ws, false) - expo;
+  const double z = block_eval_call<RES, COLS>(m, true, false, ws.par, bi, P, ws) - expo;
   for (int j = tid; j < P; j += blockDim.x) ws.q[j] = ws.par[idx[j]];
   __syncthreads();
   bool cond = false;
@@ -698,11 +820,11 @@ __device__ int rslice_transition(const HlrModelDev& m, const HlrComp& cp, const 
     for (int j = tid; j < P; j += blockDim.x) ws.q[j] = __dadd_rn(ws.q[j], __dmul_rn(step, ws.p0[j]));
     __syncthreads();
     set_block(ws.prop, idx, P, ws.q);
-    cond = block_ll_grad(m, ws.prop, idx, P, ws, false) < z;    // same value on every thread
+    cond = block_eval_call<RES, COLS>(m, true, false, ws.prop, bi, P, ws) < z;    // same value on every thread
     if (cond) {
-      block_ll_grad(m, ws.prop, idx, P, ws, true);
-      const double a1 = seq_dot(ws.p0, ws.blk_g, P, ws);
-      const double a2 = seq_dot(ws.blk_g, ws.blk_g, P, ws);
+      block_eval_call<RES, COLS>(m, false, true, ws.prop, bi, P, ws);
+      const double a1 = block_dot(ws.p0, ws.blk_g, P, ws);
+      const double a2 = block_dot(ws.blk_g, ws.blk_g, P, ws);
       const double sc = __dmul_rn(-2.0, a1 / a2);
       for (int j = tid; j < P; j += blockDim.x) ws.p0[j] = __dadd_rn(ws.p0[j], __dmul_rn(sc, ws.blk_g[j]));
       __syncthreads();
@@ -717,9 +839,10 @@ __device__ int rslice_transition(const HlrModelDev& m, const HlrComp& cp, const 
 }
 
 // ---- MWG on one scalar of par: augur_mcmclib.h:89-105,178-193 ---------------
-__device__ int mwg_transition(const HlrModelDev& m, const HlrComp& cp, const int* idx, Ws& ws,
+template <int RES, int COLS>
+__device__ int mwg_transition(const HlrModelDev& m, const HlrComp& cp, const BlockInfo bi, Ws& ws,
                               uint64_t seed, uint32_t iter, uint32_t chain, uint32_t ci) {
-  const int which = idx[0];
+  const int which = ws.idx[0];
   if (threadIdx.x == 0) {
     Stream s = make_stream(seed, chain, iter, TAG_MWG | (ci << 8));
     const double x = ws.par[which];
@@ -732,71 +855,112 @@ __device__ int mwg_transition(const HlrModelDev& m, const HlrComp& cp, const int
   __syncthreads();
   if (threadIdx.x == 0) ws.prop[which] = ws.bcast[3];
   __syncthreads();
-  const double lc = block_ll_grad(m, ws.par, idx, 1, ws, false);
-  const double lp = block_ll_grad(m, ws.prop, idx, 1, ws, false);
+  const double lc = block_eval_call<RES, COLS>(m, true, false, ws.par, bi, 1, ws);
+  const double lp = block_eval_call<RES, COLS>(m, true, false, ws.prop, bi, 1, ws);
   const int acc = log(ws.bcast[4]) < lp - lc + ws.bcast[5];
   if (acc && threadIdx.x == 0) ws.par[which] = ws.prop[which];
   __syncthreads();
   return acc;
 }
 
-__device__ Ws carve(void* base, int D) {
+// Shared memory of a chain CTA: the state vectors, the NUTS gradients and
+// stacks, then X in its own type (rows of an odd number of 4-byte words) and
+// the labels.
+struct HlrLayout {
+  int res;         // X_GLOBAL, X_F32 or X_BF16
+  int xpitch;      // elements of a row of the copy
+  int stk;         // NUTS stacks in shared memory (else the caller's scratch)
+  int nuts;        // a NUTS component is present
+};
+
+static __host__ __device__ inline size_t hlr_layout_bytes(int N, int D, const HlrLayout& l) {
+  const size_t V = (size_t)D + 2;
+  size_t d = 11 * V + HLR_THREADS + 34 + 8 + 8 + (V + 1) / 2 + 1 + ((size_t)D + 1) / 2 + 1 + HLR_CHUNK;
+  if (l.nuts) d += 3 * V;
+  if (l.stk) d += 3 * (size_t)HLR_STK * V;
+  return sizeof(double) * d +
+         (l.res ? sizeof(int) * (size_t)N + (l.res == X_F32 ? 4 : 2) * (size_t)N * l.xpitch : 0);
+}
+
+__device__ Ws carve(void* base, int N, int D, const HlrLayout& l, double*& stk) {
   Ws w;
   double* d = reinterpret_cast<double*>(base);
   const int V = D + 2;
   w.par = d; d += V; w.prop = d; d += V; w.g = d; d += V; w.blk_g = d; d += V;
   w.p0 = d; d += V; w.ps = d; d += V; w.q = d; d += V; w.aux1 = d; d += V; w.aux2 = d; d += V;
   w.aux3 = d; d += V; w.aux4 = d; d += V;
-  w.pt_ll = d; d += V; w.pt_dot = d; d += V;
   w.gpart = d; d += HLR_THREADS;
   w.red = d; d += 34;
   w.bcast = d; d += 8;
   w.ibcast = reinterpret_cast<int*>(d); d += 8;
+  w.idx = reinterpret_cast<int*>(d); d += (V + 1) / 2 + 1;
   w.th = reinterpret_cast<float*>(d); d += (D + 1) / 2 + 1;
   w.r = reinterpret_cast<float*>(d);
+  w.l = w.r + HLR_CHUNK;
+  d += HLR_CHUNK;
+  w.gfr = d; if (l.nuts) d += 3 * V;
+  stk = d; if (l.stk) d += 3 * (size_t)HLR_STK * V;
+  w.lab = reinterpret_cast<int*>(d);
+  w.xs = l.res ? w.lab + N : nullptr;
+  w.xpitch = l.xpitch;
   return w;
-}
-
-size_t hlr_smem_bytes(int D) {
-  const int V = D + 2;
-  return sizeof(double) * (13 * (size_t)V + HLR_THREADS + 34 + 8 + 8 + (D + 1) / 2 + 1) +
-         sizeof(float) * HLR_CHUNK;
 }
 
 // One CTA per chain: n_iter iterations of the schedule `comps`.
 // stats[c][ci][5] = {accepts, sum depth, sum leaves, errors, divergent iterations}.
-__global__ void __launch_bounds__(HLR_THREADS)
-hlr_chain_kernel(HlrModelDev m, const HlrComp* __restrict__ comps, int n_comps,
+// Bound: the chain of one evaluation - barriers, the compensated sums of a
+// thread's rows, binary64 reductions - at 11 evaluations an HMC iteration.
+// Measured, ten HMC iterations at N = 1000, D = 10: 870 -> 377 us; two NUTS
+// iterations of depth 5 for 48 chains at N = 2003, D = 41 (bf16): 10.5 -> 1.04 ms,
+// where every evaluation walked X a warp per row and every leaf took two.
+template <int RES, int COLS>
+__global__ void __launch_bounds__(HLR_BLOCK, 1)
+hlr_chain_kernel(const __grid_constant__ HlrModelDev m, HlrLayout l, const HlrComp* __restrict__ comps, int n_comps,
                  const int* __restrict__ idx_all, double* __restrict__ pars, int n_iter,
                  uint32_t iter0, uint64_t seed, double* __restrict__ stats,
                  double* __restrict__ nuts_stk, int stk_P) {
-  extern __shared__ double smem_d[];
-  Ws ws = carve(smem_d, m.D);
+  extern __shared__ __align__(16) double smem_d[];
+  double* stk;
+  Ws ws = carve(smem_d, m.N, m.D, l, stk);
   const int c = blockIdx.x;
+  if (!l.stk) stk = nuts_stk + (size_t)c * 3 * HLR_STK * stk_P;
+  if (RES) {
+    for (int i = threadIdx.x >> 5; i < m.N; i += HLR_BLOCK / 32)
+      for (int k = threadIdx.x & 31; k < m.D; k += 32) {
+        const size_t at = (size_t)i * m.ldx + k;
+        if (RES == X_F32) static_cast<float*>(ws.xs)[i * l.xpitch + k] = static_cast<const float*>(m.X)[at];
+        else static_cast<__nv_bfloat16*>(ws.xs)[i * l.xpitch + k] = static_cast<const __nv_bfloat16*>(m.X)[at];
+      }
+    for (int i = threadIdx.x; i < m.N; i += HLR_BLOCK) ws.lab[i] = load_label(m, i);
+  }
   double* par_g = pars + (size_t)c * (m.D + 2);
   for (int i = threadIdx.x; i < m.D + 2; i += blockDim.x) ws.par[i] = par_g[i];
   __syncthreads();
+  const bool tell = threadIdx.x == 0;
+  BlockInfo bi{false, false, false};
+  double ll_known = 0.0;
   for (int it = 0; it < n_iter; ++it) {
     const uint32_t iter = iter0 + (uint32_t)it;
     for (int ci = 0; ci < n_comps; ++ci) {
       const HlrComp cp = comps[ci];
-      const int* idx = idx_all + cp.idx_off;
+      if (n_comps > 1 || it == 0) bi = stage_block(m, idx_all + cp.idx_off, cp.P, ws);
       double* st = stats + ((size_t)c * n_comps + ci) * AB_HLR_STATS;
       if (cp.kind == COMP_HMC) {
-        const int a = hmc_transition(m, cp, idx, ws, seed, iter, (uint32_t)c, (uint32_t)ci, nullptr, nullptr);
-        if (threadIdx.x == 0) { st[0] += a & 1; st[4] += a >> 1; }
+        const int a = hmc_transition<RES, COLS>(m, cp, bi, ws, seed, iter, (uint32_t)c, (uint32_t)ci,
+                                          n_comps == 1 && it > 0, &ll_known);
+        if (tell) { st[0] += a & 1; st[4] += a >> 1; }
       } else if (cp.kind == COMP_NUTS) {
         __shared__ int sh_out[4];
-        nuts_transition(m, cp, idx, ws, nuts_stk + (size_t)c * 3 * HLR_STK * stk_P, seed, iter,
-                        (uint32_t)c, (uint32_t)ci, &sh_out[0], &sh_out[1], &sh_out[2], &sh_out[3]);
-        if (threadIdx.x == 0) { st[1] += sh_out[0]; st[2] += sh_out[1]; st[3] += sh_out[2]; st[4] += sh_out[3]; }
+        nuts_transition<RES, COLS>(m, cp, bi, ws, stk, seed, iter, (uint32_t)c, (uint32_t)ci, &sh_out[0], &sh_out[1],
+                             &sh_out[2], &sh_out[3]);
+        if (tell) { st[1] += sh_out[0]; st[2] += sh_out[1]; st[3] += sh_out[2]; st[4] += sh_out[3]; }
       } else if (cp.kind == COMP_RSLICE) {
         int refl = 0;
-        const int a = rslice_transition(m, cp, idx, ws, seed, iter, (uint32_t)c, (uint32_t)ci, &refl);
-        if (threadIdx.x == 0) { st[0] += a; st[2] += refl; }
+        const int a = rslice_transition<RES, COLS>(m, cp, bi, ws, seed, iter, (uint32_t)c, (uint32_t)ci, &refl);
+        if (tell) { st[0] += a; st[2] += refl; }
       } else {
-        const int a = mwg_transition(m, cp, idx, ws, seed, iter, (uint32_t)c, (uint32_t)ci);
-        if (threadIdx.x == 0) st[0] += a;
+        const int a = mwg_transition<RES, COLS>(m, cp, bi, ws, seed, iter, (uint32_t)c, (uint32_t)ci);
+        if (tell) st[0] += a;
       }
       __syncthreads();
     }
@@ -807,16 +971,18 @@ hlr_chain_kernel(HlrModelDev m, const HlrComp* __restrict__ comps, int n_comps,
 // Log-density and gradient of a block for C parameter vectors (one CTA per
 // vector): the data pass and priors used by the transitions, exposed for
 // parity checks and for callers that drive their own samplers.
-__global__ void __launch_bounds__(HLR_THREADS)
-hlr_ll_grad_kernel(HlrModelDev m, const int* __restrict__ idx, int P, const double* __restrict__ pars,
+template <int COLS>
+__global__ void __launch_bounds__(HLR_BLOCK, 1)
+hlr_ll_grad_kernel(const __grid_constant__ HlrModelDev m, HlrLayout l, const int* __restrict__ idx, int P, const double* __restrict__ pars,
                    double* __restrict__ ll, double* __restrict__ grad) {
-  extern __shared__ double smem_d[];
-  Ws ws = carve(smem_d, m.D);
+  extern __shared__ __align__(16) double smem_d[];
+  double* stk;
+  Ws ws = carve(smem_d, m.N, m.D, l, stk);
   const int c = blockIdx.x;
   for (int i = threadIdx.x; i < m.D + 2; i += blockDim.x) ws.par[i] = pars[(size_t)c * (m.D + 2) + i];
-  __syncthreads();
-  const double l = block_ll_grad(m, ws.par, idx, P, ws, grad != nullptr);
-  if (threadIdx.x == 0) ll[c] = l;
+  const BlockInfo bi = stage_block(m, idx, P, ws);
+  const double v = block_eval<X_GLOBAL, COLS>(m, true, grad != nullptr, ws.par, bi, P, ws);
+  if (threadIdx.x == 0) ll[c] = v;
   if (grad != nullptr)
     for (int j = threadIdx.x; j < P; j += blockDim.x) grad[(size_t)c * P + j] = ws.blk_g[j];
 }
@@ -842,7 +1008,29 @@ static int make_model(HlrModelDev& m, const ab_hlr_model* d) {
   // per-row Normal normaliser: the reference's -log(var) (compat) or -log(2 pi var) / 2
   m.ll_add = d->lik != AB_LIK_NORMAL ? 0.0
              : (double)d->N * (m.compat ? -log(d->obs_var) : -0.5 * log(2.0 * M_PI * d->obs_var));
+  m.vp_const = m.vprior == 0 ? log(m.lam) : m.a0 * log(m.s0) - lgamma(m.a0);
   return AB_OK;
+}
+
+// What a chain's CTA keeps in shared memory: X and the labels, and the NUTS
+// stacks, where they fit - 224 KB with an SM to itself, 112 KB when there are
+// more chains than SMs and two share one.  Every evaluation then reads X from
+// there instead of walking it through the caches.
+static HlrLayout choose_layout(const HlrModelDev& m, int C, bool nuts) {
+  const size_t room = (C > 148 ? 112 : 224) * 1024;
+  HlrLayout l{X_GLOBAL, 0, nuts, nuts};
+  if (hlr_layout_bytes(m.N, m.D, l) > room) l.stk = 0;
+  HlrLayout k = l;
+  k.res = m.x_bf16 ? X_BF16 : X_F32;
+  k.xpitch = m.x_bf16 ? 2 * (((m.D + 1) / 2) | 1) : (m.D | 1);
+  return hlr_layout_bytes(m.N, m.D, k) <= room ? k : l;
+}
+
+template <int COLS>
+static auto chain_kernel(int res) {
+  return res == X_F32    ? hlr_chain_kernel<X_F32, COLS>
+         : res == X_BF16 ? hlr_chain_kernel<X_BF16, COLS>
+                         : hlr_chain_kernel<X_GLOBAL, COLS>;
 }
 
 static int check_idx_host(const int* idx_host, int P, int D) {
@@ -868,9 +1056,13 @@ extern "C" int ab_hlr_ll_grad(const ab_hlr_model* model, const int* idx_dev, con
   AB_REQUIRE(idx_dev && idx_host && pars && ll, AB_ERR_ARG, "ab_hlr_ll_grad: null pointer");
   rc = check_idx_host(idx_host, P, m.D);
   if (rc) return rc;
-  const size_t smem = hlr_smem_bytes(m.D);
-  AB_CUDA(cudaFuncSetAttribute(hlr_ll_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  hlr_ll_grad_kernel<<<C, HLR_THREADS, smem, as_stream(stream)>>>(m, idx_dev, P, pars, ll, grad);
+  const HlrLayout l{X_GLOBAL, 0, 0, 0};
+  const size_t smem = hlr_layout_bytes(m.N, m.D, l);
+  const auto kernel = m.D + 2 <= 16           ? hlr_ll_grad_kernel<16>
+                      : m.D + 2 <= SMALL_COLS ? hlr_ll_grad_kernel<SMALL_COLS>
+                                              : hlr_ll_grad_kernel<0>;
+  AB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<C, HLR_BLOCK, smem, as_stream(stream)>>>(m, l, idx_dev, P, pars, ll, grad);
   AB_LAUNCH_CHECK("hlr_ll_grad_kernel");
   return AB_OK;
 }
@@ -905,12 +1097,15 @@ extern "C" int ab_hlr_run_chains(const ab_hlr_model* model, const ab_hlr_comp* c
   }
   AB_REQUIRE(!has_nuts || scratch, AB_ERR_ARG, "ab_hlr_run_chains: NUTS needs scratch");
   static_assert(sizeof(ab_hlr_comp) == sizeof(HlrComp), "component layout");
-  const size_t smem = hlr_smem_bytes(m.D);
-  AB_REQUIRE(smem <= 200 * 1024, AB_ERR_ARG, "hlr: D too large for the per-chain engine");
-  AB_CUDA(cudaFuncSetAttribute(hlr_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  hlr_chain_kernel<<<C, HLR_THREADS, smem, as_stream(stream)>>>(
-      m, reinterpret_cast<const HlrComp*>(comps_dev), n_comps, idx_dev, pars, n_iter, iter0, seed, stats,
-      reinterpret_cast<double*>(scratch), m.D + 2);
+  const HlrLayout l = choose_layout(m, C, has_nuts);
+  const size_t smem = hlr_layout_bytes(m.N, m.D, l);
+  AB_REQUIRE(smem <= 224 * 1024, AB_ERR_ARG, "hlr: D too large for the per-chain engine");
+  const auto kernel = m.D + 2 <= 16 ? chain_kernel<16>(l.res) : m.D + 2 <= SMALL_COLS ? chain_kernel<SMALL_COLS>(l.res)
+                                                                                       : chain_kernel<0>(l.res);
+  AB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<C, HLR_BLOCK, smem, as_stream(stream)>>>(m, l, reinterpret_cast<const HlrComp*>(comps_dev), n_comps, idx_dev,
+                                                    pars, n_iter, iter0, seed, stats,
+                                                    reinterpret_cast<double*>(scratch), m.D + 2);
   AB_LAUNCH_CHECK("hlr_chain_kernel");
   return AB_OK;
 }

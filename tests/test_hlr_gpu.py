@@ -95,6 +95,39 @@ def test_hmc_transition_matches_oracle(orc, has_b, vprior, block):
     assert agree >= 7
 
 
+@pytest.mark.parametrize("N,D,xd,C,kind", [
+    (7, 14, "f32", 1, "HMC"), (257, 15, "bf16", 2, "NUTS"), (600, 30, "f32", 1, "NUTS"), (1000, 31, "bf16", 1, "HMC"),
+    (1025, 41, "bf16", 2, "NUTS"), (1023, 33, "f32", 150, "HMC"), (2049, 100, "f32", 1, "HMC"), (900, 300, "bf16", 1, "HMC")])
+def test_chain_paths_match_oracle(orc, N, D, xd, C, kind):
+    """The chain engine's ways through the data (16 and 32 columns, wide; X in
+    shared memory as f32 or bf16, or too large for it; one or two chains per
+    SM; remainders of a chunk of rows): a transition of the first and the last
+    chain equals the oracle's."""
+    X, y, beta, s2, om, gd = make(N, D, N + D, True, "exponential", True, xd)
+    block = ["v", "b", "theta"]
+    idx = H.block_indices(block, D)
+    par = np.concatenate([0.5 * beta, [0.1], [1.0]])
+    eps = 0.3 / np.sqrt(N + 10.0)
+    sched = [{"kind": kind, "block": block, "eps": eps, "simlen": 5 * eps, "max_depth": 3}]
+    ch = H.HlrChains(gd, sched, C=C, init=par, seed=17)
+    ch.run(2)                                    # the second iteration starts from the first's gradient
+    got, st = ch.state(), ch.stats.cpu().numpy()
+    one = H.HlrChains(gd, sched, C=C, init=par, seed=17)
+    one.run(1)
+    one.run(1)
+    np.testing.assert_array_equal(got, one.state())
+    for c in {0, C - 1}:
+        p = par.copy()
+        tally = 0
+        for it in range(2):
+            if kind == "HMC":
+                tally += O.hlr_hmc(orc, om, p, idx, 5 * eps, eps, 17, it, chain=c)[0]
+            else:
+                tally += O.hlr_nuts(orc, om, p, idx, eps, 17, it, max_depth=3, chain=c)[0]
+        assert int(st[c, 0, 0 if kind == "HMC" else 1]) == tally
+        np.testing.assert_allclose(got[c], p, rtol=1e-4, atol=1e-5)
+
+
 def test_hmc_many_chains_distinct_streams(orc):
     X, y, beta, s2, om, gd = make(400, 5, 6, False, "invgamma", True)
     D = 5
