@@ -19,7 +19,7 @@
 //                     phi[k]   ~ Dir(beta + cnt_kw[k])       (reads, then
 //                     clears cnt_kw); one draw per thread, then a parallel
 //                     normalisation pass
-//   lda_zq_kernel     z ~ p(z | theta, phi), and the counts of the new z
+//   lda_zf_kernel     z ~ p(z | theta, phi), and the counts of the new z
 //                     (cnt_dk rows written whole, cnt_kw incremented)
 // The count statistics of the reference (conj_stat_*, rebuilt from zero each
 // step, CgKern.hs:103-107) are a function of z alone, so they are produced
@@ -827,6 +827,201 @@ int launch_lda_zf(int D, int K, int V, int Kp, const int* doc_off, const int* w,
   return fail(AB_ERR_ARG, "lda: the binary32-screened z kernel takes K <= 64 (K=%d)", K);
 }
 
+// ---------------------------------------------------------------------------
+// The z draw screened in binary32 for 64 < K <= 256.  One CTA per document,
+// of 2 to 8 warps (lda_zr_warps).  G lanes share a token, lane j of them holding UQ quads (float4) of
+// topics, [4 UQ j, 4 UQ (j + 1)): its thetas stay in registers for the document,
+// and a token's row of phi32 is read straight into registers, a step of 32 / G
+// tokens ahead.  A lane forms its
+// running sums by fused multiply-adds; a butterfly over the G lanes gives the
+// sums before each lane and the norm.  The uniforms are drawn a lane per token.
+//
+// Why a decided draw is still the reference's: every theta_k, phi_k is
+// rounded once to binary32 (relative error <= u = 2^-24), each multiply-add
+// once more, and a running sum of k nonnegative terms grouped by lanes adds at
+// most (k + 1) u relative error, so each screened running sum c_k = off + s_k
+// and the norm are within (K + 8) u of the exact sums C_k and N; u * norm adds
+// 3 u, the two bounds T = u norm (1 -+ m) - off against which s_k is compared
+// 2 u more.  Gradual underflow adds at most 2^-149 per term, below 2^-60 u of a
+// norm >= 2^-60.  The reference's running quotient sums acc_i are within 2^-50
+// of C_i / N.  So with m = (2K + 32) u: if s_j < u norm (1 - m) - off for all
+// topics before k the reference does not stop before k, and if also s_k > u norm
+// (1 + m) - off it stops at k - the draw equals the reference's.  A u within the
+// margin of a boundary (about 2 (2K + 32) u of the draws, 1e-5 at K = 50), or a
+// norm outside [2^-60, FLT_MAX], runs the reference's binary64 loop on the
+// binary64 theta and phi rows (lda_reference_draw).
+// Counts of the new z as lda_zq_kernel.
+// Measured at K = 130, V = 5003, 1.9e5 tokens in 611 documents: 90 -> 70 us, the
+// whole sweep 126 -> 105; bound by the
+// rows' round trips at 16 warps per SM.  At K = 50 this form took 39-51 us
+// against 36 for the staged one, which K <= 64 keeps: short rows leave the
+// staged kernel twice the warps.  With a whole warp per token (K = 500, 100
+// documents) the sweep took 287 us against 220 of lda_z_kernel, hence K <= 256.
+// ---------------------------------------------------------------------------
+constexpr int LDA_ZR_MAX_THREADS = 256;
+constexpr int LDA_ZR_MAX_K = 256;
+
+// Warps per document: 16 warps per SM over all documents, at most 8, so that few
+// documents do not leave the SMs idle and many short ones do not wait for idle
+// warps.
+static inline int lda_zr_warps(int D) {
+  int nw = 2;
+  while (nw < LDA_ZR_MAX_THREADS / 32 && (long long)D * nw < 148 * 16) nw *= 2;
+  return nw;
+}
+
+// Lanes per token and quads per lane for K topics.
+static inline int lda_zr_lanes(int K) { return K <= 128 ? 8 : 16; }
+static inline int lda_zr_quads(int K) {
+  const int quads = (K + 3) / 4, G = lda_zr_lanes(K);
+  return (quads + G - 1) / G;
+}
+
+template <int G, int UQ>
+__global__ void __launch_bounds__(LDA_ZR_MAX_THREADS, 2)
+lda_zr_kernel(int D, int K, int V, int Kp, const int* __restrict__ doc_off,
+              const int* __restrict__ w, const double* __restrict__ theta,
+              const double* __restrict__ phiT, const float4* __restrict__ phi32, int row_quads,
+              int* __restrict__ z, int* __restrict__ cnt_dk, int* __restrict__ cnt_kw, uint64_t seed,
+              uint32_t* iter_dev, uint32_t iter_fixed, uint32_t* done_ctr) {
+  constexpr int PER = 32 / G;              // tokens of a step
+  const int NW = blockDim.x / 32;
+  extern __shared__ int hist[];            // [K]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j = lane & (G - 1), grp = lane / G;
+  const int d = blockIdx.x;
+  const uint32_t iter = read_iter(iter_dev, iter_fixed);
+  for (int k = threadIdx.x; k < K; k += blockDim.x) hist[k] = 0;
+  const int t0 = doc_off[d], t1 = doc_off[d + 1];
+  const double* th64 = theta + (size_t)d * K;
+  float th[4 * UQ];
+#pragma unroll
+  for (int e = 0; e < 4 * UQ; ++e) {
+    const int k = 4 * UQ * j + e;
+    th[e] = k < K ? __double2float_rn(th64[k]) : 0.0f;
+  }
+  const float m = (float)(2 * K + 32) * 5.9604644775390625e-8f;
+  const float lo = 1.0f - m, hi = 1.0f + m;
+  __syncthreads();
+  float4 f0[UQ], f1[UQ];
+  int w0, w1;
+  // rows of the step st's tokens among the 32 whose ids the lanes hold
+  auto load = [&](float4 (&f)[UQ], int& wt, int ids, int st) {
+    wt = __shfl_sync(0xffffffffu, ids, st * PER + grp);
+    const float4* row = phi32 + (size_t)wt * row_quads;
+#pragma unroll
+    for (int q = 0; q < UQ; ++q) {
+      const int at = j * UQ + q;
+      f[q] = at < row_quads ? __ldg(row + at) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+  };
+  int tb = t0 + warp * 32;
+  auto draw = [&](const float4 (&f)[UQ], int wt, float uf, int st) {
+        const int tok = st * PER + grp;
+        const float u = __shfl_sync(0xffffffffu, uf, tok);
+        float c[4 * UQ];
+        float acc = 0.0f;
+#pragma unroll
+        for (int q = 0; q < UQ; ++q) {
+          acc = c[4 * q] = __fmaf_rn(th[4 * q], f[q].x, acc);
+          acc = c[4 * q + 1] = __fmaf_rn(th[4 * q + 1], f[q].y, acc);
+          acc = c[4 * q + 2] = __fmaf_rn(th[4 * q + 2], f[q].z, acc);
+          acc = c[4 * q + 3] = __fmaf_rn(th[4 * q + 3], f[q].w, acc);
+        }
+        float off = 0.0f, norm = acc;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+          const float a = __shfl_xor_sync(0xffffffffu, norm, o);
+          off = (j & o) ? __fadd_rn(off, a) : off;
+          norm = __fadd_rn(norm, a);
+        }
+        const float un = __fmul_rn(u, norm);
+        const float T1 = __fsub_rn(__fmul_rn(un, lo), off), T2 = __fsub_rn(__fmul_rn(un, hi), off);
+        // the lane's first running sum not below T1: its quad, then in it
+        float v0 = c[0], v1 = c[1], v2 = c[2], v3 = c[3];
+        int pos = 0;
+#pragma unroll
+        for (int q = 1; q < UQ; ++q) {
+          const bool past = c[4 * q - 1] < T1;
+          v0 = past ? c[4 * q] : v0;
+          v1 = past ? c[4 * q + 1] : v1;
+          v2 = past ? c[4 * q + 2] : v2;
+          v3 = past ? c[4 * q + 3] : v3;
+          pos = past ? 4 * q : pos;
+        }
+        const bool b0 = v0 < T1, b1 = v1 < T1, b2 = v2 < T1, b3 = v3 < T1;
+        pos += (int)b0 + (int)b1 + (int)b2 + (int)b3;
+        const float nxt = b0 ? (b1 ? (b2 ? v3 : v2) : v1) : v0;
+        const unsigned bal = __ballot_sync(0xffffffffu, !b3);       // b3 is the last quad's only if all are below
+        const unsigned mine = (bal >> (grp * G)) & ((1u << G) - 1u);
+        const int win = mine ? __ffs(mine) - 1 : G - 1;
+        const int t = tb + tok;
+        if (j == win && t < t1) {
+          int zk = mine ? min(4 * UQ * j + pos, K - 1) : K - 1;
+          const bool exact = !(norm >= 8.673617379884035e-19f && norm <= 3.4028234663852886e38f) ||   // [2^-60, FLT_MAX]
+                             (zk < K - 1 && !(nxt > T2));
+          if (exact) {
+            Stream se = make_stream(seed, (uint32_t)t, iter, TAG_Z);
+            zk = lda_reference_draw(K, th64, phiT + (size_t)wt * Kp, se.uniform());
+          }
+          z[t] = zk;
+          atomicAdd(&hist[zk], 1);
+          if (cnt_kw != nullptr) atomicAdd(cnt_kw + (size_t)zk * V + wt, 1);
+        }
+  };
+  int wc = tb + lane < t1 ? w[tb + lane] : 0;
+  load(f0, w0, wc, 0);
+  for (; tb < t1; tb += NW * 32) {
+    const int wn = tb + NW * 32 + lane < t1 ? w[tb + NW * 32 + lane] : 0;   // the next chunk's ids
+    Stream s = make_stream(seed, (uint32_t)(tb + lane), iter, TAG_Z);
+    const float uf = __double2float_rn(s.uniform());
+    // a step's rows are loaded while the step before it is drawn
+#pragma unroll 1
+    for (int st = 0; st < G && tb + st * PER < t1; st += 2) {
+      load(f1, w1, wc, st + 1);
+      draw(f0, w0, uf, st);
+      if (st + 2 < G) load(f0, w0, wc, st + 2);
+      else load(f0, w0, wn, 0);
+      draw(f1, w1, uf, st + 1);
+    }
+    wc = wn;
+  }
+  __syncthreads();
+  if (cnt_dk != nullptr)
+    for (int k = threadIdx.x; k < K; k += blockDim.x) cnt_dk[(size_t)d * K + k] = hist[k];
+  if (iter_dev != nullptr && done_ctr != nullptr) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      const unsigned prev = atomicAdd(done_ctr, 1u);
+      if (prev == (unsigned)(D - 1)) {
+        *done_ctr = 0u;
+        *iter_dev = iter + 1u;
+        __threadfence();
+      }
+    }
+  }
+}
+
+int launch_lda_zr(int D, int K, int V, int Kp, const int* doc_off, const int* w, const double* theta,
+                  const double* phiT, const float* phi32, int* z, int* cnt_dk, int* cnt_kw, uint64_t seed,
+                  uint32_t* iter_dev, uint32_t iter, uint32_t* done_ctr, cudaStream_t st) {
+  const int G = lda_zr_lanes(K), UQ = lda_zr_quads(K);
+  const int row_quads = lda_kq(K) / 4;
+  const float4* phi4 = reinterpret_cast<const float4*>(phi32);
+#define AB_ZR(g, uq)                                                                                              \
+  if (G == g && UQ == uq) {                                                                                       \
+    lda_zr_kernel<g, uq><<<D, 32 * lda_zr_warps(D), sizeof(int) * K, st>>>(D, K, V, Kp, doc_off, w, theta, phiT, phi4,  \
+                                                                     row_quads, z, cnt_dk, cnt_kw, seed,  \
+                                                                     iter_dev, iter, done_ctr);                   \
+    AB_LAUNCH_CHECK("lda_zr_kernel");                                                                             \
+    return AB_OK;                                                                                                 \
+  }
+  AB_ZR(8, 3) AB_ZR(8, 4) AB_ZR(16, 3) AB_ZR(16, 4)
+#undef AB_ZR
+  return fail(AB_ERR_ARG, "lda: the binary32-screened z kernel takes K <= %d (K=%d)", LDA_ZR_MAX_K, K);
+}
+
 // Count statistics of a given z (conj_stat_theta / conj_stat_phi of
 // CgConj.hs:171-177): one CTA per document; cnt_kw must be zero on entry.
 __global__ void __launch_bounds__(LDA_THREADS)
@@ -1055,11 +1250,11 @@ struct ab_lda {
 };
 
 // Sweep scratch: the phi draw's scratch, whose first 256 bytes hold the
-// runner's iteration and completion counters, then (K <= 64) the binary32
+// runner's iteration and completion counters, then (K <= 256) the binary32
 // screening copy of phi, phi32 f32 [V][Kq], zero padded, ...
 static inline size_t lda_phi32_offset(int K, int V) { return al256(lda_phi_scratch(K, V)); }
 static inline size_t lda_queue_offset(int K, int V) {
-  return lda_phi32_offset(K, V) + al256(K <= LDA_ZQ_MAX_K ? sizeof(float) * (size_t)V * lda_kq(K) : 0);
+  return lda_phi32_offset(K, V) + al256(K <= LDA_ZR_MAX_K ? sizeof(float) * (size_t)V * lda_kq(K) : 0);
 }
 // ... then the try kernel's queues: cells int2 [K * B][256], their first
 // tries' (normal, uniform) double2 [K * B][256], and lengths int [K * B]
@@ -1102,10 +1297,15 @@ static int lda_enqueue_sweep(ab_lda* h, cudaStream_t main, cudaStream_t side) {
   const ab_lda_desc& d = h->d;
   uint32_t* iter_dev = reinterpret_cast<uint32_t*>(d.scratch);
   uint32_t* done = iter_dev + 1;
-  float* phi32 = d.K <= LDA_ZQ_MAX_K
+  // Past K = 64 the screened draw needs enough documents to fill the SMs: at K =
+  // 140 with 20 documents the sweep takes 42 us against 43, at K = 192 with 40
+  // of them 88 against 86, at K = 250 with 60 132 against 119; with 611
+  // documents 107 against 126 at K = 130 and 184 against 246 at K = 256.
+  const bool screened = d.K <= LDA_ZQ_MAX_K || (d.K <= LDA_ZR_MAX_K && d.D >= (d.K <= 192 ? 148 : 2 * 148));
+  float* phi32 = screened
                      ? reinterpret_cast<float*>(static_cast<char*>(d.scratch) + lda_phi32_offset(d.K, d.V))
                      : nullptr;
-  if (phi32 != nullptr) {
+  if (d.K <= LDA_ZQ_MAX_K) {
     // phi's first tries use the whole GPU; the theta draw then runs beside the
     // phi fix-up and normalisation, which leave most SMs idle
     int rc = launch_lda_phi_sweep(0, d.K, d.V, h->Kp, d.beta, d.cnt_kw, d.phiT, d.scratch, phi32, d.seed,
@@ -1123,15 +1323,19 @@ static int lda_enqueue_sweep(ab_lda* h, cudaStream_t main, cudaStream_t side) {
     return launch_lda_zf(d.D, d.K, d.V, h->Kp, d.doc_off, d.w, d.theta, d.phiT, phi32, d.z, d.cnt_dk,
                          d.cnt_kw, d.seed, iter_dev, 0, done, main);
   }
-  // K > 64: theta beside the two-kernel phi draw, then the binary64 z kernel
+  // K > 64: theta beside the two-kernel phi draw (at K = 130 as fast as tries
+  // and fix-ups, and a launch less), then z, in binary64 past K = 256
   AB_CUDA(cudaEventRecord(h->fork, main));
   AB_CUDA(cudaStreamWaitEvent(side, h->fork, 0));
   int rc = launch_lda_theta(d.D, d.K, d.alpha, d.cnt_dk, d.theta, d.seed, iter_dev, 0, main);
   if (rc) return rc;
-  rc = launch_lda_phi(d.K, d.V, h->Kp, d.beta, d.cnt_kw, d.phiT, 1, d.scratch, d.seed, iter_dev, 0, side);
+  rc = launch_lda_phi(d.K, d.V, h->Kp, d.beta, d.cnt_kw, d.phiT, 1, d.scratch, d.seed, iter_dev, 0, side, phi32);
   if (rc) return rc;
   AB_CUDA(cudaEventRecord(h->join, side));
   AB_CUDA(cudaStreamWaitEvent(main, h->join, 0));
+  if (phi32 != nullptr)
+    return launch_lda_zr(d.D, d.K, d.V, h->Kp, d.doc_off, d.w, d.theta, d.phiT, phi32, d.z, d.cnt_dk, d.cnt_kw,
+                         d.seed, iter_dev, 0, done, main);
   return launch_lda_z(d.D, d.K, d.V, h->Kp, d.doc_off, d.w, d.theta, d.phiT, d.z, d.cnt_dk, d.cnt_kw,
                       d.seed, iter_dev, 0, done, main);
 }

@@ -131,8 +131,8 @@ int ab_lda_disc_z_f32(int D, int K, int V, const int* doc_off, const int* w, con
                       uint32_t iter, void* stream);
 
 /* Sweep runner: the whole augur_step of the LDA schedule (CgKern.hs:232-238)
- * as a captured CUDA graph of four kernels (z screened in binary32 for
- * K <= 64). */
+ * as a captured CUDA graph of five kernels (z screened in binary32 for
+ * K <= 256). */
 typedef struct ab_lda_desc {
   int D, K, V;
   const int* doc_off;   /* [D+1] */
@@ -150,7 +150,7 @@ typedef struct ab_lda_desc {
 
 typedef struct ab_lda ab_lda;
 /* Scratch of the sweep runner: its counters, the phi draw's partial sums and
- * normalisers, and the binary32 screening copy of phi (K <= 64). */
+ * normalisers, and the binary32 screening copy of phi (K <= 256). */
 size_t ab_lda_scratch_bytes(int K, int V);
 /* Replaces augur_iface_init for the LDA model (CgStInit.hs:474-510); the
  * caller owns every buffer named by the descriptor. */

@@ -301,3 +301,28 @@ def test_sweep_phi32_copy_is_phi_rounded():
     assert (phi32[:, K:] == 0).all()
     s.close()
 
+
+
+@pytest.mark.parametrize("K", [1, 3, 4, 5, 16, 17, 33, 63, 64, 65, 97, 128, 129, 193, 255, 256, 257, 300])
+def test_sweep_screen_equals_binary64(K):
+    """The sweep's z (screened in binary32 up to K = 256, whatever the lanes per
+    token and the quads per lane) and its counts equal the binary64 kernel's on
+    the sweep's own theta and phi; documents of 1 to 900 tokens."""
+    V, D = 211, 300
+    rng = np.random.default_rng(K)
+    lens = rng.integers(1, 70, D)
+    lens[5] = 900
+    lens[:4] = [1, 31, 32, 33]
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    w = rng.integers(0, V, off[-1]).astype(np.int32)
+    z0 = rng.integers(0, K, off[-1]).astype(np.int32)
+    s = LdaGibbs(K, V, off, w, 0.1, 0.01, seed=K, z=z0)
+    L = N.lib()
+    for it in range(2):
+        s.sweep(1)
+        z = torch.zeros_like(s.z)
+        dk, kw = torch.zeros_like(s.cnt_dk), torch.zeros_like(s.cnt_kw)
+        N.check(L.ab_lda_disc_z(D, K, V, N.ptr(s.doc_off), N.ptr(s.w), N.ptr(s.theta), N.ptr(s.phiT), N.ptr(z), N.ptr(dk),
+                                N.ptr(kw), K, it, N.stream_ptr()), "disc_z")
+        assert torch.equal(s.z, z)
+        assert torch.equal(s.cnt_dk, dk) and torch.equal(s.cnt_kw, kw)
