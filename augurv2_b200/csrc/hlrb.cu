@@ -321,39 +321,84 @@ struct GradEpi {
   __device__ void end(int, int, int, int, bool, int) {}
 };
 
-__device__ __forceinline__ void prior_term(int kind, double a, double b, double x, double& ll, double& g) {
-  if (kind == AB_PRIOR_NORMAL) {
+// The prior of a coefficient: kind, its parameters and the log density's
+// constant term (host).
+struct Prior {
+  int kind;
+  double a, b, c;
+};
+Prior make_prior(const ab_hlrb_model* m) {
+  const double a = m->prior_a, b = m->prior_b;
+  const double c = m->prior == AB_PRIOR_NORMAL
+                       ? -0.5 * log(2.0 * M_PI * a)
+                       : lgamma(0.5 * (a + 1.0)) - lgamma(0.5 * a) - 0.5 * log(a * M_PI) - log(b);
+  return Prior{m->prior, a, b, c};
+}
+
+__device__ __forceinline__ void prior_term(const Prior& p, double x, bool want_ll, double& ll, double& g) {
+  if (p.kind == AB_PRIOR_NORMAL) {
     // Normal(0, a): log density and derivative
-    ll = -0.5 * log(2.0 * M_PI * a) - 0.5 * x * x / a;
-    g = -x / a;
+    ll = p.c - 0.5 * x * x / p.a;
+    g = -x / p.a;
   } else {
     // Student-t(nu = a, scale = b)
-    const double nu = a, z = x / b;
-    ll = lgamma(0.5 * (nu + 1.0)) - lgamma(0.5 * nu) - 0.5 * log(nu * M_PI) - log(b) -
-         0.5 * (nu + 1.0) * log1p(z * z / nu);
-    g = -(nu + 1.0) * x / (nu * b * b + x * x);
+    const double nu = p.a, z = x / p.b;
+    ll = want_ll ? p.c - 0.5 * (nu + 1.0) * log1p(z * z / nu) : 0.0;
+    g = -(nu + 1.0) * x / (nu * p.b * p.b + x * x);
   }
 }
 
-// One block per chain: logp[c] (FP64) and grad[c][0..D-1] (FP32) from the
-// partials, in a fixed order; either output may be NULL.
-__device__ __forceinline__ void finish_chain(int c, int C, int D, int fwd_tiles, int splits, int ldw,
-                                             const float* __restrict__ llpart, const float* __restrict__ w,
-                                             const float* __restrict__ theta, int ldt, int prior, double pa,
-                                             double pb, double* __restrict__ logp, float* __restrict__ grad,
-                                             int ldg) {
-  __shared__ double red[33];
+// Sum of part[t C] over t = t0, t0 + step, ... below n, eight loads in flight,
+// added in that order.
+__device__ __forceinline__ double sum_parts(const float* __restrict__ part, int t0, int step, int n, int C) {
   double s = 0.0;
-  if (logp)
-    for (int t = threadIdx.x; t < fwd_tiles; t += blockDim.x) s += (double)llpart[(size_t)t * C + c];
+  for (int t = t0; t < n; t += 8 * step) {
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = part[(size_t)min(t + q * step, n - 1) * C];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (t + q * step < n) s += (double)v[q];
+  }
+  return s;
+}
+
+// g[i] += the splits' partial sums of coefficients d + 32 i (those below D), in
+// split order, U splits' loads in flight.
+template <int NQ, int U>
+__device__ __forceinline__ void add_splits(const float* __restrict__ w, size_t stride, int splits, int d, int step, int D,
+                                           double (&g)[NQ]) {
+  for (int k = 0; k < splits; k += U) {
+    float v[U][NQ];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < NQ; ++i)
+        v[u][i] = w[(size_t)min(k + u, splits - 1) * stride + min(d + step * i, D - 1)];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + u < splits) {
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) g[i] += (double)v[u][i];
+      }
+  }
+}
+
+// logp[c] (FP64) and grad[c][0..D-1] (FP32) from the partials, in a fixed
+// order, by one block; either output may be NULL.
+__device__ __forceinline__ void finish_block(int c, int C, int D, int fwd_tiles, int splits, int ldw,
+                                             const float* __restrict__ llpart, const float* __restrict__ w,
+                                             const float* __restrict__ theta, int ldt, const Prior& prior,
+                                             double* __restrict__ logp, float* __restrict__ grad, int ldg) {
+  __shared__ double red[33];
+  double s = logp ? sum_parts(llpart + c, threadIdx.x, blockDim.x, fwd_tiles, C) : 0.0;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    double pl, pg;
-    prior_term(prior, pa, pb, (double)theta[(size_t)c * ldt + d], pl, pg);
+    double pl, g[1];
+    prior_term(prior, (double)theta[(size_t)c * ldt + d], logp != nullptr, pl, g[0]);
     s += pl;
     if (grad) {
-      double g = pg;
-      for (int k = 0; k < splits; ++k) g += (double)w[((size_t)k * C + c) * ldw + d];
-      grad[(size_t)c * ldg + d] = (float)g;
+      add_splits<1, 8>(w + (size_t)c * ldw, (size_t)C * ldw, splits, d, 0, D, g);
+      grad[(size_t)c * ldg + d] = (float)g[0];
     }
   }
   s = block_sum_f64(s, red);
@@ -363,10 +408,34 @@ __device__ __forceinline__ void finish_chain(int c, int C, int D, int fwd_tiles,
 __global__ void __launch_bounds__(256) hlrb_finish_kernel(int C, int D, int fwd_tiles, int splits, int ldw,
                                                           const float* __restrict__ llpart,
                                                           const float* __restrict__ w, const float* __restrict__ theta,
-                                                          int ldt, int prior, double pa, double pb,
-                                                          double* __restrict__ logp, float* __restrict__ grad,
-                                                          int ldg) {
-  finish_chain(blockIdx.x, C, D, fwd_tiles, splits, ldw, llpart, w, theta, ldt, prior, pa, pb, logp, grad, ldg);
+                                                          int ldt, Prior prior, double* __restrict__ logp,
+                                                          float* __restrict__ grad, int ldg) {
+  finish_block(blockIdx.x, C, D, fwd_tiles, splits, ldw, llpart, w, theta, ldt, prior, logp, grad, ldg);
+}
+
+// The coefficients' part by one warp, 32 NQ at a time (narrow instances of a
+// group would leave most of a block idle).
+template <int NQ, int U>
+__device__ __forceinline__ double finish_coefficients(const float* __restrict__ w, size_t stride, int splits,
+                                                      const float* __restrict__ theta, const Prior& prior, int D,
+                                                      float* __restrict__ grad) {
+  const int lane = threadIdx.x & 31;
+  double s = 0.0;
+  for (int d0 = 0; d0 < D; d0 += 32 * NQ) {
+    const int d = d0 + lane;
+    double g[NQ];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      double pl;
+      prior_term(prior, (double)theta[min(d + 32 * i, D - 1)], true, pl, g[i]);
+      s += d + 32 * i < D ? pl : 0.0;
+    }
+    add_splits<NQ, U>(w, stride, splits, d, 32, D, g);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i)
+      if (d + 32 * i < D) grad[d + 32 * i] = (float)g[i];
+  }
+  return s;
 }
 
 }  // namespace
@@ -431,8 +500,8 @@ int hlrb_logp_grad(const ab_hlrb_model* m, int C, const float* theta, int ldt, d
     else rc = tc::launch_gemm<128, R_PARTS, 1>(ma, mb, bs, ge, err, st);
     if (rc) return rc;
   }
-  hlrb_finish_kernel<<<C, 256, 0, st>>>(C, D, L.fwd_tiles * L.groups, L.splits, L.ldw, llp, w, theta, ldt, m->prior,
-                                        m->prior_a, m->prior_b, logp, grad, ldg);
+  hlrb_finish_kernel<<<C, 256, 0, st>>>(C, D, L.fwd_tiles * L.groups, L.splits, L.ldw, llp, w, theta, ldt, make_prior(m),
+                                        logp, grad, ldg);
   AB_LAUNCH_CHECK("hlrb_finish_kernel");
   return AB_OK;
 }
@@ -522,8 +591,8 @@ struct GFinish {
   const float* theta;
   double* logp;
   float* grad;
-  double pa, pb;
-  int C, D, fwd_parts, splits, ldw, ldt, prior, ldg;
+  Prior prior;
+  int C, D, fwd_parts, splits, ldw, ldt, ldg;
 };
 
 // The launch header: problems in use and tiles of the forward and backward
@@ -541,13 +610,49 @@ __global__ void hlrg_split_kernel(const GSplit* __restrict__ tab, const GHeads* 
     split_elem(c, d, q.D, q.Dp, q.theta, q.ldt, q.t3);
 }
 
+// The two-GEMM grouped pass: a block per chain, each instance's own numbers.
 __global__ void __launch_bounds__(256) hlrg_finish_kernel(const GFinish* __restrict__ tab,
                                                           const GHeads* __restrict__ head) {
   if ((int)blockIdx.y >= head->fwd.n) return;
-  const GFinish q = tab[blockIdx.y];
+  const GFinish& q = tab[blockIdx.y];
   if ((int)blockIdx.x >= q.C) return;
-  finish_chain(blockIdx.x, q.C, q.D, q.fwd_parts, q.splits, q.ldw, q.llpart, q.w, q.theta, q.ldt, q.prior, q.pa, q.pb,
-               q.logp, q.grad, q.ldg);
+  finish_block(blockIdx.x, q.C, q.D, q.fwd_parts, q.splits, q.ldw, q.llpart, q.w, q.theta, q.ldt, q.prior, q.logp,
+               q.grad, q.ldg);
+}
+
+// The fused pass: a warp per chain, or from 65 coefficients on four, each with 64
+// of them, and 256 threads in all.  Against a block per chain, which
+// leaves most threads idle at D = 16 and 64: 190 -> 65 us on 24 instances of 512
+// chains, 3.5e6 rows in all (98 MB of partial sums).  One warp for all of D = 256
+// has too few loads in flight: 39 us for 512 chains x 74 segments, 23 with a block.
+__host__ __device__ constexpr int finish_warps(int D) { return D <= 64 ? 1 : 4; }
+
+__global__ void __launch_bounds__(256) hlrf_finish_kernel(const GFinish* __restrict__ tab,
+                                                          const GHeads* __restrict__ head) {
+  __shared__ double red[8];
+  if ((int)blockIdx.y >= head->fwd.n) return;
+  const GFinish& q = tab[blockIdx.y];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int D = q.D, wpc = finish_warps(D), part = warp & (wpc - 1);
+  const int c = blockIdx.x * (8 / wpc) + warp / wpc;
+  double s = 0.0;
+  if (c < q.C) {
+    s = sum_parts(q.llpart + c, part * 32 + lane, 32 * wpc, q.fwd_parts, q.C);
+    const int d0 = 64 * part, dn = min(64, D - d0);
+    const float* w = q.w + (size_t)c * q.ldw + d0;
+    const size_t stride = (size_t)q.C * q.ldw;
+    const float* theta = q.theta + (size_t)c * q.ldt + d0;
+    float* grad = q.grad + (size_t)c * q.ldg + d0;
+    if (D <= 32) s += finish_coefficients<1, 8>(w, stride, q.splits, theta, q.prior, dn, grad);
+    else if (dn > 0) s += finish_coefficients<2, 8>(w, stride, q.splits, theta, q.prior, dn, grad);
+  }
+  s = warp_sum_f64(s);
+  if (lane == 0) red[warp] = s;
+  __syncthreads();
+  if (c < q.C && lane == 0 && part == 0) {
+    for (int i = 1; i < wpc; ++i) s += red[warp + i];
+    q.logp[c] = s;
+  }
 }
 
 struct HlrgInst {
@@ -592,7 +697,15 @@ inline size_t al256(size_t a) { return (a + 255) & ~size_t(255); }
 // launch, so a group of instances gives each instance the numbers it gets
 // alone.  Roles: warp 0 lane 0 TMA producer, warp 1 lane 0 MMA issuer,
 // warps 2..17 epilogue (column group g = 32 columns, taken 16 at a time;
-// lane quarter = warp % 4).  Every wait is bounded as in gemm_kernel.
+// lane quarter = warp % 4).  No epilogue warp waits for another: each stages its
+// own labels, hands in its half of the residual on that half's own barrier and
+// waits for the previous tile's backward product only before its first residual
+// store.  At 512 chains and 600,000 rows a pass takes 389 us at D = 16, 405 at 64,
+// 493 at 128 and 737 at 256 (489, 494, 511 and 742 with a barrier over all epilogue
+// warps per tile and the wait at the tile's start).  It is bound by the epilogue's
+// chain of exponentials, logarithm and Kahan sums up to D = 64 (issue slots and the
+// special function unit each 54 % busy) and by the tensor core's operand supply
+// from there (52 % busy at D = 256).  Every wait is bounded as in gemm_kernel.
 constexpr int F_ROWS = 128;
 constexpr int F_SEG_TILES = 64;                            // row tiles per unit (8192 rows)
 constexpr int F_MAX_D = 256;
@@ -603,8 +716,8 @@ constexpr int F_STAGES = 2;
 constexpr int F_A_BYTES = 128 * 64 * 2;                    // one 128 x 64 bf16 box
 constexpr int F_STAGE_BYTES = 3 * F_A_BYTES + F_ROWS * 128; // theta parts + X tile; an Xt block uses Dn * 128
 constexpr int F_ROFF = F_STAGES * F_STAGE_BYTES;           // residual parts: [2 parts][2 K-blocks] boxes
-constexpr int F_YOFF = F_ROFF + 4 * F_A_BYTES;             // s values [2][128] f32
-constexpr int F_BAROFF = F_YOFF + 2 * F_ROWS * 4;
+constexpr int F_YOFF = F_ROFF + 4 * F_A_BYTES;             // s values of each epilogue warp's 32 rows, f32
+constexpr int F_BAROFF = F_YOFF + F_EPI_WARPS * 32 * 4;
 constexpr int F_SMEM = F_BAROFF + 256 + 1024;
 constexpr int F_TMEM_COLS = 512;                           // T0 | T1 | G
 static_assert(F_SMEM <= tc::SMEM_BUDGET, "fused pass exceeds shared memory");
@@ -636,9 +749,9 @@ hlrf_kernel(const FInst* __restrict__ insts, const FUnit* __restrict__ units, co
   uint64_t* empty = full + F_STAGES;
   uint64_t* acc_full = empty + F_STAGES;
   uint64_t* acc_empty = acc_full + 2;
-  uint64_t* r_full = acc_empty + 2;
-  uint64_t* r_empty = r_full + 1;
-  uint64_t* g_full = r_empty + 1;
+  uint64_t* r_full = acc_empty + 2;    // [2] per 64-row block of the residual
+  uint64_t* r_empty = r_full + 2;
+  uint64_t* g_full = r_empty + 2;
   uint64_t* g_empty = g_full + 1;
   uint64_t* drain = g_empty + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
@@ -649,8 +762,7 @@ hlrf_kernel(const FInst* __restrict__ insts, const FUnit* __restrict__ units, co
   if (threadIdx.x == 0) {
     for (int s = 0; s < F_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], F_EPI_WARPS); }
-    mbar_init(r_full, F_EPI_WARPS);
-    mbar_init(r_empty, 1);
+    for (int j = 0; j < 2; ++j) { mbar_init(&r_full[j], F_EPI_WARPS / 2); mbar_init(&r_empty[j], 1); }
     mbar_init(g_full, 1);
     mbar_init(g_empty, F_EPI_WARPS);
     mbar_init(drain, 1);
@@ -749,13 +861,13 @@ hlrf_kernel(const FInst* __restrict__ insts, const FUnit* __restrict__ units, co
             ++it;
           }
           if (k >= 1) {
-            if (!mbar_wait(r_full, rb & 1)) { *fail = 1; bad = true; break; }
             if (k == 1 && gu >= 1 && !mbar_wait(g_empty, (gu - 1) & 1)) { *fail = 1; bad = true; break; }
             if (*(volatile int*)fail) { bad = true; break; }
             fence_after();
             const uint32_t dg = tmem + 2u * F_ROWS;
             for (int j = 0; j < 2; ++j, ++g) {
               const int s = g % F_STAGES;
+              if (!mbar_wait(&r_full[j], rb & 1)) { *fail = 1; bad = true; break; }
               if (!mbar_wait(&full[s], (g / F_STAGES) & 1)) { *fail = 1; bad = true; break; }
               if (*(volatile int*)fail) { bad = true; break; }
               fence_after();
@@ -767,9 +879,9 @@ hlrf_kernel(const FInst* __restrict__ insts, const FUnit* __restrict__ units, co
                   mma_bf16(dg, make_desc(rbuf + (p * 2 + j) * F_A_BYTES) + 2 * kk, make_desc(b) + 2 * kk, idesc_g,
                            (k > 1 || j > 0 || kk > 0 || p > 0) ? 1u : 0u);
               mma_commit(&empty[s]);
+              mma_commit(&r_empty[j]);
             }
             if (bad) break;
-            mma_commit(r_empty);
             ++rb;
           }
         }
@@ -783,64 +895,47 @@ hlrf_kernel(const FInst* __restrict__ insts, const FUnit* __restrict__ units, co
   } else {
     const int qw = warp & 3;                 // TMEM lane quarter
     const int grp = (warp - 2) >> 2;         // column group: columns [32 grp, 32 grp + 32)
-    const int etid = (warp - 2) * 32 + lane;
     const int cl = qw * 32 + lane;           // chain within the tile
     const uint32_t lane_base = tmem + ((uint32_t)(qw * 32) << 16);
+    float* sw = ys + (warp - 2) * 32;        // this warp's s values
+    const int kb = grp >> 1;                 // residual block of the group's columns
     int it = 0, gu = 0;
-    bool bad = false;   // this thread's failure so far (uniform over the warp)
-    // y of row etid of the next tile, loaded one tile ahead (threads etid < 128)
-    int pf_y = 0;
-    bool pf_v = false;
-    auto prefetch = [&](int uu, int kk) {
-      if (etid < F_ROWS && uu < u_end) {
-        const FUnit V = units[uu];
-        const FInst* J = insts + V.inst;
-        const int nn = (V.r0 + kk) * F_ROWS + etid;
-        pf_v = nn < J->N;
-        pf_y = pf_v ? J->y[nn] : 0;
-      }
-    };
-    prefetch(u_beg, 0);
-    for (int u = u_beg; u < u_end; ++u) {
+    bool bad = false;   // a wait of this warp failed (uniform over the warp)
+    for (int u = u_beg; u < u_end && !bad; ++u) {
       const FUnit U = units[u];
       const FInst* I = insts + U.inst;
       const int n = U.r1 - U.r0, N = I->N, C = I->C, Dn = I->Dn;
       const int chain = U.m * BM + cl;
       const bool ok = chain < C;
       float acc = 0.0f, comp = 0.0f;
-      bool stop = false;
+      // y of this lane's row of the group, loaded one tile ahead
+      const int* yp = I->y + (size_t)U.r0 * F_ROWS + grp * 32 + lane;
+      int left = N - U.r0 * F_ROWS - grp * 32 - lane;   // > 0: the row exists
+      int y1 = left > 0 ? __ldg(yp) : -1;
       for (int k = 0; k < n; ++k) {
         const int buf = it & 1;
         const int row0 = (U.r0 + k) * F_ROWS;
-        if (etid < F_ROWS) ys[buf * F_ROWS + etid] = pf_v ? (pf_y ? 1.0f : -1.0f) : 0.0f;
-        if (k + 1 < n) prefetch(u, k + 1);
-        else prefetch(u + 1, 0);
-        // the barrier ORs every epilogue thread's failure flag: all stop together
-        if (epi_sync_or(32 * F_EPI_WARPS, bad)) { stop = true; break; }
-        bool okw = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (it >> 1) & 1));
-        if (it >= 1) okw = __all_sync(0xffffffffu, okw && mbar_wait(r_empty, (it - 1) & 1));
+        sw[lane] = left > 0 ? (y1 ? 1.0f : -1.0f) : 0.0f;
+        yp += F_ROWS;
+        left -= F_ROWS;
+        if (left > 0) y1 = __ldg(yp);
+        const bool okw = mbar_wait(&acc_full[buf], (it >> 1) & 1);
+        if (!__all_sync(0xffffffffu, okw && !*(volatile int*)fail)) { bad = true; break; }
         fence_after();
-        const bool have = __all_sync(0xffffffffu, okw && !*(volatile int*)fail);
-        const uint32_t tcol = (uint32_t)(buf * F_ROWS + grp * 32);
-        const float* sv0 = ys + buf * F_ROWS + grp * 32;
-        // the group's 32 columns lie in residual K-block grp / 2, 16-byte
-        // chunks 4 (grp % 2) .. +3 of each chain row
-        unsigned char* rowh = rbuf + (0 * 2 + (grp >> 1)) * F_A_BYTES + cl * 128;
-        unsigned char* rowm = rbuf + (1 * 2 + (grp >> 1)) * F_A_BYTES + cl * 128;
+        __syncwarp();   // the labels are there
+        // the group's 32 columns lie in residual block kb, 16-byte chunks
+        // 4 (grp % 2) .. +3 of each chain row
+        unsigned char* rowh = rbuf + (0 * 2 + kb) * F_A_BYTES + cl * 128;
+        unsigned char* rowm = rbuf + (1 * 2 + kb) * F_A_BYTES + cl * 128;
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
           float v[16], sv[16], rv[16];
-          if (have) {
-            uint32_t r[16];
-            tmem_ld16_issue(lane_base + tcol + cc * 16, r);
-            tmem_wait16(r);
+          uint32_t r[16];
+          tmem_ld16_issue(lane_base + (uint32_t)(buf * F_ROWS + grp * 32 + cc * 16), r);
+          tmem_wait16(r);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = 0.0f;
-          }
-          const float4* s4 = reinterpret_cast<const float4*>(sv0 + cc * 16);
+          for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+          const float4* s4 = reinterpret_cast<const float4*>(sw + cc * 16);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const float4 a = s4[i];
@@ -852,28 +947,32 @@ hlrf_kernel(const FInst* __restrict__ insts, const FUnit* __restrict__ units, co
           if (row0 + grp * 32 + cc * 16 + 16 <= N) ll_resid_chunk<true, true, true, 16>(v, sv, rv, acc, comp);
           else ll_resid_chunk<true, true, false, 16>(v, sv, rv, acc, comp);
           // residual parts into the swizzled K-major boxes: chain row cl,
-          // 16-byte chunk c16 of the row stored at c16 ^ (cl & 7)
+          // 16-byte chunk c16 of the row stored at c16 ^ (cl & 7); the boxes are
+          // free once the previous tile's backward product has read it
+          if (cc == 0 && it >= 1) {
+            const bool okr = mbar_wait(&r_empty[kb], (it - 1) & 1);
+            if (!__all_sync(0xffffffffu, okr)) bad = true;
+          }
+          if (!bad) {
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            uint32_t h[4], m[4];
+            for (int q = 0; q < 2; ++q) {
+              uint32_t h[4], m[4];
 #pragma unroll
-            for (int e2 = 0; e2 < 4; ++e2) split_pair(rv[8 * q + 2 * e2], rv[8 * q + 2 * e2 + 1], h[e2], m[e2]);
-            const int c16 = ((grp & 1) * 4 + cc * 2 + q) ^ (cl & 7);
-            *reinterpret_cast<uint4*>(rowh + c16 * 16) = make_uint4(h[0], h[1], h[2], h[3]);
-            *reinterpret_cast<uint4*>(rowm + c16 * 16) = make_uint4(m[0], m[1], m[2], m[3]);
+              for (int e2 = 0; e2 < 4; ++e2) split_pair(rv[8 * q + 2 * e2], rv[8 * q + 2 * e2 + 1], h[e2], m[e2]);
+              const int c16 = ((grp & 1) * 4 + cc * 2 + q) ^ (cl & 7);
+              *reinterpret_cast<uint4*>(rowh + c16 * 16) = make_uint4(h[0], h[1], h[2], h[3]);
+              *reinterpret_cast<uint4*>(rowm + c16 * 16) = make_uint4(m[0], m[1], m[2], m[3]);
+            }
           }
         }
+        if (bad) break;
         fence_before();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // residual writes -> tensor core
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&acc_empty[buf]);
-          mbar_arrive(r_full);
-        }
-        if (!have) bad = true;
+        if (lane == 0) { mbar_arrive(&r_full[kb]); mbar_arrive(&acc_empty[buf]); }
         ++it;
       }
-      if (stop) break;
+      if (bad) break;
       if (ok) I->llp[((size_t)U.seg * F_GROUPS + grp) * C + chain] = acc;
       // the unit's gradient: columns [64 grp, 64 grp + 64) of G
       const bool okg = __all_sync(0xffffffffu, mbar_wait(g_full, gu & 1) && !*(volatile int*)fail);
@@ -900,7 +999,10 @@ hlrf_kernel(const FInst* __restrict__ insts, const FUnit* __restrict__ units, co
       if (!okg) bad = true;
       ++gu;
     }
-    if (bad) *(volatile int*)epi_fail = 1;
+    if (bad) {   // the other warps stop at their next wait
+      *(volatile int*)fail = 1;
+      *(volatile int*)epi_fail = 1;
+    }
   }
   __syncwarp();
   if (threadIdx.x == 0 && *(volatile int*)fail) {
@@ -1136,8 +1238,8 @@ extern "C" int ab_hlrg_set_active(ab_hlrg* g, const int* active, void* stream) {
       fused_units(q, k, units);
       sp[k] = GSplit{q.theta, reinterpret_cast<__nv_bfloat16*>(q.work + q.f_t3), q.ldt, q.C, q.m.D, q.Dp};
       fin[k] = GFinish{reinterpret_cast<const float*>(q.work + q.f_llp), reinterpret_cast<const float*>(q.work + q.f_gw),
-                       q.theta, q.logp, q.grad, q.m.prior_a, q.m.prior_b, q.C, q.m.D, F_GROUPS * q.nseg, q.nseg, q.Dn, q.ldt,
-                       q.m.prior, q.ldg};
+                       q.theta, q.logp, q.grad, make_prior(&q.m), q.C, q.m.D, F_GROUPS * q.nseg, q.nseg, q.Dn, q.ldt,
+                       q.ldg};
     } else {
       fwd[k] = q.fwd;
       fwd[k].tile0 = tf;
@@ -1149,9 +1251,8 @@ extern "C" int ab_hlrg_set_active(ab_hlrg* g, const int* active, void* stream) {
       ge[k] = q.ge;
       sp[k] = GSplit{q.theta, reinterpret_cast<__nv_bfloat16*>(q.work + q.L.off_t3), q.ldt, q.C, q.m.D, q.L.Dp};
       fin[k] = GFinish{reinterpret_cast<const float*>(q.work + q.L.off_ll),
-                       reinterpret_cast<const float*>(q.work + q.L.off_w), q.theta, q.logp, q.grad, q.m.prior_a,
-                       q.m.prior_b, q.C, q.m.D, q.L.fwd_tiles * q.L.groups, q.L.splits, q.L.ldw, q.ldt, q.m.prior,
-                       q.ldg};
+                       reinterpret_cast<const float*>(q.work + q.L.off_w), q.theta, q.logp, q.grad, make_prior(&q.m),
+                       q.C, q.m.D, q.L.fwd_tiles * q.L.groups, q.L.splits, q.L.ldw, q.ldt, q.ldg};
     }
     act.push_back(i);
     ++k;
@@ -1196,8 +1297,10 @@ extern "C" int ab_hlrg_logp_grad(ab_hlrg* g, int* err, void* stream) {
             reinterpret_cast<const GradEpi*>(g->tab + g->o_ge), &head->bwd, err);
     AB_LAUNCH_CHECK("grouped_gemm_kernel (backward)");
   }
-  hlrg_finish_kernel<<<dim3(g->C_max, n), 256, 0, st>>>(reinterpret_cast<const GFinish*>(g->tab + g->o_fin), head);
-  AB_LAUNCH_CHECK("hlrg_finish_kernel");
+  const GFinish* fin = reinterpret_cast<const GFinish*>(g->tab + g->o_fin);
+  if (g->fused) hlrf_finish_kernel<<<dim3(ceil_div(g->C_max, 8 / finish_warps(g->Dp_max)), n), 256, 0, st>>>(fin, head);
+  else hlrg_finish_kernel<<<dim3(g->C_max, n), 256, 0, st>>>(fin, head);
+  AB_LAUNCH_CHECK("hlrg finish kernel");
   return AB_OK;
 }
 

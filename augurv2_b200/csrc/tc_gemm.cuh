@@ -127,19 +127,6 @@ __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::aft
 
 // Named barrier over the epilogue warps.
 __device__ __forceinline__ void epi_sync(int nthreads) { asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory"); }
-// The same barrier returning the OR of every participating thread's flag.
-__device__ __forceinline__ bool epi_sync_or(int nthreads, bool flag) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.or.pred q, 1, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)flag), "r"(nthreads)
-      : "memory");
-  return r != 0;
-}
 
 // 32 consecutive fp32 columns of this warp's 32 TMEM lanes.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
