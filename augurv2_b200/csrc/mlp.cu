@@ -14,11 +14,12 @@
 //   forward   P1 = X W1^T + b1, A1 = gelu(P1), P2 = A1 W2^T + b2,
 //             A2 = gelu(P2), Y = A2 W3^T + b3 — a product per layer when the
 //             activations are kept for the backward pass, otherwise one fused
-//             launch, a few rows per block with the activations in shared
-//             memory
+//             launch, a few rows per cluster or block with the activations in
+//             shared memory
 //   loss      mean squared error against a target, dY = 2 (Y - T) / (B d_out)
 //   backward  dW3 = dY^T A2, db3 = colsum dY, dP2 = (dY W3) . gelu'(P2), ...
 //   Adam      on the master vector, refreshing the bf16 copy.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -285,6 +286,8 @@ __global__ void sur_post_kernel(int C, int D, const float* __restrict__ theta, c
   }
 }
 
+// ---- the whole network in one launch -----------------------------------------
+
 // One dense layer for G rows held in shared memory: out[g][j] = act(b[j] +
 // sum_k W[j][k] in[g][k]).  One output feature j per thread: the thread
 // walks its bf16 weight row in 16-byte pieces (consecutive pieces share a
@@ -334,11 +337,11 @@ __device__ __forceinline__ void dense_layer(const float* __restrict__ in, int di
   }
 }
 
-// The whole network for G rows per block.  SUR: input theta with the
+// The whole network for G rows per block (large batches).  SUR: input theta with the
 // surrogate's input map z = (theta - mu) * inv_s, output the gradient
 // estimate a + h (theta - mu) + o * y; otherwise input x, output y.
 template <int G, bool SUR>
-__global__ void __launch_bounds__(256) mlp_fused_kernel(int B, int din, int h1, int h2, int dout,
+__global__ void __launch_bounds__(256) mlp_rows_kernel(int B, int din, int h1, int h2, int dout,
                                                         const float* __restrict__ x, int ldx,
                                                         const __nv_bfloat16* __restrict__ wb,
                                                         const float* __restrict__ w, float* __restrict__ y, int ldy,
@@ -381,10 +384,156 @@ __global__ void __launch_bounds__(256) mlp_fused_kernel(int B, int din, int h1, 
   }
 }
 
-constexpr int FUSED_G = 4;
+// A small batch: a cluster of eight CTAs takes G rows through the network, each CTA an eighth of
+// every layer's features.  A feature belongs to P neighbouring lanes that walk its
+// weight row in turn, 16 bytes each, so that a warp reads whole sectors; the G rows'
+// inputs come from shared memory, and a hidden feature's activations go to all
+// eight CTAs' copies.  One CTA per four rows reads every weight row by itself, each lane
+// another row: a surrogate of 512-256-256-512 with its dense linear part as a product
+// of its own takes 47 us at 16 rows, 52 at 64 and 53 at 256; this kernel 15, 22 and
+// 36 (graph replays).  It is bound by its shared-memory reads and weight loads
+// sharing one pipe, and by the latency of three layers with a cluster barrier each;
+// two features a thread halve the former and measured the same (35 us, and 17 at 16
+// rows).
+constexpr int NET_CTAS = 8, NET_THREADS = 256;
+
+// Lanes per feature when `dout` features of `n` pieces are spread over the cluster: as
+// many as leave no thread without one, at most a warp and no more than the pieces.
+__device__ __forceinline__ int net_lanes(int dout, int n) {
+  const int per = (dout + NET_CTAS - 1) / NET_CTAS;
+  int P = 32;
+  while (P > 1 && (P * per > NET_THREADS || P > n)) P >>= 1;
+  return P;
+}
+
+template <int G>
+__device__ __forceinline__ void lane_sum(float (&v)[G], int P) {
+  for (int o = P >> 1; o; o >>= 1)
+#pragma unroll
+    for (int g = 0; g < G; ++g) v[g] += __shfl_xor_sync(0xffffffffu, v[g], o);
+}
+
+// v[g] for a run-time g.
+template <int G>
+__device__ __forceinline__ float pick(const float (&v)[G], int g) {
+  float r = v[0];
+#pragma unroll
+  for (int i = 1; i < G; ++i) r = i == g ? v[i] : r;
+  return r;
+}
+
+// This CTA's features of one dense layer, out = b + W in: sink(j, g, value, linear)
+// is called once per feature j and row g.  M (k-major, [dout][dout]) adds the
+// linear = sum_k M[k][j] dt[g][k] of the surrogate; null without one.
+template <int G, class Sink>
+__device__ __forceinline__ void net_layer(const float* in, int din, const __nv_bfloat16* __restrict__ W,
+                                          const float* __restrict__ b, int dout, int rank, const float* dt,
+                                          const float* __restrict__ M, const Sink& sink) {
+  const int n8 = din >> 3, P = net_lanes(dout, n8);
+  const int slot = threadIdx.x / P, p = threadIdx.x & (P - 1), slots = NET_THREADS / P;
+  const int per = (dout + NET_CTAS - 1) / NET_CTAS, j_end = min(dout, (rank + 1) * per);
+  // lanes 4..7 of eight start with the second half of their piece: the eight
+  // 16-byte reads of a row's inputs then fall into different banks
+  const bool swap = (p >> 2) & 1;
+  for (int base = rank * per; base < j_end; base += slots) {
+    const int j = min(base + slot, dout - 1);
+    float acc[G], lin[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) acc[g] = lin[g] = 0.0f;
+    const uint4* row = reinterpret_cast<const uint4*>(W + (size_t)j * din);
+#pragma unroll 4
+    for (int k8 = p; k8 < n8; k8 += P) {
+      const uint4 raw = __ldg(row + k8);
+      const uint32_t r0 = swap ? raw.z : raw.x, r1 = swap ? raw.w : raw.y, r2 = swap ? raw.x : raw.z,
+                     r3 = swap ? raw.y : raw.w;
+      const float* x0 = in + 8 * k8 + (swap ? 4 : 0);
+      const float* x1 = in + 8 * k8 + (swap ? 0 : 4);
+      const float w0 = __uint_as_float(r0 << 16), w1 = __uint_as_float(r0 & 0xffff0000u);
+      const float w2 = __uint_as_float(r1 << 16), w3 = __uint_as_float(r1 & 0xffff0000u);
+      const float w4 = __uint_as_float(r2 << 16), w5 = __uint_as_float(r2 & 0xffff0000u);
+      const float w6 = __uint_as_float(r3 << 16), w7 = __uint_as_float(r3 & 0xffff0000u);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const float4 a = *reinterpret_cast<const float4*>(x0 + g * din);
+        const float4 c = *reinterpret_cast<const float4*>(x1 + g * din);
+        acc[g] = fmaf(w3, a.w, fmaf(w2, a.z, fmaf(w1, a.y, fmaf(w0, a.x, acc[g]))));
+        acc[g] = fmaf(w7, c.w, fmaf(w6, c.z, fmaf(w5, c.y, fmaf(w4, c.x, acc[g]))));
+      }
+    }
+    lane_sum(acc, P);
+    if (M) {
+#pragma unroll 8
+      for (int k4 = p; k4 < (dout >> 2); k4 += P) {
+        const float* m = M + (size_t)(4 * k4) * dout + j;
+        const float m0 = __ldg(m), m1 = __ldg(m + dout), m2 = __ldg(m + 2 * (size_t)dout), m3 = __ldg(m + 3 * (size_t)dout);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const float4 a = *reinterpret_cast<const float4*>(dt + g * dout + 4 * k4);
+          lin[g] = fmaf(m3, a.w, fmaf(m2, a.z, fmaf(m1, a.y, fmaf(m0, a.x, lin[g]))));
+        }
+      }
+      lane_sum(lin, P);
+    }
+    if (base + slot < j_end) {
+      const float bj = b[j];
+      for (int g = p; g < G; g += P) sink(j, g, pick(acc, g) + bj, M ? pick(lin, g) : 0.0f);
+    }
+  }
+}
+
+// SUR: input theta with the surrogate's input map z = (theta - mu) * inv_s, output the
+// gradient estimate a + h (theta - mu) + o * y, plus (theta - mu) M when M is given;
+// otherwise input x, output y.
+template <int G, bool SUR>
+__global__ void __cluster_dims__(NET_CTAS, 1, 1) __launch_bounds__(NET_THREADS, 2)
+    mlp_cluster_kernel(int B, int din, int h1, int h2, int dout, const float* __restrict__ x, int ldx,
+                     const __nv_bfloat16* __restrict__ wb, const float* __restrict__ w, float* __restrict__ y, int ldy,
+                     const float* __restrict__ mu, const float* __restrict__ inv_s, const float* __restrict__ sa,
+                     const float* __restrict__ sh, const float* __restrict__ so, const float* __restrict__ M) {
+  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  extern __shared__ float4 sm4[];
+  float* z = reinterpret_cast<float*>(sm4);   // [G][din]
+  float* a1 = z + G * din;                    // [G][h1]
+  float* a2 = a1 + G * h1;                    // [G][h2]
+  float* dt = a2 + G * h2;                    // [G][din] theta - mu (SUR)
+  const int rank = (int)cl.block_rank(), r0 = (int)(blockIdx.x / NET_CTAS) * G;
+  const size_t ob1 = (size_t)h1 * din, ow2 = ob1 + h1, ob2 = ow2 + (size_t)h2 * h1, ow3 = ob2 + h2,
+               ob3 = ow3 + (size_t)dout * h2;
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+    for (int k = threadIdx.x; k < din; k += NET_THREADS) {
+      float v = r0 + g < B ? x[(size_t)(r0 + g) * ldx + k] : 0.0f;
+      if (SUR) {
+        v = r0 + g < B ? v - mu[k] : 0.0f;
+        dt[g * din + k] = v;
+        v *= inv_s[k];
+      }
+      z[g * din + k] = v;
+    }
+  cl.sync();   // the peers run: their shared memory may be written
+  auto hidden = [&](float* out, int h) {
+    return [=](int j, int g, float v, float) {
+      const float e = gelu(v);
+#pragma unroll
+      for (int t = 0; t < NET_CTAS; ++t)
+        cooperative_groups::this_cluster().map_shared_rank(out, t)[g * h + j] = e;
+    };
+  };
+  net_layer<G>(z, din, wb, w + ob1, h1, rank, nullptr, nullptr, hidden(a1, h1));
+  cl.sync();
+  net_layer<G>(a1, h1, wb + ow2, w + ob2, h2, rank, nullptr, nullptr, hidden(a2, h2));
+  cl.sync();
+  net_layer<G>(a2, h2, wb + ow3, w + ob3, dout, rank, dt, SUR ? M : nullptr, [=](int j, int g, float v, float lin) {
+    if (r0 + g >= B) return;
+    if (SUR) v = sa[j] + sh[j] * dt[g * din + j] + so[j] * v + lin;
+    y[(size_t)(r0 + g) * ldy + j] = v;
+  });
+}
+
+constexpr int ROWS_G = 4;
 
 inline size_t fused_smem(const ab_mlp_desc* d) {
-  return sizeof(float) * FUSED_G * ((size_t)d->d_in + 2 * d->h1 + 2 * d->h2 + d->d_out);
+  return sizeof(float) * ROWS_G * ((size_t)d->d_in + 2 * d->h1 + 2 * d->h2 + d->d_out);
 }
 
 int check_fused(const ab_mlp_desc* d) {
@@ -392,18 +541,44 @@ int check_fused(const ab_mlp_desc* d) {
   return AB_OK;
 }
 
+// Rows per cluster for a batch of B, 0 for the kernel without clusters.  A cluster
+// kernel's batch is one that is resident at once, up to 32 clusters: 512 rows as 64
+// clusters of eight take 95 us against 54 of the other kernel and its product, 256
+// rows as 64 clusters of four 58 against 36 as 32 of eight.
+int net_rows(const ab_mlp_desc* d, int B) {
+  const size_t row = sizeof(float) * (2 * (size_t)d->d_in + d->h1 + d->h2);
+  for (int G : {4, 8})
+    if (B <= 32 * G && G * row <= 100 * 1024) return G;
+  return 0;
+}
+
+template <int G, bool SUR>
+int launch_net(const ab_mlp_desc* d, int B, const float* x, int ldx, float* y, int ldy, const float* mu,
+               const float* inv_s, const float* a, const float* h, const float* o, const float* M, cudaStream_t st) {
+  const size_t smem = sizeof(float) * G * ((SUR ? 2 : 1) * (size_t)d->d_in + d->h1 + d->h2);
+  AB_CUDA(cudaFuncSetAttribute(mlp_cluster_kernel<G, SUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  mlp_cluster_kernel<G, SUR><<<NET_CTAS * ceil_div(B, G), NET_THREADS, smem, st>>>(
+      B, d->d_in, d->h1, d->h2, d->d_out, x, ldx, static_cast<const __nv_bfloat16*>(d->wb), d->w, y, ldy, mu, inv_s,
+      a, h, o, M);
+  AB_LAUNCH_CHECK("mlp_cluster_kernel");
+  return AB_OK;
+}
+
+// M: only where net_rows is not 0.
 template <bool SUR>
 int launch_fused(const ab_mlp_desc* d, int B, const float* x, int ldx, float* y, int ldy, const float* mu,
-                 const float* inv_s, const float* a, const float* h, const float* o, cudaStream_t st) {
+                 const float* inv_s, const float* a, const float* h, const float* o, const float* M, cudaStream_t st) {
   int rc = check_fused(d);
   if (rc) return rc;
+  const int G = net_rows(d, B);
+  if (G == 4) return launch_net<4, SUR>(d, B, x, ldx, y, ldy, mu, inv_s, a, h, o, M, st);
+  if (G == 8) return launch_net<8, SUR>(d, B, x, ldx, y, ldy, mu, inv_s, a, h, o, M, st);
   const size_t smem = fused_smem(d);
-  AB_CUDA(cudaFuncSetAttribute(mlp_fused_kernel<FUSED_G, SUR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem));
-  mlp_fused_kernel<FUSED_G, SUR><<<ceil_div(B, FUSED_G), 256, smem, st>>>(
+  AB_CUDA(cudaFuncSetAttribute(mlp_rows_kernel<ROWS_G, SUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  mlp_rows_kernel<ROWS_G, SUR><<<ceil_div(B, ROWS_G), 256, smem, st>>>(
       B, d->d_in, d->h1, d->h2, d->d_out, x, ldx, static_cast<const __nv_bfloat16*>(d->wb), d->w, y, ldy, mu, inv_s,
       a, h, o);
-  AB_LAUNCH_CHECK("mlp_fused_kernel");
+  AB_LAUNCH_CHECK("mlp_rows_kernel");
   return AB_OK;
 }
 
@@ -476,7 +651,7 @@ extern "C" int ab_mlp_forward(const ab_mlp_desc* d, int B, const float* x, int l
   AB_REQUIRE(B > 0 && x && y && ldx >= d->d_in && ldy >= d->d_out && ldx % 4 == 0, AB_ERR_ARG,
              "ab_mlp_forward: bad arguments");
   cudaStream_t st = as_stream(stream);
-  if (!act) return launch_fused<false>(d, B, x, ldx, y, ldy, nullptr, nullptr, nullptr, nullptr, nullptr, st);
+  if (!act) return launch_fused<false>(d, B, x, ldx, y, ldy, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, st);
   // the activations are wanted anyway: one tiled product per layer, which
   // spreads every layer over the GPU (three launches, the same values; for a
   // batch of 512 through 512-256-256-512 47 us cold and 49 in the fused kernel,
@@ -499,15 +674,24 @@ extern "C" int ab_mlp_forward(const ab_mlp_desc* d, int B, const float* x, int l
                       nullptr}, nullptr, st);
 }
 
-extern "C" int ab_sur_predict(const ab_mlp_desc* d, int C, const float* theta, int ldt, const float* mu,
-                              const float* inv_s, const float* a, const float* h, const float* o, float* g, int ldg,
-                              void* stream) {
+extern "C" int ab_sur_predict_dense(const ab_mlp_desc* d, int C, const float* theta, int ldt, const float* mu,
+                                    const float* inv_s, const float* a, const float* h, const float* o, const float* M,
+                                    float* g, int ldg, void* stream) {
   int rc = check(d);
   if (rc) return rc;
   AB_REQUIRE(d->d_in == d->d_out, AB_ERR_ARG, "ab_sur_predict: the network must map D to D");
   AB_REQUIRE(C > 0 && theta && mu && inv_s && a && h && o && g && ldt >= d->d_in && ldg >= d->d_out, AB_ERR_ARG,
              "ab_sur_predict: bad arguments");
-  return launch_fused<true>(d, C, theta, ldt, g, ldg, mu, inv_s, a, h, o, as_stream(stream));
+  AB_REQUIRE(!M || net_rows(d, C), AB_ERR_ARG, "ab_sur_predict_dense: batch too large for the dense part in one launch");
+  return launch_fused<true>(d, C, theta, ldt, g, ldg, mu, inv_s, a, h, o, M, as_stream(stream));
+}
+
+extern "C" int ab_sur_dense_fits(const ab_mlp_desc* d, int C) { return d && C > 0 && net_rows(d, C) ? 1 : 0; }
+
+extern "C" int ab_sur_predict(const ab_mlp_desc* d, int C, const float* theta, int ldt, const float* mu,
+                              const float* inv_s, const float* a, const float* h, const float* o, float* g, int ldg,
+                              void* stream) {
+  return ab_sur_predict_dense(d, C, theta, ldt, mu, inv_s, a, h, o, nullptr, g, ldg, stream);
 }
 
 extern "C" int ab_mlp_mse(int B, int D, const float* y, int ldy, const float* target, int ldt, float* dy,

@@ -324,6 +324,8 @@ class MlpSurrogate(Checkpointable):
                 dt=torch.empty((B, D), dtype=torch.float32, device=dev),
                 tgt=torch.empty((B, D), dtype=torch.float32, device=dev),
                 rsq=torch.empty(B, dtype=torch.float64, device=dev),
+                # whether a prediction takes the dense linear part in its one launch
+                dense_fits=bool(N.lib().ab_sur_dense_fits(C.byref(self.desc), B)),
             )
         return self._bufs[B]
 
@@ -382,10 +384,13 @@ class MlpSurrogate(Checkpointable):
         B = theta.shape[0]
         L, st = N.lib(), N.stream_ptr(stream)
         if self.use_net:
-            N.check(L.ab_sur_predict(C.byref(self.desc), B, N.ptr(theta), theta.stride(0), N.ptr(self.mu),
-                                     N.ptr(self.inv_s), N.ptr(self.a), N.ptr(self.h), N.ptr(self.o),
-                                     N.ptr(out_grad), out_grad.stride(0), st), "ab_sur_predict")
-            self._add_dense(theta, out_grad, stream)
+            fits = self.dense and self._scratch(B)["dense_fits"]
+            N.check(L.ab_sur_predict_dense(C.byref(self.desc), B, N.ptr(theta), theta.stride(0), N.ptr(self.mu),
+                                           N.ptr(self.inv_s), N.ptr(self.a), N.ptr(self.h), N.ptr(self.o),
+                                           N.ptr(self.M) if fits else None, N.ptr(out_grad),
+                                           out_grad.stride(0), st), "ab_sur_predict_dense")
+            if self.dense and not fits:
+                self._add_dense(theta, out_grad, stream)
             return out_grad
         sc = self._scratch(B)
         N.check(L.ab_sur_pre(B, self.D, N.ptr(theta), N.ptr(self.mu), N.ptr(self.inv_s), N.ptr(sc["z"]), st),

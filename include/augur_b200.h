@@ -580,6 +580,12 @@ int ab_mlp_sync_bf16(const ab_mlp_desc* d, void* stream);
  * per coordinate, for C rows (d_in == d_out == D). */
 int ab_sur_predict(const ab_mlp_desc* d, int C, const float* theta, int ldt, const float* mu, const float* inv_s,
                    const float* a, const float* h, const float* o, float* g, int ldg, void* stream);
+/* The same plus the dense linear part (theta - mu) M, M [D][D] row-major; NULL for none,
+ * and where ab_sur_dense_fits is 0 (a batch for which a separate product is faster). */
+int ab_sur_dense_fits(const ab_mlp_desc* d, int C);
+int ab_sur_predict_dense(const ab_mlp_desc* d, int C, const float* theta, int ldt, const float* mu, const float* inv_s,
+                         const float* a, const float* h, const float* o, const float* M, float* g, int ldg,
+                         void* stream);
 /* Surrogate input/output maps around the network, per coordinate d:
  *   z = (theta - mu) * inv_s;   g = a + h (theta - mu) + o * out          */
 int ab_sur_pre(int C, int D, const float* theta, const float* mu, const float* inv_s, float* z, void* stream);

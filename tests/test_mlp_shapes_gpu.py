@@ -41,3 +41,30 @@ def test_forward_backward_match_fp64_at_ragged_sizes(D, h1, h2, Bn, pad):
     offs = [0, n1, n1 + h1, n1 + h1 + n2, n1 + h1 + n2 + h2, n1 + h1 + n2 + h2 + D * h2, len(g)]
     for a, b in zip(offs[:-1], offs[1:]):
         assert np.max(np.abs(gd[a:b] - g[a:b])) <= 1e-4 * np.max(np.abs(g[a:b])), (a, b)
+
+
+@pytest.mark.parametrize("D,h1,h2,C,pad", [(8, 8, 8, 1, 0), (16, 256, 256, 128, 0), (40, 32, 64, 129, 4), (136, 72, 264, 256, 0),
+                                           (136, 72, 264, 257, 8), (512, 256, 256, 33, 0), (1600, 24, 16, 130, 0)])
+@pytest.mark.parametrize("dense", [False, True])
+def test_surrogate_prediction_matches_fp64(D, h1, h2, C, pad, dense):
+    # both kernels of the one-launch network, four and eight rows a cluster,
+    # remainders of the rows, of the features and of the lanes; FP32 sums of at
+    # most 1,600 terms against FP64 stay within 1600 * 2^-24 = 1e-4
+    sur = H.MlpSurrogate(D, h1, h2, seed=D + C)
+    gen = torch.Generator("cuda").manual_seed(C)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    for t in (sur.mu, sur.a, sur.h, sur.o):
+        t.copy_(rnd(D))
+    sur.inv_s.copy_(0.5 + rnd(D).abs())
+    sur.dense = dense
+    if dense:
+        sur.M.copy_(rnd(D, D) / D ** 0.5)
+    mem, out = rnd(C, D + pad), torch.full((C, D), float("nan"), device="cuda")
+    theta = mem[:, :D]
+    sur.predict(theta, out)
+    torch.cuda.synchronize()
+    d64 = lambda t: t.double().cpu().numpy()
+    dt = d64(theta) - d64(sur.mu)
+    Y, _ = B.mlp_forward(d64(sur.wb), d64(sur.w), dt * d64(sur.inv_s), D, h1, h2, D)
+    want = d64(sur.a) + d64(sur.h) * dt + d64(sur.o) * Y + (dt @ d64(sur.M) if dense else 0.0)
+    assert np.max(np.abs(d64(out) - want)) <= 1e-4 * np.max(np.abs(want))
