@@ -390,11 +390,11 @@ __global__ void __launch_bounds__(256) mlp_rows_kernel(int B, int din, int h1, i
 // inputs come from shared memory, and a hidden feature's activations go to all
 // eight CTAs' copies.  One CTA per four rows reads every weight row by itself, each lane
 // another row: a surrogate of 512-256-256-512 with its dense linear part as a product
-// of its own takes 47 us at 16 rows, 52 at 64 and 53 at 256; this kernel 15, 22 and
-// 36 (graph replays).  It is bound by its shared-memory reads and weight loads
+// of its own takes 47 us at 16 rows, 52 at 64 and 53 at 256; this kernel 13, 17 and
+// 28 (graph replays).  It is bound by its shared-memory reads and weight loads
 // sharing one pipe, and by the latency of three layers with a cluster barrier each;
-// two features a thread halve the former and measured the same (35 us, and 17 at 16
-// rows).
+// two features a thread halve the former and measured the same (35 us against
+// 36 at 256 rows, and 17 against 15 at 16, before dense_slices).
 constexpr int NET_CTAS = 8, NET_THREADS = 256;
 
 // Lanes per feature when `dout` features of `n` pieces are spread over the cluster: as
@@ -481,6 +481,39 @@ __device__ __forceinline__ void net_layer(const float* in, int din, const __nv_b
   }
 }
 
+// The dense linear part of this CTA's features [j0, j0 + per), per a multiple of 4: a
+// thread takes four neighbouring features and every nsl-th group of four rows of M,
+// so that a warp reads M in whole lines and one 16-byte read of a row's dt serves
+// sixteen products (four in net_layer, whose warps read M in 32-byte pieces): 36 -> 28
+// us at D = 512 and 256 rows, 22.6 -> 17.0 at 64; 21.2 -> 19.9 at D = 256; 16.7 ->
+// 17.4 at D = 128, where 32 and more slices are left to add, hence D >= 256.
+// red[slice][g][feature] receives the slices' sums.
+template <int G>
+__device__ __forceinline__ void dense_slices(const float* dt, const float* __restrict__ M, int D, int j0, int per,
+                                             float* red) {
+  const int quads = per >> 2, nsl = NET_THREADS / quads;
+  const int q = threadIdx.x % quads, slice = threadIdx.x / quads;
+  if (slice >= nsl) return;
+  float4 acc[G];
+#pragma unroll
+  for (int g = 0; g < G; ++g) acc[g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 2
+  for (int k4 = slice; k4 < (D >> 2); k4 += nsl) {
+    const float4* m = reinterpret_cast<const float4*>(M + (size_t)(4 * k4) * D + j0) + q;
+    const float4 m0 = __ldg(m), m1 = __ldg(m + (D >> 2)), m2 = __ldg(m + 2 * (D >> 2)), m3 = __ldg(m + 3 * (D >> 2));
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const float4 a = *reinterpret_cast<const float4*>(dt + g * D + 4 * k4);
+      acc[g].x = fmaf(m3.x, a.w, fmaf(m2.x, a.z, fmaf(m1.x, a.y, fmaf(m0.x, a.x, acc[g].x))));
+      acc[g].y = fmaf(m3.y, a.w, fmaf(m2.y, a.z, fmaf(m1.y, a.y, fmaf(m0.y, a.x, acc[g].y))));
+      acc[g].z = fmaf(m3.z, a.w, fmaf(m2.z, a.z, fmaf(m1.z, a.y, fmaf(m0.z, a.x, acc[g].z))));
+      acc[g].w = fmaf(m3.w, a.w, fmaf(m2.w, a.z, fmaf(m1.w, a.y, fmaf(m0.w, a.x, acc[g].w))));
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < G; ++g) *reinterpret_cast<float4*>(red + ((size_t)slice * G + g) * per + 4 * q) = acc[g];
+}
+
 // SUR: input theta with the surrogate's input map z = (theta - mu) * inv_s, output the
 // gradient estimate a + h (theta - mu) + o * y, plus (theta - mu) M when M is given;
 // otherwise input x, output y.
@@ -522,9 +555,15 @@ __global__ void __cluster_dims__(NET_CTAS, 1, 1) __launch_bounds__(NET_THREADS, 
   net_layer<G>(z, din, wb, w + ob1, h1, rank, nullptr, nullptr, hidden(a1, h1));
   cl.sync();
   net_layer<G>(a1, h1, wb + ow2, w + ob2, h2, rank, nullptr, nullptr, hidden(a2, h2));
+  const int per = dout / NET_CTAS;
+  const bool wide = SUR && M && dout % (4 * NET_CTAS) == 0 && dout >= 256 && (reinterpret_cast<uintptr_t>(M) & 15) == 0;
+  float* red = dt + G * din;
+  if (wide) dense_slices<G>(dt, M, dout, rank * per, per, red);
   cl.sync();
-  net_layer<G>(a2, h2, wb + ow3, w + ob3, dout, rank, dt, SUR ? M : nullptr, [=](int j, int g, float v, float lin) {
+  net_layer<G>(a2, h2, wb + ow3, w + ob3, dout, rank, dt, SUR && !wide ? M : nullptr, [=](int j, int g, float v, float lin) {
     if (r0 + g >= B) return;
+    if (wide)
+      for (int t = 0; t < NET_THREADS / (per >> 2); ++t) lin += red[((size_t)t * G + g) * per + j - rank * per];
     if (SUR) v = sa[j] + sh[j] * dt[g * din + j] + so[j] * v + lin;
     y[(size_t)(r0 + g) * ldy + j] = v;
   });
@@ -544,7 +583,7 @@ int check_fused(const ab_mlp_desc* d) {
 // Rows per cluster for a batch of B, 0 for the kernel without clusters.  A cluster
 // kernel's batch is one that is resident at once, up to 32 clusters: 512 rows as 64
 // clusters of eight take 95 us against 54 of the other kernel and its product, 256
-// rows as 64 clusters of four 58 against 36 as 32 of eight.
+// rows as 64 clusters of four 58 against 36 as 32 of eight (both before dense_slices).
 int net_rows(const ab_mlp_desc* d, int B) {
   const size_t row = sizeof(float) * (2 * (size_t)d->d_in + d->h1 + d->h2);
   for (int G : {4, 8})
@@ -555,7 +594,8 @@ int net_rows(const ab_mlp_desc* d, int B) {
 template <int G, bool SUR>
 int launch_net(const ab_mlp_desc* d, int B, const float* x, int ldx, float* y, int ldy, const float* mu,
                const float* inv_s, const float* a, const float* h, const float* o, const float* M, cudaStream_t st) {
-  const size_t smem = sizeof(float) * G * ((SUR ? 2 : 1) * (size_t)d->d_in + d->h1 + d->h2);
+  const size_t smem = sizeof(float) * G * ((SUR ? 2 : 1) * (size_t)d->d_in + d->h1 + d->h2 +
+                                           (M ? 4 * NET_THREADS : 0));
   AB_CUDA(cudaFuncSetAttribute(mlp_cluster_kernel<G, SUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   mlp_cluster_kernel<G, SUR><<<NET_CTAS * ceil_div(B, G), NET_THREADS, smem, st>>>(
       B, d->d_in, d->h1, d->h2, d->d_out, x, ldx, static_cast<const __nv_bfloat16*>(d->wb), d->w, y, ldy, mu, inv_s,

@@ -44,7 +44,7 @@ def test_forward_backward_match_fp64_at_ragged_sizes(D, h1, h2, Bn, pad):
 
 
 @pytest.mark.parametrize("D,h1,h2,C,pad", [(8, 8, 8, 1, 0), (16, 256, 256, 128, 0), (40, 32, 64, 129, 4), (136, 72, 264, 256, 0),
-                                           (136, 72, 264, 257, 8), (512, 256, 256, 33, 0), (1600, 24, 16, 130, 0)])
+                                           (136, 72, 264, 257, 8), (512, 256, 256, 33, 0), (1600, 24, 16, 130, 0), (1600, 24, 16, 101, 0), (320, 32, 64, 129, 0), (256, 8, 24, 4, 8)])
 @pytest.mark.parametrize("dense", [False, True])
 def test_surrogate_prediction_matches_fp64(D, h1, h2, C, pad, dense):
     # both kernels of the one-launch network, four and eight rows a cluster,
