@@ -986,16 +986,19 @@ gmm_segment_kernel(int d, int K, int seg, int want_sum, int want_obs, const floa
 
 // Component blockIdx.y's rows added: 32 entries per CTA, eight interleaved
 // partial sums of each, then those in order; `add`: onto an earlier slab's.
+// The counts of all but the last slab gather in scratch (so_far): `cnt` is
+// stored once, with the final count, as other streams may be reading the same
+// labels' counts from an earlier pass there.
 __global__ void __launch_bounds__(GMM_THREADS)
 gmm_stats_reduce_kernel(int d, int K, int seg, int want_sum, int want_obs, const double* __restrict__ part,
-                        const int* __restrict__ start, int add, int* __restrict__ cnt, double* __restrict__ sum,
-                        double* __restrict__ obs) {
+                        const int* __restrict__ start, int add, int last, int* __restrict__ so_far,
+                        int* __restrict__ cnt, double* __restrict__ sum, double* __restrict__ obs) {
   __shared__ double red[8][33];
   const int k = blockIdx.y, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   int r0 = 0;
   for (int q = 0; q < k; ++q) r0 += (start[q + 1] - start[q] + seg - 1) / seg;
   const int n = start[k + 1] - start[k], ns = (n + seg - 1) / seg;
-  if (blockIdx.x == 0 && threadIdx.x == 0) cnt[k] = n + (add ? cnt[k] : 0);
+  if (blockIdx.x == 0 && threadIdx.x == 0) (last ? cnt : so_far)[k] = n + (add ? so_far[k] : 0);
   const int W = (want_sum ? d : 0) + (want_obs ? d * (d + 1) / 2 : 0);
   const int e = blockIdx.x * 32 + tx;
   double a = 0.0;
@@ -1567,9 +1570,9 @@ int launch_gmm_prep(int Kc, int d, const double* cov, double* Linv, double* hdet
 }
 
 // Scratch of the statistics: the component order, chunk counts, component
-// starts, and a row of partial sums per segment.
+// starts, the earlier slabs' counts, and a row of partial sums per segment.
 struct GmmStatScratch {
-  size_t perm, cnt, start, part, total;
+  size_t perm, cnt, start, so_far, part, total;
 };
 static GmmStatScratch gmm_stat_layout(int d, int K) {
   GmmStatScratch L;
@@ -1577,7 +1580,8 @@ static GmmStatScratch gmm_stat_layout(int d, int K) {
   L.perm = 0;
   L.cnt = L.perm + sizeof(int) * (size_t)GMM_SLAB;
   L.start = L.cnt + sizeof(int) * (size_t)K * GMM_ORDER_CHUNKS;
-  L.part = L.start + gmm_al256(sizeof(int) * ((size_t)K + 1));
+  L.so_far = L.start + gmm_al256(sizeof(int) * ((size_t)K + 1));
+  L.part = L.so_far + gmm_al256(sizeof(int) * (size_t)K);
   L.total = L.part + sizeof(double) * ((size_t)GMM_SEGMENTS + K) * W;
   return L;
 }
@@ -1592,6 +1596,7 @@ int launch_gmm_stats(int N, int d, int K, const float* Y, const int* z, const do
   int* perm = reinterpret_cast<int*>(base + L.perm);
   int* chunk_cnt = reinterpret_cast<int*>(base + L.cnt);
   int* start = reinterpret_cast<int*>(base + L.start);
+  int* so_far = reinterpret_cast<int*>(base + L.so_far);
   double* part = reinterpret_cast<double*>(base + L.part);
   size_t smem = want_sum ? sizeof(double) * (GMM_THREADS / 32) * GMM_MAX_D : 0;
   if (want_obs) {
@@ -1616,7 +1621,7 @@ int launch_gmm_stats(int N, int d, int K, const float* Y, const int* z, const do
       AB_LAUNCH_CHECK("gmm_segment_kernel");
     }
     gmm_stats_reduce_kernel<<<dim3(std::max(1u, ceil_div(W, 32)), K), GMM_THREADS, 0, st>>>(
-        d, K, seg, want_sum, want_obs, part, start, n0 > 0, cnt, sum, obs);
+        d, K, seg, want_sum, want_obs, part, start, n0 > 0, n0 + n == N, so_far, cnt, sum, obs);
     AB_LAUNCH_CHECK("gmm_stats_reduce_kernel");
   }
   return AB_OK;

@@ -65,6 +65,9 @@ class GmmGibbs(Checkpointable):
         self.obs = torch.zeros((K, d, d), dtype=torch.float64, device=dev)
         self.chi = torch.zeros((K, d), dtype=torch.float64, device=dev)     # Bartlett chi-square sums
         self._side = None
+        # the scatter pass's counts: a buffer of its own, as the side stream
+        # reads `cnt` beside that pass
+        self._cnt_again = torch.zeros(K, dtype=torch.int32, device=dev)
         self.scratch = torch.zeros(int(N.lib().ab_gmm_stats_scratch_bytes(d, K)) // 8 + 1,
                                    dtype=torch.float64, device=dev)
         # the screened assignment draw's tables and queue (ab_gmm_disc_z_screened)
@@ -175,7 +178,8 @@ class GmmGibbs(Checkpointable):
                                          N.ptr(self.sum), N.ptr(self.cov), N.ptr(self.mu), self.seed, it, 0, st),
                         "conj_mu")
                 N.check(L.ab_gmm_stats(self.N, d, K, N.ptr(self.Y), N.ptr(self.z), N.ptr(self.mu),
-                                       N.ptr(self.cnt), None, N.ptr(self.obs), N.ptr(self.scratch), st), "stats")
+                                       N.ptr(self._cnt_again), None, N.ptr(self.obs), N.ptr(self.scratch), st),
+                        "stats")
                 main.wait_event(join)
                 N.check(L.ab_gmm_conj_cov_chi(K, d, self.df, N.ptr(self.scale0), N.ptr(self.cnt),
                                               N.ptr(self.obs), N.ptr(self.chi), N.ptr(self.cov), self.seed, it, 0,

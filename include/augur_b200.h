@@ -270,11 +270,12 @@ int ab_gmm_disc_z_screened(int N, int d, int K, int shared_cov, const float* Y, 
                            const double* mu, const double* Linv, const double* hdet, int* z, uint64_t seed,
                            uint32_t iter, uint32_t comp, void* scratch, void* stream);
 
-/* Conjugate statistics of z (CgConj.hs:186-246): counts cnt int32 [K] always;
+/* Conjugate statistics of z (CgConj.hs:186-246): counts cnt int32 [K] always
+ * (each stored once, when it is final);
  * sum f64 [K][d] of y if `sum` is non-NULL; obs f64 [K][d][d] =
  * sum (y - mu[z])(y - mu[z])^T if `obs` is non-NULL (needs mu).  scratch:
  * ab_gmm_stats_scratch_bytes(d, K) bytes (the points in component order, and
- * rows of partial sums). */
+ * counts and rows of partial sums). */
 size_t ab_gmm_stats_scratch_bytes(int d, int K);
 int ab_gmm_stats(int N, int d, int K, const float* Y, const int* z, const double* mu, int* cnt, double* sum,
                  double* obs, void* scratch, void* stream);

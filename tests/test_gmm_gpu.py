@@ -166,6 +166,66 @@ def test_stats_sizes(orc, N_, K, d):
     np.testing.assert_allclose(g.obs.cpu().numpy(), obs, rtol=1e-12, atol=1e-8)
 
 
+SLAB = 1 << 20     # points the statistics take at a time
+
+
+@pytest.mark.parametrize("N_,K,d", [(SLAB, 3, 2), (SLAB + 1, 3, 2), (2 * SLAB + 700, 5, 3)])
+def test_stats_of_several_slabs(N_, K, d):
+    """Statistics of exactly one, and of more, slabs of points: counts and, as
+    the points are small integers, sums and scatter matrices without any
+    rounding, over stale outputs; the last component appears only in the
+    last points and one label is not a component."""
+    rng = np.random.default_rng(N_ % 1000 + d)
+    Y = rng.integers(-4, 5, (N_, d))
+    z = rng.integers(0, K - 1, N_)
+    z[-1] = K - 1
+    z[N_ // 3] = -1
+    mus = rng.integers(-2, 3, (K, d))
+    t = lambda a, dt: torch.as_tensor(np.ascontiguousarray(a), dtype=dt).cuda()
+    Yt, zt, mt = t(Y, torch.float32), t(z, torch.int32), t(mus, torch.float64)
+    cnt = torch.full((K,), 77, dtype=torch.int32, device="cuda")
+    s = torch.full((K, d), 7.0, dtype=torch.float64, device="cuda")
+    obs = torch.full((K, d, d), 7.0, dtype=torch.float64, device="cuda")
+    L = N.lib()
+    scratch = torch.full((int(L.ab_gmm_stats_scratch_bytes(d, K)),), 0x5b, dtype=torch.uint8, device="cuda")
+    N.check(L.ab_gmm_stats(N_, d, K, N.ptr(Yt), N.ptr(zt), N.ptr(mt), N.ptr(cnt), N.ptr(s), N.ptr(obs), N.ptr(scratch),
+                           N.stream_ptr()), "stats")
+    for k in range(K):
+        y = Y[z == k]
+        c = y - mus[k]
+        assert int(cnt[k]) == len(y)
+        np.testing.assert_array_equal(s[k].cpu().numpy(), y.sum(0))
+        np.testing.assert_array_equal(obs[k].cpu().numpy(), c.T @ c)
+
+
+def test_sweep_of_several_slabs_equals_one_stream():
+    """A sweep of more points than a slab and 1024 chi-square sums (more than
+    run at once) beside the scatter pass equals the same draws made one after
+    the other on one stream."""
+    N_, K, d = SLAB + 50_000, 64, 16
+    rng = np.random.default_rng(5)
+    mus = 4.0 * rng.standard_normal((K, d))
+    z = rng.integers(0, K, N_).astype(np.int32)
+    Y = (mus[z] + rng.standard_normal((N_, d))).astype(np.float32)
+    mk = lambda: GmmGibbs(Y, K, np.zeros(d), 25 * np.eye(d), alpha=np.ones(K), df=d + 2, mu=mus, z=z, seed=6)
+    a, b = mk(), mk()
+    L = N.lib()
+    st = N.stream_ptr()
+    for it in range(2):
+        a.sweep(1)
+        p = N.ptr
+        N.check(L.ab_gmm_stats(N_, d, K, p(b.Y), p(b.z), None, p(b.cnt), p(b.sum), None, p(b.scratch), st))
+        N.check(L.ab_gmm_conj_pis(K, p(b.alpha), p(b.cnt), p(b.pis), 6, it, 0, st))
+        N.check(L.ab_gmm_conj_mu(K, d, 0, p(b.mu0), p(b.cov0), p(b.cnt), p(b.sum), p(b.cov), p(b.mu), 6, it, 0, st))
+        N.check(L.ab_gmm_stats(N_, d, K, p(b.Y), p(b.z), p(b.mu), p(b.cnt), None, p(b.obs), p(b.scratch), st))
+        N.check(L.ab_gmm_conj_cov(K, d, d + 2, p(b.scale0), p(b.cnt), p(b.obs), p(b.cov), 6, it, 0, st))
+        N.check(L.ab_gmm_prep(K, d, p(b.cov), p(b.Linv), p(b.hdet), st))
+        N.check(L.ab_gmm_disc_z_screened(N_, d, K, 0, p(b.Y), p(b.pis), p(b.mu), p(b.Linv), p(b.hdet), p(b.z), 6, it, 0,
+                                         p(b.zscratch), st))
+        for name in ("pis", "mu", "cov", "z", "cnt"):
+            assert torch.equal(getattr(a, name), getattr(b, name)), (it, name)
+
+
 def test_hmvgmm_sweeps_per_sweep_contract(orc):
     N_, K, d = 1500, 4, 5
     Y, z, mus, covs, pis, om = hmodel(N_, K, d, 11)
