@@ -62,33 +62,49 @@ struct Tri {
   }
 };
 
-// sqrt(x) and 1 / sqrt(x)'s rounded root, both correctly rounded: the
-// reciprocal root (CUDA's rsqrt, within an ulp) gives the root by one
-// residual step and seeds the reciprocal, which a second one rounds
-// (Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990).  Far shorter a chain than a square root and a
-// division in turn; values outside its range take those.
-__device__ __forceinline__ void root_recip(double x, double& root, double& rec) {
-  if (x > 0x1p-900 && x < 0x1p900) {
-    const double y = rsqrt(x);
-    const double g = __dmul_rn(x, y);
-    root = __fma_rn(__fma_rn(-g, g, x), __dmul_rn(0.5, y), g);
-    rec = __fma_rn(__fma_rn(-root, y, 1.0), y, y);
-  } else {
-    root = __dsqrt_rn(x);
-    rec = __ddiv_rn(1.0, root);
-  }
+// Whether 2^-n <= |v| < 2^n, from the exponent field.
+__device__ __forceinline__ bool within_2(double v, int n) {
+  return ((unsigned)__double2hiint(v) >> 20 & 0x7ffu) - (unsigned)(1023 - n) < (unsigned)(2 * n);
 }
 
-// b / v given rec = 1 / v correctly rounded: the quotient's residual rounds it
-// correctly (the same theorem) while nothing under- or overflows.
-__device__ __forceinline__ double quotient(double b, double v, double rec) {
-  const double ab = fabs(b), av = fabs(v);
-  if ((ab > 0x1p-400 && ab < 0x1p400 && av > 0x1p-400 && av < 0x1p400) || b == 0.0) {
-    const double q = __dmul_rn(b, rec);
-    return __fma_rn(__fma_rn(-q, v, b), rec, q);
-  }
-  return __ddiv_rn(b, v);
+// Whether e, the residual b - v q rounded once, shows q to be b / v correctly
+// rounded: |e| < |v| times half the distance from q to its nearer neighbour.
+// That bound is v with another exponent (everything in range, as |v q| is near
+// |b|), and below it e is exact.  For a root, v = q and twice the bound
+// (b - q^2 is a multiple of the distance's square).  Integer operations: the
+// binary64 pipe is what the callers' chains wait for.
+template <int HALF>
+__device__ __forceinline__ bool rounds_to(double e, double v, double q) {
+  const int hq = __double2hiint(q);
+  const bool pow2 = ((hq & 0xfffff) | __double2loint(q)) == 0;   // the neighbour below is half as far
+  const int hb = (__double2hiint(v) & 0x7fffffff) + (hq & 0x7ff00000) - ((1023 + 52 + HALF + (pow2 ? 1 : 0)) << 20);
+  return (__double_as_longlong(e) & 0x7fffffffffffffffll) < __double_as_longlong(__hiloint2double(hb, __double2loint(v)));
+}
+
+// sqrt(x) and the reciprocal of that root; true if both are known to be
+// correctly rounded.  CUDA's reciprocal root (within an ulp) gives the root by
+// one residual step and seeds the reciprocal, which a second one rounds (after
+// Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990): far shorter a chain than a square root and a division in
+// turn.  The steps alone do not round every value correctly (a root just below
+// a power of two, for one), hence the tests, whose result the caller needs
+// only once it has used the values: they run beside that use.
+__device__ __forceinline__ bool root_recip(double x, double& root, double& rec) {
+  const double y = rsqrt(x);
+  const double g = __dmul_rn(x, y);
+  root = __fma_rn(__fma_rn(-g, g, x), __dmul_rn(0.5, y), g);
+  rec = __fma_rn(__fma_rn(-root, y, 1.0), y, y);
+  return __double2hiint(x) > 0 && within_2(x, 900) && rounds_to<0>(__fma_rn(-root, root, x), root, root) &&
+         rounds_to<1>(__fma_rn(-root, rec, 1.0), root, rec);
+}
+
+// b / v given rec = 1 / v correctly rounded, from the quotient's residual
+// (after the same paper); true if it is known to be correctly rounded.
+__device__ __forceinline__ bool quotient(double b, double v, double rec, double& q) {
+  q = __dmul_rn(b, rec);
+  if (b == 0.0) return within_2(v, 400);
+  q = __fma_rn(__fma_rn(-q, v, b), rec, q);
+  return within_2(v, 400) && within_2(b, 400) && rounds_to<1>(__fma_rn(-q, v, b), v, q);
 }
 
 // augur_mat_cholesky (:312-328) of A, in place (lower triangle; the upper one
@@ -97,7 +113,9 @@ __device__ __forceinline__ double quotient(double b, double v, double rec) {
 // same walk: once column k of the factor is final, so is row k of its inverse.
 // Entry (i, j) first sums A[i][k] A[j][k] over k < j, becomes final at k = j,
 // then subtracts L[i][k] O[k][j] over j <= k < i from the identity's entry and
-// gives O[i][j] at k = i.  piv: [d] scratch.
+// gives O[i][j] at k = i.  piv: [d] scratch.  A column whose root, reciprocal or
+// quotients are not known to be correctly rounded is formed again with the
+// square root and divisions.
 template <int NE, bool INV>
 __device__ __forceinline__ void g_factor(const Tri<NE>& T, double* A, double* O, double* piv, int d) {
   double acc[NE];
@@ -111,17 +129,34 @@ __device__ __forceinline__ void g_factor(const Tri<NE>& T, double* A, double* O,
       if (T.ij[q] == (k << 8 | k)) piv[k] = __dadd_rn(GP(A, k, k), -acc[q]);
     __syncthreads();
     double root, rec;
-    root_recip(piv[k], root, rec);
+    bool ok = root_recip(piv[k], root, rec);
 #pragma unroll
     for (int q = 0; q < NE; ++q) {
       const int i = T.ij[q] >> 8, j = T.ij[q] & 255;
       if (T.ij[q] < 0) continue;
       if (j == k) {
-        GP(A, i, k) = i == k ? root : __dmul_rn(rec, __dadd_rn(GP(A, i, k), -acc[q]));
+        acc[q] = __dadd_rn(GP(A, i, k), -acc[q]);
+        GP(A, i, k) = i == k ? root : __dmul_rn(rec, acc[q]);
         if (INV && i == k) GP(O, k, k) = rec;
-        acc[q] = 0.0;
       } else if (INV && i == k) {
-        GP(O, k, j) = quotient(acc[q], root, rec);
+        double b;
+        ok &= quotient(acc[q], root, rec, b);
+        GP(O, k, j) = b;
+      }
+    }
+    if (!ok) {
+      root = __dsqrt_rn(piv[k]);
+      rec = __ddiv_rn(1.0, root);
+#pragma unroll
+      for (int q = 0; q < NE; ++q) {
+        const int i = T.ij[q] >> 8, j = T.ij[q] & 255;
+        if (T.ij[q] < 0) continue;
+        if (j == k) {
+          GP(A, i, k) = i == k ? root : __dmul_rn(rec, acc[q]);
+          if (INV && i == k) GP(O, k, k) = rec;
+        } else if (INV && i == k) {
+          GP(O, k, j) = __ddiv_rn(acc[q], root);
+        }
       }
     }
     __syncthreads();
@@ -130,7 +165,7 @@ __device__ __forceinline__ void g_factor(const Tri<NE>& T, double* A, double* O,
       const int i = T.ij[q] >> 8, j = T.ij[q] & 255;
       if (T.ij[q] < 0 || i <= k || (!INV && j <= k)) continue;
       const double p = __dmul_rn(GP(A, i, k), j > k ? GP(A, j, k) : GP(O, k, j));
-      acc[q] = __dadd_rn(acc[q], j > k ? p : -p);
+      acc[q] = __dadd_rn(j == k ? 0.0 : acc[q], j > k ? p : -p);
     }
   }
   __syncthreads();
@@ -149,7 +184,12 @@ __device__ __forceinline__ void g_trmi(const Tri<NE>& T, const double* L, double
   for (int r = 0; r < d; ++r) {
 #pragma unroll
     for (int q = 0; q < NE; ++q)
-      if (T.ij[q] >= 0 && (T.ij[q] >> 8) == r) GP(O, r, T.ij[q] & 255) = quotient(b[q], GP(L, r, r), recs[r]);
+      if (T.ij[q] >= 0 && (T.ij[q] >> 8) == r) {
+        double o;
+        const bool ok = quotient(b[q], GP(L, r, r), recs[r], o);
+        GP(O, r, T.ij[q] & 255) = o;
+        if (!ok) GP(O, r, T.ij[q] & 255) = __ddiv_rn(b[q], GP(L, r, r));
+      }
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < NE; ++q) {

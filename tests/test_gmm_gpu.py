@@ -131,6 +131,100 @@ def test_factorisations_at_the_edges_of_the_dimension_ranges(orc, d):
     np.testing.assert_allclose(cov.cpu().numpy(), want, rtol=1e-9, atol=1e-9 * np.abs(want).max())
 
 
+def _tables(A):
+    """augur_mat_cholesky then augur_mat_lower_trmi of the matrices A [K][d][d]
+    in the reference's order of operations (numpy's are IEEE binary64)."""
+    L = A.copy()
+    K, d, _ = L.shape
+    for j in range(d):
+        s = np.zeros(K)
+        for k in range(j):
+            s = s + L[:, j, k] * L[:, j, k]
+        L[:, j, j] = np.sqrt(L[:, j, j] - s)
+        r = 1.0 / L[:, j, j]
+        for i in range(j + 1, d):
+            s = np.zeros(K)
+            for k in range(j):
+                s = s + L[:, i, k] * L[:, j, k]
+            L[:, i, j] = r * (L[:, i, j] - s)
+    M = np.zeros_like(L)
+    for c in range(d):
+        for m in range(c, d):
+            b = np.full(K, 1.0 if c == m else 0.0)
+            for i in range(c, m):
+                b = b - L[:, m, i] * M[:, i, c]
+            M[:, m, c] = b / L[:, m, m]
+    return M
+
+
+def _device_tables(A):
+    K, d, _ = A.shape
+    cov = torch.as_tensor(np.ascontiguousarray(A)).cuda()
+    Linv = torch.full((K, d, d), float("nan"), dtype=torch.float64, device="cuda")
+    hdet = torch.zeros(K, dtype=torch.float64, device="cuda")
+    N.check(N.lib().ab_gmm_prep(K, d, N.ptr(cov), N.ptr(Linv), N.ptr(hdet), N.stream_ptr()), "prep")
+    return Linv.cpu().numpy()
+
+
+def test_roots_reciprocals_and_quotients_are_correctly_rounded():
+    """Component tables of diagonal matrices (a reciprocal of a root an entry)
+    and of 2 x 2 blocks (a quotient each) equal IEEE arithmetic bit for bit:
+    random values of a wide range, values beside powers of four (whose roots
+    are beside powers of two), beside squares, and beyond the short steps'
+    range."""
+    rng = np.random.default_rng(8)
+    K, d = 64, 64
+    n = K * d
+    j = np.arange(1.0, 33.0)
+    edges = np.concatenate([4.0 ** e * np.concatenate([1.0 - j * 2.0 ** -53, 1.0 + j * 2.0 ** -52, [1.0]])
+                            for e in (-440, -60, -1, 0, 1, 2, 60, 440)])
+    sq = rng.integers(2 ** 26, 2 ** 27, 2000).astype(np.float64) ** 2
+    edges = np.concatenate([edges, sq, np.nextafter(sq, 0.0), np.nextafter(sq, np.inf), 2.0 ** rng.uniform(-1000, -900, 500),
+                            2.0 ** rng.uniform(900, 1000, 500)])
+    pool = [np.resize(edges, -(-len(edges) // n) * n).reshape(-1, K, d)]
+    pool.append(np.exp2(rng.uniform(-40, 40, (40, K, d))))
+    for x in np.concatenate(pool):
+        A = np.zeros((K, d, d))
+        A[:, np.arange(d), np.arange(d)] = x
+        got = _device_tables(A)
+        np.testing.assert_array_equal(got[:, np.arange(d), np.arange(d)], 1.0 / np.sqrt(x))
+        assert np.count_nonzero(got) == n
+    i = 2 * np.arange(d // 2)
+    for rep in range(40):
+        A = np.zeros((K, d, d))
+        a, c = np.exp2(rng.uniform(-20, 20, (2, K, d // 2)))
+        if rep < 8:
+            a = np.nextafter(4.0 ** rng.integers(-3, 4, a.shape), 0.0)
+        b = np.sqrt(a * c) * rng.uniform(-0.999, 0.999, a.shape)
+        if rep < 8:
+            c = np.nextafter(4.0 ** rng.integers(-3, 4, a.shape), 0.0) + (b / np.sqrt(a)) ** 2
+        A[:, i, i], A[:, i + 1, i], A[:, i, i + 1], A[:, i + 1, i + 1] = a, b, b, c
+        got = _device_tables(A)
+        r0 = 1.0 / np.sqrt(a)
+        l10 = r0 * b
+        l11 = np.sqrt(c - l10 * l10)
+        np.testing.assert_array_equal(got[:, i, i], r0)
+        np.testing.assert_array_equal(got[:, i + 1, i + 1], 1.0 / l11)
+        np.testing.assert_array_equal(got[:, i + 1, i], -(l10 * r0) / l11)
+    # zero over an infinite pivot is zero
+    np.testing.assert_array_equal(_device_tables(np.diag([1.0, np.inf])[None]), [[[1.0, 0.0], [0.0, 0.0]]])
+
+
+@pytest.mark.parametrize("d", [1, 7, 16, 33])
+def test_component_tables_bit_exact(d):
+    """Tables of covariances, and of correlation-like ones whose diagonal is
+    just below 1, equal the reference's order of operations bit for bit."""
+    rng = np.random.default_rng(d)
+    K = 48
+    A = rng.standard_normal((K, d, d + 3))
+    cov = np.einsum("kij,klj->kil", A, A) / (d + 3) + 0.1 * np.eye(d)
+    sd = np.sqrt(np.einsum("kii->ki", cov))
+    cor = 0.5 * cov / (sd[:, :, None] * sd[:, None, :])
+    cor[:, np.arange(d), np.arange(d)] = np.nextafter(1.0, 0.0)
+    for m in (cov, cor):
+        np.testing.assert_array_equal(_device_tables(m), _tables(m))
+
+
 @pytest.mark.parametrize("N_,K,d", [(300_000, 16, 32), (250_000, 3, 40), (1, 2, 3), (900, 16, 2)])
 def test_stats_sizes(orc, N_, K, d):
     """Statistics at sizes where a CTA's chunk spans several shared-memory
