@@ -1415,11 +1415,14 @@ gmm_move_kernel(int N, int d, int shared_cov, const float* __restrict__ Y, const
     for (int r = 1; r < GMM_MOVE_CLUSTER; ++r) n += *cl.map_shared_rank(&count, r);
   cl.sync();                 // the other CTAs' shared memory has been read
   if (rank > 0 || tid >= 32) return;
+  bool finite = true;                        // S is, unless a point or the mean is not
   for (int i = lane; i < d; i += 32) {       // R = P S
     double a = 0.0;
     for (int j = 0; j <= i; ++j) a = __fma_rn(GP(P, i, j), x[j], a);
     R[i] = a;
+    finite = finite && isfinite(x[i]);
   }
+  finite = __all_sync(0xffffffffu, finite);
   __syncwarp();
   double q0, unused;
   for (int i = lane; i < d; i += 32) x[i] = __dadd_rn(cur[i], -mu0s[i]);
@@ -1428,7 +1431,7 @@ gmm_move_kernel(int N, int d, int shared_cov, const float* __restrict__ Y, const
   // a density that is not finite at any point rejects every candidate, as its
   // comparison would
   const double scale = (n > 0 ? hdet[kc] : 0.0) + hdet[prior_slot];
-  const double bad = isfinite(scale) ? 0.0 : NAN;
+  const double bad = finite && isfinite(scale) ? 0.0 : NAN;
   // log density at `m` minus the one at the current mean
   auto gain = [&](const double* m) {
     double q1, sq, dot;

@@ -395,6 +395,34 @@ def test_mean_moves_at_ragged_sizes(orc, move, N_, K, d):
         np.testing.assert_allclose(g.mu.cpu().numpy(), want, rtol=1e-9, atol=1e-9)
 
 
+@pytest.mark.parametrize("move", ["eslice", "mwg"])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_mean_moves_beside_a_point_that_is_not_finite(orc, move, value):
+    """A component with such a point has no finite density anywhere: its mean
+    stays where it is, as in the oracle; the other component moves."""
+    N_, K = 200, 2
+    for d in (1, 3):
+        rng = np.random.default_rng(d)
+        z = (np.arange(N_) % K).astype(np.int32)
+        Y = rng.standard_normal((N_, d)).astype(np.float32)
+        Y[4, d - 1] = value
+        om = O.GmmModel(Y.astype(np.float64), K, np.zeros(d), 4 * np.eye(d), True)
+        cov, prop = np.eye(d), 0.02 * np.eye(d)
+        g = GmmGibbs(Y, K, np.zeros(d), 4 * np.eye(d), pis=np.full(K, 0.5), covs=cov, mu=np.zeros((K, d)), z=z, move=move,
+                     prop_cov=prop, seed=5)
+        moved = 0
+        for it in range(6):
+            prev = g.mu.cpu().numpy()
+            g.z.copy_(torch.as_tensor(z))
+            g.sweep(1)
+            got = g.mu.cpu().numpy()
+            want = O.gmm_eslice(orc, om, prev, cov, z, 5, it) if move == "eslice" else O.gmm_mwg(orc, om, prev, cov, z, prop, 5, it)
+            np.testing.assert_array_equal(got[0], prev[0])
+            np.testing.assert_allclose(got, want, rtol=1e-9, atol=1e-9)
+            moved += bool((got[1] != prev[1]).any())
+        assert moved > 0
+
+
 def test_bench_shape_properties():
     """K=16, d=32, N=2e5 (the benchmark shape): statistics sum to N, the
     covariances stay symmetric positive definite, assignments recover most
