@@ -369,9 +369,10 @@ __device__ __forceinline__ double normal_ll(const HlrModelDev& m, double pt, dou
   if (!(var > 0.0)) return -INFINITY;
   return -0.5 * log(2.0 * 3.14159265358979323846 * var) - 0.5 * t * t / var;
 }
-// d/dvar of the former at mean 0, iv = 1 / var.
+// d/dvar of the former at mean 0, iv = 1 / var, whose square may be out of range.
 __device__ __forceinline__ double normal_dvar(const HlrModelDev& m, double t, double var, double iv) {
-  return (m.compat ? -0.5 * var : -0.5 * iv) + 0.5 * (t * t) * (iv * iv);
+  const double ti = t * iv;
+  return (m.compat ? -0.5 * var : -0.5 * iv) + 0.5 * (ti * ti);
 }
 __device__ __forceinline__ double vprior_ll(const HlrModelDev& m, double v) {
   if (m.vprior == 0) return (m.lam > 0.0 && v > 0.0) ? m.vp_const - m.lam * v : (m.compat ? -1e8 : -INFINITY);
@@ -380,7 +381,7 @@ __device__ __forceinline__ double vprior_ll(const HlrModelDev& m, double v) {
 }
 __device__ __forceinline__ double vprior_dot(const HlrModelDev& m, double v, double iv) {
   if (m.vprior == 0) return (m.lam > 0.0 && v > 0.0) ? -m.lam : 0.0;
-  return -(m.a0 + 1.0) * iv + m.s0 * (iv * iv);
+  return -(m.a0 + 1.0) * iv + (m.s0 * iv) * iv;
 }
 
 __device__ __forceinline__ BlockInfo block_info(const HlrModelDev& m, const int* idx, int P) {

@@ -128,6 +128,26 @@ def test_chain_paths_match_oracle(orc, N, D, xd, C, kind):
         np.testing.assert_allclose(got[c], p, rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("compat", [True, False])
+@pytest.mark.parametrize("vprior", ["exponential", "invgamma"])
+@pytest.mark.parametrize("v", [1e-158, 1e-156, 3e-155, 1e-100, 1e150])
+def test_variance_gradient_at_the_ends_of_the_range(v, vprior, compat):
+    """The prior's derivative in the variance where 1 / v^2 is out of binary64's
+    range and the derivative is not: some coefficients zero, some far below
+    the root of v, an inverse-gamma scale as small."""
+    D = 7
+    s0 = v * v * 2.0 ** 90
+    gd = H.HlrData(np.ones((3, D)), np.array([0, 1, 1]), has_b=True, vprior=vprior, lam=0.5, a0=2.0, s0=s0, compat=compat)
+    par = np.zeros((1, D + 2))
+    par[0, 2], par[0, D] = 0.25 * v * 2.0 ** 60, -3.0 * v
+    par[0, D + 1] = v
+    _, g = H.ll_grad(gd, par, [D + 1])
+    q = np.array([par[0, 2], par[0, D]]) / v
+    want = (D + 1) * (-0.5 * v if compat else -0.5 / v) + 0.5 * (q * q).sum()
+    want += -0.5 if vprior == "exponential" else -3.0 / v + s0 / v / v
+    np.testing.assert_allclose(g[0, 0], want, rtol=1e-12)
+
+
 def test_hmc_many_chains_distinct_streams(orc):
     X, y, beta, s2, om, gd = make(400, 5, 6, False, "invgamma", True)
     D = 5
