@@ -1,6 +1,10 @@
 // Library-wide C ABI: error reporting and version.
 #include <string.h>
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include "common.cuh"
 
 namespace ab {
@@ -17,6 +21,20 @@ int fail(int code, const char* fmt, ...) {
 
 int cuda_status(cudaError_t e, const char* what) {
   return fail(AB_ERR_CUDA, "%s: %s (%s)", what, cudaGetErrorString(e), cudaGetErrorName(e));
+}
+
+cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  static std::mutex lock;
+  static std::map<std::pair<int, const void*>, size_t> limits;   // one entry a kernel and device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const std::lock_guard<std::mutex> hold(lock);
+  size_t& limit = limits[{dev, kernel}];
+  if (bytes <= limit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) limit = bytes;
+  return e;
 }
 
 }  // namespace ab

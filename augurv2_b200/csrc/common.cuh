@@ -17,6 +17,14 @@ int fail(int code, const char* fmt, ...);
 // Converts a CUDA error into a status, recording where it came from.
 int cuda_status(cudaError_t e, const char* what);
 
+// Lets `kernel` be launched with `bytes` of dynamic shared memory on the
+// current device.  The limit belongs to the kernel in the whole process, so it
+// is only ever raised, and under a lock: if every call set its own size, one of
+// a smaller shape could lower the limit between another thread's setting and
+// its launch, which would then be refused.  For kernels whose size depends on
+// the call.
+cudaError_t allow_smem(const void* kernel, size_t bytes);
+
 #define AB_CUDA(call)                                           \
   do {                                                          \
     cudaError_t _e = (call);                                    \

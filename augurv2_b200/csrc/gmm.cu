@@ -1547,7 +1547,7 @@ template <int DT>
 static int launch_zs_t(int N, int d, int K, const float* Y, const float* tab, const int* perm, const int* flag,
                        int* queue, int* qn, int* z, uint64_t seed, uint32_t iter, uint32_t comp, cudaStream_t st) {
   const size_t smem = gmm_zs_smem(d, K);
-  AB_CUDA(cudaFuncSetAttribute(gmm_zs_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)gmm_zs_kernel<DT>, smem));
   const int vec = d % 4 == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
   const unsigned grid = std::min(ceil_div(N, 64), 148u * 3u);   // few points: a warp's tile each
   gmm_zs_kernel<DT><<<grid, GMM_ZS_THREADS, smem, st>>>(N, d, K, vec, Y, tab, perm, flag, queue, qn, z, seed, iter, comp);
@@ -1600,7 +1600,7 @@ int launch_gmm_z_screened(int N, int d, int K, int shared, const float* Y, const
 template <int DT>
 static int launch_prep_t(int Kc, int d, const double* cov, double* Linv, double* hdet, cudaStream_t st) {
   const size_t smem = sizeof(double) * 2 * (size_t)d * pitch(d);
-  AB_CUDA(cudaFuncSetAttribute(gmm_prep_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)gmm_prep_kernel<DT>, smem));
   gmm_prep_kernel<DT><<<Kc, GMM_THREADS, smem, st>>>(d, cov, Linv, hdet);
   AB_LAUNCH_CHECK("gmm_prep_kernel");
   return AB_OK;
@@ -1649,7 +1649,7 @@ int launch_gmm_stats(int N, int d, int K, const float* Y, const int* z, const do
   const int pts_at = (int)(smem / sizeof(double));   // then the segment's points
   smem += sizeof(int) * (size_t)std::max(32, (int)ceil_div(std::min(N, GMM_SLAB), GMM_SEGMENTS));
   const auto segments = d <= 16 ? gmm_segment_kernel<16> : d <= 32 ? gmm_segment_kernel<32> : gmm_segment_kernel<64>;
-  AB_CUDA(cudaFuncSetAttribute(segments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)segments, smem));
   for (int n0 = 0; n0 < N; n0 += GMM_SLAB) {
     const int n = std::min(GMM_SLAB, N - n0);
     const int chunks = (int)ceil_div(n, GMM_ORDER_CHUNK);
@@ -1675,7 +1675,7 @@ static int launch_conj_mu_t(int K, int d, int shared, const double* mu0, const d
                             const double* sum, const double* cov, double* mu, uint64_t seed, uint32_t iter,
                             uint32_t comp, cudaStream_t st) {
   const size_t smem = sizeof(double) * (4 * (size_t)d * pitch(d) + 6 * (size_t)d);
-  AB_CUDA(cudaFuncSetAttribute(gmm_conj_mu_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)gmm_conj_mu_kernel<DT>, smem));
   gmm_conj_mu_kernel<DT><<<K, GMM_THREADS, smem, st>>>(d, shared, mu0, cov0, cnt, sum, cov, mu, seed, iter, comp);
   AB_LAUNCH_CHECK("gmm_conj_mu_kernel");
   return AB_OK;
@@ -1705,7 +1705,7 @@ static int launch_conj_cov_t(int K, int d, int df, const double* scale0, const i
                              const double* chi, int sk, int si, double* cov, uint64_t seed, uint32_t iter,
                              uint32_t comp, cudaStream_t st) {
   const size_t smem = sizeof(double) * 4 * (size_t)d * pitch(d);
-  AB_CUDA(cudaFuncSetAttribute(gmm_conj_cov_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)gmm_conj_cov_kernel<DT>, smem));
   gmm_conj_cov_kernel<DT><<<K, GMM_THREADS, smem, st>>>(d, df, scale0, cnt, obs, chi, sk, si, cov, seed, iter, comp);
   AB_LAUNCH_CHECK("gmm_conj_cov_kernel");
   return AB_OK;
@@ -1738,7 +1738,7 @@ static int launch_move_t(int N, int d, int K, int shared, const float* Y, const 
   const size_t tables = sizeof(double) * 3 * (size_t)d * pitch(d);
   const size_t sums = (GMM_THREADS / 32) * (sizeof(double) * GMM_MAX_D + sizeof(int) * GMM_MOVE_BATCH);
   const size_t smem = std::max(tables, sums);
-  AB_CUDA(cudaFuncSetAttribute(gmm_move_kernel<DT, SLICE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)gmm_move_kernel<DT, SLICE>, smem));
   gmm_move_kernel<DT, SLICE><<<K * GMM_MOVE_CLUSTER, GMM_THREADS, smem, st>>>(
       N, d, shared, Y, z, mu0, cov, Linv, hdet, prior_slot, prop_slot, compat, mu, seed, iter, comp, tally);
   AB_LAUNCH_CHECK("gmm_move_kernel");

@@ -1062,7 +1062,7 @@ extern "C" int ab_hlr_ll_grad(const ab_hlr_model* model, const int* idx_dev, con
   const auto kernel = m.D + 2 <= 16           ? hlr_ll_grad_kernel<16>
                       : m.D + 2 <= SMALL_COLS ? hlr_ll_grad_kernel<SMALL_COLS>
                                               : hlr_ll_grad_kernel<0>;
-  AB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)kernel, smem));
   kernel<<<C, HLR_BLOCK, smem, as_stream(stream)>>>(m, l, idx_dev, P, pars, ll, grad);
   AB_LAUNCH_CHECK("hlr_ll_grad_kernel");
   return AB_OK;
@@ -1103,7 +1103,7 @@ extern "C" int ab_hlr_run_chains(const ab_hlr_model* model, const ab_hlr_comp* c
   AB_REQUIRE(smem <= 224 * 1024, AB_ERR_ARG, "hlr: D too large for the per-chain engine");
   const auto kernel = m.D + 2 <= 16 ? chain_kernel<16>(l.res) : m.D + 2 <= SMALL_COLS ? chain_kernel<SMALL_COLS>(l.res)
                                                                                        : chain_kernel<0>(l.res);
-  AB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)kernel, smem));
   kernel<<<C, HLR_BLOCK, smem, as_stream(stream)>>>(m, l, reinterpret_cast<const HlrComp*>(comps_dev), n_comps, idx_dev,
                                                     pars, n_iter, iter0, seed, stats,
                                                     reinterpret_cast<double*>(scratch), m.D + 2);

@@ -596,7 +596,7 @@ int launch_net(const ab_mlp_desc* d, int B, const float* x, int ldx, float* y, i
                const float* inv_s, const float* a, const float* h, const float* o, const float* M, cudaStream_t st) {
   const size_t smem = sizeof(float) * G * ((SUR ? 2 : 1) * (size_t)d->d_in + d->h1 + d->h2 +
                                            (M ? 4 * NET_THREADS : 0));
-  AB_CUDA(cudaFuncSetAttribute(mlp_cluster_kernel<G, SUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)mlp_cluster_kernel<G, SUR>, smem));
   mlp_cluster_kernel<G, SUR><<<NET_CTAS * ceil_div(B, G), NET_THREADS, smem, st>>>(
       B, d->d_in, d->h1, d->h2, d->d_out, x, ldx, static_cast<const __nv_bfloat16*>(d->wb), d->w, y, ldy, mu, inv_s,
       a, h, o, M);
@@ -614,7 +614,7 @@ int launch_fused(const ab_mlp_desc* d, int B, const float* x, int ldx, float* y,
   if (G == 4) return launch_net<4, SUR>(d, B, x, ldx, y, ldy, mu, inv_s, a, h, o, M, st);
   if (G == 8) return launch_net<8, SUR>(d, B, x, ldx, y, ldy, mu, inv_s, a, h, o, M, st);
   const size_t smem = fused_smem(d);
-  AB_CUDA(cudaFuncSetAttribute(mlp_rows_kernel<ROWS_G, SUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  AB_CUDA(allow_smem((const void*)mlp_rows_kernel<ROWS_G, SUR>, smem));
   mlp_rows_kernel<ROWS_G, SUR><<<ceil_div(B, ROWS_G), 256, smem, st>>>(
       B, d->d_in, d->h1, d->h2, d->d_out, x, ldx, static_cast<const __nv_bfloat16*>(d->wb), d->w, y, ldy, mu, inv_s,
       a, h, o);
