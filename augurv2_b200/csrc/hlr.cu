@@ -907,6 +907,41 @@ __device__ Ws carve(void* base, int N, int D, const HlrLayout& l, double*& stk) 
   return w;
 }
 
+// X and the labels into shared memory, STAGE_DEPTH values of a thread in flight
+// (a row a warp, one load after another, took 45 us for 1000 x 10 values, as
+// long as ten evaluations).
+constexpr int STAGE_DEPTH = 8;
+template <typename T>
+__device__ __forceinline__ void stage_rows(const HlrModelDev& m, const T* __restrict__ X, T* xs, int pitch) {
+  const int N = m.N, D = m.D, di = HLR_BLOCK / D, dk = HLR_BLOCK % D;
+  int i = threadIdx.x / D, k = threadIdx.x % D;
+  while (i < N) {
+    T v[STAGE_DEPTH];
+    int at[STAGE_DEPTH];
+#pragma unroll
+    for (int u = 0; u < STAGE_DEPTH; ++u) {
+      at[u] = i < N ? i * pitch + k : -1;
+      if (i < N) v[u] = X[(size_t)i * m.ldx + k];
+      i += di;
+      k += dk;
+      if (k >= D) { k -= D; ++i; }
+    }
+#pragma unroll
+    for (int u = 0; u < STAGE_DEPTH; ++u)
+      if (at[u] >= 0) xs[at[u]] = v[u];
+  }
+}
+__device__ __forceinline__ void stage_labels(const HlrModelDev& m, int* lab) {
+  for (int i0 = threadIdx.x; i0 < m.N; i0 += STAGE_DEPTH * HLR_BLOCK) {
+    int v[STAGE_DEPTH];
+#pragma unroll
+    for (int u = 0; u < STAGE_DEPTH; ++u) v[u] = load_label(m, min(i0 + u * HLR_BLOCK, m.N - 1));
+#pragma unroll
+    for (int u = 0; u < STAGE_DEPTH; ++u)
+      if (i0 + u * HLR_BLOCK < m.N) lab[i0 + u * HLR_BLOCK] = v[u];
+  }
+}
+
 // One CTA per chain: n_iter iterations of the schedule `comps`.
 // stats[c][ci][5] = {accepts, sum depth, sum leaves, errors, divergent iterations}.
 // Bound: the chain of one evaluation - barriers, the compensated sums of a
@@ -925,15 +960,9 @@ hlr_chain_kernel(const __grid_constant__ HlrModelDev m, HlrLayout l, const HlrCo
   Ws ws = carve(smem_d, m.N, m.D, l, stk);
   const int c = blockIdx.x;
   if (!l.stk) stk = nuts_stk + (size_t)c * 3 * HLR_STK * stk_P;
-  if (RES) {
-    for (int i = threadIdx.x >> 5; i < m.N; i += HLR_BLOCK / 32)
-      for (int k = threadIdx.x & 31; k < m.D; k += 32) {
-        const size_t at = (size_t)i * m.ldx + k;
-        if (RES == X_F32) static_cast<float*>(ws.xs)[i * l.xpitch + k] = static_cast<const float*>(m.X)[at];
-        else static_cast<__nv_bfloat16*>(ws.xs)[i * l.xpitch + k] = static_cast<const __nv_bfloat16*>(m.X)[at];
-      }
-    for (int i = threadIdx.x; i < m.N; i += HLR_BLOCK) ws.lab[i] = load_label(m, i);
-  }
+  if (RES == X_F32) stage_rows(m, static_cast<const float*>(m.X), static_cast<float*>(ws.xs), l.xpitch);
+  if (RES == X_BF16) stage_rows(m, static_cast<const __nv_bfloat16*>(m.X), static_cast<__nv_bfloat16*>(ws.xs), l.xpitch);
+  if (RES) stage_labels(m, ws.lab);
   double* par_g = pars + (size_t)c * (m.D + 2);
   for (int i = threadIdx.x; i < m.D + 2; i += blockDim.x) ws.par[i] = par_g[i];
   __syncthreads();
@@ -1013,14 +1042,16 @@ static int make_model(HlrModelDev& m, const ab_hlr_model* d) {
   return AB_OK;
 }
 
-// What a chain's CTA keeps in shared memory: X and the labels, and the NUTS
-// stacks, where they fit - 224 KB with an SM to itself, 112 KB when there are
-// more chains than SMs and two share one.  Every evaluation then reads X from
-// there instead of walking it through the caches.
-static HlrLayout choose_layout(const HlrModelDev& m, int C, bool nuts) {
+// What a chain's CTA keeps in shared memory: X and the labels, if a component
+// evaluates the data, and the NUTS stacks, where they fit - 224 KB with an SM
+// to itself, 112 KB when there are more chains than SMs and two share one.
+// Every evaluation then reads X from there instead of walking it through the
+// caches.
+static HlrLayout choose_layout(const HlrModelDev& m, int C, bool nuts, bool data) {
   const size_t room = (C > 148 ? 112 : 224) * 1024;
   HlrLayout l{X_GLOBAL, 0, nuts, nuts};
   if (hlr_layout_bytes(m.N, m.D, l) > room) l.stk = 0;
+  if (!data) return l;
   HlrLayout k = l;
   k.res = m.x_bf16 ? X_BF16 : X_F32;
   k.xpitch = m.x_bf16 ? 2 * (((m.D + 1) / 2) | 1) : (m.D | 1);
@@ -1080,7 +1111,7 @@ extern "C" int ab_hlr_run_chains(const ab_hlr_model* model, const ab_hlr_comp* c
              HLR_MAX_COMPS);
   AB_REQUIRE(comps_host && comps_dev && idx_dev && idx_host && pars && stats, AB_ERR_ARG,
              "ab_hlr_run_chains: null pointer");
-  bool has_nuts = false;
+  bool has_nuts = false, data = false;
   for (int i = 0; i < n_comps; ++i) {
     const ab_hlr_comp& c = comps_host[i];
     AB_REQUIRE(c.kind >= 0 && c.kind <= 3, AB_ERR_ARG, "component %d: unknown kind", i);
@@ -1095,10 +1126,11 @@ extern "C" int ab_hlr_run_chains(const ab_hlr_model* model, const ab_hlr_comp* c
     rc = check_idx_host(idx_host + c.idx_off, c.P, m.D);
     if (rc) return rc;
     has_nuts |= c.kind == 1;
+    for (int j = 0; j < c.P; ++j) data |= idx_host[c.idx_off + j] < m.D + (m.has_b ? 1 : 0);
   }
   AB_REQUIRE(!has_nuts || scratch, AB_ERR_ARG, "ab_hlr_run_chains: NUTS needs scratch");
   static_assert(sizeof(ab_hlr_comp) == sizeof(HlrComp), "component layout");
-  const HlrLayout l = choose_layout(m, C, has_nuts);
+  const HlrLayout l = choose_layout(m, C, has_nuts, data);
   const size_t smem = hlr_layout_bytes(m.N, m.D, l);
   AB_REQUIRE(smem <= 224 * 1024, AB_ERR_ARG, "hlr: D too large for the per-chain engine");
   const auto kernel = m.D + 2 <= 16 ? chain_kernel<16>(l.res) : m.D + 2 <= SMALL_COLS ? chain_kernel<SMALL_COLS>(l.res)

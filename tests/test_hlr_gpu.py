@@ -128,6 +128,39 @@ def test_chain_paths_match_oracle(orc, N, D, xd, C, kind):
         np.testing.assert_allclose(got[c], p, rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("N,D,xd,C", [(9, 3, "f32", 1), (1000, 10, "bf16", 2), (1500, 20, "f32", 150), (300, 33, "f32", 1),
+                                      (9001, 9, "f32", 2), (900, 120, "bf16", 150), (4000, 60, "f32", 1)])
+def test_slice_and_metropolis_moves_on_every_path(orc, N, D, xd, C):
+    """Reflective-slice and Metropolis moves with X in shared memory (f32,
+    bf16) or too large for it, 16, 32 and more columns, one or more chains an
+    SM: the first and the last chain's moves equal the oracle's.  A component
+    a launch, so that every chain starts from the oracle's state; an FP32
+    data term may flip one decision of the lot."""
+    X, y, beta, s2, om, gd = make(N, D, N + D, True, "exponential", True, xd)
+    theta = H.block_indices(["theta"], D)
+    eps = 0.4 / np.sqrt(N + 10.0)
+    par = np.concatenate([beta, [0.1], [max(s2, 0.5)]])
+    agree = total = 0
+    for it in range(4):
+        for comp in ({"kind": "RSlice", "block": ["theta"], "simlen": 4 * eps, "eps": eps},
+                     {"kind": "MWG", "var": "b", "scale": 0.05}, {"kind": "MWG", "var": "v", "scale": 0.3}):
+            got, st = run_one(gd, [comp], par, it, 31, C)
+            refs = {}
+            for c in {0, C - 1}:
+                p = par.copy()
+                if comp["kind"] == "RSlice":
+                    moved = O.hlr_rslice(orc, om, p, theta, 4 * eps, eps, 31, it, chain=c)[0]
+                else:
+                    moved = O.hlr_mwg(orc, om, p, D if comp["var"] == "b" else D + 1, comp["scale"], 31, it, chain=c)
+                refs[c] = p
+                total += 1
+                if int(st[c, 0, 0]) == moved:
+                    agree += 1
+                    np.testing.assert_allclose(got[c], p, rtol=1e-4, atol=1e-6)
+            par = refs[0]
+    assert agree >= total - 1
+
+
 @pytest.mark.parametrize("compat", [True, False])
 @pytest.mark.parametrize("vprior", ["exponential", "invgamma"])
 @pytest.mark.parametrize("v", [1e-158, 1e-156, 3e-155, 1e-100, 1e150])
