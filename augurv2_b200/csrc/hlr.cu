@@ -1043,19 +1043,22 @@ static int make_model(HlrModelDev& m, const ab_hlr_model* d) {
 }
 
 // What a chain's CTA keeps in shared memory: X and the labels, if a component
-// evaluates the data, and the NUTS stacks, where they fit - 224 KB with an SM
-// to itself, 112 KB when there are more chains than SMs and two share one.
+// evaluates the data, and the NUTS stacks, where they fit 224 KB (an SM holds
+// one CTA, whatever its shared memory: 288 threads of 155 to 168 registers).
 // Every evaluation then reads X from there instead of walking it through the
 // caches.
-static HlrLayout choose_layout(const HlrModelDev& m, int C, bool nuts, bool data) {
-  const size_t room = (C > 148 ? 112 : 224) * 1024;
+static HlrLayout choose_layout(const HlrModelDev& m, bool nuts, bool data) {
+  const size_t room = 224 * 1024;
+  const auto fits = [&](const HlrLayout& l) { return hlr_layout_bytes(m.N, m.D, l) <= room; };
+  if (data) {
+    HlrLayout x{m.x_bf16 ? X_BF16 : X_F32, m.x_bf16 ? 2 * (((m.D + 1) / 2) | 1) : (m.D | 1), nuts, nuts};
+    if (fits(x)) return x;
+    x.stk = 0;
+    if (fits(x)) return x;
+  }
   HlrLayout l{X_GLOBAL, 0, nuts, nuts};
-  if (hlr_layout_bytes(m.N, m.D, l) > room) l.stk = 0;
-  if (!data) return l;
-  HlrLayout k = l;
-  k.res = m.x_bf16 ? X_BF16 : X_F32;
-  k.xpitch = m.x_bf16 ? 2 * (((m.D + 1) / 2) | 1) : (m.D | 1);
-  return hlr_layout_bytes(m.N, m.D, k) <= room ? k : l;
+  if (!fits(l)) l.stk = 0;
+  return l;
 }
 
 template <int COLS>
@@ -1130,7 +1133,7 @@ extern "C" int ab_hlr_run_chains(const ab_hlr_model* model, const ab_hlr_comp* c
   }
   AB_REQUIRE(!has_nuts || scratch, AB_ERR_ARG, "ab_hlr_run_chains: NUTS needs scratch");
   static_assert(sizeof(ab_hlr_comp) == sizeof(HlrComp), "component layout");
-  const HlrLayout l = choose_layout(m, C, has_nuts, data);
+  const HlrLayout l = choose_layout(m, has_nuts, data);
   const size_t smem = hlr_layout_bytes(m.N, m.D, l);
   AB_REQUIRE(smem <= 224 * 1024, AB_ERR_ARG, "hlr: D too large for the per-chain engine");
   const auto kernel = m.D + 2 <= 16 ? chain_kernel<16>(l.res) : m.D + 2 <= SMALL_COLS ? chain_kernel<SMALL_COLS>(l.res)

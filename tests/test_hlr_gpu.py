@@ -161,6 +161,24 @@ def test_slice_and_metropolis_moves_on_every_path(orc, N, D, xd, C):
     assert agree >= total - 1
 
 
+@pytest.mark.parametrize("N,D,xd,C", [(200, 300, "bf16", 1), (200, 300, "bf16", 150), (1600, 28, "f32", 150), (700, 300, "f32", 2)])
+def test_nuts_with_rows_or_stacks_in_shared_memory(orc, N, D, xd, C):
+    """NUTS where shared memory holds X but not the walk's stacks, the stacks
+    but not X, or both, for fewer and more chains than SMs: the first and the
+    last chain's trees and states equal the oracle's."""
+    X, y, beta, s2, om, gd = make(N, D, N + D, True, "exponential", True, xd)
+    block = ["v", "b", "theta"]
+    idx = H.block_indices(block, D)
+    par = np.concatenate([0.5 * beta, [0.1], [1.0]])
+    eps = 0.2 / np.sqrt(N + 10.0)
+    got, st = run_one(gd, [{"kind": "NUTS", "block": block, "eps": eps, "max_depth": 3}], par, 0, 23, C)
+    for c in {0, C - 1}:
+        p = par.copy()
+        depth = O.hlr_nuts(orc, om, p, idx, eps, 23, 0, max_depth=3, chain=c)[0]
+        assert int(st[c, 0, 1]) == depth
+        np.testing.assert_allclose(got[c], p, rtol=1e-4, atol=1e-5)
+
+
 @pytest.mark.parametrize("compat", [True, False])
 @pytest.mark.parametrize("vprior", ["exponential", "invgamma"])
 @pytest.mark.parametrize("v", [1e-158, 1e-156, 3e-155, 1e-100, 1e150])
