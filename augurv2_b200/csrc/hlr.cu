@@ -454,13 +454,6 @@ __device__ __forceinline__ double block_eval(const HlrModelDev& m, bool want_ll,
   return ll;
 }
 
-// The same as a call, for the moves that evaluate a few times an iteration.
-template <int RES, int COLS>
-__device__ __noinline__ double block_eval_call(const HlrModelDev& m, bool want_ll, bool want_grad, const double* par,
-                                               const BlockInfo bi, int P, Ws& ws) {
-  return block_eval<RES, COLS>(m, want_ll, want_grad, par, bi, P, ws);
-}
-
 __device__ __forceinline__ void set_block(double* par, const int* idx, int P, const double* q) {
   for (int j = threadIdx.x; j < P; j += blockDim.x) par[idx[j]] = q[j];
   __syncthreads();
@@ -812,25 +805,35 @@ __device__ int rslice_transition(const HlrModelDev& m, const HlrComp& cp, const 
   const double expo = ws.bcast[3];
   const int L = ws.ibcast[0];
   const double step = cp.eps;
-  const double z = block_eval_call<RES, COLS>(m, true, false, ws.par, bi, P, ws) - expo;
   for (int j = tid; j < P; j += blockDim.x) ws.q[j] = ws.par[idx[j]];
-  __syncthreads();
+  // l = 0: the log density at the current state; then at each of L points, and
+  // where it is outside the slice (cond) the gradient there: one evaluation a
+  // turn, so that the kernel holds its code once
   bool cond = false;
   int refl = 0;
-  for (int l = 0; l < L; ++l) {
-    for (int j = tid; j < P; j += blockDim.x) ws.q[j] = __dadd_rn(ws.q[j], __dmul_rn(step, ws.p0[j]));
-    __syncthreads();
-    set_block(ws.prop, idx, P, ws.q);
-    cond = block_eval_call<RES, COLS>(m, true, false, ws.prop, bi, P, ws) < z;    // same value on every thread
+  double z = 0.0;
+  for (int l = 0;;) {
+    const double ll = block_eval<RES, COLS>(m, !cond, cond, l == 0 ? ws.par : ws.prop, bi, P, ws);
     if (cond) {
-      block_eval_call<RES, COLS>(m, false, true, ws.prop, bi, P, ws);
       const double a1 = block_dot(ws.p0, ws.blk_g, P, ws);
       const double a2 = block_dot(ws.blk_g, ws.blk_g, P, ws);
       const double sc = __dmul_rn(-2.0, a1 / a2);
       for (int j = tid; j < P; j += blockDim.x) ws.p0[j] = __dadd_rn(ws.p0[j], __dmul_rn(sc, ws.blk_g[j]));
       __syncthreads();
       ++refl;
+      if (l == L) break;
+      cond = false;
+    } else if (l == 0) {
+      z = ll - expo;
+    } else {
+      cond = ll < z;                     // same value on every thread
+      if (cond) continue;
+      if (l == L) break;
     }
+    for (int j = tid; j < P; j += blockDim.x) ws.q[j] = __dadd_rn(ws.q[j], __dmul_rn(step, ws.p0[j]));
+    __syncthreads();
+    set_block(ws.prop, idx, P, ws.q);
+    ++l;
   }
   if (!cond)
     for (int i = tid; i < m.D + 2; i += blockDim.x) ws.par[i] = ws.prop[i];
@@ -856,8 +859,12 @@ __device__ int mwg_transition(const HlrModelDev& m, const HlrComp& cp, const Blo
   __syncthreads();
   if (threadIdx.x == 0) ws.prop[which] = ws.bcast[3];
   __syncthreads();
-  const double lc = block_eval_call<RES, COLS>(m, true, false, ws.par, bi, 1, ws);
-  const double lp = block_eval_call<RES, COLS>(m, true, false, ws.prop, bi, 1, ws);
+  double lc = 0.0, lp = 0.0;
+#pragma unroll 1
+  for (int l = 0; l < 2; ++l) {
+    lc = lp;
+    lp = block_eval<RES, COLS>(m, true, false, l == 0 ? ws.par : ws.prop, bi, 1, ws);
+  }
   const int acc = log(ws.bcast[4]) < lp - lc + ws.bcast[5];
   if (acc && threadIdx.x == 0) ws.par[which] = ws.prop[which];
   __syncthreads();
