@@ -848,12 +848,14 @@ int launch_lda_zf(int D, int K, int V, int Kp, const int* doc_off, const int* w,
 // topics before k the reference does not stop before k, and if also s_k > u norm
 // (1 + m) - off it stops at k - the draw equals the reference's.  A u within the
 // margin of a boundary (about 2 (2K + 32) u of the draws, 1e-5 at K = 50), or a
-// norm outside [2^-60, FLT_MAX], runs the reference's binary64 loop on the
-// binary64 theta and phi rows (lda_reference_draw).
+// norm outside [2^-60, FLT_MAX], is drawn in binary64 from the binary64 theta
+// and phi rows (lda_warp_draw).
 // Counts of the new z as lda_zq_kernel.
 // Measured at K = 130, V = 5003, 1.9e5 tokens in 611 documents: 90 -> 70 us, the
-// whole sweep 126 -> 105; bound by the
-// rows' round trips at 16 warps per SM.  At K = 50 this form took 39-51 us
+// whole sweep 134 -> 113; bound by the rows' round trips at 16 warps per SM.
+// Faster than the binary64 kernel down to a single document (450 shapes with K
+// = 65 to 256, 1 to 400 documents of 10 to 1500 tokens: sweep 0.5 to 0.99 of its
+// time).  At K = 50 this form took 39-51 us
 // against 36 for the staged one, which K <= 64 keeps: short rows leave the
 // staged kernel twice the warps.  With a whole warp per token (K = 500, 100
 // documents) the sweep took 287 us against 220 of lda_z_kernel, hence K <= 256.
@@ -861,12 +863,64 @@ int launch_lda_zf(int D, int K, int V, int Kp, const int* doc_off, const int* w,
 constexpr int LDA_ZR_MAX_THREADS = 256;
 constexpr int LDA_ZR_MAX_K = 256;
 
-// Warps per document: 16 warps per SM over all documents, at most 8, so that few
-// documents do not leave the SMs idle and many short ones do not wait for idle
-// warps.
+// A token that binary32 does not decide, by a whole warp: token_draw's binary64
+// test with eight topics a lane (running sums grouped by lanes, which its margin
+// covers), and the reference's loop only where that does not decide either.
+// The loop alone is a chain of K divisions on one lane, longer than the rest
+// of the draw of a small corpus, and about every second sweep of 10^4 tokens has
+// such a token: with it, K = 256 and 297 documents of 30 tokens, a sweep took
+// 121 us, 91 with this.
+__device__ __noinline__ int lda_warp_draw(int K, const double* __restrict__ th, const double* __restrict__ row,
+                                          double u) {
+  constexpr int PER = LDA_ZR_MAX_K / 32;
+  const int lane = threadIdx.x & 31;
+  double c[PER];
+#pragma unroll
+  for (int e = 0; e < PER; ++e) {
+    const int k = PER * lane + e;
+    c[e] = k < K ? __dmul_rn(th[k], row[k]) : 0.0;
+  }
+#pragma unroll
+  for (int e = 1; e < PER; ++e) c[e] = __dadd_rn(c[e - 1], c[e]);
+  double incl = c[PER - 1];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double a = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl = __dadd_rn(a, incl);
+  }
+  const double norm = __shfl_sync(0xffffffffu, incl, 31);
+  double off = __shfl_up_sync(0xffffffffu, incl, 1);
+  if (lane == 0) off = 0.0;
+  if (norm >= 1e-290 && norm <= 1.7976931348623157e308) {
+    const double m = (6.0 * K + 32.0) * 1.1102230246251565e-16;
+    const double lo = 1.0 - m, hi = 1.0 + m, un = __dmul_rn(u, norm);
+    int first = -1;                       // the lane's first topic at which the reference may stop
+    bool sure = false;                    // and does
+#pragma unroll
+    for (int e = 0; e < PER; ++e) {
+      const int k = PER * lane + e;
+      const double ck = __dadd_rn(off, c[e]);
+      if (first < 0 && k < K - 1 && un <= __dmul_rn(ck, hi)) {
+        first = k;
+        sure = un < __dmul_rn(ck, lo);
+      }
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, first >= 0);
+    if (bal == 0u) return K - 1;
+    const int win = __ffs(bal) - 1;
+    if (__shfl_sync(0xffffffffu, (int)sure, win)) return __shfl_sync(0xffffffffu, first, win);
+  }
+  return lda_reference_draw(K, th, row, u);
+}
+
+// Warps per document: the most with which all documents run at once, 16 warps
+// per SM (128 registers), at least 2 and at most 8.  At D = 400 documents of 30
+// tokens, K = 128, the sweep takes 51.9 us with 4 and 57.5 with the 8 that would
+// wait for a second wave (300 tokens: 68 and 78); at D = 1000 55.7 with 2 and
+// 60.9 with 4 (89 and 95).
 static inline int lda_zr_warps(int D) {
-  int nw = 2;
-  while (nw < LDA_ZR_MAX_THREADS / 32 && (long long)D * nw < 148 * 16) nw *= 2;
+  int nw = LDA_ZR_MAX_THREADS / 32;
+  while (nw > 2 && (long long)D * nw > 148 * 16) nw /= 2;
   return nw;
 }
 
@@ -915,7 +969,9 @@ lda_zr_kernel(int D, int K, int V, int Kp, const int* __restrict__ doc_off,
       f[q] = at < row_quads ? __ldg(row + at) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   };
-  int tb = t0 + warp * 32;
+  // tokens a warp takes at a time: 32, or what spreads a short document over the warps
+  const int chunk = min(32, ((t1 - t0 + NW - 1) / NW + 2 * PER - 1) / (2 * PER) * (2 * PER));
+  int tb = t0 + warp * chunk;
   auto draw = [&](const float4 (&f)[UQ], int wt, float uf, int st) {
         const int tok = st * PER + grp;
         const float u = __shfl_sync(0xffffffffu, uf, tok);
@@ -956,31 +1012,36 @@ lda_zr_kernel(int D, int K, int V, int Kp, const int* __restrict__ doc_off,
         const unsigned mine = (bal >> (grp * G)) & ((1u << G) - 1u);
         const int win = mine ? __ffs(mine) - 1 : G - 1;
         const int t = tb + tok;
-        if (j == win && t < t1) {
-          int zk = mine ? min(4 * UQ * j + pos, K - 1) : K - 1;
-          const bool exact = !(norm >= 8.673617379884035e-19f && norm <= 3.4028234663852886e38f) ||   // [2^-60, FLT_MAX]
-                             (zk < K - 1 && !(nxt > T2));
-          if (exact) {
-            Stream se = make_stream(seed, (uint32_t)t, iter, TAG_Z);
-            zk = lda_reference_draw(K, th64, phiT + (size_t)wt * Kp, se.uniform());
-          }
+        const bool mark = j == win && t < t1;
+        int zk = mine ? min(4 * UQ * j + pos, K - 1) : K - 1;
+        const bool exact = !(norm >= 8.673617379884035e-19f && norm <= 3.4028234663852886e38f) ||   // [2^-60, FLT_MAX]
+                           (zk < K - 1 && !(nxt > T2));
+        for (unsigned open = __ballot_sync(0xffffffffu, mark && exact); open; open &= open - 1u) {
+          const int src = __ffs(open) - 1;
+          const int ws = __shfl_sync(0xffffffffu, wt, src);
+          Stream se = make_stream(seed, (uint32_t)__shfl_sync(0xffffffffu, t, src), iter, TAG_Z);
+          const int zs = lda_warp_draw(K, th64, phiT + (size_t)ws * Kp, se.uniform());
+          if (lane == src) zk = zs;
+        }
+        if (mark) {
           z[t] = zk;
           atomicAdd(&hist[zk], 1);
           if (cnt_kw != nullptr) atomicAdd(cnt_kw + (size_t)zk * V + wt, 1);
         }
   };
-  int wc = tb + lane < t1 ? w[tb + lane] : 0;
+  auto ids = [&](int at) { return lane < chunk && at + lane < t1 ? w[at + lane] : 0; };
+  int wc = ids(tb);
   load(f0, w0, wc, 0);
-  for (; tb < t1; tb += NW * 32) {
-    const int wn = tb + NW * 32 + lane < t1 ? w[tb + NW * 32 + lane] : 0;   // the next chunk's ids
+  for (; tb < t1; tb += NW * chunk) {
+    const int wn = ids(tb + NW * chunk);   // the next chunk's ids
     Stream s = make_stream(seed, (uint32_t)(tb + lane), iter, TAG_Z);
     const float uf = __double2float_rn(s.uniform());
     // a step's rows are loaded while the step before it is drawn
 #pragma unroll 1
-    for (int st = 0; st < G && tb + st * PER < t1; st += 2) {
+    for (int st = 0; st * PER < chunk && tb + st * PER < t1; st += 2) {
       load(f1, w1, wc, st + 1);
       draw(f0, w0, uf, st);
-      if (st + 2 < G) load(f0, w0, wc, st + 2);
+      if ((st + 2) * PER < chunk) load(f0, w0, wc, st + 2);
       else load(f0, w0, wn, 0);
       draw(f1, w1, uf, st + 1);
     }
@@ -1297,11 +1358,7 @@ static int lda_enqueue_sweep(ab_lda* h, cudaStream_t main, cudaStream_t side) {
   const ab_lda_desc& d = h->d;
   uint32_t* iter_dev = reinterpret_cast<uint32_t*>(d.scratch);
   uint32_t* done = iter_dev + 1;
-  // Past K = 64 the screened draw needs enough documents to fill the SMs: at K =
-  // 140 with 20 documents the sweep takes 42 us against 43, at K = 192 with 40
-  // of them 88 against 86, at K = 250 with 60 132 against 119; with 611
-  // documents 107 against 126 at K = 130 and 184 against 246 at K = 256.
-  const bool screened = d.K <= LDA_ZQ_MAX_K || (d.K <= LDA_ZR_MAX_K && d.D >= (d.K <= 192 ? 148 : 2 * 148));
+  const bool screened = d.K <= LDA_ZR_MAX_K;
   float* phi32 = screened
                      ? reinterpret_cast<float*>(static_cast<char*>(d.scratch) + lda_phi32_offset(d.K, d.V))
                      : nullptr;

@@ -326,3 +326,34 @@ def test_sweep_screen_equals_binary64(K):
                                 N.ptr(kw), K, it, N.stream_ptr()), "disc_z")
         assert torch.equal(s.z, z)
         assert torch.equal(s.cnt_dk, dk) and torch.equal(s.cnt_kw, kw)
+
+
+@pytest.mark.parametrize("K,D,alpha,beta", [(65, 1, 0.1, 0.01), (128, 40, 0.1, 0.01), (130, 297, 0.1, 0.01), (256, 700, 0.1, 0.01),
+                                            (70, 60, 0.002, 0.002), (129, 400, 0.003, 0.002), (256, 90, 0.001, 0.001),
+                                            (200, 700, 1e-4, 1e-4)])
+def test_sweep_screen_of_short_documents_and_tiny_weights(K, D, alpha, beta):
+    """The screened draw past K = 64 with 2, 4 and 8 warps a document, on empty
+    documents and ones shorter than a warp's share; and with so small
+    hyper-parameters that norms leave binary32's range, vanish or overflow
+    nothing but the reference's loop: z and its counts equal the binary64
+    kernel's on the sweep's own theta and phi."""
+    V = 157
+    rng = np.random.default_rng(K + D)
+    lens = rng.integers(0, 45, D)
+    lens[-1] = 700
+    if D > 4:
+        lens[:4] = [0, 1, 33, 0]
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    w = rng.integers(0, V, off[-1]).astype(np.int32)
+    z0 = rng.integers(0, K, off[-1]).astype(np.int32)
+    s = LdaGibbs(K, V, off, w, alpha, beta, seed=K, z=z0)
+    L = N.lib()
+    for it in range(2):
+        s.sweep(1)
+        z = torch.zeros_like(s.z)
+        dk, kw = torch.zeros_like(s.cnt_dk), torch.zeros_like(s.cnt_kw)
+        N.check(L.ab_lda_disc_z(D, K, V, N.ptr(s.doc_off), N.ptr(s.w), N.ptr(s.theta), N.ptr(s.phiT), N.ptr(z), N.ptr(dk),
+                                N.ptr(kw), K, it, N.stream_ptr()), "disc_z")
+        assert torch.equal(s.z, z)
+        assert torch.equal(s.cnt_dk, dk) and torch.equal(s.cnt_kw, kw)
+    s.close()
