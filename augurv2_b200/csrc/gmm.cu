@@ -317,7 +317,7 @@ gmm_z_kernel(int N, int d, int K, int shared_cov, const float* __restrict__ Y, c
 //   gmm_zs_prep_kernel  per component (once per call): the lower triangle of
 //                       Linv_k and mu_k rounded to binary32, and the constants
 //                       of the error bound below; log(pis_k) + c - hdet_k;
-//   gmm_zs_kernel       two points a thread: t_k = log p_k in binary32 with a
+//   gmm_zs_kernel       one or two points a thread: t_k = log p_k in binary32 with a
 //                       rigorous bound eps_k on its error against the exact
 //                       value, p_k / p_max = exp(t_k - t_max), the running
 //                       sums, and the reference's draw when u lies outside the
@@ -355,6 +355,7 @@ gmm_z_kernel(int N, int d, int K, int shared_cov, const float* __restrict__ Y, c
 // c - hdet_k > 700, take the exact path.
 constexpr int GMM_ZS_MAXK = 32;
 constexpr int GMM_ZS_THREADS = 128;
+constexpr int gmm_zs_ctas(int DT, int H) { return H == 2 ? 3 : DT <= 8 ? 10 : 5; }   // per SM
 
 // Per component, floats: L~ with row i padded to whole float4s (zeros) at
 // gmm_zs_row(i), then a, mh and ml, each padded to whole float4s (zeros), then
@@ -438,20 +439,25 @@ __device__ __forceinline__ unsigned long long pack2(float x, float y) {
 __device__ __forceinline__ float lo2(unsigned long long a) { return __uint_as_float((unsigned)a); }
 __device__ __forceinline__ float hi2(unsigned long long a) { return __uint_as_float((unsigned)(a >> 32)); }
 
-// A thread takes two points at a time, so that every 16-byte read of the
-// factor's rows (a shared-memory broadcast) feeds eight multiply-adds, and
-// pairs of a row's columns go through one packed multiply-add: 338 -> 210 us
-// for N = 200,000, K = 16, d = 32, where one point a thread with scalar
-// operations waited for the factor reads and for the conversions of a
-// binary64 y - mu.  Warps walk the points 64 at a time over a grid of three
-// CTAs per SM, each of which reads the tables once.
-template <int DT>
-__global__ void __launch_bounds__(GMM_ZS_THREADS, 3)
+// H = 1: a point a thread, pairs of a row's columns in one packed multiply-add,
+// five CTAs per SM: 370 -> 235 us for the whole draw at N = 200,000, K = 16, d =
+// 32, where scalar operations on a binary64 y - mu took most of the time.  Up to
+// d = 8 the exponentials and running sums are most of the work, and ten CTAs per
+// SM faster than the registers of five (K = 30, d = 2, N = 400,000: 104 and 117 us).
+// H = 2: two points a thread, so that every 16-byte read of the factor's rows
+// (a shared-memory broadcast) feeds eight multiply-adds, at three CTAs per SM.
+// Only in label order, where most of the work is left out: 155 us there with
+// components apart, 171 with H = 1.  Without the order it is slower than H = 1 at
+// every size (252 us there; 63 against 46 at N = 3,000, K = 30, d = 12).
+// Warps walk the points 32 H at a time; each CTA reads the tables once.
+template <int DT, int H>
+__global__ void __launch_bounds__(GMM_ZS_THREADS, gmm_zs_ctas(DT, H))
 gmm_zs_kernel(int N, int d, int K, int vec, const float* __restrict__ Y, const float* __restrict__ tab,
-              const int* __restrict__ perm, const int* __restrict__ flag, int* __restrict__ queue, int* __restrict__ qn, int* __restrict__ z,
-              uint64_t seed, uint32_t iter, uint32_t comp) {
+              const int* __restrict__ perm, const int* __restrict__ flag, int* __restrict__ queue, int* __restrict__ qn,
+              int* __restrict__ z, uint64_t seed, uint32_t iter, uint32_t comp) {
   extern __shared__ __align__(16) float ts[];   // the K components' tables
   constexpr int DW = (DT + 3) / 4 * 4;          // whole float4s of row entries
+  constexpr bool ORDERED = H == 2;              // the points in the order of their labels (perm)
   const int stride = gmm_zs_stride(d), dq = gmm_zs_dq(d);
   {
     const float4* src = reinterpret_cast<const float4*>(tab);
@@ -463,20 +469,24 @@ gmm_zs_kernel(int N, int d, int K, int vec, const float* __restrict__ Y, const f
   const bool all_exact = *flag != 0;
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (GMM_ZS_THREADS / 32);
-  for (int tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; tile < (N + 63) / 64; tile += warps) {
-    int n2[2];
+  for (int tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; tile < (N + 32 * H - 1) / (32 * H); tile += warps) {
+    int n2[H];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int i = tile * 64 + lane + 32 * h;
-      n2[h] = i < N ? (perm ? perm[i] : i) : -1;
+    for (int h = 0; h < H; ++h) {
+      const int i = tile * 32 * H + lane + 32 * h;
+      n2[h] = i < N ? (ORDERED ? perm[i] : i) : -1;
     }
-    bool exact[2] = {all_exact, all_exact};
-    float tk[2][GMM_ZS_MAXK], ek[2][GMM_ZS_MAXK];
-    float tmax[2] = {-INFINITY, -INFINITY};
-    if (!all_exact) {
-      unsigned long long y[2][DW / 2];
+    bool exact[H];
+    float tk[H][GMM_ZS_MAXK], ek[H][GMM_ZS_MAXK], tmax[H];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < H; ++h) {
+      exact[h] = all_exact;
+      tmax[h] = -INFINITY;
+    }
+    if (!all_exact) {
+      unsigned long long y[H][DW / 2];
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
         const float* yr = Y + (size_t)max(n2[h], 0) * d;
         if (vec) {   // d a multiple of 4, rows 16-byte aligned
 #pragma unroll
@@ -495,65 +505,92 @@ gmm_zs_kernel(int N, int d, int K, int vec, const float* __restrict__ Y, const f
       // their draws too: those components first, then - where a point does not
       // look like any of them - the component its first coordinates suggest,
       // so that the other components can be found far away early.
-      float low[2] = {-INFINITY, -INFINITY};   // a lower bound of log p_max so far
-      bool likely[2] = {n2[0] < 0, n2[1] < 0};
+      float low[H];                            // a lower bound of log p_max so far
+      bool likely[H];
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        low[h] = -INFINITY;
+        likely[h] = n2[h] < 0;
+      }
       unsigned todo = K == 32 ? 0xffffffffu : (1u << K) - 1u, pend = todo;
-      bool suggest = perm != nullptr;
-      if (perm) {
+      bool suggest = ORDERED;
+      if constexpr (ORDERED) {
         unsigned m = 0u;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < H; ++h) {
           const int l = n2[h] >= 0 ? z[n2[h]] : -1;
           m |= l >= 0 && l < K ? 1u << l : 0u;
         }
         pend = __reduce_or_sync(0xffffffffu, m);
       }
-      while (todo) {
-        if (pend == 0u && suggest) {
-          suggest = false;
-          if (__any_sync(0xffffffffu, !likely[0] || !likely[1])) {
-            float best[2] = {-INFINITY, -INFINITY};
-            int at[2] = {0, 0};
-            for (int k = 0; k < K; ++k) {
-              const float* L32 = ts + k * stride;
-              const float* a = L32 + gmm_zs_row(d - 1) + dq;
-              const ulonglong2 mh = *reinterpret_cast<const ulonglong2*>(a + dq);
-              const float lpc = a[3 * dq];
+      for (int k0 = 0; ORDERED ? todo != 0u : k0 < K; ++k0) {
+        int k = k0;
+        if constexpr (ORDERED) {
+          if (pend == 0u && suggest) {
+            suggest = false;
+            bool odd = false;
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const unsigned long long w0 = add2(y[h][0], mh.x), w1 = DW > 2 ? add2(y[h][1], mh.y) : 0ull;
-                float e = 0.0f;
+            for (int h = 0; h < H; ++h) odd = odd || !likely[h];
+            if (__any_sync(0xffffffffu, odd)) {
+              float best[H];
+              int at[H];
 #pragma unroll
-                for (int i = 0; i < (DT < 4 ? DT : 4); ++i) {
-                  const ulonglong2 l = *reinterpret_cast<const ulonglong2*>(L32 + gmm_zs_row(i));
-                  const unsigned long long sr = fma2(l.y, w1, fma2(l.x, w0, 0ull));
-                  const float r = lo2(sr) + hi2(sr);
-                  e += r * r;
-                }
-                if (lpc - 0.5f * e > best[h]) {
-                  best[h] = lpc - 0.5f * e;
-                  at[h] = k;
+              for (int h = 0; h < H; ++h) {
+                best[h] = -INFINITY;
+                at[h] = 0;
+              }
+              for (int c = 0; c < K; ++c) {
+                const float* L32 = ts + c * stride;
+                const float* a = L32 + gmm_zs_row(d - 1) + dq;
+                const ulonglong2 mh = *reinterpret_cast<const ulonglong2*>(a + dq);
+                const float lpc = a[3 * dq];
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                  const unsigned long long w0 = add2(y[h][0], mh.x), w1 = add2(y[h][1], mh.y);
+                  float e = 0.0f;
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) {
+                    const ulonglong2 l = *reinterpret_cast<const ulonglong2*>(L32 + gmm_zs_row(i));
+                    const unsigned long long sr = fma2(l.y, w1, fma2(l.x, w0, 0ull));
+                    const float r = lo2(sr) + hi2(sr);
+                    e += r * r;
+                  }
+                  if (lpc - 0.5f * e > best[h]) {
+                    best[h] = lpc - 0.5f * e;
+                    at[h] = c;
+                  }
                 }
               }
+              unsigned want = 0u;
+#pragma unroll
+              for (int h = 0; h < H; ++h) want |= likely[h] ? 0u : 1u << at[h];
+              pend = __reduce_or_sync(0xffffffffu, want) & todo;
             }
-            pend = __reduce_or_sync(0xffffffffu, (likely[0] ? 0u : 1u << at[0]) | (likely[1] ? 0u : 1u << at[1])) & todo;
           }
+          if (pend == 0u) pend = todo;
+          k = __ffs(pend) - 1;
+          pend &= pend - 1u;
+          todo &= ~(1u << k);
         }
-        if (pend == 0u) pend = todo;
-        const int k = __ffs(pend) - 1;
-        pend &= pend - 1u;
-        todo &= ~(1u << k);
         const float* L32 = ts + k * stride;
         const float* a = L32 + gmm_zs_row(d - 1) + dq;
         const float4 sc = *reinterpret_cast<const float4*>(a + 3 * dq);
         const float lpc = sc.x;
         if (lpc == -INFINITY) {   // weight 0: the term is exactly 0 here and in the reference
-          tk[0][k] = tk[1][k] = -INFINITY;
-          ek[0][k] = ek[1][k] = 0.0f;
+#pragma unroll
+          for (int h = 0; h < H; ++h) {
+            tk[h][k] = -INFINITY;
+            ek[h][k] = 0.0f;
+          }
           continue;
         }
-        unsigned long long w[2][DW / 2], W2[2] = {0ull, 0ull};
-        float e[2] = {0.0f, 0.0f}, t1[2] = {0.0f, 0.0f};
+        unsigned long long w[H][DW / 2], W2[H];
+        float e[H], t1[H];
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          W2[h] = 0ull;
+          e[h] = t1[h] = 0.0f;
+        }
         float4 a4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         bool far = false;
 #pragma unroll
@@ -565,30 +602,36 @@ gmm_zs_kernel(int N, int d, int K, int vec, const float* __restrict__ Y, const f
               const ulonglong2 ml = reinterpret_cast<const ulonglong2*>(a + 2 * dq)[i / 4];
               a4 = reinterpret_cast<const float4*>(a)[i / 4];
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
+              for (int h = 0; h < H; ++h) {
                 w[h][i / 2] = add2(add2(y[h][i / 2], mh.x), ml.x);
-                w[h][i / 2 + 1] = add2(add2(y[h][i / 2 + 1], mh.y), ml.y);
                 W2[h] = fma2(w[h][i / 2], w[h][i / 2], W2[h]);
-                W2[h] = fma2(w[h][i / 2 + 1], w[h][i / 2 + 1], W2[h]);
+                if (DT > 2) {
+                  w[h][i / 2 + 1] = add2(add2(y[h][i / 2 + 1], mh.y), ml.y);
+                  W2[h] = fma2(w[h][i / 2 + 1], w[h][i / 2 + 1], W2[h]);
+                }
               }
             }
             // row i in float4s; its padding is zero (exact zero products)
             const ulonglong2* Li = reinterpret_cast<const ulonglong2*>(L32 + gmm_zs_row(i));
-            unsigned long long s0 = 0ull, s1 = 0ull;
+            unsigned long long s[H];
+#pragma unroll
+            for (int h = 0; h < H; ++h) s[h] = 0ull;
 #pragma unroll
             for (int q = 0; q <= i / 4; ++q) {
               const ulonglong2 l = Li[q];
-              s0 = fma2(l.x, w[0][2 * q], s0);
-              s1 = fma2(l.x, w[1][2 * q], s1);
-              s0 = fma2(l.y, w[0][2 * q + 1], s0);
-              s1 = fma2(l.y, w[1][2 * q + 1], s1);
+#pragma unroll
+              for (int h = 0; h < H; ++h) s[h] = fma2(l.x, w[h][2 * q], s[h]);
+#pragma unroll
+              for (int h = 0; h < H; ++h)
+                if (DT > 2) s[h] = fma2(l.y, w[h][2 * q + 1], s[h]);
             }
-            const float r0 = __fadd_rn(lo2(s0), hi2(s0)), r1 = __fadd_rn(lo2(s1), hi2(s1));
             const float ai = i % 4 == 0 ? a4.x : i % 4 == 1 ? a4.y : i % 4 == 2 ? a4.z : a4.w;
-            e[0] = __fmaf_rn(r0, r0, e[0]);
-            e[1] = __fmaf_rn(r1, r1, e[1]);
-            t1[0] = __fmaf_rn(fabsf(r0), ai, t1[0]);
-            t1[1] = __fmaf_rn(fabsf(r1), ai, t1[1]);
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+              const float r = __fadd_rn(lo2(s[h]), hi2(s[h]));
+              e[h] = __fmaf_rn(r, r, e[h]);
+              t1[h] = __fmaf_rn(fabsf(r), ai, t1[h]);
+            }
             // After 4, 8 and 16 rows: log p_k <= lpc - (1 - 2^-9) e~ / 2 + 1 (e's
             // remaining terms are nonnegative, its error far below 2^-9 e~ + 1
             // while |lpc| < 2^20 and the bound on e~'s error is below 1), so
@@ -596,10 +639,10 @@ gmm_zs_kernel(int N, int d, int K, int vec, const float* __restrict__ Y, const f
             // points adds less than 2^-59 of p_max to the sums - all of them
             // far less than the band's own rounding slack of 2^-38 - and its
             // remaining rows are left out.
-            if ((i == 3 || i == 7 || i == 15) && perm) {
+            if ((i == 3 || i == 7 || i == 15) && ORDERED) {
               bool f = true;
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
+              for (int h = 0; h < H; ++h) {
                 const float W = __fadd_ru(__fsqrt_ru(2.0f * __fadd_ru(lo2(W2[h]), hi2(W2[h]))), sc.z);
                 const float err = __fmul_ru(4.0f * u32, __fmul_ru(W, t1[h]));
                 f = f && err < 0.25f + 0x1p-11f * e[h] && fabsf(lpc) < 0x1p20f &&
@@ -610,12 +653,15 @@ gmm_zs_kernel(int N, int d, int K, int vec, const float* __restrict__ Y, const f
           }
         }
         if (far) {
-          tk[0][k] = tk[1][k] = -INFINITY;
-          ek[0][k] = ek[1][k] = 0.0f;
+#pragma unroll
+          for (int h = 0; h < H; ++h) {
+            tk[h][k] = -INFINITY;
+            ek[h][k] = 0.0f;
+          }
           continue;
         }
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < H; ++h) {
           // W >= ||w~|| + 2^-23 ||mu|| (the sum of squares' rounding and the root's covered)
           const float ww = __fadd_ru(lo2(W2[h]), hi2(W2[h]));
           const float W = __fadd_ru(__fsqrt_ru(__fmul_ru(ww, 1.0f + (float)(DT + 2) * u32)), sc.z);
@@ -637,7 +683,7 @@ gmm_zs_kernel(int N, int d, int K, int vec, const float* __restrict__ Y, const f
       }
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < H; ++h) {
       const int n = n2[h];
       if (n < 0) continue;
       if (!(tmax[h] >= -690.0f && tmax[h] <= 690.0f)) exact[h] = true;
@@ -1530,12 +1576,14 @@ static inline size_t gmm_zs_smem(int d, int K) { return sizeof(float) * (size_t)
 // Whether the screened draw takes the points in the order of their current
 // labels (two small launches, about 11 us at 200,000 points): then a warp's
 // points are near one component and the others' rows are mostly left out.
-// Worth it where the whole triangular products take several times that: the
-// whole draw 227 -> 145 us at N = 200,000, K = 16, d = 32 (3.3e9 here) with
-// components apart, 250 us while 5 % of the labels are wrong; at 20,011
-// points, K = 7, d = 13 (2.4e7) the draw takes 27 us, no more than the two
-// launches would leave to gain.
-static inline bool gmm_zs_ordered(int N, int d, int K) { return d > 8 && K > 2 && (double)N * K * d * d >= 4e8; }
+// That depends on a state the host does not see, so the line lies where the
+// order gains more with components apart and most labels right than it loses
+// with random labels or components in one another: at N = 200,000 the draw takes,
+// in order so, otherwise, and without the order,
+//   d = 32: K = 30  298, 649, 597 us;  K = 16  155, 290, 235;  K = 8  107, 167, 136;
+//   d = 24: K = 30  209, 390, 297 us;  K = 16  134, 227, 164;  K = 8  92, 132, 94;
+// at N = 30,000, d = 32, K = 30 and 16 171, 232, 138 and 101, 137, 89.
+static inline bool gmm_zs_ordered(int N, int d, int K) { return d > 24 && (double)N * K * d * d >= 1.5e9; }
 static inline size_t gmm_zs_queue_bytes(int N) { return gmm_al256(sizeof(int) * (size_t)N); }
 size_t gmm_zs_scratch(int N, int d, int K) {
   return gmm_al256(gmm_zs_smem(d, K)) + 256 + gmm_zs_queue_bytes(N) +
@@ -1543,14 +1591,21 @@ size_t gmm_zs_scratch(int N, int d, int K) {
 }
 bool gmm_zs_fits(int d, int K) { return K <= GMM_ZS_MAXK && d <= 32 && gmm_zs_smem(d, K) <= 100 * 1024; }
 
-template <int DT>
+template <int DT, int H>
 static int launch_zs_t(int N, int d, int K, const float* Y, const float* tab, const int* perm, const int* flag,
                        int* queue, int* qn, int* z, uint64_t seed, uint32_t iter, uint32_t comp, cudaStream_t st) {
   const size_t smem = gmm_zs_smem(d, K);
-  AB_CUDA(allow_smem((const void*)gmm_zs_kernel<DT>, smem));
+  AB_CUDA(allow_smem((const void*)gmm_zs_kernel<DT, H>, smem));
   const int vec = d % 4 == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
-  const unsigned grid = std::min(ceil_div(N, 64), 148u * 3u);   // few points: a warp's tile each
-  gmm_zs_kernel<DT><<<grid, GMM_ZS_THREADS, smem, st>>>(N, d, K, vec, Y, tab, perm, flag, queue, qn, z, seed, iter, comp);
+  // a tile of 32 H points for each of a CTA's warps; with fewer, still a CTA per
+  // SM, and where the tables that each reads are large, not more CTAs than run
+  // at once (K = 30, d = 24 to 32: 1 to 3 % faster; K = 30, d = 2 at 400,000 points
+  // 10 % slower)
+  const unsigned tiles = ceil_div(N, 32 * H), warps = GMM_ZS_THREADS / 32;
+  const unsigned resident = 148u * std::min<unsigned>(gmm_zs_ctas(DT, H), 227 * 1024 / (smem + 1024));
+  const unsigned grid = std::min(std::max(ceil_div(tiles, warps), std::min(tiles, 148u)), smem > 10 * 1024 ? resident : ~0u);
+  gmm_zs_kernel<DT, H><<<grid, GMM_ZS_THREADS, smem, st>>>(N, d, K, vec, Y, tab, perm, flag, queue, qn, z, seed,
+                                                                 iter, comp);
   AB_LAUNCH_CHECK("gmm_zs_kernel");
   return AB_OK;
 }
@@ -1581,11 +1636,14 @@ int launch_gmm_z_screened(int N, int d, int K, int shared, const float* Y, const
     }
   }
   int rc;
-  if (d <= 2) rc = launch_zs_t<2>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
-  else if (d <= 4) rc = launch_zs_t<4>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
-  else if (d <= 8) rc = launch_zs_t<8>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
-  else if (d <= 16) rc = launch_zs_t<16>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
-  else rc = launch_zs_t<32>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st);
+#define AB_ZS(DT, H) launch_zs_t<DT, H>(N, d, K, Y, tab, perm, flag, queue, qn, z, seed, iter, comp, st)
+  rc = d <= 2   ? AB_ZS(2, 1)
+       : d <= 4 ? AB_ZS(4, 1)
+       : d <= 8 ? AB_ZS(8, 1)
+       : d <= 16 ? AB_ZS(16, 1)
+       : perm    ? AB_ZS(32, 2)
+                 : AB_ZS(32, 1);
+#undef AB_ZS
   if (rc) return rc;
   gmm_zx_kernel<<<592, 32 * K, 0, st>>>(d, K, shared, Y, pis, mu, Linv, hdet, queue, qn, z, seed, iter, comp);
   AB_LAUNCH_CHECK("gmm_zx_kernel");

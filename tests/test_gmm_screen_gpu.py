@@ -90,6 +90,25 @@ def test_screen_in_label_order_equals_binary64(N_, K, d, spread, labels):
     np.testing.assert_array_equal(b, a)
 
 
+@pytest.mark.parametrize("N_,K,d,spread,labels", [(60_001, 32, 32, 5.0, "generating"), (60_001, 32, 32, 0.4, "random"),
+                                                  (90_013, 27, 25, 5.0, "none"), (70_000, 23, 31, 5.0, "random"),
+                                                  (1_060_000, 3, 25, 3.0, "generating")])
+def test_large_screen_in_label_order_equals_binary64(N_, K, d, spread, labels):
+    """The sizes from which the points go in the order of the labels z holds on
+    entry, two a thread: as above, with more points than are ordered at a time
+    and a dimension that is no multiple of four."""
+    test_screen_in_label_order_equals_binary64(N_, K, d, spread, labels)
+
+
+@pytest.mark.parametrize("N_,K,d", [(1, 2, 1), (31, 5, 9), (33, 30, 32), (4737, 30, 32), (18_945, 32, 32), (94_721, 6, 5),
+                                    (94_719, 20, 17), (47_361, 31, 30)])
+def test_screen_at_the_edges_of_its_grid(N_, K, d):
+    """Less than a warp of points, less than a tile for every warp of a CTA per
+    SM, and one point more or less than the CTAs that run at once take in
+    one turn, also where the tables leave room for two of them per SM."""
+    test_screen_in_label_order_equals_binary64(N_, K, d, 2.0, "random")
+
+
 def test_screen_exact_path_cases():
     rng = np.random.default_rng(7)
     N_, K, d = 4000, 6, 6
