@@ -791,7 +791,7 @@ gmm_zx_kernel(int d, int K, int shared_cov, const float* __restrict__ Y, const d
 // ---- conjugate statistics ----------------------------------------------------
 // Counts, sums of y and scatter matrices sum (y - mu_k)(y - mu_k)^T (the
 // reference's full-matrix update augur_mat_atm_inc_vtmt is symmetric
-// elementwise) of the points of each component, in four launches:
+// elementwise) of the points of each component.  Of many points in four launches:
 //   order    the points are brought in component order, stable in the point
 //            index: counts per chunk of 1024 points (gmm_count_kernel), then
 //            every chunk's ranks behind the counts before it
@@ -801,6 +801,8 @@ gmm_zx_kernel(int d, int K, int shared_cov, const float* __restrict__ Y, const d
 //            the whole segment, and only one row of them is written;
 //   reduce   the rows of each component added in a fixed order
 //            (gmm_stats_reduce_kernel).
+// Of fewer (gmm_stats_share) without the order: a CTA per component and share
+// of the points, then the reduction if there is more than one share.
 // Deterministic; the reference adds in point order.  Before, each of 296 CTAs
 // kept a table of all components over its own points, so every pass wrote and
 // read back 296 K-component tables (20 MB at K = 16, d = 32) and summed them in
@@ -937,8 +939,42 @@ __host__ __device__ inline int gmm_obs_groups(int d) {
 }
 __host__ __device__ inline int gmm_seg_pitch(int d) { return (d + 3) / 4 * 4 + 2; }
 
+// The points p_lo .. p_hi - 1 with label k, in order, into pts, and their
+// number: every warp takes an equal share of the labels, counts, and places
+// behind the warps before it.
+__device__ __forceinline__ int gmm_gather_points(int p_lo, int p_hi, int k, const int* __restrict__ z, int* pts) {
+  constexpr int NW = GMM_THREADS / 32;
+  __shared__ int found[NW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int share = (p_hi - p_lo + GMM_THREADS - 1) / GMM_THREADS * 32;
+  const int p0 = p_lo + warp * share, p1 = min(p_hi, p0 + share);
+  int c = 0;
+#pragma unroll 8
+  for (int p = p0; p < p1; p += 32) c += __popc(__ballot_sync(0xffffffffu, z[min(p + lane, p_hi - 1)] == k && p + lane < p1));
+  if (lane == 0) found[warp] = c;
+  __syncthreads();
+  int at = 0, m = 0;
+#pragma unroll
+  for (int w = 0; w < NW; ++w) {
+    at += w < warp ? found[w] : 0;
+    m += found[w];
+  }
+#pragma unroll 8
+  for (int p = p0; p < p1; p += 32) {
+    const bool in = z[min(p + lane, p_hi - 1)] == k && p + lane < p1;
+    const unsigned bal = __ballot_sync(0xffffffffu, in);
+    if (in) pts[at + __popc(bal & ((1u << lane) - 1u))] = p + lane;
+    at += __popc(bal);
+  }
+  return m;
+}
+
 // One row of part per segment: sums [d] if wanted, then the scatter's lower
 // triangle, row by row, if wanted.
+// GATHER (small n): no order and no segments; a CTA per component and share of
+// `seg` points finds the component's points in its share itself.  Its row is
+// k gridDim.y + share, and cnt_part there its number of points; a component's
+// only share stores the results.
 // Sums: a group of pow2(d) lanes (32 lanes taking two coordinates each past
 // d = 32) takes points in turn, one coordinate a lane.
 // Scatter: the points are centred in binary64 once each, 64 at a time, into
@@ -949,24 +985,42 @@ __host__ __device__ inline int gmm_seg_pitch(int d) { return (d + 3) / 4 * 4 + 2
 // a round are issued together, their indices clamped into the segment rather
 // than guarded one by one (guarded loads waited for each other: 71 us for the
 // scatter pass at K = 16, d = 32, N = 200,000).
-template <int CW>
+template <int CW, bool GATHER>
 __global__ void __launch_bounds__(GMM_THREADS)
-gmm_segment_kernel(int d, int K, int seg, int want_sum, int want_obs, const float* __restrict__ Y,
-                   const double* __restrict__ mu, const int* __restrict__ perm, const int* __restrict__ start,
-                   double* __restrict__ part, int pts_at) {
+gmm_segment_kernel(int n, int d, int K, int seg, int want_sum, int want_obs, const float* __restrict__ Y,
+                   const int* __restrict__ z, const double* __restrict__ mu, const int* __restrict__ perm,
+                   const int* __restrict__ start, double* __restrict__ part, int pts_at, int* __restrict__ cnt_part,
+                   int* __restrict__ cnt, double* __restrict__ sum, double* __restrict__ obs) {
   extern __shared__ __align__(16) double sh[];
   __shared__ double mk[GMM_MAX_D];
   __shared__ int where[4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < 32) gmm_find_segment(start, K, seg, blockIdx.x, where);
-  __syncthreads();
-  const int k = where[0], m = where[3];
-  if (k < 0) return;   // uniform
   int* pts = reinterpret_cast<int*>(sh + pts_at);
-  for (int p = tid; p < m; p += GMM_THREADS) pts[p] = perm[where[2] + p];
-  __syncthreads();
+  const bool whole = GATHER && gridDim.y == 1;
   const int W = (want_sum ? d : 0) + (want_obs ? d * (d + 1) / 2 : 0);
-  double* row = part + (size_t)blockIdx.x * W;
+  int k, m, at;
+  if (GATHER) {
+    k = blockIdx.x;
+    at = k * gridDim.y + blockIdx.y;
+    m = gmm_gather_points(blockIdx.y * seg, min(n, (int)(blockIdx.y + 1) * seg), k, z, pts);
+    if (tid == 0) *(whole ? cnt + k : cnt_part + at) = m;
+    if (m == 0) {        // uniform
+      for (int e = tid; e < (whole ? 0 : W); e += GMM_THREADS) part[(size_t)at * W + e] = 0.0;
+      for (int e = tid; e < (whole && want_sum ? d : 0); e += GMM_THREADS) sum[(size_t)k * d + e] = 0.0;
+      for (int e = tid; e < (whole && want_obs ? d * d : 0); e += GMM_THREADS) obs[(size_t)k * d * d + e] = 0.0;
+      return;
+    }
+  } else {
+    if (tid < 32) gmm_find_segment(start, K, seg, blockIdx.x, where);
+    __syncthreads();
+    k = where[0];
+    m = where[3];
+    if (k < 0) return;   // uniform
+    at = blockIdx.x;
+    for (int p = tid; p < m; p += GMM_THREADS) pts[p] = perm[where[2] + p];
+  }
+  __syncthreads();
+  double* row = part + (size_t)at * W;
   if (want_sum) {
     int dp = 1;
     while (dp < d && dp < 32) dp <<= 1;
@@ -998,7 +1052,7 @@ gmm_segment_kernel(int d, int K, int seg, int want_sum, int want_obs, const floa
     if (tid < d) {
       double a = 0.0;
       for (int w = 0; w < GMM_THREADS / 32; ++w) a = __dadd_rn(a, sh[w * GMM_MAX_D + tid]);
-      row[tid] = a;
+      (whole ? sum + (size_t)k * d : row)[tid] = a;
     }
     __syncthreads();
     row += d;
@@ -1066,24 +1120,41 @@ gmm_segment_kernel(int d, int K, int seg, int want_sum, int want_obs, const floa
     int t = e >> 4, r = 0;
     while (t >= r + 1) { t -= r + 1; ++r; }
     const int ii = 4 * r + ((e >> 2) & 3), jj = 4 * t + (e & 3);
-    if (ii < d && jj <= ii) row[ii * (ii + 1) / 2 + jj] = a;
+    if (ii >= d || jj > ii) continue;
+    if (whole) {
+      obs[(size_t)k * d * d + ii * d + jj] = a;
+      obs[(size_t)k * d * d + jj * d + ii] = a;
+    } else {
+      row[ii * (ii + 1) / 2 + jj] = a;
+    }
   }
 }
 
-// Component blockIdx.y's rows added: 32 entries per CTA, eight interleaved
+// Component blockIdx.y's rows (its segments', or `shares` rows of a gathering
+// pass) added: 32 entries per CTA, eight interleaved
 // partial sums of each, then those in order; `add`: onto an earlier slab's.
 // The counts of all but the last slab gather in scratch (so_far): `cnt` is
 // stored once, with the final count, as other streams may be reading the same
 // labels' counts from an earlier pass there.
 __global__ void __launch_bounds__(GMM_THREADS)
-gmm_stats_reduce_kernel(int d, int K, int seg, int want_sum, int want_obs, const double* __restrict__ part,
-                        const int* __restrict__ start, int add, int last, int* __restrict__ so_far,
+gmm_stats_reduce_kernel(int d, int K, int seg, int shares, int want_sum, int want_obs,
+                        const double* __restrict__ part, const int* __restrict__ start,
+                        const int* __restrict__ cnt_part, int add, int last, int* __restrict__ so_far,
                         int* __restrict__ cnt, double* __restrict__ sum, double* __restrict__ obs) {
   __shared__ double red[8][33];
   const int k = blockIdx.y, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  int r0 = 0;
-  for (int q = 0; q < k; ++q) r0 += (start[q + 1] - start[q] + seg - 1) / seg;
-  const int n = start[k + 1] - start[k], ns = (n + seg - 1) / seg;
+  int r0 = 0, n = 0, ns = shares;
+  if (shares > 0) {
+    r0 = k * shares;
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+      for (int r = tx; r < shares; r += 32) n += cnt_part[r0 + r];
+      n = __reduce_add_sync(0xffffffffu, n);
+    }
+  } else {
+    for (int q = 0; q < k; ++q) r0 += (start[q + 1] - start[q] + seg - 1) / seg;
+    n = start[k + 1] - start[k];
+    ns = (n + seg - 1) / seg;
+  }
   if (blockIdx.x == 0 && threadIdx.x == 0) (last ? cnt : so_far)[k] = n + (add ? so_far[k] : 0);
   const int W = (want_sum ? d : 0) + (want_obs ? d * (d + 1) / 2 : 0);
   const int e = blockIdx.x * 32 + tx;
@@ -1688,6 +1759,21 @@ static GmmStatScratch gmm_stat_layout(int d, int K) {
 }
 size_t gmm_stats_scratch(int d, int K) { return gmm_stat_layout(d, K).total; }
 
+// The points of a share of the gathering pass, 0 for the ordered one.  One or
+// two launches instead of four, which is what a sweep of few points in few
+// dimensions waits for (N = 2,000, K = 3, d = 2: 122 us with the ordered pass,
+// 92 with this), and no ordering: per pass 5 and 9 us (sums, scatter) against
+// 11 and 12 at N = 8,000, K = 2, d = 2, 6 and 15 against 13 and 22 at N = 32,000, d =
+// 32.  A share bounds what a CTA does if all labels are equal (16 turns of the
+// scatter's loop, 8 or 2 of the slower ones of wide d); twice that where the
+// rows of partial sums would not suffice otherwise, and the ordered pass beyond.
+static inline int gmm_stats_share(int N, int d, int K) {
+  const int base = d <= 16 ? 1024 : d <= 32 ? 512 : 128;
+  for (int share : {base, 2 * base})
+    if (N <= 131072 && K * (int)ceil_div(N, share) <= GMM_SEGMENTS) return share;
+  return 0;
+}
+
 int launch_gmm_stats(int N, int d, int K, const float* Y, const int* z, const double* mu, int want_sum,
                      int want_obs, int* cnt, double* sum, double* obs, void* scratch, cudaStream_t st) {
   const int W = (want_sum ? d : 0) + (want_obs ? d * (d + 1) / 2 : 0);
@@ -1705,8 +1791,26 @@ int launch_gmm_stats(int N, int d, int K, const float* Y, const int* z, const do
     smem = std::max(smem, sizeof(double) * 16 * (size_t)gmm_obs_groups(d) * gmm_obs_tiles(d));
   }
   const int pts_at = (int)(smem / sizeof(double));   // then the segment's points
+  if (const int share = gmm_stats_share(N, d, K)) {
+    const int shares = (int)ceil_div(N, share);
+    smem += sizeof(int) * (size_t)std::min(N, share);
+    const auto gather = d <= 16   ? gmm_segment_kernel<16, true>
+                        : d <= 32 ? gmm_segment_kernel<32, true>
+                                  : gmm_segment_kernel<64, true>;
+    AB_CUDA(allow_smem((const void*)gather, smem));
+    gather<<<dim3(K, shares), GMM_THREADS, smem, st>>>(N, d, K, share, want_sum, want_obs, Y, z, mu, nullptr, nullptr, part,
+                                                       pts_at, chunk_cnt, cnt, sum, obs);
+    AB_LAUNCH_CHECK("gmm_segment_kernel");
+    if (shares == 1) return AB_OK;
+    gmm_stats_reduce_kernel<<<dim3(std::max(1u, ceil_div(W, 32)), K), GMM_THREADS, 0, st>>>(
+        d, K, 0, shares, want_sum, want_obs, part, nullptr, chunk_cnt, 0, 1, so_far, cnt, sum, obs);
+    AB_LAUNCH_CHECK("gmm_stats_reduce_kernel");
+    return AB_OK;
+  }
   smem += sizeof(int) * (size_t)std::max(32, (int)ceil_div(std::min(N, GMM_SLAB), GMM_SEGMENTS));
-  const auto segments = d <= 16 ? gmm_segment_kernel<16> : d <= 32 ? gmm_segment_kernel<32> : gmm_segment_kernel<64>;
+  const auto segments = d <= 16   ? gmm_segment_kernel<16, false>
+                        : d <= 32 ? gmm_segment_kernel<32, false>
+                                  : gmm_segment_kernel<64, false>;
   AB_CUDA(allow_smem((const void*)segments, smem));
   for (int n0 = 0; n0 < N; n0 += GMM_SLAB) {
     const int n = std::min(GMM_SLAB, N - n0);
@@ -1717,12 +1821,13 @@ int launch_gmm_stats(int N, int d, int K, const float* Y, const int* z, const do
     gmm_place_kernel<<<chunks, GMM_THREADS, 0, st>>>(n, K, K, 0, z + n0, chunk_cnt, perm, start);
     AB_LAUNCH_CHECK("gmm_place_kernel");
     if (W > 0) {
-      segments<<<ceil_div(n, seg) + K, GMM_THREADS, smem, st>>>(d, K, seg, want_sum, want_obs, Y + (size_t)n0 * d, mu,
-                                                                perm, start, part, pts_at);
+      segments<<<ceil_div(n, seg) + K, GMM_THREADS, smem, st>>>(n, d, K, seg, want_sum, want_obs, Y + (size_t)n0 * d,
+                                                                z + n0, mu, perm, start, part, pts_at, nullptr, nullptr,
+                                                                nullptr, nullptr);
       AB_LAUNCH_CHECK("gmm_segment_kernel");
     }
     gmm_stats_reduce_kernel<<<dim3(std::max(1u, ceil_div(W, 32)), K), GMM_THREADS, 0, st>>>(
-        d, K, seg, want_sum, want_obs, part, start, n0 > 0, n0 + n == N, so_far, cnt, sum, obs);
+        d, K, seg, 0, want_sum, want_obs, part, start, nullptr, n0 > 0, n0 + n == N, so_far, cnt, sum, obs);
     AB_LAUNCH_CHECK("gmm_stats_reduce_kernel");
   }
   return AB_OK;

@@ -260,6 +260,37 @@ def test_stats_sizes(orc, N_, K, d):
     np.testing.assert_allclose(g.obs.cpu().numpy(), obs, rtol=1e-12, atol=1e-8)
 
 
+@pytest.mark.parametrize("N_,K,d", [(1, 1, 1), (1023, 3, 2), (1024, 64, 16), (1025, 3, 16), (2048, 5, 17), (513, 2, 32), (129, 4, 33),
+                                    (6143, 64, 2), (12_289, 64, 2), (14_337, 64, 2), (131_072, 3, 1), (131_073, 3, 1), (3000, 7, 62)])
+@pytest.mark.parametrize("same", [False, True])
+def test_stats_of_few_points(N_, K, d, same):
+    """The pass without the points' order, one and more shares of them, up to
+    the number of partial sums and points from which the ordered pass takes over:
+    small integers, so without any rounding; each output wanted and not; labels
+    outside [0, K), empty components, all points in one."""
+    rng = np.random.default_rng(N_ + d)
+    Y = rng.integers(-4, 5, (N_, d))
+    z = np.full(N_, K - 1) if same else rng.integers(-1, max(1, K - 1), N_)
+    mus = rng.integers(-2, 3, (K, d))
+    t = lambda a, dt: torch.as_tensor(np.ascontiguousarray(a), dtype=dt).cuda()
+    Yt, zt, mt = t(Y, torch.float32), t(z, torch.int32), t(mus, torch.float64)
+    L = N.lib()
+    want_cnt = np.bincount(z[z >= 0], minlength=K)
+    want_sum = np.zeros((K, d))
+    np.add.at(want_sum, z[z >= 0], Y[z >= 0])
+    want_obs = np.stack([(Y[z == k] - mus[k]).T @ (Y[z == k] - mus[k]) for k in range(K)])
+    for ws, wo in ((True, True), (True, False), (False, True), (False, False)):
+        cnt = torch.full((K,), 77, dtype=torch.int32, device="cuda")
+        s = torch.full((K, d), 7.0, dtype=torch.float64, device="cuda")
+        obs = torch.full((K, d, d), 7.0, dtype=torch.float64, device="cuda")
+        scratch = torch.full((int(L.ab_gmm_stats_scratch_bytes(d, K)),), 0x5b, dtype=torch.uint8, device="cuda")
+        N.check(L.ab_gmm_stats(N_, d, K, N.ptr(Yt), N.ptr(zt), N.ptr(mt) if wo else None, N.ptr(cnt), N.ptr(s) if ws else None,
+                               N.ptr(obs) if wo else None, N.ptr(scratch), N.stream_ptr()), "stats")
+        np.testing.assert_array_equal(cnt.cpu().numpy(), want_cnt)
+        np.testing.assert_array_equal(s.cpu().numpy(), want_sum if ws else 7.0)
+        np.testing.assert_array_equal(obs.cpu().numpy(), want_obs if wo else 7.0)
+
+
 SLAB = 1 << 20     # points the statistics take at a time
 
 
