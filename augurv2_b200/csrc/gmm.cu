@@ -1698,8 +1698,8 @@ int launch_gmm_z_screened(int N, int d, int K, int shared, const float* Y, const
   if (gmm_zs_ordered(N, d, K)) {
     perm = reinterpret_cast<int*>(reinterpret_cast<char*>(queue) + gmm_zs_queue_bytes(N));
     int* chunk_cnt = reinterpret_cast<int*>(reinterpret_cast<char*>(perm) + gmm_zs_queue_bytes(N));
-    for (int n0 = 0; n0 < N; n0 += GMM_SLAB) {
-      const int n = std::min(GMM_SLAB, N - n0), chunks = (int)ceil_div(n, GMM_ORDER_CHUNK);
+    for (long long at = 0; at < N; at += GMM_SLAB) {   // 64 bits: past the last slab the offset may not fit 32
+      const int n0 = (int)at, n = std::min(GMM_SLAB, N - n0), chunks = (int)ceil_div(n, GMM_ORDER_CHUNK);
       gmm_count_kernel<<<chunks, GMM_THREADS, 0, st>>>(n, K, K + 1, z + n0, chunk_cnt);
       AB_LAUNCH_CHECK("gmm_count_kernel");
       gmm_place_kernel<<<chunks, GMM_THREADS, 0, st>>>(n, K, K + 1, n0, z + n0, chunk_cnt, perm + n0, nullptr);
@@ -1812,7 +1812,8 @@ int launch_gmm_stats(int N, int d, int K, const float* Y, const int* z, const do
                         : d <= 32 ? gmm_segment_kernel<32, false>
                                   : gmm_segment_kernel<64, false>;
   AB_CUDA(allow_smem((const void*)segments, smem));
-  for (int n0 = 0; n0 < N; n0 += GMM_SLAB) {
+  for (long long at = 0; at < N; at += GMM_SLAB) {   // 64 bits: past the last slab the offset may not fit 32
+    const int n0 = (int)at;
     const int n = std::min(GMM_SLAB, N - n0);
     const int chunks = (int)ceil_div(n, GMM_ORDER_CHUNK);
     const int seg = std::max(32, (int)ceil_div(n, GMM_SEGMENTS));   // at most GMM_SEGMENTS + K segments
