@@ -1048,6 +1048,23 @@ def run_reference(args, rank, world):
             "e2e": {"value": value, "unit": "tokens/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
 
 
+# What the default line keeps of the other configurations: readers of the line
+# may see only the last few thousand characters of the output.
+BRIEF = {"hlr_surrogate": ("value", "unit", "gain_vs_plain", "ms_per_iteration", "posterior_mean_diff_in_sd", "fallback"),
+         "hlr_small": ("value", "unit", "chains", "gain_single_chain_vs_cpu"),
+         "gmm": ("value", "unit", "ms_per_sweep"),
+         "hlr_nuts": ("value", "unit", "seconds", "gain_vs_cpu_core")}
+
+
+def brief(line):
+    """The line with its other configurations cut to their main figures (six
+    digits), and what was cut, whole, by configuration."""
+    short = lambda v: float("%.6g" % v) if isinstance(v, float) else {k: short(x) for k, x in v.items()} if isinstance(v, dict) else v
+    full = {k: line[k] for k in BRIEF if isinstance(line.get(k), dict)}
+    cut = {k: {n: short(v[n]) for n in BRIEF[k] + ("error",) if n in v} for k, v in full.items()}
+    return dict(line, **cut), full
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -1106,6 +1123,10 @@ def main():
                          "data": "synthetic (X ~ N(0,1) bf16, beta ~ Student-t(3), seed 5)"})
     else:
         line = run_ours(args, rank, world, local_rank)
+        if rank == 0 and line is not None:
+            line, full = brief(line)
+            for k, v in full.items():      # the whole of each, one line apiece
+                print(json.dumps({k: v}), file=sys.stderr, flush=True)
     if rank == 0 and line is not None:
         print(json.dumps(line), flush=True)
 
