@@ -7,9 +7,12 @@
 //   [W1 (h1 x d_in), b1 (h1), W2 (h2 x h1), b2 (h2), W3 (d_out x h2), b3 (d_out)]
 // with a bf16 copy of the same layout; forward passes multiply by the bf16
 // weights with FP32 accumulation and FP32 biases.  The layer products run on
-// the CUDA cores (mlp_gemm_kernel), every output one chain of multiply-adds
-// in k order: they are a few hundred MFLOP per step, small beside the exact
-// HLR pass.
+// the CUDA cores: they are a few hundred MFLOP per step, small beside the exact
+// HLR pass.  An output is one chain of multiply-adds in k order in
+// mlp_gemm_kernel and mlp_rows_kernel; mlp_cluster_kernel splits it over up to 32
+// lanes and adds their parts in a tree.  So a prediction's last bits depend on
+// whether its batch is one for clusters, and a forward pass's on whether it
+// keeps the activations; each repeats bit for bit.
 //
 //   forward   P1 = X W1^T + b1, A1 = gelu(P1), P2 = A1 W2^T + b2,
 //             A2 = gelu(P2), Y = A2 W3^T + b3 — a product per layer when the
@@ -581,9 +584,10 @@ int check_fused(const ab_mlp_desc* d) {
 }
 
 // Rows per cluster for a batch of B, 0 for the kernel without clusters.  A cluster
-// kernel's batch is one that is resident at once, up to 32 clusters: 512 rows as 64
-// clusters of eight take 95 us against 54 of the other kernel and its product, 256
-// rows as 64 clusters of four 58 against 36 as 32 of eight (both before dense_slices).
+// kernel's batch is one that is resident at once, up to 32 clusters.  At D = 512, 512
+// rows as 64 clusters of eight take 45 us against 41 of the other kernel without the
+// linear part, 56 against 60 with it (the other kernel's being a product of its own);
+// 256 rows as 64 clusters of four 36 against 29 as 32 of eight.
 int net_rows(const ab_mlp_desc* d, int B) {
   const size_t row = sizeof(float) * (2 * (size_t)d->d_in + d->h1 + d->h2);
   for (int G : {4, 8})
@@ -693,7 +697,7 @@ extern "C" int ab_mlp_forward(const ab_mlp_desc* d, int B, const float* x, int l
   cudaStream_t st = as_stream(stream);
   if (!act) return launch_fused<false>(d, B, x, ldx, y, ldy, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, st);
   // the activations are wanted anyway: one tiled product per layer, which
-  // spreads every layer over the GPU (three launches, the same values; for a
+  // spreads every layer over the GPU (three launches; for a
   // batch of 512 through 512-256-256-512 47 us cold and 49 in the fused kernel,
   // whose CTAs each read every weight)
   if ((rc = check_fused(d))) return rc;

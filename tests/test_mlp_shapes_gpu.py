@@ -68,3 +68,31 @@ def test_surrogate_prediction_matches_fp64(D, h1, h2, C, pad, dense):
     Y, _ = B.mlp_forward(d64(sur.wb), d64(sur.w), dt * d64(sur.inv_s), D, h1, h2, D)
     want = d64(sur.a) + d64(sur.h) * dt + d64(sur.o) * Y + (dt @ d64(sur.M) if dense else 0.0)
     assert np.max(np.abs(d64(out) - want)) <= 1e-4 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("D,h1,h2", [(64, 256, 256), (512, 264, 40)])
+def test_passes_agree_across_their_kernels(D, h1, h2):
+    # the same rows in batches on both sides of each kernel's limit, and the
+    # forward pass with and without kept activations: FP32 sums of at most 512
+    # terms in two orders stay within 2 * 512 * 2^-24 = 6e-5 of one another,
+    # through three layers within 2e-4 of the largest output
+    sur = H.MlpSurrogate(D, h1, h2, seed=D)
+    gen = torch.Generator("cuda").manual_seed(D)
+    x = torch.randn(300, D, device="cuda", generator=gen)
+    sur.M.copy_(torch.randn(D, D, device="cuda", generator=gen) / D ** 0.5)
+    L = H.N.lib()
+    for dense in (False, True):
+        sur.dense = dense
+        full = sur.predict(x, torch.empty_like(x)).clone()
+        for C in (1, 128, 129, 256, 257):
+            got = sur.predict(x[:C], torch.empty(C, D, device="cuda"))
+            again = sur.predict(x[:C], torch.empty(C, D, device="cuda"))
+            assert torch.equal(got, again)
+            assert float((got - full[:C]).abs().max()) <= 2e-4 * float(full.abs().max())
+    for Bn in (5, 200, 300):
+        sc = sur._scratch(Bn)
+        y = torch.empty(Bn, D, device="cuda")
+        for act, out in ((sc["act"], sc["out"]), (None, y)):
+            H.N.check(L.ab_mlp_forward(H.C.byref(sur.desc), Bn, H.N.ptr(x), D, H.N.ptr(out), D, H.N.ptr(act), None))
+        torch.cuda.synchronize()
+        assert float((y - sc["out"]).abs().max()) <= 2e-4 * float(y.abs().max())
