@@ -9,7 +9,10 @@
 // Linv f64 [Kc][d][d] and hdet f64 [Kc] are per-sweep derived tables.
 //
 // Arithmetic is binary64 without contraction (this file is compiled with
-// -fmad=false and uses _rn intrinsics).  The reference's d x d routines
+// -fmad=false and uses _rn intrinsics), but for the scatter matrices and the
+// mean moves' gains, which are summed in another order than the reference's and
+// use multiply-adds (held to 1e-12 and 1e-9 of the oracle), and the draw's
+// binary32 screen.  The reference's d x d routines
 // (cbits/augur_matop.c:312-420) are in-place sequential loops; the routines
 // below compute every element with the same operand order, reading the values
 // the in-place reference would read at that point, so their results are
@@ -81,19 +84,20 @@ __device__ __forceinline__ bool rounds_to(double e, double v, double q) {
   return (__double_as_longlong(e) & 0x7fffffffffffffffll) < __double_as_longlong(__hiloint2double(hb, __double2loint(v)));
 }
 
-// sqrt(x) and the reciprocal of that root; true if both are known to be
-// correctly rounded.  CUDA's reciprocal root (within an ulp) gives the root by
-// one residual step and seeds the reciprocal, which a second one rounds (after
-// Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990): far shorter a chain than a square root and a division in
-// turn.  The steps alone do not round every value correctly (a root just below
-// a power of two, for one), hence the tests, whose result the caller needs
-// only once it has used the values: they run beside that use.
-__device__ __forceinline__ bool root_recip(double x, double& root, double& rec) {
+// sqrt(x) and the reciprocal of that root.  CUDA's reciprocal root (within an
+// ulp) gives the root by one residual step and seeds the reciprocal, which a
+// second one rounds (after Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990): far shorter a chain than a square
+// root and a division in turn.  The steps alone do not round every value
+// correctly (a root just below a power of two, for one), hence the test, whose
+// result is needed only once the values have been used: it runs beside that use.
+__device__ __forceinline__ void root_recip(double x, double& root, double& rec) {
   const double y = rsqrt(x);
   const double g = __dmul_rn(x, y);
   root = __fma_rn(__fma_rn(-g, g, x), __dmul_rn(0.5, y), g);
   rec = __fma_rn(__fma_rn(-root, y, 1.0), y, y);
+}
+__device__ __forceinline__ bool root_recip_rounded(double x, double root, double rec) {
   return __double2hiint(x) > 0 && within_2(x, 900) && rounds_to<0>(__fma_rn(-root, root, x), root, root) &&
          rounds_to<1>(__fma_rn(-root, rec, 1.0), root, rec);
 }
@@ -129,7 +133,8 @@ __device__ __forceinline__ void g_factor(const Tri<NE>& T, double* A, double* O,
       if (T.ij[q] == (k << 8 | k)) piv[k] = __dadd_rn(GP(A, k, k), -acc[q]);
     __syncthreads();
     double root, rec;
-    bool ok = root_recip(piv[k], root, rec);
+    root_recip(piv[k], root, rec);
+    bool ok = true;
 #pragma unroll
     for (int q = 0; q < NE; ++q) {
       const int i = T.ij[q] >> 8, j = T.ij[q] & 255;
@@ -144,7 +149,9 @@ __device__ __forceinline__ void g_factor(const Tri<NE>& T, double* A, double* O,
         GP(O, k, j) = b;
       }
     }
-    if (!ok) {
+    // one warp of each half of the CTA tests the values that all of them share
+    if ((threadIdx.x & 96) == 0) ok &= root_recip_rounded(piv[k], root, rec);
+    if (__syncthreads_or(!ok)) {
       root = __dsqrt_rn(piv[k]);
       rec = __ddiv_rn(1.0, root);
 #pragma unroll
@@ -158,8 +165,8 @@ __device__ __forceinline__ void g_factor(const Tri<NE>& T, double* A, double* O,
           GP(O, k, j) = __ddiv_rn(acc[q], root);
         }
       }
+      __syncthreads();
     }
-    __syncthreads();
 #pragma unroll
     for (int q = 0; q < NE; ++q) {
       const int i = T.ij[q] >> 8, j = T.ij[q] & 255;

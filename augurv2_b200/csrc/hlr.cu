@@ -782,7 +782,7 @@ __device__ int nuts_transition(const HlrModelDev& m, const HlrComp& cp, const Bl
 // with the exponential from (c, iter, RSLICE|ci<<8); augur_max(1,
 // round(simlen / eps)) steps of q += eps p0, each followed by the log density
 // at the new point and, outside the slice, a reflection of p0 off the block
-// gradient there (p0 += -2 (p0.g)/(g.g) g, sequential dot products).  The
+// gradient there (p0 += -2 (p0.g)/(g.g) g, dot products in block_dot's tree).  The
 // move is kept only if the last point is inside the slice.
 template <int RES, int COLS>
 __device__ int rslice_transition(const HlrModelDev& m, const HlrComp& cp, const BlockInfo bi, Ws& ws,
@@ -953,9 +953,11 @@ __device__ __forceinline__ void stage_labels(const HlrModelDev& m, int* lab) {
 // stats[c][ci][5] = {accepts, sum depth, sum leaves, errors, divergent iterations}.
 // Bound: the chain of one evaluation - barriers, the compensated sums of a
 // thread's rows, binary64 reductions - at 11 evaluations an HMC iteration.
-// Measured, ten HMC iterations at N = 1000, D = 10: 870 -> 377 us; two NUTS
-// iterations of depth 5 for 48 chains at N = 2003, D = 41 (bf16): 10.5 -> 1.04 ms,
+// Measured, ten HMC iterations at N = 1000, D = 10: 890 -> 338 us; a NUTS
+// iteration of depth 5 for 48 chains at N = 2003, D = 41 (bf16): 5.30 -> 0.40 ms,
 // where every evaluation walked X a warp per row and every leaf took two.
+// Issue slots 37 and 52 % busy, no pipe near its limit, stalls on fixed latencies
+// and barriers.
 template <int RES, int COLS>
 __global__ void __launch_bounds__(HLR_BLOCK, 1)
 hlr_chain_kernel(const __grid_constant__ HlrModelDev m, HlrLayout l, const HlrComp* __restrict__ comps, int n_comps,
