@@ -700,12 +700,12 @@ inline size_t al256(size_t a) { return (a + 255) & ~size_t(255); }
 // lane quarter = warp % 4).  No epilogue warp waits for another: each stages its
 // own labels, hands in its half of the residual on that half's own barrier and
 // waits for the previous tile's backward product only before its first residual
-// store.  At 512 chains and 600,000 rows a pass takes 389 us at D = 16, 405 at 64,
-// 493 at 128 and 737 at 256 (489, 494, 511 and 742 with a barrier over all epilogue
+// store.  At 512 chains and 600,000 rows a pass takes 391 us at D = 16, 403 at 64,
+// 493 at 128 and 714 at 256 (489, 495, 510 and 725 with a barrier over all epilogue
 // warps per tile and the wait at the tile's start).  It is bound by the epilogue's
-// chain of exponentials, logarithm and Kahan sums up to D = 64 (issue slots and the
-// special function unit each 54 % busy) and by the tensor core's operand supply
-// from there (52 % busy at D = 256).  Every wait is bounded as in gemm_kernel.
+// chain of exponentials, logarithm and Kahan sums up to D = 64 (issue slots 52 %, the
+// special function unit 55 % busy) and by the tensor core's operand supply
+// from there (53 % busy at D = 256).  Every wait is bounded as in gemm_kernel.
 constexpr int F_ROWS = 128;
 constexpr int F_SEG_TILES = 64;                            // row tiles per unit (8192 rows)
 constexpr int F_MAX_D = 256;
