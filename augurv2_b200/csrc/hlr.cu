@@ -29,7 +29,8 @@
 namespace ab {
 
 constexpr int HLR_THREADS = 256;         // threads that walk the rows: each row's place in the compensated sums
-constexpr int HLR_BLOCK = HLR_THREADS + 32;   // and a warp for the prior and, past D = 30, the log-likelihood sums
+constexpr int HLR_BLOCK = HLR_THREADS + 32;   // and, in the chain kernel, a warp for the prior and, past D = 30, the
+                                              // log-likelihood sums (otherwise the last of the row threads' warps)
 constexpr int HLR_CHUNK = 1024;          // rows per data-pass chunk (r buffer)
 constexpr int HLR_MAX_COLS = 4;          // columns per thread in the gradient pass
 constexpr int HLR_MAX_D = HLR_THREADS * HLR_MAX_COLS - 1;
@@ -54,11 +55,6 @@ struct HlrComp {
   int kind, P, idx_off, max_depth;
   double simlen, eps, mwg_var;
 };
-
-__device__ __forceinline__ float load_x(const HlrModelDev& m, size_t i) {
-  if (m.x_bf16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(m.X)[i]);
-  return __ldg(reinterpret_cast<const float*>(m.X) + i);
-}
 
 __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
   const float yv = x - c;
@@ -157,17 +153,23 @@ __device__ __forceinline__ void warp_transpose_sum(double (&v)[COLS], int lane) 
   if (COLS == 16) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
 }
 
-// Where the rows are read: global memory, or the shared copy in X's type.
-enum { X_GLOBAL = 0, X_F32 = 1, X_BF16 = 2 };
+// Where the rows are read: the shared copy in X's type, or global memory (the
+// data passes then take X's type as a template argument too, G_F32 or G_BF16:
+// a test of it at every load kept the loads of a row from being in flight
+// together; with row_dot's groups, 20,000 rows of D = 20 176 -> 87 us).
+enum { X_GLOBAL = 0, X_F32 = 1, X_BF16 = 2, G_F32 = 3, G_BF16 = 4 };
+__host__ __device__ constexpr bool in_shared(int res) { return res == X_F32 || res == X_BF16; }
 template <int RES>
 __device__ __forceinline__ float row_x(const HlrModelDev& m, const Ws& ws, int i, int k) {
   if (RES == X_F32) return static_cast<const float*>(ws.xs)[i * ws.xpitch + k];
   if (RES == X_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(ws.xs)[i * ws.xpitch + k]);
-  return load_x(m, (size_t)i * m.ldx + k);
+  const size_t at = (size_t)i * m.ldx + k;
+  if (RES == G_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(m.X)[at]);
+  return __ldg(static_cast<const float*>(m.X) + at);
 }
 template <int RES>
 __device__ __forceinline__ int row_label(const HlrModelDev& m, const Ws& ws, int i) {
-  return RES ? ws.lab[i] : load_label(m, i);
+  return in_shared(RES) ? ws.lab[i] : load_label(m, i);
 }
 
 // Data pass for D + 2 <= COLS: one row per thread (t, the log-likelihood term
@@ -176,6 +178,29 @@ __device__ __forceinline__ int row_label(const HlrModelDev& m, const Ws& ws, int
 // fixed-order sum over the warps, all in FP64: the row-per-thread walk keeps
 // every thread busy at small N.  By the row threads; leaves the sums in ws.g and
 // ws.red[33].
+// A row's values (zeros past D) and their dot product with th.  From global
+// memory eight at a time without a test between them, so that they are issued
+// together.
+template <int RES, int K>
+__device__ __forceinline__ float row_dot(const HlrModelDev& m, const Ws& ws, int i, const float (&th)[K], float (&x)[K]) {
+  const int D = m.D;
+#pragma unroll
+  for (int k0 = 0; k0 < K; k0 += 8) {
+    const bool whole = !in_shared(RES) && k0 + 8 <= K && k0 + 8 <= D;
+    if (whole) {
+#pragma unroll
+      for (int k = k0; k < k0 + 8 && k < K; ++k) x[k] = row_x<RES>(m, ws, i, k);
+    } else {
+#pragma unroll
+      for (int k = k0; k < k0 + 8 && k < K; ++k) x[k] = k < D ? row_x<RES>(m, ws, i, k) : 0.0f;
+    }
+  }
+  float t = 0.0f;
+#pragma unroll
+  for (int k = 0; k < K; ++k) t += x[k] * th[k];
+  return t;
+}
+
 template <int COLS, int RES>
 __device__ __forceinline__ void data_rows_small(const HlrModelDev& m, bool want_ll, bool want_grad, float bias, const Ws& ws) {
   const int D = m.D;
@@ -184,22 +209,36 @@ __device__ __forceinline__ void data_rows_small(const HlrModelDev& m, bool want_
     float th[COLS - 2];
 #pragma unroll
     for (int k = 0; k < COLS - 2; ++k) th[k] = k < D ? ws.th[k] : 0.0f;
-    float s[COLS], c[COLS];
-#pragma unroll
-    for (int j = 0; j < COLS; ++j) { s[j] = 0.0f; c[j] = 0.0f; }
+    double v[COLS];
+    if (!want_grad) {
+      // two rows in flight, which the gradient's sums leave no registers for
+      float ls = 0.0f, lc = 0.0f;
 #pragma unroll 1
-    for (int i = tid; i < m.N; i += HLR_THREADS) {
-      float x[COLS - 2];
-      float t = 0.0f;
-#pragma unroll
-      for (int k = 0; k < COLS - 2; ++k) {
-        x[k] = k < D ? row_x<RES>(m, ws, i, k) : 0.0f;
-        t += x[k] * th[k];
+      for (int i = tid; i < m.N; i += 2 * HLR_THREADS) {
+        const int i1 = min(i + HLR_THREADS, m.N - 1);
+        float x0[COLS - 2], x1[COLS - 2];
+        const float t0 = row_dot<RES>(m, ws, i, th, x0), t1 = row_dot<RES>(m, ws, i1, th, x1);
+        const int y0 = row_label<RES>(m, ws, i), y1 = row_label<RES>(m, ws, i1);
+        float l0, l1, rv;
+        lik_terms(m, true, y0, t0 + bias, l0, rv);
+        lik_terms(m, true, y1, t1 + bias, l1, rv);
+        kahan_add(ls, lc, l0);
+        if (i + HLR_THREADS < m.N) kahan_add(ls, lc, l1);
       }
-      float llv, rv;
-      lik_terms(m, want_ll, row_label<RES>(m, ws, i), t + bias, llv, rv);
-      if (want_ll) kahan_add(s[COLS - 1], c[COLS - 1], llv);
-      if (want_grad) {
+#pragma unroll
+      for (int j = 0; j < COLS - 1; ++j) v[j] = 0.0;
+      v[COLS - 1] = (double)ls - (double)lc;
+    } else {
+      float s[COLS], c[COLS];
+#pragma unroll
+      for (int j = 0; j < COLS; ++j) { s[j] = 0.0f; c[j] = 0.0f; }
+#pragma unroll 1
+      for (int i = tid; i < m.N; i += HLR_THREADS) {
+        float x[COLS - 2];
+        const float t = row_dot<RES>(m, ws, i, th, x);
+        float llv, rv;
+        lik_terms(m, want_ll, row_label<RES>(m, ws, i), t + bias, llv, rv);
+        if (want_ll) kahan_add(s[COLS - 1], c[COLS - 1], llv);
 #pragma unroll
         for (int k = 0; k < COLS - 2; ++k)
           if (k < D) kahan_add(s[k], c[k], rv * x[k]);
@@ -207,10 +246,9 @@ __device__ __forceinline__ void data_rows_small(const HlrModelDev& m, bool want_
         for (int k = 0; k < COLS - 1; ++k)
           if (k == D) kahan_add(s[k], c[k], rv);
       }
-    }
-    double v[COLS];
 #pragma unroll
-    for (int j = 0; j < COLS; ++j) v[j] = (double)s[j] - (double)c[j];
+      for (int j = 0; j < COLS; ++j) v[j] = (double)s[j] - (double)c[j];
+    }
     warp_transpose_sum<COLS>(v, lane);
     if (lane < COLS) ws.gpart[warp * COLS + lane] = v[0];
   }
@@ -232,9 +270,9 @@ __device__ __forceinline__ void data_rows_small(const HlrModelDev& m, bool want_
 // otherwise a warp per row) and their terms; then the row threads, owners of
 // gradient columns, walk the chunk's residuals, while eight lanes of the last
 // warp walk its log-likelihood terms.
-template <int RES>
+template <int RES, int BLOCK>
 __device__ __forceinline__ void data_rows_wide(const HlrModelDev& m, bool want_ll, bool want_grad, float bias, const Ws& ws) {
-  constexpr int NW = HLR_THREADS / 32;
+  constexpr int NW = HLR_THREADS / 32, LAST = BLOCK / 32 - 1;
   const int D = m.D, N = m.N;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // gradient accumulators: thread owns columns c = tid + i*HLR_THREADS (cols
@@ -250,8 +288,8 @@ __device__ __forceinline__ void data_rows_wide(const HlrModelDev& m, bool want_l
   float lls = 0.0f, llc = 0.0f;   // log-likelihood terms of rows = lane (mod NW), lanes below NW of the last warp
   for (int n0 = 0; n0 < N; n0 += HLR_CHUNK) {
     const int nc = min(HLR_CHUNK, N - n0);
-    if (RES) {
-      for (int i = tid; i < nc; i += HLR_BLOCK) {
+    if (in_shared(RES)) {
+      for (int i = tid; i < nc; i += BLOCK) {
         float p[32];
 #pragma unroll
         for (int q = 0; q < 32; ++q) p[q] = 0.0f;
@@ -334,13 +372,13 @@ __device__ __forceinline__ void data_rows_wide(const HlrModelDev& m, bool want_l
         }
       }
     }
-    if (want_ll && warp == NW && lane < NW) {
+    if (want_ll && warp == LAST && lane < NW) {
 #pragma unroll 4
       for (int i = lane; i < nc; i += NW) kahan_add(lls, llc, ws.l[i]);
     }
     if (n0 + HLR_CHUNK < N) __syncthreads();
   }
-  if (want_ll && warp == NW) {
+  if (want_ll && warp == LAST) {
     const double v = warp_sum_f64((double)lls - (double)llc);
     if (lane == 0) ws.red[33] = v;
   }
@@ -360,6 +398,12 @@ __device__ __forceinline__ void data_rows_wide(const HlrModelDev& m, bool want_l
       }
     }
   }
+}
+
+template <int COLS, int RES, int BLOCK>
+__device__ __forceinline__ void data_rows(const HlrModelDev& m, bool want_ll, bool want_grad, float bias, const Ws& ws) {
+  if constexpr (COLS > 0) data_rows_small<COLS, RES>(m, want_ll, want_grad, bias, ws);
+  else data_rows_wide<RES, BLOCK>(m, want_ll, want_grad, bias, ws);
 }
 
 // ---- priors (binary64; reference formulas when compat) ----------------------
@@ -403,28 +447,42 @@ __device__ __forceinline__ BlockInfo block_info(const HlrModelDev& m, const int*
 // operations of an evaluation - while the row threads pass over the data.
 // COLS: the data pass, 16 or 32 columns of the row-per-thread one, or 0 for the
 // wide one.
-template <int RES, int COLS>
+template <int RES, int COLS, int BLOCK = HLR_BLOCK>
 __device__ __forceinline__ double block_eval(const HlrModelDev& m, bool want_ll, bool want_grad, const double* par,
                                           const BlockInfo bi, int P, Ws& ws) {
   const int D = m.D, tid = threadIdx.x, lane = tid & 31;
   const bool data = bi.th || bi.b;
   const double v = par[D + 1];
   if (data)
-    for (int k = tid; k < D; k += HLR_BLOCK) ws.th[k] = (float)par[k];
+    for (int k = tid; k < D; k += BLOCK) ws.th[k] = (float)par[k];
   const float bias = m.has_b ? (float)par[D] : 0.0f;
   const double iv = 1.0 / v;
   __syncthreads();
-  if (tid >= HLR_THREADS && (want_ll || bi.v)) {
-    // the prior: lanes take the coefficients, lane 0 the variance and the bias
+  if ((tid >= BLOCK - 32 || !data) && (want_ll || bi.v)) {
+    // the prior: lanes take the coefficients (of all warps if none passes over
+    // the data), lane 0 of the last warp the variance and the bias
     double pl = 0.0, pd = 0.0;
     if (bi.th || bi.v)
-      for (int k = lane; k < D; k += 32) {
+      for (int k = data ? lane : tid; k < D; k += data ? 32 : BLOCK) {
         if (want_ll) pl += normal_ll(m, par[k], 0.0, v);
         if (bi.v) pd += normal_dvar(m, par[k], v, iv);
       }
     if (want_ll) pl = warp_sum_f64(pl);
     if (bi.v) pd = warp_sum_f64(pd);
-    if (lane == 0) {
+    if (!data) {
+      constexpr int NW = BLOCK / 32;
+      if (lane == 0) {
+        ws.gpart[tid >> 5] = pl;
+        ws.gpart[NW + (tid >> 5)] = pd;
+      }
+      __syncthreads();
+      pl = pd = 0.0;
+      for (int w = 0; w < NW; ++w) {
+        pl += ws.gpart[w];
+        pd += ws.gpart[NW + w];
+      }
+    }
+    if (tid == BLOCK - 32) {
       double ll = 0.0, gv = 0.0;
       if (bi.v) {
         if (want_ll) ll += vprior_ll(m, v);
@@ -439,12 +497,13 @@ __device__ __forceinline__ double block_eval(const HlrModelDev& m, bool want_ll,
     }
   }
   if (data) {
-    if constexpr (COLS > 0) data_rows_small<COLS, RES>(m, want_ll, want_grad, bias, ws);
-    else data_rows_wide<RES>(m, want_ll, want_grad, bias, ws);
+    if constexpr (RES != X_GLOBAL) data_rows<COLS, RES, BLOCK>(m, want_ll, want_grad, bias, ws);
+    else if (m.x_bf16) data_rows<COLS, G_BF16, BLOCK>(m, want_ll, want_grad, bias, ws);
+    else data_rows<COLS, G_F32, BLOCK>(m, want_ll, want_grad, bias, ws);
   }
   __syncthreads();
   if (want_grad) {
-    for (int j = tid; j < P; j += HLR_BLOCK) {
+    for (int j = tid; j < P; j += BLOCK) {
       const int i = ws.idx[j];
       ws.blk_g[j] = i < D ? -par[i] * iv + ws.g[i] : i == D ? (m.has_b ? -par[D] * iv + ws.g[D] : 0.0) : ws.bcast[1];
     }
@@ -953,7 +1012,7 @@ __device__ __forceinline__ void stage_labels(const HlrModelDev& m, int* lab) {
 // stats[c][ci][5] = {accepts, sum depth, sum leaves, errors, divergent iterations}.
 // Bound: the chain of one evaluation - barriers, the compensated sums of a
 // thread's rows, binary64 reductions - at 11 evaluations an HMC iteration.
-// Measured, ten HMC iterations at N = 1000, D = 10: 890 -> 338 us; a NUTS
+// Measured, ten HMC iterations at N = 1000, D = 10: 890 -> 334 us; a NUTS
 // iteration of depth 5 for 48 chains at N = 2003, D = 41 (bf16): 5.30 -> 0.40 ms,
 // where every evaluation walked X a warp per row and every leaf took two.
 // Issue slots 37 and 52 % busy, no pipe near its limit, stalls on fixed latencies
@@ -1010,8 +1069,11 @@ hlr_chain_kernel(const __grid_constant__ HlrModelDev m, HlrLayout l, const HlrCo
 // Log-density and gradient of a block for C parameter vectors (one CTA per
 // vector): the data pass and priors used by the transitions, exposed for
 // parity checks and for callers that drive their own samplers.
+// 256 threads of at most 128 registers, two CTAs per SM: with many vectors that
+// counts for more than a warp for the prior (500 vectors of D = 28, 5000 rows:
+// 104 us, 150 with one CTA of 288 threads per SM).
 template <int COLS>
-__global__ void __launch_bounds__(HLR_BLOCK, 1)
+__global__ void __launch_bounds__(HLR_THREADS, 2)
 hlr_ll_grad_kernel(const __grid_constant__ HlrModelDev m, HlrLayout l, const int* __restrict__ idx, int P, const double* __restrict__ pars,
                    double* __restrict__ ll, double* __restrict__ grad) {
   extern __shared__ __align__(16) double smem_d[];
@@ -1020,7 +1082,7 @@ hlr_ll_grad_kernel(const __grid_constant__ HlrModelDev m, HlrLayout l, const int
   const int c = blockIdx.x;
   for (int i = threadIdx.x; i < m.D + 2; i += blockDim.x) ws.par[i] = pars[(size_t)c * (m.D + 2) + i];
   const BlockInfo bi = stage_block(m, idx, P, ws);
-  const double v = block_eval<X_GLOBAL, COLS>(m, true, grad != nullptr, ws.par, bi, P, ws);
+  const double v = block_eval<X_GLOBAL, COLS, HLR_THREADS>(m, true, grad != nullptr, ws.par, bi, P, ws);
   if (threadIdx.x == 0) ll[c] = v;
   if (grad != nullptr)
     for (int j = threadIdx.x; j < P; j += blockDim.x) grad[(size_t)c * P + j] = ws.blk_g[j];
@@ -1053,7 +1115,7 @@ static int make_model(HlrModelDev& m, const ab_hlr_model* d) {
 
 // What a chain's CTA keeps in shared memory: X and the labels, if a component
 // evaluates the data, and the NUTS stacks, where they fit 224 KB (an SM holds
-// one CTA, whatever its shared memory: 288 threads of 155 to 168 registers).
+// one CTA, whatever its shared memory: 288 threads of 153 to 168 registers).
 // Every evaluation then reads X from there instead of walking it through the
 // caches.
 static HlrLayout choose_layout(const HlrModelDev& m, bool nuts, bool data) {
@@ -1106,7 +1168,7 @@ extern "C" int ab_hlr_ll_grad(const ab_hlr_model* model, const int* idx_dev, con
                       : m.D + 2 <= SMALL_COLS ? hlr_ll_grad_kernel<SMALL_COLS>
                                               : hlr_ll_grad_kernel<0>;
   AB_CUDA(allow_smem((const void*)kernel, smem));
-  kernel<<<C, HLR_BLOCK, smem, as_stream(stream)>>>(m, l, idx_dev, P, pars, ll, grad);
+  kernel<<<C, HLR_THREADS, smem, as_stream(stream)>>>(m, l, idx_dev, P, pars, ll, grad);
   AB_LAUNCH_CHECK("hlr_ll_grad_kernel");
   return AB_OK;
 }

@@ -161,6 +161,45 @@ def test_slice_and_metropolis_moves_on_every_path(orc, N, D, xd, C):
     assert agree >= total - 1
 
 
+@pytest.mark.parametrize("N,D,xd", [(1, 1, "f32"), (255, 7, "bf16"), (257, 8, "f32"), (511, 9, "bf16"), (513, 14, "f32"),
+                                    (700, 15, "bf16"), (769, 16, "f32"), (300, 22, "bf16"), (1025, 24, "f32"), (256, 30, "bf16"),
+                                    (1030, 31, "f32"), (90, 254, "bf16"), (60, 255, "f32"), (60, 600, "f32")])
+def test_ll_and_gradient_at_the_edges_of_the_row_walk(orc, N, D, xd):
+    """Rows and columns around the groups in which the evaluation loads them,
+    with and without the gradient (two rows at a time without), the variance
+    alone: the same density with and without, within 1e-5 of its terms'
+    magnitudes of the oracle's, and gradients that do not depend on columns of
+    zeros beside them."""
+    X, y, beta, s2, om, gd = make(N, D, N + D, True, "exponential", True, xd)
+    rng = np.random.default_rng(D)
+    par = np.concatenate([beta + 0.2 * rng.standard_normal(D), [0.2], [0.7]])
+    pars = np.stack([par, par * 0.5, par])
+    pars[:, D + 1] = [0.7, 1.3, 0.7]
+    L, C_ = H.N.lib(), len(pars)
+    for idx in ([D + 1, D] + list(range(D)), list(range(D)), [D + 1]):
+        ll, g = H.ll_grad(gd, pars, idx)
+        pt = torch.as_tensor(pars).cuda()
+        ih = np.ascontiguousarray(idx, np.int32)
+        only = torch.zeros(C_, dtype=torch.float64, device="cuda")
+        H.N.check(L.ab_hlr_ll_grad(H.C.byref(gd.c), H.N.ptr(torch.as_tensor(ih).cuda()), ih.ctypes.data_as(H.C.c_void_p), len(ih),
+                                   C_, H.N.ptr(pt), H.N.ptr(only), None, H.N.stream_ptr()))
+        np.testing.assert_array_equal(only.cpu().numpy(), ll)
+        np.testing.assert_array_equal(g[0], g[2])
+        for c in range(2):
+            p = pars[c]
+            t = X @ p[:D] + p[D]
+            l_ref = O.hlr_ll(orc, om, p, idx)
+            size = np.abs(y * t).sum() + np.logaddexp(0.0, t).sum() if idx != [D + 1] else 0.0
+            assert abs(ll[c] - l_ref) <= 1e-5 * size + 1e-9 * max(1.0, abs(l_ref))
+    if D <= 30:
+        # columns of zeros up to the walk's width change no bit of the others' sums
+        W = 14 if D <= 14 else 30
+        wide = H.HlrData(np.hstack([X, np.zeros((N, W - D))]), y, has_b=True, vprior="exponential", compat=True, x_dtype=xd)
+        wp = np.hstack([pars[:, :D], np.zeros((len(pars), W - D)), pars[:, D:]])
+        gw = H.ll_grad(wide, wp, list(range(D)) + [W])[1]
+        np.testing.assert_array_equal(H.ll_grad(gd, pars, list(range(D)) + [D])[1], gw)
+
+
 @pytest.mark.parametrize("N,D,xd,C", [(200, 300, "bf16", 1), (200, 300, "bf16", 150), (1600, 28, "f32", 150), (700, 300, "f32", 2)])
 def test_nuts_with_rows_or_stacks_in_shared_memory(orc, N, D, xd, C):
     """NUTS where shared memory holds X but not the walk's stacks, the stacks
